@@ -228,7 +228,11 @@ void map_product_dev(ds_map* map, ds_operator* op, const double* x_dev, double* 
   a.mask = map->pairs.mask.p;
   a.row_order = map->pairs.row_order.p;
   a.n_row_tiles = map->pts.n_tiles;
+  a.n_rows = map->pts.n;
+  a.n_cols = op->pix.n;
   a.v = op->tmp.p;
+  op->u.alloc(op->pix.n_pad);
+  a.u = op->u.p;
   a.out = m_dev;
   a.row_perm = map->pts.perm.p;
   a.table = op->table.p;
@@ -687,7 +691,7 @@ int ds_smp_product(ds_context* ctx, int n_pix, const double* pixel_points, int n
     const ds_kernel_params k = checked_kp(kp);
     const KernelConsts kc = make_consts(k);
     cudaStream_t st = ctx->stream;
-    DevBuf<double> table, dpix, dmap, dx, xs, dm;
+    DevBuf<double> table, dpix, dmap, dx, xs, us, dm;
     load_table(table, k, st);
     upload(pixel_points, (size_t)n_pix * 3, dpix, st);
     upload(map_points, (size_t)n_map * 3, dmap, st);
@@ -709,7 +713,11 @@ int ds_smp_product(ds_context* ctx, int n_pix, const double* pixel_points, int n
     a.mask = pl.mask.p;
     a.row_order = pl.row_order.p;
     a.n_row_tiles = mp.n_tiles;
+    a.n_rows = n_map;
+    a.n_cols = n_pix;
     a.v = xs.p;
+    us.alloc(pix.n_pad);
+    a.u = us.p;
     a.out = dm.p;
     a.row_perm = mp.perm.p;
     a.table = table.p;
@@ -729,7 +737,7 @@ int ds_sigma_m_noise_dom(ds_context* ctx, int n_pix, const double* npixels, int 
     const ds_kernel_params k = checked_kp(kp);
     const KernelConsts kc = make_consts(k);
     cudaStream_t st = ctx->stream;
-    DevBuf<double> table, drec, dmap, u, dm;
+    DevBuf<double> table, drec, dmap, u, us, dm;
     load_table(table, k, st);
     upload(npixels, (size_t)n_pix * 5, drec, st);
     upload(map_points, (size_t)n_map * 3, dmap, st);
@@ -752,7 +760,11 @@ int ds_sigma_m_noise_dom(ds_context* ctx, int n_pix, const double* npixels, int 
     a.mask = pl.mask.p;
     a.row_order = pl.row_order.p;
     a.n_row_tiles = mp.n_tiles;
+    a.n_rows = n_map;
+    a.n_cols = n_pix;
     a.v = u.p;
+    us.alloc(pix.n_pad);
+    a.u = us.p;
     a.out = dm.p;
     a.row_perm = mp.perm.p;
     a.table = table.p;

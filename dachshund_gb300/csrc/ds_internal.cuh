@@ -222,12 +222,12 @@ void build_pair_list(PairList& pl, const PointSet& rows, const PointSet& cols,
 void build_slice_items(PairList& pl, cudaStream_t st);
 
 // ---- pair kernels (FP64) -------------------------------------------------
-// Column weight u_j and epilogue selection.
+// Column weight u_j (formed by form_u) and epilogue selection.
 enum PairEpi {
-  EPI_PRODUCT = 0,   // out_i = wl_i acc + e_i v_i      (u_j = wr_j v_j)
+  EPI_PRODUCT = 0,   // out_i = wl_i acc + e_i v_i      (u_j = var_s wr_j v_j)
   EPI_RESIDUAL = 1,  // out_i = b_i - (wl_i acc + e_i v_i)
-  EPI_MAP = 2,       // out[perm_i] = acc               (u_j = v_j)
-  EPI_NOISE = 3      // out[perm_i] = sum S^2 u_j       (u_j = 1 / N_j)
+  EPI_MAP = 2,       // out[perm_i] = acc               (u_j = var_s v_j)
+  EPI_NOISE = 3      // out[perm_i] = sum S^2 u_j       (u_j = var_s^2 / N_j)
 };
 
 struct PairArgs {
@@ -236,11 +236,13 @@ struct PairArgs {
   const double* cx; const double* cy; const double* cz;
   const int* row_ptr; const int* cols;
   int n_row_tiles;
+  int n_rows, n_cols;          // points of each side (the rest is padding)
   const unsigned short* mask;  // sub-tile interaction mask per tile pair
   const int* row_order;        // blockIdx -> row tile (heaviest first), or null
   // coefficients (sorted order)
   const double* wl; const double* wr; const double* e; const double* b;
   const double* v;      // the vector being multiplied (column side)
+  double* u;            // its column weights (the FP64 kernel's)
   const double* vrow;   // the same vector on the row side (diagonal term)
   double* out;
   const int* row_perm;  // EPI_MAP / EPI_NOISE scatter
@@ -285,6 +287,9 @@ struct Profiler {
 
 void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a,
                      cudaStream_t st);
+// u_j = scale (w_j v_j), or scale v_j without w (n_pad entries).
+void form_u(int n_pad, double scale, const double* w, const double* v, double* u,
+            const int* skip, cudaStream_t st);
 
 // ---- PCG -----------------------------------------------------------------
 struct PcgState {
@@ -330,6 +335,7 @@ struct ds_operator {
   double norm_b = 0.0;
   // PCG work space (sorted, padded)
   ds::DevBuf<double> x, r, d, q, s, tmp, tmp2;
+  ds::DevBuf<double> u;            // column weights of the vector being multiplied
   ds::DevBuf<double> partial;      // per-block partial sums
   ds::DevBuf<double> partial2;
   ds::DevBuf<ds::PcgState> state;

@@ -1,14 +1,17 @@
 // FP64 matrix-free pair kernel: one CTA per row tile, one row per thread,
-// looping over the row tile's culled column tiles.  Column coordinates and
-// weights are staged in shared memory and read as broadcasts; the 200-knot
-// table lives in shared memory.  Serves
+// looping over the row tile's culled column tiles: an FP32 search finds the
+// interacting pairs, which alone are evaluated in FP64.  The 200-knot table
+// lives in shared memory.  Serves
 //   * WFVector{SN,W}::A_product / A_residual (lib/wf_vector.cc:51-103,
 //     196-251), with the CG dot d.q fused into the product epilogue;
 //   * smp_product (lib/map.cc:20-43);
 //   * sigma_m_noise_dom (lib/map_covar.cc:11-38).
-// Roofline: FP64 pipe (about 16 FP64 instructions per pair in table mode,
-// plus exp() in exact mode); no HBM traffic beyond the tiles (L2 resident).
+// Roofline: FP64 pipe (about 19 FP64 instructions per interacting pair with
+// either kernel); no HBM traffic beyond the tiles (L2 resident).
+#include <algorithm>
+
 #include "ds_device.cuh"
+#include "ds_pairhit.cuh"
 
 namespace ds {
 
@@ -23,16 +26,29 @@ __device__ __forceinline__ double g_exact_fast(double dx, double dy, double dz,
   return g;
 }
 
-// Each warp's 32 rows form a k-d sub-tile with its own box; a staged column
-// tile is four 32-column sub-tiles, and a warp skips every column sub-tile
-// whose box is beyond the cutoff from its own (a warp-uniform branch).
+// Each warp's 32 rows form a k-d sub-tile with its own box; a column tile is
+// four 32-column sub-tiles, and a warp visits only the column sub-tiles whose
+// box is within the cutoff of its own (the pair mask).  Per visited block the
+// FP32 test (ds_pairhit.cuh) gives every lane the columns that may interact
+// with its row; they go to the lane's queue in shared memory, in column
+// order, and are evaluated in FP64 from there.  A row's sum takes its
+// interacting columns in ascending tile, sub-tile and column order (the terms
+// left out are exact zeros).
+//
+// Bound: the FP64 pipe, ~20 instructions per interacting pair (2 lanes per
+// clock per SM).  A queue of QLEN columns per lane is drained only when one
+// fills, so a step that evaluates one pair per lane finds almost all lanes
+// busy (rows of a sub-tile have similar neighbourhoods, single blocks do
+// not).  Measured against evaluating every pair of the visited blocks: the
+// 409,600-point exact map of 32,768 pixels 45.0 -> 35.2 ms, the table-kernel
+// solve and 131,072-point map of 4,096 pixels 115 -> 63 ms, the same bits.
+constexpr int QLEN = 64;  // a block adds at most 32
+
 template <int EVAL, int EPI, bool DOT>
 __global__ void __launch_bounds__(TILE) k_pair_f64(KernelConsts kc, PairArgs a) {
   if (a.skip_flag && *a.skip_flag) return;
-  // Warp-private staging of one 32-column sub-tile at a time: a warp loads
-  // only the column sub-tiles its own row sub-tile interacts with, and the
-  // warps of a CTA never wait for each other inside the loop.
-  __shared__ double sw[TILE / 32][4][SUBTILE];
+  __shared__ float4 scol[TILE / 32][SUBTILE];
+  __shared__ int queue[TILE / 32][QLEN][32];
   __shared__ double tf[EVAL == DS_EVAL_TABLE ? TABLE_N : 32];
   __shared__ double red[TILE / 32];
   const int t = a.row_order ? a.row_order[blockIdx.x] : blockIdx.x;  // heaviest tiles first
@@ -44,15 +60,22 @@ __global__ void __launch_bounds__(TILE) k_pair_f64(KernelConsts kc, PairArgs a) 
     tf[tid] = exp2(-(double)tid / 32.0);
   }
   __syncthreads();
-  // var_s, folded into the column weights (squared for the S^2 sum)
-  const double wscale = EPI == EPI_NOISE ? kc.var_s * kc.var_s : kc.var_s;
   const double xi = a.rx[i], yi = a.ry[i], zi = a.rz[i];
+  float3 row;
+  const HitFrame frame = hit_frame(kc, xi, yi, zi, row);
   double acc = 0.0;
-  unsigned long long evaluated = 0;  // pairs this warp evaluates (profiling)
-  double* sxw = sw[warp][0];
-  double* syw = sw[warp][1];
-  double* szw = sw[warp][2];
-  double* suw = sw[warp][3];
+  int head = 0, tail = 0;  // this lane's queue
+  auto step = [&] {
+    if (head < tail) {
+      const int j = queue[warp][head & (QLEN - 1)][lane];
+      ++head;
+      const double dx = xi - a.cx[j], dy = yi - a.cy[j], dz = zi - a.cz[j];
+      double g = EVAL == DS_EVAL_TABLE ? gp_table_fast(dx, dy, dz, kc, tf)
+                                       : g_exact_fast(dx, dy, dz, kc, tf);
+      if (EPI == EPI_NOISE) g = g * g;
+      acc = fma(g, a.u[j], acc);
+    }
+  };
   const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
   for (int p = p0; p < p1; ++p) {
     const unsigned m = (a.mask[p] >> (4 * warp)) & 0xFu;  // this warp's row sub-tile
@@ -60,28 +83,27 @@ __global__ void __launch_bounds__(TILE) k_pair_f64(KernelConsts kc, PairArgs a) 
     const int ct = a.cols[p];
     for (int cs = 0; cs < TILE / SUBTILE; ++cs) {
       if (!((m >> cs) & 1u)) continue;
-      const int j = ct * TILE + cs * SUBTILE + lane;
+      const int j0 = ct * TILE + cs * SUBTILE;
+      const float3 c = hit_point(frame, a.cx[j0 + lane], a.cy[j0 + lane], a.cz[j0 + lane]);
       __syncwarp();
-      sxw[lane] = a.cx[j];
-      syw[lane] = a.cy[j];
-      szw[lane] = a.cz[j];
-      if (EPI == EPI_PRODUCT || EPI == EPI_RESIDUAL)
-        suw[lane] = wscale * (a.wr[j] * a.v[j]);
-      else
-        suw[lane] = wscale * a.v[j];
+      scol[warp][lane] = make_float4(c.x, c.y, c.z, 0.f);
       __syncwarp();
-      evaluated += SUBTILE * SUBTILE;
-#pragma unroll 4
-      for (int jj = 0; jj < SUBTILE; ++jj) {
-        const double dx = xi - sxw[jj], dy = yi - syw[jj], dz = zi - szw[jj];
-        double g = EVAL == DS_EVAL_TABLE ? gp_table_fast(dx, dy, dz, kc, tf)
-                                         : g_exact_fast(dx, dy, dz, kc, tf);
-        if (EPI == EPI_NOISE) g = g * g;
-        acc = fma(g, suw[jj], acc);
+      unsigned h = hit_mask(frame, row, scol[warp]);
+      if (i >= a.n_rows) h = 0;  // padding rows and columns carry no term
+      if (a.n_cols - j0 < SUBTILE) h &= (1u << max(a.n_cols - j0, 0)) - 1u;
+      while (h) {
+        queue[warp][tail & (QLEN - 1)][lane] = j0 + __ffs(h) - 1;
+        ++tail;
+        h &= h - 1;
       }
+      while (__any_sync(0xffffffffu, tail - head > QLEN - SUBTILE)) step();
     }
   }
-  if (a.prof_pairs && (tid & 31) == 0) atomicAdd(a.prof_pairs, evaluated);
+  while (__any_sync(0xffffffffu, head < tail)) step();
+  if (a.prof_pairs) {
+    const int evaluated = __reduce_add_sync(0xffffffffu, tail);
+    if (lane == 0) atomicAdd(a.prof_pairs, (unsigned long long)evaluated);
+  }
   if (EPI == EPI_PRODUCT || EPI == EPI_RESIDUAL) {
     const double q = a.wl[i] * acc + a.e[i] * a.v[i];
     const double o = (EPI == EPI_RESIDUAL) ? a.b[i] - q : q;
@@ -102,6 +124,14 @@ __global__ void __launch_bounds__(TILE) k_pair_f64(KernelConsts kc, PairArgs a) 
     const int dst = a.row_perm[i];
     if (dst >= 0) a.out[dst] = acc;
   }
+}
+
+__global__ void k_form_u(int n, double scale, const double* __restrict__ w,
+                         const double* __restrict__ v, double* __restrict__ u,
+                         const int* skip) {
+  if (skip && *skip) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    u[i] = scale * (w ? w[i] * v[i] : v[i]);
 }
 
 template <int EVAL>
@@ -130,9 +160,19 @@ void launch_eval(const KernelConsts& kc, int epi, const PairArgs& a, cudaStream_
 
 }  // namespace
 
+void form_u(int n_pad, double scale, const double* w, const double* v, double* u,
+            const int* skip, cudaStream_t st) {
+  k_form_u<<<std::max(1, std::min(1024, (n_pad + 255) / 256)), 256, 0, st>>>(n_pad, scale, w, v, u,
+                                                                            skip);
+  DS_CHECK_LAUNCH();
+}
+
 void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a0, cudaStream_t st) {
   if (a0.n_row_tiles <= 0) return;
   PairArgs a = a0;
+  const bool op = epi == EPI_PRODUCT || epi == EPI_RESIDUAL;
+  form_u((a.n_cols + TILE - 1) / TILE * TILE, epi == EPI_NOISE ? kc.var_s * kc.var_s : kc.var_s,
+         op ? a.wr : nullptr, a.v, a.u, a.skip_flag, st);
   cudaEvent_t ev = nullptr;
   const int kind = epi == EPI_MAP ? 2 : 0;
   if (a.prof && a.prof->enabled) {

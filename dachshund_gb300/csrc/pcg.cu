@@ -167,6 +167,9 @@ PairArgs op_pair_args(ds_operator* op, const double* v, double* out) {
   a.mask = op->pairs.mask.p;
   a.row_order = op->pairs.row_order.p;
   a.n_row_tiles = op->pix.n_tiles;
+  a.n_rows = a.n_cols = op->pix.n;
+  op->u.alloc(op->pix.n_pad);
+  a.u = op->u.p;
   a.wl = op->wl.p;
   a.wr = op->wr.p;
   a.e = op->e.p;
