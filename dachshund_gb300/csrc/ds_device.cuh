@@ -135,6 +135,15 @@ __device__ __forceinline__ double exp_neg_f64(double a, const double* tab) {
   return __longlong_as_double(__double_as_longlong(v) - ((long long)(k >> 5) << 52));
 }
 
+// Exact kernel without var_s, zero at and beyond the cutoff.
+__device__ __forceinline__ double g_exact_fast(double dx, double dy, double dz,
+                                               const KernelConsts& k, const double* tab) {
+  const double arg = fma(k.c_perp, fma(dx, dx, dy * dy), k.c_para * (dz * dz));
+  double g = 0.0;
+  if (arg < k.exact_cut) g = exp_neg_f64(arg, tab);
+  return g;
+}
+
 // Sub-tile / tile box test: true when the nearest corners of two boxes
 // (lo x, y, z, hi x, y, z in raw coordinates) are inside the cutoff.
 __device__ __forceinline__ bool boxes_interact(const double* __restrict__ bi,

@@ -291,6 +291,18 @@ void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a,
 void form_u(int n_pad, double scale, const double* w, const double* v, double* u,
             const int* skip, cudaStream_t st);
 
+// The FP64 operator's interacting pairs as stored values (pair_vals.cu):
+// slices of 32 rows, entry e of lane l of slice s at (start[s] + e) * 32 + l.
+struct PairVals {
+  bool tried = false;  // built or given up
+  bool ok = false;
+  DevBuf<int> cnt;          // entries per row
+  DevBuf<long long> start;  // per slice (+ 1)
+  DevBuf<double> val;       // kernel values without var_s
+  DevBuf<unsigned short> col16;  // column indices (one of the two)
+  DevBuf<int> col32;
+};
+
 // ---- PCG -----------------------------------------------------------------
 struct PcgState {
   double delta;       // r . s (current)
@@ -335,7 +347,7 @@ struct ds_operator {
   double norm_b = 0.0;
   // PCG work space (sorted, padded)
   ds::DevBuf<double> x, r, d, q, s, tmp, tmp2;
-  ds::DevBuf<double> u;            // column weights of the vector being multiplied
+  ds::DevBuf<double> u, ud;        // column weights of the vector being multiplied, of d
   ds::DevBuf<double> partial;      // per-block partial sums
   ds::DevBuf<double> partial2;
   ds::DevBuf<ds::PcgState> state;
@@ -357,6 +369,7 @@ struct ds_operator {
   ds::DevBuf<double> dense_part, dense_dot;
   ds::DevBuf<unsigned int> dense_cnt;
   bool pairs_built = false;  // `pairs` (ensure_op_pairs)
+  ds::PairVals vals;         // the pairs' values (ensure_pair_vals)
   int inner_variant = 0;     // inner matvec of the mixed form (InnerVariant)
   int iter_form = 0;         // DS_ITER_AUTO / DS_ITER_GRAPH
   // skewer-band preconditioner of the mixed form (null: Jacobi)

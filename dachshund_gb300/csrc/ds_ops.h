@@ -61,6 +61,12 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
 // (pcg.cu; op_pair_args calls it).
 void ensure_op_pairs(ds_operator* op);
 
+// The operator's pair values, built on the first FP64 product; false when
+// they would take too much memory (pair_vals.cu).
+bool ensure_pair_vals(ds_operator* op);
+// out = A v or b - A v from them (a as for launch_pair_f64, a.u formed).
+void launch_pair_vals(ds_operator* op, int epi, const PairArgs& a, cudaStream_t st);
+
 // The map's tiled point set, built on the first call that needs it (the
 // structured column-grid map reads the points as given).
 void ensure_map_points(ds_map* map);

@@ -17,15 +17,6 @@ namespace ds {
 
 namespace {
 
-// Exact kernel without var_s, zero at and beyond the cutoff.
-__device__ __forceinline__ double g_exact_fast(double dx, double dy, double dz,
-                                               const KernelConsts& k, const double* tab) {
-  const double arg = fma(k.c_perp, fma(dx, dx, dy * dy), k.c_para * (dz * dz));
-  double g = 0.0;
-  if (arg < k.exact_cut) g = exp_neg_f64(arg, tab);
-  return g;
-}
-
 // Each warp's 32 rows form a k-d sub-tile with its own box; a column tile is
 // four 32-column sub-tiles, and a warp visits only the column sub-tiles whose
 // box is within the cutoff of its own (the pair mask).  Per visited block the

@@ -101,14 +101,20 @@ __global__ void __launch_bounds__(VB) k_pcg_update(int n, PcgState* st, double* 
   }
 }
 
-// d = s + beta d (lib/pcg.h:62-64).
+// d = s + beta d (lib/pcg.h:62-64) and, with u, the column weights of d
+// for the next product.
 __global__ void __launch_bounds__(VB) k_pcg_direction(int n, const PcgState* st,
                                                       const double* __restrict__ s,
-                                                      double* __restrict__ d) {
+                                                      double* __restrict__ d, double var_s,
+                                                      const double* __restrict__ wr,
+                                                      double* __restrict__ u) {
   if (st->done) return;
   const double beta = st->beta;
-  for (int i = blockIdx.x * VB + threadIdx.x; i < n; i += gridDim.x * VB)
-    d[i] = fma(beta, d[i], s[i]);
+  for (int i = blockIdx.x * VB + threadIdx.x; i < n; i += gridDim.x * VB) {
+    const double di = fma(beta, d[i], s[i]);
+    d[i] = di;
+    if (u) u[i] = var_s * (wr[i] * di);
+  }
 }
 
 __global__ void k_gather(int n_pad, const int* __restrict__ perm, const double* __restrict__ src,
@@ -189,7 +195,12 @@ void op_apply_sorted(ds_operator* op, int epi, const double* v, double* out, cud
     return;
   }
   PairArgs a = op_pair_args(op, v, out);
-  launch_pair_f64(op->kc, epi, a, st);
+  if (ensure_pair_vals(op)) {
+    form_u(op->pix.n_pad, op->kc.var_s, a.wr, v, a.u, nullptr, st);
+    launch_pair_vals(op, epi, a, st);
+  } else {
+    launch_pair_f64(op->kc, epi, a, st);
+  }
 }
 
 void ensure_pcg_workspace(ds_operator* op) {
@@ -202,7 +213,7 @@ void ensure_pcg_workspace(ds_operator* op) {
   op->partial.alloc(std::max<size_t>(2 * VGRID_MAX, op->pix.n_tiles));
   // + 2 n_pad: the per-skewer (r.z, |r|^2) partials of the preconditioned
   // mixed form, after the n_tiles p.q partials
-  op->partial2.alloc(std::max((size_t)2 * VGRID_MAX, (size_t)op->pix.n_tiles) +
+  op->partial2.alloc(std::max((size_t)2 * VGRID_MAX, (size_t)op->pix.n_pad / 32) +
                      2 * (size_t)op->pix.n_pad);
   op->state.alloc(1);
   op->h_flag.alloc(64);
@@ -244,6 +255,13 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   prod.skip_flag = &S->done;
   PairArgs resid = op_pair_args(op, op->x.p, op->r.p);
   resid.skip_flag = &S->done;
+  const bool vals = !op->use_dense && ensure_pair_vals(op);
+  double* u = nullptr;  // the weights of d, kept by k_pcg_direction
+  if (vals) {
+    op->ud.alloc(np);
+    u = prod.u = op->ud.p;
+    form_u(np, op->kc.var_s, prod.wr, op->d.p, u, nullptr, st);
+  }
 
   constexpr int CHECK = 8;     // read the done flag every CHECK iterations
   constexpr int NSLOT = 64;
@@ -253,6 +271,8 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   for (int it = 1; it < pp.max_iter; ++it) {
     if (op->use_dense)  // q = A d, alpha
       dense_apply(op, false, op->d.p, op->q.p, op->d.p, S, &S->done, st);
+    else if (vals)
+      launch_pair_vals(op, EPI_PRODUCT, prod, st);
     else
       launch_pair_f64(op->kc, EPI_PRODUCT, prod, st);
     if (it % pp.step_r == 0) {
@@ -261,7 +281,10 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
       DS_CHECK_LAUNCH();
       if (op->use_dense)  // r = b - A x
         dense_apply(op, true, op->x.p, op->r.p, nullptr, nullptr, &S->done, st);
-      else
+      else if (vals) {
+        form_u(np, op->kc.var_s, resid.wr, op->x.p, resid.u, resid.skip_flag, st);
+        launch_pair_vals(op, EPI_RESIDUAL, resid, st);
+      } else
         launch_pair_f64(op->kc, EPI_RESIDUAL, resid, st);
       k_pcg_update<2><<<g, VB, 0, st>>>(np, S, op->x.p, op->r.p, op->d.p, op->q.p, op->s.p,
                                         op->pdiag.p, op->partial.p, op->hist.p, op->dhist.p);
@@ -270,7 +293,7 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
                                         op->pdiag.p, op->partial.p, op->hist.p, op->dhist.p);
     }
     DS_CHECK_LAUNCH();
-    k_pcg_direction<<<g, VB, 0, st>>>(np, S, op->s.p, op->d.p);
+    k_pcg_direction<<<g, VB, 0, st>>>(np, S, op->s.p, op->d.p, op->kc.var_s, op->wr.p, u);
     DS_CHECK_LAUNCH();
     if (it % CHECK == 0) {
       const int slot = issued % NSLOT;

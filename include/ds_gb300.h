@@ -179,7 +179,13 @@ typedef struct {
 } ds_operator_info;
 int ds_operator_get_info(ds_operator* op, ds_operator_info* info);
 
-/* WFVector{SN,W}::A_product, b = A a (lib/wf_vector.cc:51-74, 196-220). */
+/* WFVector{SN,W}::A_product, b = A a (lib/wf_vector.cc:51-74, 196-220).  The
+ * operator's first FP64 product (here, in A_residual or in solve_pcg) evaluates
+ * every interacting pair once and keeps the values on the device (10 to 12
+ * bytes per pair: about 0.6 GB at 32,768 pixels and 8 GB at 262,144 with the
+ * exact kernel); later products read them.  An operator whose values would take
+ * more than an eighth of the free device memory evaluates its pairs on every
+ * call instead, with the same results to rounding. */
 int ds_A_product(ds_operator* op, const double* a, double* b);
 int ds_A_product_dev(ds_operator* op, const double* a, double* b);
 
