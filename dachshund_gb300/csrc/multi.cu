@@ -15,7 +15,7 @@
 // return at once when all have.
 //
 // Vectors are n_pad x R doubles in the operator's sorted order with the
-// right-hand side fastest (v[i * R + r]), R a power of two from 16 to 256.
+// right-hand side fastest (v[i * R + r]), R a power of two from 32 to 256.
 // Reductions are deterministic (fixed tree and partial orders, no floating
 // atomics).
 #include <algorithm>
@@ -30,6 +30,7 @@ namespace ds {
 namespace {
 
 constexpr int MR = 16;       // right-hand sides per CTA of the pair kernel
+constexpr int MR_MIN = 32;   // right-hand sides per solve at least (a warp of the list product)
 constexpr int MR_MAX = 256;  // right-hand sides per solve at most
 constexpr int MVB = 256;     // threads per vector-kernel CTA (R divides it)
 constexpr int MVGRID = 304;  // vector-kernel CTAs at most
@@ -45,7 +46,9 @@ struct MShared {
   int max_iter;
   int R;  // right-hand sides of this solve
   int pad;
-  unsigned int counter[4];
+  // arrivals: [0, 8) products, [8, 16) updates (one per 32 right-hand sides),
+  // 16 finished groups of an update, 17 |b|, 18 sigma, 19 evaluating products
+  unsigned int counter[20];
 };
 
 struct MPairArgs {
@@ -161,7 +164,7 @@ __global__ void __launch_bounds__(TILE) k_mpair(KernelConsts kc, MPairArgs a) {
   }
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = atomicAdd(&a.sh->counter[0], 1u) == gridDim.x * gridDim.y - 1;
+  if (tid == 0) last = atomicAdd(&a.sh->counter[19], 1u) == gridDim.x * gridDim.y - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
@@ -175,7 +178,124 @@ __global__ void __launch_bounds__(TILE) k_mpair(KernelConsts kc, MPairArgs a) {
       st.alpha = st.delta / dq;  // lib/pcg.h:37
     }
   }
-  if (tid == 0) a.sh->counter[0] = 0;
+  if (tid == 0) a.sh->counter[19] = 0;
+}
+
+// True in the last of `n` CTAs to arrive on a counter (left at 0).
+__device__ __forceinline__ bool last_of_group(unsigned int* counter, unsigned int n) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == n - 1;
+    if (last) *counter = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Sum of n values part[k * stride] (each lane its own part), valid in warp 0:
+// warp w takes k = w, w + 8, ..., then the warps in order.
+__device__ __forceinline__ double sum_rows(const double* part, int stride, int n, double* red) {
+  constexpr int W = MVB / 32;
+  const int warp = threadIdx.x >> 5;
+  double v = 0.0;
+#pragma unroll 8
+  for (int k = warp; k < n; k += W) v += __ldcg(part + (size_t)k * stride);
+  __syncthreads();  // red may still be read by a previous call
+  red[threadIdx.x] = v;
+  __syncthreads();
+  if (warp == 0)
+    for (int w = 1; w < W; ++w) v += red[w * 32 + threadIdx.x];
+  return v;
+}
+
+// The same products from the operator's stored values: a warp takes one row of
+// 32 right-hand sides (its lanes), CTA (x, y) the rows [8 x, 8 x + 8) and the
+// right-hand sides [32 y, 32 y + 32).  The lanes load 32 entries of a row at a
+// time and hand them round by shuffles; the neighbour's 32 values are one
+// 256-byte load per entry.  Rows are summed in list order.  Bound by the FP64
+// FMAs (83% of the pipe while an SM is busy); one row a warp rather than four
+// keeps enough CTAs for an even spread over the SMs (548 -> 445 us per product
+// of 4,096 rows and 256 right-hand sides; the evaluating kernel 4.0 ms).
+template <bool RESID, bool DOT, class I>
+__global__ void __launch_bounds__(MVB) k_mvals(double var_s, MPairArgs a,
+                                               const int* __restrict__ cnt,
+                                               const long long* __restrict__ start,
+                                               const I* __restrict__ cols,
+                                               const double* __restrict__ val) {
+  constexpr unsigned full = 0xffffffffu;
+  constexpr int W = MVB / 32;
+  if (a.sh->all_done) return;
+  __shared__ double red[MVB];
+  const int R = a.sh->R, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.y * 32 + lane;
+  const bool live = !a.st[r].done;
+  double dot = 0.0;
+  if (__any_sync(full, live)) {
+    const int i = blockIdx.x * W + warp;
+    const int n = cnt[i];
+    const size_t at = (size_t)start[i >> 5] * 32 + (i & 31);
+    double acc = 0.0;
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      int j = 0;
+      double g = 0.0;
+      if (e0 + lane < n) {
+        j = cols[at + (size_t)(e0 + lane) * 32];
+        g = val[at + (size_t)(e0 + lane) * 32] * (var_s * a.wr[j]);
+      }
+      const int m = min(32, n - e0);
+#pragma unroll 8
+      for (int e = 0; e < m; ++e) {
+        const int je = __shfl_sync(full, j, e);
+        const double ge = __shfl_sync(full, g, e);
+        acc = fma(ge, a.v[(size_t)je * R + r], acc);
+      }
+    }
+    const size_t o = (size_t)i * R + r;
+    const double q = a.wl[i] * acc + a.e[i] * a.v[o];
+    const double out = RESID ? a.b[o] - q : q;
+    if (live) a.out[o] = out;  // a converged right-hand side stays as it was
+    if (DOT) dot = a.dotv[o] * out;
+  }
+  if (!DOT) return;
+  red[threadIdx.x] = dot;
+  __syncthreads();
+  if (warp == 0) {  // the warps in order
+    for (int w = 1; w < W; ++w) dot += red[w * 32 + lane];
+    a.part[(size_t)blockIdx.x * R + r] = dot;
+  }
+  if (!last_of_group(&a.sh->counter[blockIdx.y], gridDim.x)) return;
+  // the group's last CTA: d.q per right-hand side
+  const double dq = sum_rows(a.part + r, R, gridDim.x, red);
+  if (warp == 0 && live) {
+    MState& st = a.st[r];
+    st.dq = dq;
+    st.alpha = st.delta / dq;  // lib/pcg.h:37
+  }
+}
+
+// A product (RESID: residual) of R vectors: from the stored values when the
+// operator has them, else evaluating.
+template <bool RESID, bool DOT>
+void mproduct(ds_operator* op, const MPairArgs& a, int R, bool vals, cudaStream_t st) {
+  const PairVals& pv = op->vals;
+  const dim3 grid(op->pix.n_pad / (MVB / 32), R / 32);
+  if (!vals)
+    k_mpair<RESID, DOT><<<dim3(op->pix.n_tiles, R / MR), TILE, 0, st>>>(op->kc, a);
+  else if (pv.col16.p)
+    k_mvals<RESID, DOT><<<grid, MVB, 0, st>>>(op->kc.var_s, a, pv.cnt.p, pv.start.p, pv.col16.p,
+                                              pv.val.p);
+  else
+    k_mvals<RESID, DOT><<<grid, MVB, 0, st>>>(op->kc.var_s, a, pv.cnt.p, pv.start.p, pv.col32.p,
+                                              pv.val.p);
+  DS_CHECK_LAUNCH();
+}
+
+__global__ void k_recip(int n, const double* __restrict__ v, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = 1.0 / v[i];
 }
 
 // Per right-hand side sums over the grid of two values each thread holds
@@ -221,7 +341,7 @@ __global__ void __launch_bounds__(MVB) k_mnorm(size_t n, const double* __restric
   double bb = 0.0;
   for (size_t e = (size_t)blockIdx.x * MVB + threadIdx.x; e < n; e += (size_t)gridDim.x * MVB)
     bb = fma(b[e], b[e], bb);
-  if (!grid_sum_by_rhs(R, bb, 0.0, part, &sh->counter[1], tot)) return;
+  if (!grid_sum_by_rhs(R, bb, 0.0, part, &sh->counter[17], tot)) return;
   for (int r = threadIdx.x; r < R; r += MVB) {
     MState& s = st[r];
     s.norm_b = sqrt(tot[r]);
@@ -237,57 +357,73 @@ __global__ void __launch_bounds__(MVB) k_mnorm(size_t n, const double* __restric
 // mode 1: x update only (full-residual step, before the residual kernel)
 // mode 2: precondition + dots only (full-residual step, after the residual)
 // mode 3: start from x = 0: r = b, d = M^-1 r + dots
+// CTA (x, y): right-hand sides [32 y, 32 y + 32) (the lanes) of rows 8 x + warp,
+// + 8 gridDim.x, ..., four rows in flight; ipd = 1 / the Jacobi diagonal.
 template <int MODE>
-__global__ void __launch_bounds__(MVB) k_mupdate(size_t n, MState* st, MShared* sh,
+__global__ void __launch_bounds__(MVB) k_mupdate(int n, MState* st, MShared* sh,
                                                  double* __restrict__ x, double* __restrict__ r,
                                                  double* __restrict__ d,
                                                  const double* __restrict__ q,
                                                  double* __restrict__ s,
                                                  const double* __restrict__ b,
-                                                 const double* __restrict__ pdiag,
+                                                 const double* __restrict__ ipd,
                                                  double* part, double* hist, int hist_stride) {
   if (MODE != 3 && sh->all_done) return;
-  __shared__ double tot[2 * MR_MAX];
-  const int R = sh->R;
-  const int rr = threadIdx.x % R;  // this thread's right-hand side (R divides the stride)
+  __shared__ double red[MVB];
+  constexpr int W = MVB / 32;
+  const int R = sh->R, warp = threadIdx.x >> 5, rr = blockIdx.y * 32 + (threadIdx.x & 31);
   const bool live = !st[rr].done;
   const double alpha = st[rr].alpha;
   double rs = 0.0, r2 = 0.0;
-  for (size_t e = (size_t)blockIdx.x * MVB + threadIdx.x; e < n; e += (size_t)gridDim.x * MVB) {
-    if (!live) break;
-    if (MODE == 0 || MODE == 1) x[e] = fma(alpha, d[e], x[e]);  // lib/pcg.h:39
-    if (MODE == 1) continue;
-    double ri;
-    if (MODE == 3) {
-      ri = b[e];  // r = b - A x with x = 0
-      r[e] = ri;
-    } else {
-      ri = r[e];
+  if (live) {
+#pragma unroll 4
+    for (int i = blockIdx.x * W + warp; i < n; i += gridDim.x * W) {
+      const size_t e = (size_t)i * R + rr;
+      if (MODE == 0 || MODE == 1) x[e] = fma(alpha, d[e], x[e]);  // lib/pcg.h:39
+      if (MODE == 1) continue;
+      double ri;
+      if (MODE == 3) {
+        ri = b[e];  // r = b - A x with x = 0
+        r[e] = ri;
+      } else {
+        ri = r[e];
+      }
+      if (MODE == 0) {
+        ri = fma(-alpha, q[e], ri);  // lib/pcg.h:48
+        r[e] = ri;
+      }
+      const double si = ri * ipd[i];  // lib/pcg.h:52
+      s[e] = si;
+      if (MODE == 3) d[e] = si;
+      rs = fma(ri, si, rs);
+      r2 = fma(ri, ri, r2);
     }
-    if (MODE == 0) {
-      ri = fma(-alpha, q[e], ri);  // lib/pcg.h:48
-      r[e] = ri;
-    }
-    const double si = ri / pdiag[e / R];  // lib/pcg.h:52
-    s[e] = si;
-    if (MODE == 3) d[e] = si;
-    rs = fma(ri, si, rs);
-    r2 = fma(ri, ri, r2);
   }
   if (MODE == 1) return;
-  if (!grid_sum_by_rhs(R, rs, r2, part, &sh->counter[1], tot)) return;
-  for (int rq = threadIdx.x; rq < R; rq += MVB) {
-    MState& S = st[rq];
-    const double trs = tot[rq], trr = tot[R + rq];
-    double* h = hist + (size_t)rq * hist_stride;
+  red[threadIdx.x] = rs;
+  __syncthreads();
+  if (warp == 0)
+    for (int w = 1; w < W; ++w) rs += red[w * 32 + threadIdx.x];
+  __syncthreads();
+  red[threadIdx.x] = r2;
+  __syncthreads();
+  if (warp == 0) {
+    for (int w = 1; w < W; ++w) r2 += red[w * 32 + threadIdx.x];
+    part[(size_t)blockIdx.x * 2 * R + rr] = rs;
+    part[(size_t)blockIdx.x * 2 * R + R + rr] = r2;
+  }
+  if (!last_of_group(&sh->counter[8 + blockIdx.y], gridDim.x)) return;
+  const double trs = sum_rows(part + rr, 2 * R, gridDim.x, red);
+  const double trr = sum_rows(part + R + rr, 2 * R, gridDim.x, red);
+  if (warp == 0 && live) {
+    MState& S = st[rr];
+    double* h = hist + (size_t)rr * hist_stride;
     if (MODE == 3) {
-      if (!S.done) {
-        S.delta = trs;  // lib/pcg.h:104
-        S.norm_r = sqrt(trr);
-        h[0] = S.norm_r;
-        if (sh->max_iter <= 1) S.done = 1;
-      }
-    } else if (!S.done) {
+      S.delta = trs;  // lib/pcg.h:104
+      S.norm_r = sqrt(trr);
+      h[0] = S.norm_r;
+      if (sh->max_iter <= 1) S.done = 1;
+    } else {
       S.delta_old = S.delta;
       S.delta = trs;                        // lib/pcg.h:58
       S.beta = S.delta / S.delta_old;       // lib/pcg.h:61
@@ -303,12 +439,12 @@ __global__ void __launch_bounds__(MVB) k_mupdate(size_t n, MState* st, MShared* 
       }
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int all = 1;
-    for (int k = 0; k < R; ++k) all &= st[k].done;
-    sh->all_done = all;
-  }
+  // the last group to finish sees every right-hand side's state
+  if (!last_of_group(&sh->counter[16], gridDim.y)) return;
+  int running = 0;
+  for (int k = threadIdx.x; k < R; k += MVB) running |= !__ldcg(&st[k].done);
+  running = __syncthreads_or(running);
+  if (threadIdx.x == 0) sh->all_done = !running;
 }
 
 // d = s + beta d (lib/pcg.h:62-64) for the right-hand sides still running.
@@ -316,7 +452,7 @@ __global__ void __launch_bounds__(MVB) k_mdir(size_t n, const MState* st, const 
                                               const double* __restrict__ s,
                                               double* __restrict__ d) {
   if (sh->all_done) return;
-  const int rr = threadIdx.x % sh->R;
+  const int R = sh->R, rr = threadIdx.x % R;
   if (st[rr].done) return;
   const double beta = st[rr].beta;
   for (size_t e = (size_t)blockIdx.x * MVB + threadIdx.x; e < n; e += (size_t)gridDim.x * MVB)
@@ -368,15 +504,18 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
   cudaStream_t st = op->ctx->stream;
   require(pp.max_iter >= 0, "max_iter must be >= 0");
   require(pp.step_r > 0, "step_r must be > 0");
-  // right-hand sides per solve: a power of two from 16 to 256 covering the
-  // map points (or at least enough CTAs for the device)
-  int R = MR;
+  // right-hand sides per solve: a power of two from 32 to 256 covering the
+  // map points
+  int R = MR_MIN;
   while (R < MR_MAX && R < n_map) R *= 2;
   const int np = op->pix.n_pad;
   const size_t nv = (size_t)np * R;
   const int g = mgrid(nv);
+  const int gd = (int)std::max<size_t>(1, std::min<size_t>(2432, (nv + MVB - 1) / MVB));
+  const dim3 ug(std::min(np / (MVB / 32), std::max(1, 1216 * 32 / R)), R / 32);
   const int hist_stride = std::max(pp.max_iter, 1) + 1;
-  DevBuf<double> b, x, r, d, q, s, part, hist, mp, sig;
+  const bool vals = ensure_pair_vals(op);
+  DevBuf<double> b, x, r, d, q, s, part, hist, mp, sig, ipd;
   DevBuf<MState> dst;
   DevBuf<MShared> dsh;
   b.alloc(nv);
@@ -385,7 +524,10 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
   d.alloc(nv);
   q.alloc(nv);
   s.alloc(nv);
-  part.alloc(std::max<size_t>((size_t)2 * R * g, (size_t)op->pix.n_tiles * R));
+  part.alloc(std::max<size_t>((size_t)2 * R * std::max<size_t>(g, ug.x), (size_t)np / 8 * R));
+  ipd.alloc(np);
+  k_recip<<<(np + MVB - 1) / MVB, MVB, 0, st>>>(np, op->pdiag.p, ipd.p);
+  DS_CHECK_LAUNCH();
   hist.alloc((size_t)R * hist_stride);
   mp.alloc(3 * (size_t)R);
   sig.alloc(R);
@@ -414,7 +556,6 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
   resid.v = x.p;
   resid.b = b.p;
   resid.out = r.p;
-  const dim3 pgrid(op->pix.n_tiles, R / MR), pblock(TILE);
 
   std::vector<double> hp(3 * (size_t)R), hs(R);
   std::vector<MState> hst(R);
@@ -436,26 +577,24 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
     k_mnorm<<<g, MVB, 0, st>>>(nv, b.p, pp.tol, dst.p, dsh.p, part.p);
     DS_CHECK_LAUNCH();
     // r = b (x = 0), d = M^-1 r, delta, |r|  (lib/pcg.h:95-108)
-    k_mupdate<3><<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                    op->pdiag.p, part.p, hist.p, hist_stride);
+    k_mupdate<3><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
+                                    ipd.p, part.p, hist.p, hist_stride);
     DS_CHECK_LAUNCH();
     for (int it = 1; it < pp.max_iter; ++it) {
-      k_mpair<false, true><<<pgrid, pblock, 0, st>>>(op->kc, prod);
-      DS_CHECK_LAUNCH();
+      mproduct<false, true>(op, prod, R, vals, st);
       if (it % pp.step_r == 0) {
-        k_mupdate<1><<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        op->pdiag.p, part.p, hist.p, hist_stride);
+        k_mupdate<1><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
+                                        ipd.p, part.p, hist.p, hist_stride);
         DS_CHECK_LAUNCH();
-        k_mpair<true, false><<<pgrid, pblock, 0, st>>>(op->kc, resid);
-        DS_CHECK_LAUNCH();
-        k_mupdate<2><<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        op->pdiag.p, part.p, hist.p, hist_stride);
+        mproduct<true, false>(op, resid, R, vals, st);
+        k_mupdate<2><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
+                                        ipd.p, part.p, hist.p, hist_stride);
       } else {
-        k_mupdate<0><<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        op->pdiag.p, part.p, hist.p, hist_stride);
+        k_mupdate<0><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
+                                        ipd.p, part.p, hist.p, hist_stride);
       }
       DS_CHECK_LAUNCH();
-      k_mdir<<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, s.p, d.p);
+      k_mdir<<<gd, MVB, 0, st>>>(nv, dst.p, dsh.p, s.p, d.p);
       DS_CHECK_LAUNCH();
       if (it % MCHECK == 0) {
         DS_CUDA(cudaMemcpyAsync(&h_done, &dsh.p->all_done, sizeof(int), cudaMemcpyDeviceToHost,
@@ -464,7 +603,7 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
         if (h_done) break;
       }
     }
-    k_msigma<<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, b.p, x.p, &dsh.p->counter[2], part.p, sig.p);
+    k_msigma<<<g, MVB, 0, st>>>(nv, dst.p, dsh.p, b.p, x.p, &dsh.p->counter[18], part.p, sig.p);
     DS_CHECK_LAUNCH();
     DS_CUDA(cudaMemcpyAsync(hs.data(), sig.p, R * sizeof(double), cudaMemcpyDeviceToHost, st));
     DS_CUDA(cudaMemcpyAsync(hst.data(), dst.p, R * sizeof(MState), cudaMemcpyDeviceToHost, st));
