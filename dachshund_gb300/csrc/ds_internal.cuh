@@ -368,6 +368,9 @@ struct ds_operator {
   ds::DevBuf<float2> dense_vff;
   ds::DevBuf<double> dense_part, dense_dot;
   ds::DevBuf<unsigned int> dense_cnt;
+  // nonzero 64 x 64 blocks (a word per work item), their words per row block
+  // and a flag (dense.cu)
+  ds::DevBuf<unsigned int> dense_mask, dense_need;
   bool pairs_built = false;  // `pairs` (ensure_op_pairs)
   ds::PairVals vals;         // the pairs' values (ensure_pair_vals)
   int inner_variant = 0;     // inner matvec of the mixed form (InnerVariant)

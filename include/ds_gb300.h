@@ -138,7 +138,7 @@ typedef struct {
   double map_evaluated;
   long long dense_launches;  /* dense-operator matvecs (ds_operator_set_dense) */
   double dense_ms;
-  double dense_entries;      /* matrix entries read (n_pad^2 per matvec) */
+  double dense_entries;      /* matrix entries read (its nonzero 64 x 64 blocks) */
 } ds_profile;
 int ds_context_set_profiling(ds_context* ctx, int enable);
 int ds_context_get_profile(ds_context* ctx, ds_profile* out);
