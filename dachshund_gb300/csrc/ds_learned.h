@@ -61,8 +61,9 @@ struct LearnedNet {
 // = record, blocks of n_per consecutive records) or per cluster of
 // neighbouring skewers (crec: the record of each slot, -1 on padding).
 bool layer_tc_usable(int M, int N, int K);
-void launch_layer_tc(int M, const float* A, const __nv_bfloat16* W, const float* bias, float* Z,
-                     float* out, const float* res, float* wt, int* err, cudaStream_t st);
+void launch_layer_tc(int M, int n_per, const float* h, const int* nbr, const float* gw,
+                     const __nv_bfloat16* W, const float* bias, float* out, float* wt, int* err,
+                     cudaStream_t st);
 
 struct SkewerPC {
   int n_sk = 0, n_per = 0, band = 0;  // blocks, slots per block, bandwidth

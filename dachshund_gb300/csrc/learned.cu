@@ -240,6 +240,67 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* 
   }
 }
 
+// h0 = relu(X W_in + b_in) (Z: the sum before relu, kept for training): CTA of
+// EMB_ROWS rows, W_in as FP32 in shared memory, a thread 4 channels of a row at
+// a time (stores are whole rows).  Bound by the 4 H bytes written per row.
+constexpr int EMB_ROWS = 64;
+__global__ void __launch_bounds__(256) k_embed(int n, int H, const float* __restrict__ X,
+                                               const __nv_bfloat16* __restrict__ W,
+                                               const float* __restrict__ bias,
+                                               float* __restrict__ Z, float* __restrict__ h) {
+  __shared__ __align__(16) float w[(F_IN + 1) * 512];  // H <= 512; the bias last
+  for (int q = threadIdx.x; q < F_IN * H; q += 256) w[q] = __bfloat162float(W[q]);
+  for (int q = threadIdx.x; q < H; q += 256) w[F_IN * H + q] = bias[q];
+  __syncthreads();
+  const int H4 = H >> 2, r0 = blockIdx.x * EMB_ROWS;
+  for (int q = threadIdx.x; q < EMB_ROWS * H4; q += 256) {
+    const int i = r0 + q / H4, c = 4 * (q % H4);
+    if (i >= n) break;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < F_IN; ++k) {
+      const float x = X[(size_t)i * F_IN + k];
+      const float4 wk = *reinterpret_cast<const float4*>(&w[k * H + c]);
+      a = make_float4(fmaf(x, wk.x, a.x), fmaf(x, wk.y, a.y), fmaf(x, wk.z, a.z),
+                      fmaf(x, wk.w, a.w));
+    }
+    const float4 b = *reinterpret_cast<const float4*>(&w[F_IN * H + c]);
+    a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    if (Z) *reinterpret_cast<float4*>(Z + (size_t)i * H + c) = a;
+    *reinterpret_cast<float4*>(h + (size_t)i * H + c) =
+        make_float4(fmaxf(a.x, 0.f), fmaxf(a.y, 0.f), fmaxf(a.z, 0.f), fmaxf(a.w, 0.f));
+  }
+}
+
+// Y = h W_o + b_o (4 outputs), a thread per row: bound by reading h.
+__global__ void __launch_bounds__(128) k_head(int n, int H, const float* __restrict__ h,
+                                              const __nv_bfloat16* __restrict__ W,
+                                              const float* __restrict__ bias,
+                                              float* __restrict__ Y) {
+  __shared__ __align__(16) float w[4 * 512];
+  for (int q = threadIdx.x; q < 4 * H; q += 128) w[q] = __bfloat162float(W[q]);
+  __syncthreads();
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= n) return;
+  const float4* hr = reinterpret_cast<const float4*>(h + (size_t)i * H);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto mac = [&](float x, int k) {
+    const float4 wk = *reinterpret_cast<const float4*>(&w[4 * k]);
+    a = make_float4(fmaf(x, wk.x, a.x), fmaf(x, wk.y, a.y), fmaf(x, wk.z, a.z),
+                    fmaf(x, wk.w, a.w));
+  };
+#pragma unroll 8
+  for (int q = 0; q < H / 4; ++q) {
+    const float4 v = hr[q];
+    mac(v.x, 4 * q);
+    mac(v.y, 4 * q + 1);
+    mac(v.z, 4 * q + 2);
+    mac(v.w, 4 * q + 3);
+  }
+  reinterpret_cast<float4*>(Y)[i] =
+      make_float4(a.x + bias[0], a.y + bias[1], a.z + bias[2], a.w + bias[3]);
+}
+
 // Partial products for C[K x N] = A^T D over a chunk of rows: A [M x K],
 // D [M x N] FP32 row-major; each CTA (ky, nx, chunk) writes its 64 x 64 block
 // of the chunk's contribution; k_reduce_chunks sums the chunks (fixed order).
@@ -702,25 +763,32 @@ void LearnedNet::forward(int n_sk, int n_per, const double* rec) {
   DS_CHECK_LAUNCH();
   k_features<<<grid1(n), 256, 0, st>>>(n, n_per, rec, gw.p, X.p);
   DS_CHECK_LAUNCH();
-  gemm_fwd(n, H, F_IN, X.p, F_IN, W_in, b_in, Z[0].p, h[0].p, nullptr, 1);
+  const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(wbf.p);
+  k_embed<<<(n + EMB_ROWS - 1) / EMB_ROWS, 256, 0, st>>>(n, H, X.p, wb + W_in.off,
+                                                         params.p + b_in.off,
+                                                         tc_active ? nullptr : Z[0].p, h[0].p);
+  DS_CHECK_LAUNCH();
   for (int l = 0; l < N_LAYERS; ++l) {
-    k_agg_fwd<<<grid1((size_t)n * (H / 4)), 256, 0, st>>>(n, n_per, H, h[l].p, nbr.p, gw.p,
-                                                          cat[l].p);
-    DS_CHECK_LAUNCH();
     if (tc_active && layer_tc_usable(n, H, 3 * H)) {
       if (!wt.p) wt.alloc((size_t)3 * H * H);
       if (!tc_err.p) {
         tc_err.alloc(1);
         DS_CUDA(cudaMemsetAsync(tc_err.p, 0, sizeof(int), st));
       }
-      // inference only: no Z (the backward pass alone reads it)
-      launch_layer_tc(n, cat[l].p, reinterpret_cast<const __nv_bfloat16*>(wbf.p) + W_l[l].off,
-                      params.p + b_l[l].off, nullptr, h[l + 1].p, h[l].p, wt.p, tc_err.p, st);
+      // inference only: no aggregated activations and no Z (the backward pass
+      // alone reads them)
+      launch_layer_tc(n, n_per, h[l].p, nbr.p, gw.p, wb + W_l[l].off, params.p + b_l[l].off,
+                      h[l + 1].p, wt.p, tc_err.p, st);
     } else {
+      k_agg_fwd<<<grid1((size_t)n * (H / 4)), 256, 0, st>>>(n, n_per, H, h[l].p, nbr.p, gw.p,
+                                                            cat[l].p);
+      DS_CHECK_LAUNCH();
       gemm_fwd(n, H, 3 * H, cat[l].p, 3 * H, W_l[l], b_l[l], Z[l + 1].p, h[l + 1].p, h[l].p, 2);
     }
   }
-  gemm_fwd(n, NO, H, h[N_LAYERS].p, H, W_o, b_o, nullptr, Y.p, nullptr, 0);
+  k_head<<<grid1(n, 128), 128, 0, st>>>(n, H, h[N_LAYERS].p, wb + W_o.off, params.p + b_o.off,
+                                        Y.p);
+  DS_CHECK_LAUNCH();
 }
 
 void LearnedNet::outputs(int n_sk, int n_per, double* y0, float* Lrows) {
