@@ -11,6 +11,13 @@ namespace ds {
 constexpr int F_IN = 11;      // input features per pixel
 constexpr int N_LAYERS = 4;   // message-passing layers
 
+// The skewers that name each skewer as a neighbour (learned_gemm.cu), CSR.
+struct RevLists {
+  DevBuf<int> ptr, cnt, src, idx;
+  DevBuf<float> w;
+  DevBuf<unsigned char> tmp;
+};
+
 struct LearnedNet {
   struct Slot {
     size_t off = 0, rows = 0, cols = 0;
@@ -30,8 +37,11 @@ struct LearnedNet {
   int nsk_cur = 0;
   DevBuf<int> nbr;
   DevBuf<double2> skxy;  // (x, y) per skewer
-  DevBuf<float> gw, X, h[N_LAYERS + 1], Z[N_LAYERS + 1], cat[N_LAYERS], Y, dY, dh, dh2, dZ, dcat,
-      part;
+  DevBuf<float> gw, X, h[N_LAYERS + 1], Y, wf;
+  DevBuf<float> agg[N_LAYERS];  // [A_z h | A_n h] per layer (without training: the first alone)
+  // training
+  DevBuf<float> Z[N_LAYERS + 1], dY, dh, dZ, dZ2, aggT, part;
+  RevLists rev;
   DevBuf<double> dpart;
   // inference: message-passing layers on the tensor cores (learned_tc.cu)
   bool tc_infer = true;
@@ -42,13 +52,11 @@ struct LearnedNet {
   LearnedNet(ds_context* c, int hidden, int band, const KernelConsts& k, unsigned seed);
   void sync_weights();
   void ensure(int n_sk, int n_per);
-  void gemm_fwd(int M, int N, int K, const float* A, int lda, const Slot& W, const Slot& b,
-                float* Zp, float* out, const float* res, int epi);
-  void grad_w(int M, int K, int N, const float* A, int lda, const float* D, const Slot& W,
-              const Slot& b);
+  void ensure_train();
   // records: W-form records (x, y, z, w, w d) of n_sk skewers x n_per pixels,
   // skewer-contiguous, on the device
-  void forward(int n_sk, int n_per, const double* rec);
+  // train: keeps Z and the aggregated activations for backward()
+  void forward(int n_sk, int n_per, const double* rec, bool train);
   void outputs(int n_sk, int n_per, double* y0, float* Lrows);
   void loss_and_grad(int n_sk, int n_per, const double* rec, const double* ystar,
                      const float* probe, float wx, float wp, double* losses);
@@ -64,6 +72,24 @@ bool layer_tc_usable(int M, int N, int K);
 void launch_layer_tc(int M, int n_per, const float* h, const int* nbr, const float* gw,
                      const __nv_bfloat16* W, const float* bias, float* out, float* wt, int* err,
                      cudaStream_t st);
+
+// FP32 layers, forward and backward (learned_gemm.cu).
+size_t layer_grad_parts(int M, int H, int sms);
+size_t small_grad_parts(int H, int sms);
+void layer_forward(int M, int n_per, int H, const float* h, const int* nbr, const float* g,
+                   const __nv_bfloat16* W, const float* bias, float* agg, float* wf, float* Z,
+                   float* out, cudaStream_t st);
+void layer_backward(int M, int n_per, int H, int sms, const float* h, const float* agg,
+                    const RevLists& rev, const __nv_bfloat16* W, const float* Z_below,
+                    const float* dZ, float* dZ_below, float* dh, bool last, float* aggT, float* wf,
+                    float* part, float* dW, float* db, cudaStream_t st);
+void head_backward(int n, int H, const float* dY, const __nv_bfloat16* W, const float* Z,
+                   float* dh, float* dZ, cudaStream_t st);
+void head_grad(int M, int H, int sms, const float* h, const float* dY, float* part, float* dW,
+               float* db, cudaStream_t st);
+void embed_grad(int M, int H, int sms, const float* X, const float* dZ, float* part, float* dW,
+                float* db, cudaStream_t st);
+void build_rev_lists(int n_sk, const int* nbr, const float* g, RevLists& rev, cudaStream_t st);
 
 struct SkewerPC {
   int n_sk = 0, n_per = 0, band = 0;  // blocks, slots per block, bandwidth

@@ -172,74 +172,6 @@ __global__ void k_features(int n, int n_per, const double* __restrict__ rec,
 
 // ---- dense layers -------------------------------------------------------------------
 
-// C[M x N] = A[M x K] B + bias, A FP32 row-major (lda), B BF16: row-major
-// K x N (ldb) or, with TB, stored N x K (B(k, n) = Bm[n ldb + k]).  Epilogue
-// (EPI): 0 plain store; 1 Z = C stored, out = relu(Z); 2 Z stored,
-// out = res + relu(Z).  64 x 64 tiles, K steps of 16, 256 threads with 4 x 4
-// outputs each.
-template <bool TB, int EPI>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A,
-                                              int lda, const __nv_bfloat16* __restrict__ Bm,
-                                              int ldb, const float* __restrict__ bias,
-                                              float* __restrict__ Z, float* __restrict__ out,
-                                              const float* __restrict__ res, int ldc) {
-  __shared__ float As[16][64 + 1];
-  __shared__ float Bs[16][64];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int tr = tid / 16, tc = tid % 16;  // 4 rows x 4 cols each
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int q = tid; q < 64 * 16; q += 256) {
-      const int r = q / 16, kk = q % 16;
-      const int m = m0 + r, k = k0 + kk;
-      As[kk][r] = (m < M && k < K) ? A[(size_t)m * lda + k] : 0.f;
-    }
-    for (int q = tid; q < 16 * 64; q += 256) {
-      const int kk = q / 64, c = q % 64;
-      const int k = k0 + kk, n = n0 + c;
-      float v = 0.f;
-      if (k < K && n < N)
-        v = __bfloat162float(TB ? Bm[(size_t)n * ldb + k] : Bm[(size_t)k * ldb + n]);
-      Bs[kk][c] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a[u] = As[kk][tr * 4 + u];
-        b[u] = Bs[kk][tc * 4 + u];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int m = m0 + tr * 4 + u;
-    if (m >= M) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int n = n0 + tc * 4 + v;
-      if (n >= N) continue;
-      const float c = acc[u][v] + (bias ? bias[n] : 0.f);
-      const size_t o = (size_t)m * ldc + n;
-      if (EPI == 0) {
-        out[o] = c;
-      } else {
-        Z[o] = c;
-        const float r = fmaxf(c, 0.f);
-        out[o] = EPI == 2 ? res[o] + r : r;
-      }
-    }
-  }
-}
-
 // h0 = relu(X W_in + b_in) (Z: the sum before relu, kept for training): CTA of
 // EMB_ROWS rows, W_in as FP32 in shared memory, a thread 4 channels of a row at
 // a time (stores are whole rows).  Bound by the 4 H bytes written per row.
@@ -299,143 +231,6 @@ __global__ void __launch_bounds__(128) k_head(int n, int H, const float* __restr
   }
   reinterpret_cast<float4*>(Y)[i] =
       make_float4(a.x + bias[0], a.y + bias[1], a.z + bias[2], a.w + bias[3]);
-}
-
-// Partial products for C[K x N] = A^T D over a chunk of rows: A [M x K],
-// D [M x N] FP32 row-major; each CTA (ky, nx, chunk) writes its 64 x 64 block
-// of the chunk's contribution; k_reduce_chunks sums the chunks (fixed order).
-constexpr int ATB_CHUNK = 2048;
-__global__ void __launch_bounds__(256) k_gemm_atb(int M, int K, int N, const float* __restrict__ A,
-                                                  int lda, const float* __restrict__ D, int ldd,
-                                                  float* __restrict__ part) {
-  __shared__ float As[16][64 + 1];
-  __shared__ float Ds[16][64];
-  const int tid = threadIdx.x;
-  const int k0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int mc = blockIdx.z * ATB_CHUNK;
-  const int m_end = min(M, mc + ATB_CHUNK);
-  const int tr = tid / 16, tc = tid % 16;
-  float acc[4][4] = {};
-  for (int mm = mc; mm < m_end; mm += 16) {
-    for (int q = tid; q < 16 * 64; q += 256) {
-      const int r = q / 64, c = q % 64;
-      const int m = mm + r;
-      As[r][c] = (m < m_end && k0 + c < K) ? A[(size_t)m * lda + k0 + c] : 0.f;
-      Ds[r][c] = (m < m_end && n0 + c < N) ? D[(size_t)m * ldd + n0 + c] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      float a[4], d[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a[u] = As[r][tr * 4 + u];
-        d[u] = Ds[r][tc * 4 + u];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], d[v], acc[u][v]);
-    }
-    __syncthreads();
-  }
-  float* P = part + (size_t)blockIdx.z * K * N;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int k = k0 + tr * 4 + u;
-    if (k >= K) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int n = n0 + tc * 4 + v;
-      if (n < N) P[(size_t)k * N + n] = acc[u][v];
-    }
-  }
-}
-
-__global__ void k_reduce_chunks(int n_chunks, size_t len, const float* __restrict__ part,
-                                float* __restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
-  float s = 0.f;
-  for (int c = 0; c < n_chunks; ++c) s += part[(size_t)c * len + i];
-  out[i] = s;
-}
-
-// Column sums of D [M x N] (bias gradients), in chunks then a fixed-order sum.
-__global__ void k_colsum_part(int M, int N, const float* __restrict__ D,
-                              float* __restrict__ part) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const int mc = blockIdx.y * ATB_CHUNK, me = min(M, mc + ATB_CHUNK);
-  float s = 0.f;
-  for (int m = mc; m < me; ++m) s += D[(size_t)m * N + n];
-  part[(size_t)blockIdx.y * N + n] = s;
-}
-
-// ---- message passing ---------------------------------------------------------------
-
-// cat_i = [h_i | h_{i-1} + h_{i+1} | sum_n g_n h_{nb_n, k}], four channels
-// per thread (H % 4 == 0; 128-bit loads and stores).
-__global__ void k_agg_fwd(int n, int n_per, int H, const float* __restrict__ h,
-                          const int* __restrict__ nbr, const float* __restrict__ g,
-                          float* __restrict__ cat) {
-  const int H4 = H >> 2;
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)n * H4) return;
-  const int i = (int)(q / H4), c4 = (int)(q % H4);
-  const int s = i / n_per, k = i % n_per;
-  const float4* h4 = reinterpret_cast<const float4*>(h);
-  const float4 hi = h4[q];
-  float4 az = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (k > 0) {
-    const float4 v = h4[q - H4];
-    az = make_float4(az.x + v.x, az.y + v.y, az.z + v.z, az.w + v.w);
-  }
-  if (k + 1 < n_per) {
-    const float4 v = h4[q + H4];
-    az = make_float4(az.x + v.x, az.y + v.y, az.z + v.z, az.w + v.w);
-  }
-  float4 an = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int m = 0; m < NB_K; ++m) {
-    const float gm = g[s * NB_K + m];
-    const float4 v = h4[((size_t)nbr[s * NB_K + m] * n_per + k) * H4 + c4];
-    an = make_float4(fmaf(gm, v.x, an.x), fmaf(gm, v.y, an.y), fmaf(gm, v.z, an.z),
-                     fmaf(gm, v.w, an.w));
-  }
-  float4* o = reinterpret_cast<float4*>(cat + (size_t)i * 3 * H);
-  o[c4] = hi;
-  o[H4 + c4] = az;
-  o[2 * H4 + c4] = an;
-}
-
-// dh += adjoint of the aggregation applied to dcat (the neighbour part
-// scattered with atomics: several skewers may share a neighbour).
-__global__ void k_agg_bwd(int n, int n_per, int H, const float* __restrict__ dcat,
-                          const int* __restrict__ nbr, const float* __restrict__ g,
-                          float* __restrict__ dh) {
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)n * H) return;
-  const int i = (int)(q / H), c = (int)(q % H);
-  const int s = i / n_per, k = i % n_per;
-  const float* d = dcat + (size_t)i * 3 * H;
-  float v = d[c];
-  if (k > 0) v += dcat[(size_t)(i - 1) * 3 * H + H + c];
-  if (k + 1 < n_per) v += dcat[(size_t)(i + 1) * 3 * H + H + c];
-  atomicAdd(&dh[q], v);
-  const float dn = d[2 * H + c];
-#pragma unroll
-  for (int m = 0; m < NB_K; ++m) {
-    const float gm = g[s * NB_K + m];
-    if (gm != 0.f) atomicAdd(&dh[((size_t)nbr[s * NB_K + m] * n_per + k) * H + c], gm * dn);
-  }
-}
-
-// dZ = dh * (Z > 0).
-__global__ void k_relu_bwd(size_t len, const float* __restrict__ dh, const float* __restrict__ Z,
-                           float* __restrict__ dZ) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < len) dZ[i] = Z[i] > 0.f ? dh[i] : 0.f;
 }
 
 // ---- head, outputs and losses -------------------------------------------------------
@@ -704,56 +499,26 @@ void LearnedNet::ensure(int n_sk, int n_per) {
   gw.alloc((size_t)n_sk * NB_K);
   skxy.alloc(n_sk);
   X.alloc(n * F_IN);
-  for (int l = 0; l <= N_LAYERS; ++l) {
-    h[l].alloc(n * H);
-    Z[l].alloc(n * H);
-  }
-  for (int l = 0; l < N_LAYERS; ++l) cat[l].alloc(n * 3 * H);
+  for (int l = 0; l <= N_LAYERS; ++l) h[l].alloc(n * H);
   Y.alloc(n * NO);
-  dY.alloc(n * NO);
-  dh.alloc(n * H);
-  dh2.alloc(n * H);
-  dZ.alloc(n * H);
-  dcat.alloc(n * 3 * H);
-  const size_t chunks = (n + ATB_CHUNK - 1) / ATB_CHUNK;
-  part.alloc(chunks * std::max<size_t>(3 * (size_t)H * H, (size_t)H * NO));
   dpart.alloc(std::max<size_t>(2 * grid1(n), (size_t)n_sk) + 2);
 }
 
-void LearnedNet::gemm_fwd(int M, int N, int K, const float* A, int lda, const Slot& W, const Slot& b,
-                          float* Zp, float* out, const float* res, int epi) {
-  const dim3 grid((N + 63) / 64, (M + 63) / 64);
-  const __nv_bfloat16* Wp = reinterpret_cast<const __nv_bfloat16*>(wbf.p) + W.off;
-  const float* bp = params.p + b.off;
-  cudaStream_t st = ctx->stream;
-  if (epi == 0)
-    k_gemm<false, 0><<<grid, 256, 0, st>>>(M, N, K, A, lda, Wp, N, bp, Zp, out, res, N);
-  else if (epi == 1)
-    k_gemm<false, 1><<<grid, 256, 0, st>>>(M, N, K, A, lda, Wp, N, bp, Zp, out, res, N);
-  else
-    k_gemm<false, 2><<<grid, 256, 0, st>>>(M, N, K, A, lda, Wp, N, bp, Zp, out, res, N);
-  DS_CHECK_LAUNCH();
+void LearnedNet::ensure_train() {
+  for (auto& z : Z) z.alloc(n_cur * H);
+  for (auto& a : agg) a.alloc(n_cur * 2 * H);
+  dY.alloc(n_cur * NO);
+  dh.alloc(n_cur * H);
+  dZ.alloc(n_cur * H);
+  dZ2.alloc(n_cur * H);
+  aggT.alloc(n_cur * 2 * H);
+  part.alloc(std::max(layer_grad_parts((int)n_cur, H, ctx->num_sms),
+                      small_grad_parts(H, ctx->num_sms)));
 }
 
-// dW (slot) = A^T D over M rows; db = column sums of D.
-void LearnedNet::grad_w(int M, int K, int N, const float* A, int lda, const float* D,
-                        const Slot& W, const Slot& b) {
-  cudaStream_t st = ctx->stream;
-  const int chunks = (M + ATB_CHUNK - 1) / ATB_CHUNK;
-  const dim3 grid((N + 63) / 64, (K + 63) / 64, chunks);
-  k_gemm_atb<<<grid, 256, 0, st>>>(M, K, N, A, lda, D, N, part.p);
-  DS_CHECK_LAUNCH();
-  k_reduce_chunks<<<grid1((size_t)K * N), 256, 0, st>>>(chunks, (size_t)K * N, part.p,
-                                                        grads.p + W.off);
-  DS_CHECK_LAUNCH();
-  k_colsum_part<<<dim3(grid1(N, 128), chunks), 128, 0, st>>>(M, N, D, part.p);
-  DS_CHECK_LAUNCH();
-  k_reduce_chunks<<<grid1(N), 256, 0, st>>>(chunks, (size_t)N, part.p, grads.p + b.off);
-  DS_CHECK_LAUNCH();
-}
-
-void LearnedNet::forward(int n_sk, int n_per, const double* rec) {
+void LearnedNet::forward(int n_sk, int n_per, const double* rec, bool train) {
   ensure(n_sk, n_per);
+  if (train) ensure_train();
   rec_cur = rec;
   cudaStream_t st = ctx->stream;
   const int n = n_sk * n_per;
@@ -766,7 +531,7 @@ void LearnedNet::forward(int n_sk, int n_per, const double* rec) {
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(wbf.p);
   k_embed<<<(n + EMB_ROWS - 1) / EMB_ROWS, 256, 0, st>>>(n, H, X.p, wb + W_in.off,
                                                          params.p + b_in.off,
-                                                         tc_active ? nullptr : Z[0].p, h[0].p);
+                                                         train ? Z[0].p : nullptr, h[0].p);
   DS_CHECK_LAUNCH();
   for (int l = 0; l < N_LAYERS; ++l) {
     if (tc_active && layer_tc_usable(n, H, 3 * H)) {
@@ -780,10 +545,11 @@ void LearnedNet::forward(int n_sk, int n_per, const double* rec) {
       launch_layer_tc(n, n_per, h[l].p, nbr.p, gw.p, wb + W_l[l].off, params.p + b_l[l].off,
                       h[l + 1].p, wt.p, tc_err.p, st);
     } else {
-      k_agg_fwd<<<grid1((size_t)n * (H / 4)), 256, 0, st>>>(n, n_per, H, h[l].p, nbr.p, gw.p,
-                                                            cat[l].p);
-      DS_CHECK_LAUNCH();
-      gemm_fwd(n, H, 3 * H, cat[l].p, 3 * H, W_l[l], b_l[l], Z[l + 1].p, h[l + 1].p, h[l].p, 2);
+      DevBuf<float>& A = agg[train ? l : 0];
+      A.alloc((size_t)n * 2 * H);
+      wf.alloc((size_t)3 * H * H);
+      layer_forward(n, n_per, H, h[l].p, nbr.p, gw.p, wb + W_l[l].off, params.p + b_l[l].off, A.p,
+                    wf.p, train ? Z[l + 1].p : nullptr, h[l + 1].p, st);
     }
   }
   k_head<<<grid1(n, 128), 128, 0, st>>>(n, H, h[N_LAYERS].p, wb + W_o.off, params.p + b_o.off,
@@ -801,7 +567,7 @@ void LearnedNet::loss_and_grad(int n_sk, int n_per, const double* rec, const dou
                                const float* probe, float wx, float wp, double* losses) {
   cudaStream_t st = ctx->stream;
   const int n = n_sk * n_per;
-  forward(n_sk, n_per, rec);
+  forward(n_sk, n_per, rec, true);
   DS_CUDA(cudaMemsetAsync(dY.p, 0, (size_t)n * NO * sizeof(float), st));
   // warm-start loss
   const unsigned gb = grid1(n);
@@ -839,37 +605,21 @@ void LearnedNet::loss_and_grad(int n_sk, int n_per, const double* rec, const dou
 
 void LearnedNet::backward(int n_sk, int n_per) {
   cudaStream_t st = ctx->stream;
-  const int n = n_sk * n_per;
+  const int n = n_sk * n_per, sms = ctx->num_sms;
+  const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(wbf.p);
+  build_rev_lists(n_sk, nbr.p, gw.p, rev, st);
+  wf.alloc((size_t)3 * H * H);
   // head: dW_o = h4^T dY, dh4 = dY W_o^T
-  grad_w(n, H, NO, h[N_LAYERS].p, H, dY.p, W_o, b_o);
-  {
-    const dim3 grid((H + 63) / 64, (n + 63) / 64);
-    const __nv_bfloat16* Wp = reinterpret_cast<const __nv_bfloat16*>(wbf.p) + W_o.off;
-    k_gemm<true, 0><<<grid, 256, 0, st>>>(n, H, NO, dY.p, NO, Wp, NO, nullptr, nullptr, dh.p,
-                                          nullptr, H);
-    DS_CHECK_LAUNCH();
-  }
+  head_grad(n, H, sms, h[N_LAYERS].p, dY.p, part.p, grads.p + W_o.off, grads.p + b_o.off, st);
+  head_backward(n, H, dY.p, wb + W_o.off, Z[N_LAYERS].p, dh.p, dZ.p, st);
   for (int l = N_LAYERS - 1; l >= 0; --l) {
-    // h_{l+1} = h_l + relu(Z_{l+1}), Z_{l+1} = cat_l W_l + b_l
-    k_relu_bwd<<<grid1((size_t)n * H), 256, 0, st>>>((size_t)n * H, dh.p, Z[l + 1].p, dZ.p);
-    DS_CHECK_LAUNCH();
-    grad_w(n, 3 * H, H, cat[l].p, 3 * H, dZ.p, W_l[l], b_l[l]);
-    const dim3 grid((3 * H + 63) / 64, (n + 63) / 64);
-    const __nv_bfloat16* Wp = reinterpret_cast<const __nv_bfloat16*>(wbf.p) + W_l[l].off;
-    k_gemm<true, 0><<<grid, 256, 0, st>>>(n, 3 * H, H, dZ.p, H, Wp, H, nullptr, nullptr, dcat.p,
-                                          nullptr, 3 * H);
-    DS_CHECK_LAUNCH();
-    // dh_l = dh_{l+1} (residual) + aggregation adjoint of dcat
-    DS_CUDA(cudaMemcpyAsync(dh2.p, dh.p, (size_t)n * H * sizeof(float), cudaMemcpyDeviceToDevice,
-                            st));
-    k_agg_bwd<<<grid1((size_t)n * H), 256, 0, st>>>(n, n_per, H, dcat.p, nbr.p, gw.p, dh2.p);
-    DS_CHECK_LAUNCH();
-    std::swap(dh, dh2);
+    layer_backward(n, n_per, H, sms, h[l].p, agg[l].p, rev, wb + W_l[l].off, Z[l].p, dZ.p, dZ2.p,
+                   dh.p, l == 0, aggT.p, wf.p, part.p, grads.p + W_l[l].off,
+                   grads.p + b_l[l].off, st);
+    std::swap(dZ, dZ2);
   }
   // embed: h0 = relu(Z0)
-  k_relu_bwd<<<grid1((size_t)n * H), 256, 0, st>>>((size_t)n * H, dh.p, Z[0].p, dZ.p);
-  DS_CHECK_LAUNCH();
-  grad_w(n, F_IN, H, X.p, F_IN, dZ.p, W_in, b_in);
+  embed_grad(n, H, sms, X.p, dZ.p, part.p, grads.p + W_in.off, grads.p + b_in.off, st);
 }
 
 void LearnedNet::adam_step(float lr) {
@@ -1034,7 +784,7 @@ int ds_learned_forward_dev(ds_learned* h, int n_skewers, int n_per, const double
   return guarded(net.ctx, [&] {
     net.tc_active = net.tc_infer;
     try {
-      net.forward(n_skewers, n_per, records);
+      net.forward(n_skewers, n_per, records, false);
     } catch (...) {
       net.tc_active = false;
       throw;
