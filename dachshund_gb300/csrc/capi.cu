@@ -238,7 +238,7 @@ void map_product_dev(ds_map* map, ds_operator* op, const double* x_dev, double* 
   a.table = op->table.p;
   a.n_tile_pairs = map->pairs.n_pairs;
   a.prof = &map->ctx->prof;
-  launch_pair_f64(op->kc, EPI_MAP, a, st);
+  launch_pair_f64(op->kc, EPI_MAP, a, st, &map->pts, &op->pix);
 }
 
 }  // namespace
@@ -723,7 +723,7 @@ int ds_smp_product(ds_context* ctx, int n_pix, const double* pixel_points, int n
     a.table = table.p;
     a.n_tile_pairs = pl.n_pairs;
     a.prof = &ctx->prof;
-    launch_pair_f64(kc, EPI_MAP, a, st);
+    launch_pair_f64(kc, EPI_MAP, a, st, &mp, &pix);
     DS_CUDA(cudaMemcpyAsync(m, dm.p, n_map * sizeof(double), cudaMemcpyDeviceToHost, st));
     DS_CUDA(cudaStreamSynchronize(st));
   });
@@ -770,7 +770,7 @@ int ds_sigma_m_noise_dom(ds_context* ctx, int n_pix, const double* npixels, int 
     a.table = table.p;
     a.n_tile_pairs = pl.n_pairs;
     a.prof = &ctx->prof;
-    launch_pair_f64(kc, EPI_NOISE, a, st);
+    launch_pair_f64(kc, EPI_NOISE, a, st, &mp, &pix);
     DS_CUDA(cudaMemcpyAsync(sigma_m, dm.p, n_map * sizeof(double), cudaMemcpyDeviceToHost, st));
     DS_CUDA(cudaStreamSynchronize(st));
   });

@@ -176,6 +176,7 @@ struct PointSet {
   int n = 0;
   int n_pad = 0;
   int n_tiles = 0;
+  double lo[3], hi[3];     // bounding box
   DevBuf<double> x, y, z;  // sorted + padded
   DevBuf<int> perm;        // sorted position -> caller index (-1 on padding)
   DevBuf<double> box;      // 6 per tile: lo x, y, z, hi x, y, z
@@ -285,11 +286,20 @@ struct Profiler {
   ~Profiler();
 };
 
-void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a,
-                     cudaStream_t st);
+// With rows and cols (the point sets), the exact kernel's map and noise sums run
+// in fixed point where that applies.
+void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a, cudaStream_t st,
+                     const PointSet* rows = nullptr, const PointSet* cols = nullptr);
 // u_j = scale (w_j v_j), or scale v_j without w (n_pad entries).
 void form_u(int n_pad, double scale, const double* w, const double* v, double* u,
             const int* skip, cudaStream_t st);
+
+// A point set's scaled coordinates in fixed point (pair_fx.cu): units of 2^-60
+// modulo 2^64, three runs of n_pad, and coarse 32-bit ones for the pair search.
+struct FxPoints {
+  DevBuf<unsigned long long> fx;
+  DevBuf<int4> c;
+};
 
 // The FP64 operator's interacting pairs as stored values (pair_vals.cu):
 // slices of 32 rows, entry e of lane l of slice s at (start[s] + e) * 32 + l.

@@ -67,6 +67,12 @@ bool ensure_pair_vals(ds_operator* op);
 // out = A v or b - A v from them (a as for launch_pair_f64, a.u formed).
 void launch_pair_vals(ds_operator* op, int epi, const PairArgs& a, cudaStream_t st);
 
+// Pair values in fixed point (pair_fx.cu).
+bool fx_usable(const KernelConsts& kc, const PointSet& rows, const PointSet& cols);
+void launch_pair_fx(const KernelConsts& kc, int epi, const PairArgs& a, const PointSet& rows,
+                    const PointSet& cols, cudaStream_t st);
+void fill_vals_fx(ds_operator* op, const dim3& grid, cudaStream_t st);
+
 // The map's tiled point set, built on the first call that needs it (the
 // structured column-grid map reads the points as given).
 void ensure_map_points(ds_map* map);

@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "ds_device.cuh"
+#include "ds_ops.h"
 #include "ds_pairhit.cuh"
 
 namespace ds {
@@ -158,7 +159,8 @@ void form_u(int n_pad, double scale, const double* w, const double* v, double* u
   DS_CHECK_LAUNCH();
 }
 
-void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a0, cudaStream_t st) {
+void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a0, cudaStream_t st,
+                     const PointSet* rows, const PointSet* cols) {
   if (a0.n_row_tiles <= 0) return;
   PairArgs a = a0;
   const bool op = epi == EPI_PRODUCT || epi == EPI_RESIDUAL;
@@ -172,7 +174,9 @@ void launch_pair_f64(const KernelConsts& kc, int epi, const PairArgs& a0, cudaSt
   } else {
     a.prof_pairs = nullptr;
   }
-  if (kc.eval == DS_EVAL_TABLE)
+  if (rows && fx_usable(kc, *rows, *cols))
+    launch_pair_fx(kc, epi, a, *rows, *cols, st);
+  else if (kc.eval == DS_EVAL_TABLE)
     launch_eval<DS_EVAL_TABLE>(kc, epi, a, st);
   else
     launch_eval<DS_EVAL_EXACT>(kc, epi, a, st);

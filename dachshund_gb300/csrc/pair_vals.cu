@@ -200,6 +200,10 @@ void fill(ds_operator* op, PairVals& pv, const PairArgs& a, DevBuf<I>& cols, cud
   // enough CTAs for 16 per SM (152) when there are few slices
   const int ns = op->pix.n_pad / 32;
   const dim3 grid(ns, std::max(1, std::min(32, (2432 + ns - 1) / ns)));
+  if (fx_usable(op->kc, op->pix, op->pix)) {
+    fill_vals_fx(op, grid, st);
+    return;
+  }
   if (op->kc.eval == DS_EVAL_TABLE)
     k_vals_eval<DS_EVAL_TABLE, I>
         <<<grid, TILE, 0, st>>>(op->kc, a, pv.cnt.p, pv.start.p, cols.p, pv.val.p);

@@ -607,6 +607,10 @@ void build_point_set(PointSet& ps, const double* d_rec, int n, int stride, doubl
   // Bounding box of all points.
   double lo[3], hi[3];
   point_bbox(d_rec, n, stride, lo, hi, st);
+  for (int c = 0; c < 3; ++c) {
+    ps.lo[c] = lo[c];
+    ps.hi[c] = hi[c];
+  }
   const double ext = std::max({(hi[0] - lo[0]) * sx, (hi[1] - lo[1]) * sy,
                                (hi[2] - lo[2]) * sz, 1e-300});
   const double inv_h = 1023.0 / ext;

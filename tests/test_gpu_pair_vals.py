@@ -87,6 +87,32 @@ def test_map_vs_oracle(ctx, exact, n, m, spread):
     op.close()
 
 
+@pytest.mark.parametrize("cutoff,spread", [(5.0, 1), (48.0, 1), (47.99, 1), (48.01, 1),
+                                           (40.0, 3e3), (40.0, 3e4)])
+def test_fixed_point_and_fp64_ranges(ctx, cutoff, spread):
+    """The exact kernel on both sides of the fixed-point range (cutoff 48, extent
+    2^16 scaled units; spread 3e3 is 2^15.1 of them, 3e4 beyond), products and map:
+    the oracle has no cutoff, the terms beyond it are at most exp(-cutoff)."""
+    n, m = 3001, 777
+    rec = records("w", n, n, spread)
+    rec[:3000:3, :3] = rec[1:3000:3, :3] + 0.5  # close pairs in the sparse sets
+    pts = rec[:m, :3] + 1.25
+    a = np.random.default_rng(1).standard_normal(n)
+    op = WFVectorW(ctx, rec, SignalCovarParams(VS, LP, LQ, eval="exact", exact_cutoff=cutoff))
+    lim = oracle.A_product("w", rec, np.abs(a), VS, LP, LQ, exact=True)
+    w = rec[:, 3]
+    lim = (n + 128) * 2.0 ** -53 * lim + np.exp(-cutoff) * VS * w * np.sum(w * np.abs(a))
+    assert np.all(np.abs(op.A_product(a) - oracle.A_product("w", rec, a, VS, LP, LQ, exact=True))
+                  <= lim)
+    grid = MapGrid(ctx, pts)
+    ref = oracle.smp_product(rec[:, :3], pts, a, VS, LP, LQ, exact=True)
+    lim = oracle.smp_product(rec[:, :3], pts, np.abs(a), VS, LP, LQ, exact=True)
+    lim = (n + 128) * 2.0 ** -53 * lim + np.exp(-cutoff) * VS * np.sum(np.abs(a))
+    assert np.all(np.abs(grid.product(op, a) - ref) <= lim)
+    grid.close()
+    op.close()
+
+
 def test_residual_evaluated_on_every_call(ctx):
     """A cutoff beyond the float-float range: the mixed form's outer residual is
     the evaluating FP64 kernel's; its solution is the FP64 solve's to tol."""
