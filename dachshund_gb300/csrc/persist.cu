@@ -121,12 +121,11 @@ enum { B_LEVELS = 1, B_PRODUCT, B_STEP, B_LEVELS64, B_UPDATE, B_CALIB };
 constexpr int N_CALIB = 1;
 
 // Phase timers (%globaltimer, ns), accumulated over launches until read:
-// CTA 0 records, per barrier code, the time from the previous barrier's exit
-// to this one's exit and the number of visits; every CTA records, per code,
+// CTA 0 records, per barrier code (0 unused), the time from the previous
+// barrier's exit to this one's exit and the number of visits; every CTA records, per code,
 // its own work (from its previous exit to its arrival), so the slowest CTA
 // and the barrier's wait are told apart.
 enum {
-  PT_LAST = 0,       // CTA 0's last exit
   PT_PHASE = 0,      // + code: exit-to-exit totals (codes 1..6)
   PT_VISITS = 8,     // + code
   PT_START = 16,     // kernel start (CTA 0)
@@ -159,16 +158,48 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // may work on its own data (writing nothing another CTA reads in the next
 // phase), which hides that work behind the barrier's latency.
 constexpr int BAR_WORDS = 32;  // one 128-byte line
-struct BarState {                  // thread 0's barrier state
+// Thread 0's barrier state.  The phase timers accumulate in shared memory and
+// go to global memory once, at the kernel's end: a read-modify-write of global
+// memory in front of the arrival's release held up every barrier.
+struct BarState {
   unsigned int epoch = 0;          // barriers passed
   unsigned long long exit_ns = 0;  // last exit (%globaltimer)
   int last = 0;                    // this CTA completed the current epoch
 };
+struct PhaseTimers {
+  unsigned long long phase[8], visits[8], work[8];
+};
+__shared__ PhaseTimers s_timers;
+
+__device__ void timers_start(const PersistArgs& a, BarState& b) {
+  if (threadIdx.x < 8)
+    s_timers.phase[threadIdx.x] = s_timers.visits[threadIdx.x] = s_timers.work[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    b.exit_ns = global_ns();
+    if (blockIdx.x == 0) {
+      a.pt[PT_START] = b.exit_ns;
+      a.pt[PT_GRID] = gridDim.x;
+      a.pt[PT_LAUNCHES] += 1;
+    }
+  }
+}
+
+__device__ void timers_end(const PersistArgs& a) {
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    a.pt[PT_CTA + 8 * blockIdx.x + threadIdx.x] += s_timers.work[threadIdx.x];
+    if (blockIdx.x == 0) {
+      a.pt[PT_PHASE + threadIdx.x] += s_timers.phase[threadIdx.x];
+      a.pt[PT_VISITS + threadIdx.x] += s_timers.visits[threadIdx.x];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.pt[PT_KERNEL] += global_ns() - a.pt[PT_START];
+}
 
 __device__ void grid_arrive(const PersistArgs& a, int code, BarState& b) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (b.epoch > 0) a.pt[PT_CTA + 8 * blockIdx.x + code] += global_ns() - b.exit_ns;
+    if (b.epoch > 0) s_timers.work[code] += global_ns() - b.exit_ns;
     ++b.epoch;
     const unsigned int target = b.epoch * gridDim.x;
     unsigned int old;
@@ -207,12 +238,9 @@ __device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
       ok = 0;
     }
     const unsigned long long now = global_ns();
+    s_timers.phase[code] += now - b.exit_ns;  // reported for CTA 0
+    s_timers.visits[code] += 1;
     b.exit_ns = now;
-    if (blockIdx.x == 0) {
-      a.pt[PT_PHASE + code] += now - a.pt[PT_LAST];
-      a.pt[PT_LAST] = now;
-      a.pt[PT_VISITS + code] += 1;
-    }
     ok_s = ok;
   }
   __syncthreads();
@@ -224,15 +252,38 @@ __device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code, BarSta
   return grid_wait(a, code, b);
 }
 
-// Sum of n partials in a fixed order, valid in every thread of every CTA
-// alike: warp 0 alone sums them in FP64 (lane l takes l, l + 32, ..., then a
-// shuffle tree), so the FP64 pipe (2 operations per clock per SM on GB300)
-// sees n + 5 additions per CTA instead of a CTA-wide tree.
+// Sum of n partials in a fixed order by one warp (valid in lane 0), the same in
+// every CTA: lane l takes l, l + 32, ..., then a shuffle tree, so the FP64 pipe
+// (2 operations per clock per SM on GB300) sees n + 5 additions per CTA instead
+// of a CTA-wide tree.
+__device__ __forceinline__ double warp_total(const double* part, int n) {
+  double v = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += 32) v += __ldcg(part + i);
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The same for n pairs of partials (both sums from one pass over them).
+__device__ __forceinline__ double2 warp_total2(const double* part, int n) {
+  double v0 = 0.0, v1 = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += 32) {
+    const double2 pr = __ldcg(reinterpret_cast<const double2*>(part) + i);
+    v0 += pr.x;
+    v1 += pr.y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    v0 += __shfl_down_sync(0xffffffffu, v0, o);
+    v1 += __shfl_down_sync(0xffffffffu, v1, o);
+  }
+  return make_double2(v0, v1);
+}
+
+// The totals in every thread of the CTA (the general form).
 __device__ __forceinline__ double partial_total(const double* part, int n, double* out) {
   if (threadIdx.x < 32) {
-    double v = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) v += __ldcg(part + i);
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    const double v = warp_total(part, n);
     if (threadIdx.x == 0) *out = v;
   }
   __syncthreads();
@@ -241,22 +292,12 @@ __device__ __forceinline__ double partial_total(const double* part, int n, doubl
   return t;
 }
 
-// The same for n pairs of partials (both sums from one pass over them).
 __device__ __forceinline__ double2 partial_total2(const double* part, int n, double* out) {
   if (threadIdx.x < 32) {
-    double v0 = 0.0, v1 = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) {
-      const double2 pr = __ldcg(reinterpret_cast<const double2*>(part) + i);
-      v0 += pr.x;
-      v1 += pr.y;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      v0 += __shfl_down_sync(0xffffffffu, v0, o);
-      v1 += __shfl_down_sync(0xffffffffu, v1, o);
-    }
+    const double2 v = warp_total2(part, n);
     if (threadIdx.x == 0) {
-      out[0] = v0;
-      out[1] = v1;
+      out[0] = v.x;
+      out[1] = v.y;
     }
   }
   __syncthreads();
@@ -265,25 +306,35 @@ __device__ __forceinline__ double2 partial_total2(const double* part, int n, dou
   return t;
 }
 
-// Sum over the CTA of one float pair per thread (fixed order: a float-pair
-// shuffle tree within each warp, then the warps' sums in FP64 by thread 0,
-// where the result is valid).  The FP32 Krylov vectors' dot products are
-// summed this way: exact products (FMA) and compensated sums keep about 44
-// bits, and the FP64 pipe sees NT/32 additions per CTA.
-__device__ __forceinline__ double block_sum_ff(ff v, double* sm /* NT/32 */) {
+// Sums over the CTA of two float pairs per thread (fixed order: a float-pair
+// shuffle tree within each warp, then the warps' sums in FP64), valid in lanes 0
+// and 16 of warp 0.  The FP32 Krylov vectors' dot products are summed this way:
+// exact products (FMA) and compensated sums keep about 44 bits.  The warps' sums
+// are added by a shuffle tree in each half of warp 0: one thread's chain of NT /
+// 32 FP64 additions was the longest part of a short phase.
+__device__ __forceinline__ double block_sum2_ff(ff v, ff w, double* sm /* 2 NT/32 */) {
+  static_assert(NT / 32 == 16, "two sums share a warp");
+  constexpr unsigned full = 0xffffffffu;
   for (int o = 16; o > 0; o >>= 1) {
-    ff w;
-    w.h = __shfl_down_sync(0xffffffffu, v.h, o);
-    w.l = __shfl_down_sync(0xffffffffu, v.l, o);
-    v = ff_add(v, w);
+    ff a, b;
+    a.h = __shfl_down_sync(full, v.h, o);
+    a.l = __shfl_down_sync(full, v.l, o);
+    b.h = __shfl_down_sync(full, w.h, o);
+    b.l = __shfl_down_sync(full, w.l, o);
+    v = ff_add(v, a);
+    w = ff_add(w, b);
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sm[wid] = (double)v.h + (double)v.l;
+  if (lane == 0) {
+    sm[wid] = (double)v.h + (double)v.l;
+    sm[16 + wid] = (double)w.h + (double)w.l;
+  }
   __syncthreads();
   double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < NT / 32; ++w) s += sm[w];
+  if (wid == 0) {
+    s = sm[lane];
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_down_sync(full, s, o, 16);
+  }
   return s;
 }
 
@@ -507,13 +558,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
   const size_t ns = (size_t)a.n_blocks * a.S;
   BarState bst;  // barrier state (thread 0)
   if (tid == 0) sS = *a.S_;
-  if (tid == 0 && blockIdx.x == 0) {
-    const unsigned long long now = global_ns();
-    a.pt[PT_LAST] = now;
-    a.pt[PT_START] = now;
-    a.pt[PT_GRID] = gridDim.x;
-    a.pt[PT_LAUNCHES] += 1;
-  }
+  timers_start(a, bst);
   __syncthreads();
   for (int k = 0; k < N_CALIB; ++k) grid_sync(a, B_CALIB, bst);
   // the recurrence sets done by iteration max_iter at the latest (the
@@ -673,8 +718,8 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
       __syncthreads();
     }
   }
+  timers_end(a);
   if (blockIdx.x == 0 && tid == 0) {
-    a.pt[PT_KERNEL] += global_ns() - a.pt[PT_START];
     sS.skip_update = 1;
     *a.S_ = sS;
   }
@@ -840,8 +885,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   int* sk = reinterpret_cast<int*>(smraw + ResLayout::sk);
   __half* Lh = reinterpret_cast<__half*>(smraw + ResLayout::lh);
   __shared__ MixedState sS;
-  __shared__ double red[NT / 32];
-  __shared__ double tot[2];
+  __shared__ double red[2 * (NT / 32)];
   __shared__ ff s_alpha;  // alpha as a float pair (x update)
   __shared__ float s_ab;  // alpha or beta in FP32
   __shared__ size_t s_off[MAX_G * NB_R];  // staged FP64 lists (the update's residual)
@@ -857,13 +901,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   const size_t ns = (size_t)a.n_blocks * a.S;
   BarState bst;  // barrier state (thread 0)
   if (tid == 0) sS = *a.S_;
-  if (tid == 0 && blockIdx.x == 0) {
-    const unsigned long long now = global_ns();
-    a.pt[PT_LAST] = now;
-    a.pt[PT_START] = now;
-    a.pt[PT_GRID] = gridDim.x;
-    a.pt[PT_LAUNCHES] += 1;
-  }
+  timers_start(a, bst);
   if (tid < MAX_G) sk[tid] = tid < a.g ? skewer_of(a, blk, tid) : -1;
   {  // the block's product items
     const size_t i0 = (size_t)blk * NI;
@@ -967,8 +1005,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   // accumulator per skewer (acc).  The rows of the block's own skewers (the
   // first items) are done between the arrival at the barrier that publishes
   // the levels and its wait; the others after it.
-  const int tk = NT / npr;  // threads per pixel
+  // tk = NT / n_per threads per pixel; the last NT % n_per threads have no pixel
+  const int tk = NT / npr;
   const int kq = tid % npr, part = tid / npr;
+  const bool has_pixel = part < tk;
   float acc[GI];
   auto product_rows = [&](int e0, int e1) {
     for (int e = e0; e < e1; e += UFI) {
@@ -990,7 +1030,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
 #pragma unroll
     for (int j = 0; j < GI; ++j) acc[j] = 0.f;
     const int no = s_nit[1];
-    product_rows(part * no / tk, (part + 1) * no / tk);
+    if (has_pixel) product_rows(part * no / tk, (part + 1) * no / tk);
   };
   levels_z();
   grid_arrive(a, B_LEVELS, bst);
@@ -1008,9 +1048,11 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         if (tid == 0) s_ab = (float)sS.beta;
         float* red_w = reinterpret_cast<float*>(us);  // (NT / n_per) x GI x n_per
         const int ni = s_nit[0] - s_nit[1], i0 = s_nit[1];  // the other blocks' rows
-        product_rows(i0 + part * ni / tk, i0 + (part + 1) * ni / tk);
+        if (has_pixel) {
+          product_rows(i0 + part * ni / tk, i0 + (part + 1) * ni / tk);
 #pragma unroll
-        for (int j = 0; j < GI; ++j) red_w[(part * GI + j) * npr + kq] = acc[j];
+          for (int j = 0; j < GI; ++j) red_w[(part * GI + j) * npr + kq] = acc[j];
+        }
         __syncthreads();  // red_w, s_ab
         const float beta = s_ab;
 #pragma unroll
@@ -1029,20 +1071,23 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       {
-        const double bs = block_sum_ff(dq, red);
+        const double bs = block_sum2_ff(dq, ff{0.f, 0.f}, red);
         if (tid == 0) a.part[blk] = bs;
       }
       if (!grid_sync(a, B_PRODUCT, bst)) break;
-      // ---- step: alpha; x, r, z of the block; levels of z; partials
-      const double pq = partial_total(a.part, G, tot);
-      if (tid == 0) {
-        const double al = sS.rz / pq;
-        tot[0] = al;
-        s_alpha = ff_from_double(al);
-        s_ab = (float)al;
+      // ---- step: alpha; x, r, z of the block; levels of z; partials.  Warp 0
+      // alone adds the CTAs' partials and forms the scalars.
+      if (tid < 32) {
+        const double pq = warp_total(a.part, G);
+        if (tid == 0) {
+          const double al = sS.rz / pq;
+          sS.pq = pq;
+          sS.alpha = al;
+          s_alpha = ff_from_double(al);
+          s_ab = (float)al;
+        }
       }
       __syncthreads();
-      const double alpha_d = tot[0];
       const float alpha = s_ab;
       const ff alpha_ff = s_alpha;
       ff rz{0.f, 0.f}, rr{0.f, 0.f};
@@ -1070,24 +1115,19 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           ff_acc_prod(rr, ri, ri);
         }
       }
-
+      levels_z();  // published first: the stores drain while the sums are formed
       {
-        const double b1 = block_sum_ff(rz, red);
-        const double b2 = block_sum_ff(rr, red);
-        if (tid == 0) {
-          a.part[(size_t)P2 + 2 * blk] = b1;
-          a.part[(size_t)P2 + 2 * blk + 1] = b2;
-        }
+        const double bs = block_sum2_ff(rz, rr, red);
+        if (tid == 0 || tid == 16) a.part[(size_t)P2 + 2 * blk + (tid >> 4)] = bs;
       }
-      levels_z();
       grid_arrive(a, B_STEP, bst);
       own_rows();
       if (!grid_wait(a, B_STEP, bst)) break;
-      {
-        const double2 t2 = partial_total2(a.part + P2, G, tot);
-        if (tid == 0) step_scalars(sS, a, it, alpha_d, pq, t2.x, t2.y);
-        __syncthreads();
+      if (tid < 32) {
+        const double2 t2 = warp_total2(a.part + P2, G);
+        if (tid == 0) step_scalars(sS, a, it, sS.alpha, sS.pq, t2.x, t2.y);
       }
+      __syncthreads();
       if (!sS.need_update) continue;
       // ---- FP64-accurate update in float pairs (GB300 issues FP64 at 1/64 of
       // FP32): levels of u = wr x, stored as float pairs in the FP64 levels'
@@ -1161,7 +1201,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       {
-        const double b1 = block_sum_ff(rz_u, red);
+        const double b1 = block_sum2_ff(rz_u, ff{0.f, 0.f}, red);
         const double b2 = block_sum<NT>(rr_u, red);
         if (tid == 0) {
           a.part[(size_t)P2 + 2 * blk] = b1;
@@ -1172,18 +1212,18 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       grid_arrive(a, B_UPDATE, bst);
       own_rows();
       if (!grid_wait(a, B_UPDATE, bst)) break;
-      {
-        const double2 t2 = partial_total2(a.part + P2, G, tot);
+      if (tid < 32) {
+        const double2 t2 = warp_total2(a.part + P2, G);
         if (tid == 0) update_scalars(sS, a, t2.x, t2.y);
-        __syncthreads();
       }
+      __syncthreads();
     }
   // the iterate back to global memory (record order)
 #pragma unroll
   for (int t = 0; t < RPT; ++t)
     if (jj[t] >= 0) a.x[rg[t]] = (double)xs[tid + t * NT].h + (double)xs[tid + t * NT].l;
+  timers_end(a);
   if (blockIdx.x == 0 && tid == 0) {
-    a.pt[PT_KERNEL] += global_ns() - a.pt[PT_START];
     sS.skip_update = 1;
     *a.S_ = sS;
   }
@@ -1376,7 +1416,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   const bool off31 = (double)(g.inner.lmax + 1) * (double)op->n < 2147483647.0;
   if (g.res_pc != pc || g.res_cut != g.inner.cut) {
     g.res_max_list = NI + 1;  // unusable unless built
-    if (off31 && pc->g <= GI && NT % g.n_per == 0 && g.inner.idx.n < (1u << 28)) {
+    if (off31 && pc->g <= GI && g.n_per <= NT && g.inner.idx.n < (1u << 28)) {
       g.it_cnt.alloc(pc->n_sk + 1);  // last: the largest count (or an overflow mark)
       g.it_own.alloc(pc->n_sk);
       g.it_off.alloc((size_t)pc->n_sk * NI);
@@ -1408,7 +1448,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   }
   const int nsm = op->ctx->num_sms;
   // the item form: 32-bit offsets into the levels, <= GI skewers per block,
-  // n_per dividing the CTA, every block's items in shared memory
+  // a thread for every pixel, every block's items in shared memory
   const bool resident = g.res_max_list <= NI && per_sm1[bi] * nsm >= pc->n_sk;
   const int grid = resident ? pc->n_sk : std::min(per_sm0[bi] * nsm, pc->n_sk);
   if (grid <= 0) return false;
