@@ -141,18 +141,17 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // Grid-wide barrier (all CTAs resident: cooperative launch).  Every CTA's
-// thread 0 arrives on one monotonic count (atom.acq_rel: it releases the
-// CTA's writes, ordered before it by the CTA barrier) and polls the same
-// count (ld.acquire) until it reaches epoch x CTAs: reading the last
-// arrival's value synchronises with every arrival (the arrivals form one
-// release sequence), and the CTA whose arrival completes the epoch does not
-// poll at all.  (Measured on GB300 against a broadcast in which that CTA
-// writes the epoch into a flag line per CTA after a fence: 2.90 against
-// 3.07 ms per 262,144-pixel solve; the broadcast adds a fence and a store
-// round trip to every barrier.)  A wait that runs out (`limit` SM cycles,
-// checked before each poll) records `code` in the error word and returns
-// false, as does a CTA that finds the error word set (read every 16 polls,
-// and by the last arrival).
+// thread 0 adds itself to one monotonic count (red.release: it releases the
+// CTA's writes, ordered before it by the CTA barrier; nothing waits for the
+// addition's return) and polls the same count (ld.acquire) until it reaches
+// epoch x CTAs: reading the last arrival's value synchronises with every
+// arrival (the arrivals form one release sequence).  (Measured on GB300 against
+// a broadcast in which the last CTA to arrive writes the epoch into a flag line
+// per CTA after a fence: 2.90 against 3.07 ms per 262,144-pixel solve; the
+// broadcast adds a fence and a store round trip to every barrier.)  A wait that
+// runs out (`limit` SM cycles, checked before each poll) records `code` in the
+// error word and returns false, as does a CTA that finds the error word set
+// (read every 16 polls).
 // Words: [0] count, [1] error code.
 // The barrier comes in two halves: between grid_arrive and grid_wait a CTA
 // may work on its own data (writing nothing another CTA reads in the next
@@ -164,7 +163,6 @@ constexpr int BAR_WORDS = 32;  // one 128-byte line
 struct BarState {
   unsigned int epoch = 0;          // barriers passed
   unsigned long long exit_ns = 0;  // last exit (%globaltimer)
-  int last = 0;                    // this CTA completed the current epoch
 };
 struct PhaseTimers {
   unsigned long long phase[8], visits[8], work[8];
@@ -201,13 +199,7 @@ __device__ void grid_arrive(const PersistArgs& a, int code, BarState& b) {
   if (threadIdx.x == 0) {
     if (b.epoch > 0) s_timers.work[code] += global_ns() - b.exit_ns;
     ++b.epoch;
-    const unsigned int target = b.epoch * gridDim.x;
-    unsigned int old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
-                 : "=r"(old)
-                 : "l"(a.bar)
-                 : "memory");
-    b.last = old + 1 == target;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
   }
 }
 
@@ -215,7 +207,7 @@ __device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
   __shared__ int ok_s;
   if (threadIdx.x == 0) {
     int ok = 1;
-    if (!b.last) {
+    {
       const unsigned int target = b.epoch * gridDim.x;
       const long long t0 = clock64();
       for (int k = 0;; ++k) {
@@ -234,8 +226,6 @@ __device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
           break;
         }
       }
-    } else if (*(volatile int*)a.err) {
-      ok = 0;
     }
     const unsigned long long now = global_ns();
     s_timers.phase[code] += now - b.exit_ns;  // reported for CTA 0
@@ -306,36 +296,140 @@ __device__ __forceinline__ double2 partial_total2(const double* part, int n, dou
   return t;
 }
 
-// Sums over the CTA of two float pairs per thread (fixed order: a float-pair
-// shuffle tree within each warp, then the warps' sums in FP64), valid in lanes 0
-// and 16 of warp 0.  The FP32 Krylov vectors' dot products are summed this way:
-// exact products (FMA) and compensated sums keep about 44 bits.  The warps' sums
-// are added by a shuffle tree in each half of warp 0: one thread's chain of NT /
-// 32 FP64 additions was the longest part of a short phase.
-__device__ __forceinline__ double block_sum2_ff(ff v, ff w, double* sm /* 2 NT/32 */) {
+__device__ __forceinline__ ff ff_shfl_down(ff v, int o, int width = 32) {
+  ff r;
+  r.h = __shfl_down_sync(0xffffffffu, v.h, o, width);
+  r.l = __shfl_down_sync(0xffffffffu, v.l, o, width);
+  return r;
+}
+
+// Sums over the CTA of two float pairs per thread (float-pair shuffle trees, a
+// fixed order), valid in lanes 0 and 16 of warp 0.  The Krylov vectors' dot
+// products are summed this way from the threads to the grid (exact products by
+// FMA, compensated sums, about 44 bits): a chain of dependent FP64 instructions
+// has a latency of a hundred clocks or more each on GB300, and the FP64 sums and
+// scalars of an iteration took 14,000 of its 22,000 clocks at 16 CTAs.
+__device__ __forceinline__ ff block_sum2_ff(ff v, ff w, float2* sm /* 2 NT/32 */) {
   static_assert(NT / 32 == 16, "two sums share a warp");
-  constexpr unsigned full = 0xffffffffu;
   for (int o = 16; o > 0; o >>= 1) {
-    ff a, b;
-    a.h = __shfl_down_sync(full, v.h, o);
-    a.l = __shfl_down_sync(full, v.l, o);
-    b.h = __shfl_down_sync(full, w.h, o);
-    b.l = __shfl_down_sync(full, w.l, o);
+    const ff a = ff_shfl_down(v, o), b = ff_shfl_down(w, o);
     v = ff_add(v, a);
     w = ff_add(w, b);
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) {
-    sm[wid] = (double)v.h + (double)v.l;
-    sm[16 + wid] = (double)w.h + (double)w.l;
+    sm[wid] = make_float2(v.h, v.l);
+    sm[16 + wid] = make_float2(w.h, w.l);
   }
   __syncthreads();
-  double s = 0.0;
+  ff s{0.f, 0.f};
   if (wid == 0) {
-    s = sm[lane];
-    for (int o = 8; o > 0; o >>= 1) s += __shfl_down_sync(full, s, o, 16);
+    const float2 t = sm[lane];
+    s = ff{t.x, t.y};
+    for (int o = 8; o > 0; o >>= 1) s = ff_add(s, ff_shfl_down(s, o, 16));
   }
   return s;
+}
+
+// Sum of n float-pair partials by one warp (valid in lane 0), the same in every
+// CTA: lane l takes l, l + 32, ..., then a shuffle tree.
+__device__ __forceinline__ ff warp_total_ff(const double* part, int n) {
+  ff v{0.f, 0.f};
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += 32) {
+    const float2 t = __ldcg(reinterpret_cast<const float2*>(part) + i);
+    v = ff_add(v, ff{t.x, t.y});
+  }
+  for (int o = 16; o > 0; o >>= 1) v = ff_add(v, ff_shfl_down(v, o));
+  return v;
+}
+
+// The same for n pairs of float pairs.
+__device__ __forceinline__ void warp_total2_ff(const double* part, int n, ff& v, ff& w) {
+  v = w = ff{0.f, 0.f};
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += 32) {
+    const float4 t = __ldcg(reinterpret_cast<const float4*>(part) + i);
+    v = ff_add(v, ff{t.x, t.y});
+    w = ff_add(w, ff{t.z, t.w});
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const ff a = ff_shfl_down(v, o), b = ff_shfl_down(w, o);
+    v = ff_add(v, a);
+    w = ff_add(w, b);
+  }
+}
+
+// a / b as a float pair (the quotient of the heads and its correction).
+__device__ __forceinline__ ff ff_div(ff a, ff b) {
+  const float q = __fdiv_rn(a.h, b.h);
+  const float p = __fmul_rn(q, b.h), pe = __fmaf_rn(q, b.h, -p);
+  float e = __fsub_rn(__fsub_rn(a.h, p), pe);  // a.h - q b.h (a.h - p is exact)
+  e = __fadd_rn(e, __fmaf_rn(-q, b.l, a.l));
+  ff r;
+  fast_two_sum(q, __fdiv_rn(e, b.h), r.h, r.l);
+  return r;
+}
+
+__device__ __forceinline__ void store_part(double* part, ff v) {
+  *reinterpret_cast<float2*>(part) = make_float2(v.h, v.l);
+}
+
+__device__ __forceinline__ double ff_double(ff v) { return (double)v.h + (double)v.l; }
+
+// The recurrence's scalars of the resident form between two updates, in float
+// pairs and FP32 (thread 0 of every CTA alike; the MixedState holds them at the
+// ends and across updates).  The norms only decide when an update is due, whose
+// FP64-accurate residual decides the solve.
+struct FastState {
+  ff rz, rz_old, alpha, pq;
+  float beta, rnorm, rmax, rbest, delta, tol;
+  int it_best;
+};
+
+__device__ __forceinline__ void fast_from(FastState& f, const MixedState& s) {
+  f.rz = ff_from_double(s.rz);
+  f.rz_old = ff_from_double(s.rz_old);
+  f.beta = (float)s.beta;
+  f.rnorm = (float)s.rnorm;
+  f.rmax = (float)s.rmax;
+  f.rbest = (float)s.rbest;
+  f.delta = (float)s.delta;
+  f.tol = (float)s.tol_norm_b;
+  f.it_best = s.it_best;
+}
+
+__device__ __forceinline__ void fast_to(const FastState& f, MixedState& s) {
+  s.rz = ff_double(f.rz);
+  s.rz_old = ff_double(f.rz_old);
+  s.alpha = ff_double(f.alpha);
+  s.pq = ff_double(f.pq);
+  s.beta = f.beta;
+  s.rnorm = f.rnorm;
+  s.rmax = f.rmax;
+  s.rbest = f.rbest;
+  s.it_best = f.it_best;
+}
+
+// The step's scalars, as step_scalars and update_due; CTA 0 leaves |r|^2 as a
+// float pair in the history (k_hist_sqrt takes the root after the launch).
+__device__ __forceinline__ void fast_step(FastState& f, MixedState& s, const PersistArgs& a,
+                                          int it, ff trz, ff trr) {
+  f.rz_old = f.rz;
+  f.rz = trz;
+  f.rnorm = sqrtf(trr.h);
+  s.iter = it;
+  if (blockIdx.x == 0) store_part(a.hist + it, trr);
+  f.rmax = fmaxf(f.rmax, f.rnorm);
+  if (f.rnorm < 0.5f * f.rbest) {
+    f.rbest = f.rnorm;
+    f.it_best = it;
+  }
+  const bool stall = it - f.it_best >= STALL_ITERS;
+  if (stall) s.stalled = 1;
+  s.need_update =
+      f.rnorm < f.delta * f.rmax || f.rnorm <= f.tol || it >= s.max_iter || stall ? 1 : 0;
+  f.beta = ff_div(f.rz, f.rz_old).h;
 }
 
 // a += x y exactly rounded to a float pair (the product's error by FMA).
@@ -885,7 +979,9 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   int* sk = reinterpret_cast<int*>(smraw + ResLayout::sk);
   __half* Lh = reinterpret_cast<__half*>(smraw + ResLayout::lh);
   __shared__ MixedState sS;
-  __shared__ double red[2 * (NT / 32)];
+  __shared__ FastState sF;
+  __shared__ float2 red[2 * (NT / 32)];
+  __shared__ double red64[NT / 32];
   __shared__ ff s_alpha;  // alpha as a float pair (x update)
   __shared__ float s_ab;  // alpha or beta in FP32
   __shared__ size_t s_off[MAX_G * NB_R];  // staged FP64 lists (the update's residual)
@@ -900,7 +996,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   const size_t n = (size_t)a.n;
   const size_t ns = (size_t)a.n_blocks * a.S;
   BarState bst;  // barrier state (thread 0)
-  if (tid == 0) sS = *a.S_;
+  if (tid == 0) {
+    sS = *a.S_;
+    fast_from(sF, sS);
+  }
   timers_start(a, bst);
   if (tid < MAX_G) sk[tid] = tid < a.g ? skewer_of(a, blk, tid) : -1;
   {  // the block's product items
@@ -1045,7 +1144,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       // memory (us, free in this phase).
       ff dq{0.f, 0.f};
       {
-        if (tid == 0) s_ab = (float)sS.beta;
+        if (tid == 0) s_ab = sF.beta;
         float* red_w = reinterpret_cast<float*>(us);  // (NT / n_per) x GI x n_per
         const int ni = s_nit[0] - s_nit[1], i0 = s_nit[1];  // the other blocks' rows
         if (has_pixel) {
@@ -1071,20 +1170,18 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       {
-        const double bs = block_sum2_ff(dq, ff{0.f, 0.f}, red);
-        if (tid == 0) a.part[blk] = bs;
+        const ff bs = block_sum2_ff(dq, ff{0.f, 0.f}, red);
+        if (tid == 0) store_part(a.part + blk, bs);
       }
       if (!grid_sync(a, B_PRODUCT, bst)) break;
       // ---- step: alpha; x, r, z of the block; levels of z; partials.  Warp 0
       // alone adds the CTAs' partials and forms the scalars.
       if (tid < 32) {
-        const double pq = warp_total(a.part, G);
+        const ff pq = warp_total_ff(a.part, G);
         if (tid == 0) {
-          const double al = sS.rz / pq;
-          sS.pq = pq;
-          sS.alpha = al;
-          s_alpha = ff_from_double(al);
-          s_ab = (float)al;
+          sF.pq = pq;
+          sF.alpha = s_alpha = ff_div(sF.rz, pq);
+          s_ab = s_alpha.h;
         }
       }
       __syncthreads();
@@ -1117,15 +1214,16 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       }
       levels_z();  // published first: the stores drain while the sums are formed
       {
-        const double bs = block_sum2_ff(rz, rr, red);
-        if (tid == 0 || tid == 16) a.part[(size_t)P2 + 2 * blk + (tid >> 4)] = bs;
+        const ff bs = block_sum2_ff(rz, rr, red);
+        if (tid == 0 || tid == 16) store_part(a.part + (size_t)P2 + 2 * blk + (tid >> 4), bs);
       }
       grid_arrive(a, B_STEP, bst);
       own_rows();
       if (!grid_wait(a, B_STEP, bst)) break;
       if (tid < 32) {
-        const double2 t2 = warp_total2(a.part + P2, G);
-        if (tid == 0) step_scalars(sS, a, it, sS.alpha, sS.pq, t2.x, t2.y);
+        ff trz, trr;
+        warp_total2_ff(a.part + P2, G, trz, trr);
+        if (tid == 0) fast_step(sF, sS, a, it, trz, trr);
       }
       __syncthreads();
       if (!sS.need_update) continue;
@@ -1201,10 +1299,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       {
-        const double b1 = block_sum2_ff(rz_u, ff{0.f, 0.f}, red);
-        const double b2 = block_sum<NT>(rr_u, red);
+        const ff b1 = block_sum2_ff(rz_u, ff{0.f, 0.f}, red);
+        const double b2 = block_sum<NT>(rr_u, red64);
         if (tid == 0) {
-          a.part[(size_t)P2 + 2 * blk] = b1;
+          a.part[(size_t)P2 + 2 * blk] = ff_double(b1);
           a.part[(size_t)P2 + 2 * blk + 1] = b2;
         }
       }
@@ -1214,7 +1312,12 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       if (!grid_wait(a, B_UPDATE, bst)) break;
       if (tid < 32) {
         const double2 t2 = warp_total2(a.part + P2, G);
-        if (tid == 0) update_scalars(sS, a, t2.x, t2.y);
+        if (tid == 0) {
+          fast_to(sF, sS);
+          update_scalars(sS, a, t2.x, t2.y);
+          if (blockIdx.x == 0) store_part(a.hist + sS.iter, ff_from_double(t2.y));
+          fast_from(sF, sS);
+        }
       }
       __syncthreads();
     }
@@ -1224,6 +1327,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     if (jj[t] >= 0) a.x[rg[t]] = (double)xs[tid + t * NT].h + (double)xs[tid + t * NT].l;
   timers_end(a);
   if (blockIdx.x == 0 && tid == 0) {
+    fast_to(sF, sS);
     sS.skip_update = 1;
     *a.S_ = sS;
   }
@@ -1350,6 +1454,15 @@ __global__ void __launch_bounds__(NT) k_build_items(int g, int n_per, int n,
     cnt[blk] = n_items;
     own[blk] = n_own;
     atomicMax(cnt + gridDim.x, n_items);
+  }
+}
+
+// The roots of the |r|^2 that the resident form left in hist[1 .. iter].
+__global__ void k_hist_sqrt(const MixedState* st, double* __restrict__ hist) {
+  for (int i = 1 + blockIdx.x * blockDim.x + threadIdx.x; i <= st->iter;
+       i += gridDim.x * blockDim.x) {
+    const float2 v = reinterpret_cast<const float2*>(hist)[i];
+    hist[i] = sqrt((double)v.x + (double)v.y);
   }
 }
 
@@ -1527,6 +1640,10 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   DS_CUDA(cudaLaunchCooperativeKernel(pick(resident), dim3(grid), dim3(NT), args,
                                       resident ? res_bytes : 0, st));
   DS_CHECK_LAUNCH();
+  if (resident) {
+    k_hist_sqrt<<<std::min(64, (max_iter + 255) / 256), 256, 0, st>>>(f.state.p, f.hist.p);
+    DS_CHECK_LAUNCH();
+  }
   return true;
 }
 
