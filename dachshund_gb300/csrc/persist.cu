@@ -925,18 +925,84 @@ struct ResLayout {
   static size_t bytes(int band, int S) { return lh + ((size_t)(band + 1) * S * 2 + 15) / 16 * 16; }
 };
 
+// The thread's slots of the resident form: neighbours where a block has more
+// slots than the CTA threads, else one.
+__device__ __forceinline__ int slot_of(int S, int t) {
+  return S > NT ? 2 * (int)threadIdx.x + t : (int)threadIdx.x + t * NT;
+}
+
 // z = G G^T r over the CTA's block from r in shared memory, with the block's
 // factor in shared memory in FP16 (plane m, slot i at Lh[m S + i]; a
 // preconditioner needs no more: M^-1 = G G^T stays symmetric positive
 // definite whatever the rounding of G).
+//
+// With more slots than threads a thread takes slots 2 tid and 2 tid + 1: its
+// window of r (or t) comes as pairs and serves both slots, and so does a pair of
+// factor entries where it is aligned.  The passes are bound by the shared-memory
+// wavefronts (2 x 17 taps of three operands): 68 per warp, slot pair and pass
+// slot by slot, ~40 this way.  The sums are the same, in the same order.
 template <int BAND>
 __device__ __forceinline__ void block_precond_h(const PersistArgs& a, const __half* Lh,
                                                 const float* rs, float* ts, float (&zk)[RPT]) {
+  static_assert(RPT == 2, "two slots per thread");
   const int band = BAND >= 0 ? BAND : a.band;
   const int S = a.S;
+  if (BAND > 0 && BAND % 2 == 0 && S > NT && S % 2 == 0) {
+    constexpr int B = BAND > 0 ? BAND : 2;
+    const int i0 = 2 * threadIdx.x;
+    const bool in = i0 < S;
+    float w[B + 2];  // w[k] = r[i0 + k]
+    if (in) {
+#pragma unroll
+      for (int k = 0; k < B + 2; k += 2) {
+        const bool ok = i0 + k < S;
+        const float2 v = ok ? *reinterpret_cast<const float2*>(rs + i0 + k) : make_float2(0.f, 0.f);
+        w[k] = v.x;
+        w[k + 1] = v.y;
+      }
+      float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+      for (int m = 0; m <= B; ++m) {  // L[m][i + m], i = i0, i0 + 1
+        __half l0 = __float2half_rn(0.f), l1 = l0;
+        if (m % 2 == 0) {
+          if (i0 + m < S) {
+            const __half2 l = *reinterpret_cast<const __half2*>(Lh + m * S + i0 + m);
+            l0 = __low2half(l);
+            l1 = __high2half(l);
+          }
+        } else {
+          if (i0 + m < S) l0 = Lh[m * S + i0 + m];
+          if (i0 + 1 + m < S) l1 = Lh[m * S + i0 + 1 + m];
+        }
+        v0 = fmaf(__half2float(l0), w[m], v0);
+        v1 = fmaf(__half2float(l1), w[m + 1], v1);
+      }
+      *reinterpret_cast<float2*>(ts + i0) = make_float2(v0, v1);
+    }
+    __syncthreads();
+    float z0 = 0.f, z1 = 0.f;
+    if (in) {
+#pragma unroll
+      for (int k = 0; k < B + 2; k += 2) {  // w[k] = t[i0 - B + k]
+        const int q = i0 - B + k;
+        const float2 v = q >= 0 ? *reinterpret_cast<const float2*>(ts + q) : make_float2(0.f, 0.f);
+        w[k] = v.x;
+        w[k + 1] = v.y;
+      }
+#pragma unroll
+      for (int m = 0; m <= B; ++m) {  // L[m][i] t[i - m]
+        const __half2 l = *reinterpret_cast<const __half2*>(Lh + m * S + i0);
+        z0 = fmaf(__low2float(l), w[B - m], z0);
+        z1 = fmaf(__high2float(l), w[B + 1 - m], z1);
+      }
+    }
+    zk[0] = z0;
+    zk[1] = z1;
+    return;
+  }
 #pragma unroll
   for (int t = 0; t < RPT; ++t) {
-    const int i = threadIdx.x + t * NT;
+    const int i = slot_of(S, t);
     if (i < S) {
       float v = 0.f;
 #pragma unroll(BAND >= 0 ? BAND + 1 : 1)
@@ -948,7 +1014,7 @@ __device__ __forceinline__ void block_precond_h(const PersistArgs& a, const __ha
   __syncthreads();
 #pragma unroll
   for (int t = 0; t < RPT; ++t) {
-    const int i = threadIdx.x + t * NT;
+    const int i = slot_of(S, t);
     float v = 0.f;
     if (i < S) {
 #pragma unroll(BAND >= 0 ? BAND + 1 : 1)
@@ -1191,7 +1257,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       int li[RPT];
 #pragma unroll
       for (int t = 0; t < RPT; ++t) {
-        const int i = tid + t * NT;
+        const int i = slot_of(a.S, t);
         li[t] = i < a.S ? loc[i] : -1;
         if (li[t] >= 0) {
           const int l = li[t];
@@ -1206,7 +1272,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
 #pragma unroll
         for (int t = 0; t < RPT; ++t) {
           if (li[t] < 0) continue;
-          const float ri = rs[tid + t * NT];
+          const float ri = rs[slot_of(a.S, t)];
           zs[li[t]] = zk[t];
           ff_acc_prod(rz, ri, zk[t]);
           ff_acc_prod(rr, ri, ri);
@@ -1277,7 +1343,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       double rr_u = 0.0;
 #pragma unroll
       for (int t = 0; t < RPT; ++t) {
-        const int i = tid + t * NT;
+        const int i = slot_of(a.S, t);
         if (i >= a.S) continue;
         float rv = 0.f;
         if (li[t] >= 0) {
@@ -1295,7 +1361,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         for (int t = 0; t < RPT; ++t) {
           if (li[t] < 0) continue;
           zs[li[t]] = zk[t];
-          ff_acc_prod(rz_u, rs[tid + t * NT], zk[t]);
+          ff_acc_prod(rz_u, rs[slot_of(a.S, t)], zk[t]);
         }
       }
       {
