@@ -4,6 +4,8 @@
 
 #include <cuda_bf16.h>
 
+#include <atomic>
+
 #include "ds_internal.cuh"
 
 namespace ds {
@@ -91,7 +93,14 @@ void embed_grad(int M, int H, int sms, const float* X, const float* dZ, float* p
                 float* db, cudaStream_t st);
 void build_rev_lists(int n_sk, const int* nbr, const float* g, RevLists& rev, cudaStream_t st);
 
+inline unsigned long long next_pc_serial() {
+  static std::atomic<unsigned long long> n{0};
+  return ++n;
+}
+
 struct SkewerPC {
+  // identity for what is built from it (an address can come back)
+  const unsigned long long serial = next_pc_serial();
   int n_sk = 0, n_per = 0, band = 0;  // blocks, slots per block, bandwidth
   DevBuf<float> L;    // band + 1 planes of n_sk n_per slots: L[k][k - m] at plane m
   DevBuf<int> crec;   // record of each slot (empty: slot = record)

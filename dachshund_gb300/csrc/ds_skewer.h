@@ -45,7 +45,7 @@ struct SkewerGrid {
   DevBuf<float2> ff_wl, ff_wr, ff_e, ff_b, ff_op, ff_taps;
   // the persistent solve's product items (for the preconditioner and inner
   // cutoff they were built for)
-  const void* res_pc = nullptr;
+  unsigned long long res_pc = 0;  // SkewerPC::serial
   double res_cut = 0.0;
   int res_max_list = 0;  // the most items of a block (above the limit: not built)
   DevBuf<int> it_cnt;            // per block: its items (n_blocks + 1: the largest)

@@ -1593,7 +1593,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   // (neighbour, level) rows its skewers' FP32 lists name, ordered by offset,
   // with each skewer's factor, in slots of NI per block.
   const bool off31 = (double)(g.inner.lmax + 1) * (double)op->n < 2147483647.0;
-  if (g.res_pc != pc || g.res_cut != g.inner.cut) {
+  if (g.res_pc != pc->serial || g.res_cut != g.inner.cut) {
     g.res_max_list = NI + 1;  // unusable unless built
     if (off31 && pc->g <= GI && g.n_per <= NT && g.inner.idx.n < (1u << 28)) {
       g.it_cnt.alloc(pc->n_sk + 1);  // last: the largest count (or an overflow mark)
@@ -1612,7 +1612,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
       DS_CUDA(cudaStreamSynchronize(st));
       g.res_max_list = mx;
     }
-    g.res_pc = pc;
+    g.res_pc = pc->serial;
     g.res_cut = g.inner.cut;
   }
   const size_t res_bytes = ResLayout::bytes(band, pc->n_per);
@@ -1737,7 +1737,7 @@ int persistent_profile(ds_operator* op, double* out, int n, bool reset) {
   const int grid = (int)v[PT_GRID];
   // the resident form's product: neighbour values loaded per product
   // (items x n_per); 0 for the general form
-  if (g.it_cnt.p && g.res_max_list <= NI && g.res_pc == op->pc.get()) {
+  if (g.it_cnt.p && g.res_max_list <= NI && op->pc && g.res_pc == op->pc->serial) {
     std::vector<int> cnt(g.it_cnt.n);
     DS_CUDA(cudaMemcpyAsync(cnt.data(), g.it_cnt.p, cnt.size() * sizeof(int),
                             cudaMemcpyDeviceToHost, st));
