@@ -50,6 +50,7 @@ struct SkewerGrid {
   int res_max_list = 0;  // the most items of a block (above the limit: not built)
   DevBuf<int> it_cnt;            // per block: its items (n_blocks + 1: the largest)
   DevBuf<int> it_own;            // per block: its items on its own skewers (the first)
+  DevBuf<int> it_order;          // block of each CTA (launch order)
   DevBuf<unsigned int> it_off;   // item (slots of 512 per block): offset of its
                                  // (neighbour, level) row in the levels
   DevBuf<float4> it_coef;        // item: the factor for each of the block's skewers

@@ -45,6 +45,7 @@
 // timers (%globaltimer) accumulate per launch for the profile.
 #include <algorithm>
 #include <cmath>
+#include <numeric>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -103,6 +104,7 @@ struct PersistArgs {
   // offset into the levels and the factor for each of the block's (<= 4)
   // skewers, 0 where unused)
   const int* it_cnt;
+  const int* it_order;  // block of each CTA
   const int* it_own;  // per block: its items on the block's own skewers (the first ones)
   const unsigned int* it_off;
   const float4* it_coef;
@@ -1056,7 +1058,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   const int tid = threadIdx.x;
   const int G = gridDim.x;
   const int P2 = (G + 1) & ~1;
-  const int blk = blockIdx.x;
+  const int blk = a.it_order[blockIdx.x];
   const int npr = a.n_per;
   const int m = a.g * npr;  // records of the block (record-local index j n_per + k)
   const size_t n = (size_t)a.n;
@@ -1564,6 +1566,25 @@ int resident_per_sm(const void* fn, size_t smem) {
   return per_sm;
 }
 
+// The block of each CTA.  The slowest block sets the product phase (an interior
+// cluster has up to 1.7 times the mean's rows), and the first CTAs of a launch
+// go one to an SM, the rest second to the same SMs in order: the blocks with the
+// most items get the SMs that hold one CTA, the others are paired most with
+// fewest.
+std::vector<int> launch_order(const std::vector<int>& cnt, int n, int sms) {
+  std::vector<int> by(n), order(n);
+  std::iota(by.begin(), by.end(), 0);
+  std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return cnt[x] > cnt[y]; });
+  const int second = std::max(0, n - sms), alone = n - 2 * second;
+  if (alone < 0) return by;
+  for (int i = 0; i < alone; ++i) order[second + i] = by[i];
+  for (int i = 0; i < second; ++i) {
+    order[i] = by[alone + i];
+    order[sms + i] = by[n - 1 - i];
+  }
+  return order;
+}
+
 template <int BAND>
 const void* kernel_of(bool resident) {
   return resident ? (const void*)k_mixed_resident<BAND> : (const void*)k_mixed_persistent<BAND>;
@@ -1606,11 +1627,16 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
                                              g.it_cnt.p, g.it_own.p, g.it_off.p,
                                              g.it_coef.p);
       DS_CHECK_LAUNCH();
-      int mx = 0;
-      DS_CUDA(cudaMemcpyAsync(&mx, g.it_cnt.p + pc->n_sk, sizeof(int), cudaMemcpyDeviceToHost,
+      std::vector<int> cnt(pc->n_sk + 1), order;
+      DS_CUDA(cudaMemcpyAsync(cnt.data(), g.it_cnt.p, g.it_cnt.bytes(), cudaMemcpyDeviceToHost,
                               st));
       DS_CUDA(cudaStreamSynchronize(st));
-      g.res_max_list = mx;
+      g.res_max_list = cnt.back();
+      order = launch_order(cnt, pc->n_sk, op->ctx->num_sms);
+      g.it_order.alloc(pc->n_sk);
+      DS_CUDA(cudaMemcpyAsync(g.it_order.p, order.data(), g.it_order.bytes(),
+                              cudaMemcpyHostToDevice, st));
+      DS_CUDA(cudaStreamSynchronize(st));  // order is on this stack frame
     }
     g.res_pc = pc->serial;
     g.res_cut = g.inner.cut;
@@ -1684,6 +1710,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   a.limit = op->ctx->wait_limit > 0 ? op->ctx->wait_limit : 4000000000LL;
   a.pt = g.p_time.p;
   a.it_cnt = g.it_cnt.p;
+  a.it_order = g.it_order.p;
   a.it_own = g.it_own.p;
   a.it_off = g.it_off.p;
   a.it_coef = g.it_coef.p;
