@@ -383,6 +383,7 @@ struct ds_operator {
   ds::DevBuf<unsigned int> dense_mask, dense_need;
   bool pairs_built = false;  // `pairs` (ensure_op_pairs)
   ds::PairVals vals;         // the pairs' values (ensure_pair_vals)
+  ds::DevBuf<unsigned int> pcg_sync;  // barrier count and error word (pcg_persist.cu)
   int inner_variant = 0;     // inner matvec of the mixed form (InnerVariant)
   int iter_form = 0;         // DS_ITER_AUTO / DS_ITER_GRAPH
   // skewer-band preconditioner of the mixed form (null: Jacobi)

@@ -67,6 +67,10 @@ bool ensure_pair_vals(ds_operator* op);
 // out = A v or b - A v from them (a as for launch_pair_f64, a.u formed).
 void launch_pair_vals(ds_operator* op, int epi, const PairArgs& a, cudaStream_t st);
 
+// The iteration of run_pcg as one cooperative launch, where that applies
+// (pcg_persist.cu).
+bool run_pcg_persistent(ds_operator* op, const ds_pcg_params& pp, cudaStream_t st);
+
 // Pair values in fixed point (pair_fx.cu).
 bool fx_usable(const KernelConsts& kc, const PointSet& rows, const PointSet& cols);
 void launch_pair_fx(const KernelConsts& kc, int epi, const PairArgs& a, const PointSet& rows,

@@ -241,11 +241,17 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
 
   PcgState* S = op->state.p;
   const int g = vgrid(np);
-  // r = b - A x; d = M^-1 r; delta = r.d; |r|  (lib/pcg.h:95-108)
-  op_apply_sorted(op, EPI_RESIDUAL, op->x.p, op->r.p, st);
-  k_pcg_update<3><<<g, VB, 0, st>>>(np, S, op->x.p, op->r.p, op->q.p, op->q.p, op->d.p,
-                                    op->pdiag.p, op->partial.p, op->hist.p, op->dhist.p);
-  DS_CHECK_LAUNCH();
+  const bool vals = !op->use_dense && ensure_pair_vals(op);
+  // (profiling times the products one by one)
+  const bool persistent =
+      vals && !op->ctx->prof.enabled && run_pcg_persistent(op, pp, st);
+  if (!persistent) {
+    // r = b - A x; d = M^-1 r; delta = r.d; |r|  (lib/pcg.h:95-108)
+    op_apply_sorted(op, EPI_RESIDUAL, op->x.p, op->r.p, st);
+    k_pcg_update<3><<<g, VB, 0, st>>>(np, S, op->x.p, op->r.p, op->q.p, op->q.p, op->d.p,
+                                      op->pdiag.p, op->partial.p, op->hist.p, op->dhist.p);
+    DS_CHECK_LAUNCH();
+  }
 
   PairArgs prod = op_pair_args(op, op->d.p, op->q.p);
   prod.dotv = op->d.p;
@@ -255,9 +261,8 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   prod.skip_flag = &S->done;
   PairArgs resid = op_pair_args(op, op->x.p, op->r.p);
   resid.skip_flag = &S->done;
-  const bool vals = !op->use_dense && ensure_pair_vals(op);
   double* u = nullptr;  // the weights of d, kept by k_pcg_direction
-  if (vals) {
+  if (vals && !persistent) {
     op->ud.alloc(np);
     u = prod.u = op->ud.p;
     form_u(np, op->kc.var_s, prod.wr, op->d.p, u, nullptr, st);
@@ -268,7 +273,7 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   cudaEvent_t evs[NSLOT];
   for (auto& e : evs) DS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   int issued = 0, waited = 0;
-  for (int it = 1; it < pp.max_iter; ++it) {
+  for (int it = 1; it < pp.max_iter && !persistent; ++it) {
     if (op->use_dense)  // q = A d, alpha
       dense_apply(op, false, op->d.p, op->q.p, op->d.p, S, &S->done, st);
     else if (vals)
@@ -318,6 +323,14 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   for (auto& e : evs) cudaEventDestroy(e);
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
+  if (persistent) {
+    unsigned int code = 0;
+    DS_CUDA(cudaMemcpyAsync(&code, op->pcg_sync.p + 1, sizeof(code), cudaMemcpyDeviceToHost, st));
+    DS_CUDA(cudaStreamSynchronize(st));
+    if (code)
+      throw Error{DS_ERR_TIMEOUT, "persistent PCG: a grid barrier wait timed out (barrier " +
+                                      std::to_string(code) + ")"};
+  }
 
   const int n_hist = h.iter + 1;
   std::vector<double> hh(n_hist), dh(n_hist);

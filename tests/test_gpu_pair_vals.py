@@ -124,3 +124,38 @@ def test_residual_evaluated_on_every_call(ctx):
     # both residuals <= 1e-11 |b|, A >= I in the W form (x = w y, w in [3.3, 20])
     assert np.linalg.norm((x - xp) / rec[:, 3]) <= 2.1e-11 * res.norm_b
     op.close()
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("n", [1, 33, 129, 4000, 5000, 9700, 9800])
+def test_pcg_forms_vs_oracle_residual(ctx, n, exact):
+    """One CTA per slice (up to one per SM, two, and beyond the cooperative form):
+    the recurrence's |r| and the true residual by the oracle's operator.  FP64 CG
+    drifts from the true residual by rounding alone, below 1e-13 |b| here (200
+    iterations of 2^-53 |A| |x| each, |A| |x| < 30 |b|)."""
+    rec = records("w", n, n)
+    op = WFVectorW(ctx, rec, SignalCovarParams(VS, LP, LQ, eval="exact" if exact else "table"))
+    x, res = op.solve_pcg(PCGParams(2000, 50, 1e-10))
+    assert res.success and res.final_norm <= 1e-10 * res.norm_b
+    assert res.residual_norms.size == res.num_iters + 1
+    r = oracle.A_residual("w", rec, x / rec[:, 3], VS, LP, LQ, exact=exact)
+    assert abs(np.linalg.norm(r) - res.final_norm) <= 1e-12 * res.norm_b
+    # a start from the solution stops after the first iteration's test; the cap counts
+    x2, r2 = op.solve_pcg(PCGParams(3, 2, 0.0), x / rec[:, 3])
+    assert not r2.success and r2.num_iters == 3 and r2.residual_norms.size == 3
+    op.close()
+
+
+def test_pcg_barrier_timeout(ctx):
+    from dachshund_gb300 import DsError
+
+    op = WFVectorW(ctx, records("w", 1000, 3), SignalCovarParams(VS, LP, LQ))
+    ctx.set_wait_limit(1)
+    try:
+        with pytest.raises(DsError) as e:
+            op.solve_pcg(PCGParams(100, 50, 1e-8))
+        assert e.value.code == 8
+    finally:
+        ctx.set_wait_limit(0)
+    assert op.solve_pcg(PCGParams(1000, 50, 1e-8))[1].success
+    op.close()
