@@ -55,6 +55,7 @@
 #include "ds_f32.h"
 #include "ds_learned.h"
 #include "ds_mixed_dev.cuh"
+#include "ds_ffsum.cuh"
 #include "ds_ops.h"
 #include "ds_skewer.h"
 
@@ -296,150 +297,6 @@ __device__ __forceinline__ double2 partial_total2(const double* part, int n, dou
   const double2 t = make_double2(out[0], out[1]);
   __syncthreads();
   return t;
-}
-
-__device__ __forceinline__ ff ff_shfl_down(ff v, int o, int width = 32) {
-  ff r;
-  r.h = __shfl_down_sync(0xffffffffu, v.h, o, width);
-  r.l = __shfl_down_sync(0xffffffffu, v.l, o, width);
-  return r;
-}
-
-// Sums over the CTA of two float pairs per thread (float-pair shuffle trees, a
-// fixed order), valid in lanes 0 and 16 of warp 0.  The Krylov vectors' dot
-// products are summed this way from the threads to the grid (exact products by
-// FMA, compensated sums, about 44 bits): a chain of dependent FP64 instructions
-// has a latency of a hundred clocks or more each on GB300, and the FP64 sums and
-// scalars of an iteration took 14,000 of its 22,000 clocks at 16 CTAs.
-__device__ __forceinline__ ff block_sum2_ff(ff v, ff w, float2* sm /* 2 NT/32 */) {
-  static_assert(NT / 32 == 16, "two sums share a warp");
-  for (int o = 16; o > 0; o >>= 1) {
-    const ff a = ff_shfl_down(v, o), b = ff_shfl_down(w, o);
-    v = ff_add(v, a);
-    w = ff_add(w, b);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    sm[wid] = make_float2(v.h, v.l);
-    sm[16 + wid] = make_float2(w.h, w.l);
-  }
-  __syncthreads();
-  ff s{0.f, 0.f};
-  if (wid == 0) {
-    const float2 t = sm[lane];
-    s = ff{t.x, t.y};
-    for (int o = 8; o > 0; o >>= 1) s = ff_add(s, ff_shfl_down(s, o, 16));
-  }
-  return s;
-}
-
-// Sum of n float-pair partials by one warp (valid in lane 0), the same in every
-// CTA: lane l takes l, l + 32, ..., then a shuffle tree.
-__device__ __forceinline__ ff warp_total_ff(const double* part, int n) {
-  ff v{0.f, 0.f};
-#pragma unroll 4
-  for (int i = threadIdx.x; i < n; i += 32) {
-    const float2 t = __ldcg(reinterpret_cast<const float2*>(part) + i);
-    v = ff_add(v, ff{t.x, t.y});
-  }
-  for (int o = 16; o > 0; o >>= 1) v = ff_add(v, ff_shfl_down(v, o));
-  return v;
-}
-
-// The same for n pairs of float pairs.
-__device__ __forceinline__ void warp_total2_ff(const double* part, int n, ff& v, ff& w) {
-  v = w = ff{0.f, 0.f};
-#pragma unroll 4
-  for (int i = threadIdx.x; i < n; i += 32) {
-    const float4 t = __ldcg(reinterpret_cast<const float4*>(part) + i);
-    v = ff_add(v, ff{t.x, t.y});
-    w = ff_add(w, ff{t.z, t.w});
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const ff a = ff_shfl_down(v, o), b = ff_shfl_down(w, o);
-    v = ff_add(v, a);
-    w = ff_add(w, b);
-  }
-}
-
-// a / b as a float pair (the quotient of the heads and its correction).
-__device__ __forceinline__ ff ff_div(ff a, ff b) {
-  const float q = __fdiv_rn(a.h, b.h);
-  const float p = __fmul_rn(q, b.h), pe = __fmaf_rn(q, b.h, -p);
-  float e = __fsub_rn(__fsub_rn(a.h, p), pe);  // a.h - q b.h (a.h - p is exact)
-  e = __fadd_rn(e, __fmaf_rn(-q, b.l, a.l));
-  ff r;
-  fast_two_sum(q, __fdiv_rn(e, b.h), r.h, r.l);
-  return r;
-}
-
-__device__ __forceinline__ void store_part(double* part, ff v) {
-  *reinterpret_cast<float2*>(part) = make_float2(v.h, v.l);
-}
-
-__device__ __forceinline__ double ff_double(ff v) { return (double)v.h + (double)v.l; }
-
-// The recurrence's scalars of the resident form between two updates, in float
-// pairs and FP32 (thread 0 of every CTA alike; the MixedState holds them at the
-// ends and across updates).  The norms only decide when an update is due, whose
-// FP64-accurate residual decides the solve.
-struct FastState {
-  ff rz, rz_old, alpha, pq;
-  float beta, rnorm, rmax, rbest, delta, tol;
-  int it_best;
-};
-
-__device__ __forceinline__ void fast_from(FastState& f, const MixedState& s) {
-  f.rz = ff_from_double(s.rz);
-  f.rz_old = ff_from_double(s.rz_old);
-  f.beta = (float)s.beta;
-  f.rnorm = (float)s.rnorm;
-  f.rmax = (float)s.rmax;
-  f.rbest = (float)s.rbest;
-  f.delta = (float)s.delta;
-  f.tol = (float)s.tol_norm_b;
-  f.it_best = s.it_best;
-}
-
-__device__ __forceinline__ void fast_to(const FastState& f, MixedState& s) {
-  s.rz = ff_double(f.rz);
-  s.rz_old = ff_double(f.rz_old);
-  s.alpha = ff_double(f.alpha);
-  s.pq = ff_double(f.pq);
-  s.beta = f.beta;
-  s.rnorm = f.rnorm;
-  s.rmax = f.rmax;
-  s.rbest = f.rbest;
-  s.it_best = f.it_best;
-}
-
-// The step's scalars, as step_scalars and update_due; CTA 0 leaves |r|^2 as a
-// float pair in the history (k_hist_sqrt takes the root after the launch).
-__device__ __forceinline__ void fast_step(FastState& f, MixedState& s, const PersistArgs& a,
-                                          int it, ff trz, ff trr) {
-  f.rz_old = f.rz;
-  f.rz = trz;
-  f.rnorm = sqrtf(trr.h);
-  s.iter = it;
-  if (blockIdx.x == 0) store_part(a.hist + it, trr);
-  f.rmax = fmaxf(f.rmax, f.rnorm);
-  if (f.rnorm < 0.5f * f.rbest) {
-    f.rbest = f.rnorm;
-    f.it_best = it;
-  }
-  const bool stall = it - f.it_best >= STALL_ITERS;
-  if (stall) s.stalled = 1;
-  s.need_update =
-      f.rnorm < f.delta * f.rmax || f.rnorm <= f.tol || it >= s.max_iter || stall ? 1 : 0;
-  f.beta = ff_div(f.rz, f.rz_old).h;
-}
-
-// a += x y exactly rounded to a float pair (the product's error by FMA).
-__device__ __forceinline__ void ff_acc_prod(ff& a, float x, float y) {
-  ff p;
-  p.h = __fmul_rn(x, y);
-  p.l = __fmaf_rn(x, y, -p.h);
-  a = ff_add(a, p);
 }
 
 __device__ __forceinline__ int skewer_of(const PersistArgs& a, int blk, int j) {
@@ -1066,7 +923,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   BarState bst;  // barrier state (thread 0)
   if (tid == 0) {
     sS = *a.S_;
-    fast_from(sF, sS);
+    fast_init(sF, sS);
   }
   timers_start(a, bst);
   if (tid < MAX_G) sk[tid] = tid < a.g ? skewer_of(a, blk, tid) : -1;
@@ -1083,6 +940,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     }
   }
   __syncthreads();
+  const float sr = sF.sr, sz = sF.sz;  // the sums' scales
   for (int i = tid; i < m; i += NT) {
     const int j = i / npr;
     const int s = sk[j];
@@ -1234,11 +1092,11 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           const float qv = fmaf(beta, qs[i], wv);
           ps[i] = pv;
           qs[i] = qv;
-          ff_acc_prod(dq, pv, qv);
+          ff_acc_prod(dq, sz * pv, sr * qv);
         }
       }
       {
-        const ff bs = block_sum2_ff(dq, ff{0.f, 0.f}, red);
+        const ff bs = block_sum2_ff<NT>(dq, ff{0.f, 0.f}, red);
         if (tid == 0) store_part(a.part + blk, bs);
       }
       if (!grid_sync(a, B_PRODUCT, bst)) break;
@@ -1276,13 +1134,14 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           if (li[t] < 0) continue;
           const float ri = rs[slot_of(a.S, t)];
           zs[li[t]] = zk[t];
-          ff_acc_prod(rz, ri, zk[t]);
-          ff_acc_prod(rr, ri, ri);
+          const float rs_i = sr * ri;
+          ff_acc_prod(rz, rs_i, sz * zk[t]);
+          ff_acc_prod(rr, rs_i, rs_i);
         }
       }
       levels_z();  // published first: the stores drain while the sums are formed
       {
-        const ff bs = block_sum2_ff(rz, rr, red);
+        const ff bs = block_sum2_ff<NT>(rz, rr, red);
         if (tid == 0 || tid == 16) store_part(a.part + (size_t)P2 + 2 * blk + (tid >> 4), bs);
       }
       grid_arrive(a, B_STEP, bst);
@@ -1291,7 +1150,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       if (tid < 32) {
         ff trz, trr;
         warp_total2_ff(a.part + P2, G, trz, trr);
-        if (tid == 0) fast_step(sF, sS, a, it, trz, trr);
+        if (tid == 0) fast_step(sF, sS, blockIdx.x == 0 ? a.hist : nullptr, it, trz, trr);
       }
       __syncthreads();
       if (!sS.need_update) continue;
@@ -1363,14 +1222,14 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         for (int t = 0; t < RPT; ++t) {
           if (li[t] < 0) continue;
           zs[li[t]] = zk[t];
-          ff_acc_prod(rz_u, rs[slot_of(a.S, t)], zk[t]);
+          ff_acc_prod(rz_u, sr * rs[slot_of(a.S, t)], sz * zk[t]);
         }
       }
       {
-        const ff b1 = block_sum2_ff(rz_u, ff{0.f, 0.f}, red);
+        const ff b1 = block_sum2_ff<NT>(rz_u, ff{0.f, 0.f}, red);
         const double b2 = block_sum<NT>(rr_u, red64);
         if (tid == 0) {
-          a.part[(size_t)P2 + 2 * blk] = ff_double(b1);
+          a.part[(size_t)P2 + 2 * blk] = ff_double(b1) * (1.0 / ((double)sr * (double)sz));
           a.part[(size_t)P2 + 2 * blk + 1] = b2;
         }
       }
@@ -1383,7 +1242,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         if (tid == 0) {
           fast_to(sF, sS);
           update_scalars(sS, a, t2.x, t2.y);
-          if (blockIdx.x == 0) store_part(a.hist + sS.iter, ff_from_double(t2.y));
+          if (blockIdx.x == 0) store_hist(a.hist + sS.iter, sF, t2.y);
           fast_from(sF, sS);
         }
       }
@@ -1397,6 +1256,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   if (blockIdx.x == 0 && tid == 0) {
     fast_to(sF, sS);
     sS.skip_update = 1;
+    sS.fast = sF;
     *a.S_ = sS;
   }
 }
@@ -1525,12 +1385,14 @@ __global__ void __launch_bounds__(NT) k_build_items(int g, int n_per, int n,
   }
 }
 
-// The roots of the |r|^2 that the resident form left in hist[1 .. iter].
-__global__ void k_hist_sqrt(const MixedState* st, double* __restrict__ hist) {
+// The roots of the |sr r|^2 that a form with float-pair sums left in
+// hist[1 .. iter].
+__global__ void k_hist_roots(const MixedState* st, double* __restrict__ hist) {
+  const double ur = 1.0 / (double)st->fast.sr;
   for (int i = 1 + blockIdx.x * blockDim.x + threadIdx.x; i <= st->iter;
        i += gridDim.x * blockDim.x) {
     const float2 v = reinterpret_cast<const float2*>(hist)[i];
-    hist[i] = sqrt((double)v.x + (double)v.y);
+    hist[i] = sqrt((double)v.x + (double)v.y) * ur;
   }
 }
 
@@ -1733,11 +1595,13 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   DS_CUDA(cudaLaunchCooperativeKernel(pick(resident), dim3(grid), dim3(NT), args,
                                       resident ? res_bytes : 0, st));
   DS_CHECK_LAUNCH();
-  if (resident) {
-    k_hist_sqrt<<<std::min(64, (max_iter + 255) / 256), 256, 0, st>>>(f.state.p, f.hist.p);
-    DS_CHECK_LAUNCH();
-  }
+  if (resident) launch_hist_roots(f.state.p, f.hist.p, max_iter, st);
   return true;
+}
+
+void launch_hist_roots(const MixedState* s, double* hist, int max_iter, cudaStream_t st) {
+  k_hist_roots<<<std::max(1, std::min(64, (max_iter + 255) / 256)), 256, 0, st>>>(s, hist);
+  DS_CHECK_LAUNCH();
 }
 
 int persistent_error(ds_operator* op, cudaStream_t st) {
