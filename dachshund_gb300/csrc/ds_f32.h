@@ -45,6 +45,12 @@ struct F32Args {
   double* alpha_out;
   double* den_out;
   const int* skip_flag;
+  // the mixed form's fused direction step (launch_pair_f32_dir): v = z + beta p,
+  // p the one of the two buffers that the iteration count names, the new p to the
+  // other
+  const float* z;
+  float* p[2];
+  struct MixedState* mst;
   // EPI_MAP
   const int* row_perm;
   double* out64;
@@ -57,6 +63,7 @@ struct F32Args {
 };
 
 void launch_pair_f32(int formula, int epi, const F32Args& a, cudaStream_t st);
+void launch_pair_f32_dir(int formula, const F32Args& a, cudaStream_t st);
 
 // The inner product q = A32 p with the pair exponents on the tensor cores
 // (pair_tc.cu): EXPANDED formula, EPI_PRODUCT epilogue, a.err set.
