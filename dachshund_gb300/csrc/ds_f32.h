@@ -139,6 +139,9 @@ struct MixedState {
   FastState fast;     // the scalars of the forms that sum in float pairs
 };
 
+bool mixed_pairs_usable(ds_operator* op, struct OpF32& f);
+void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, cudaStream_t st);
+
 // The |r| history of a form that sums in float pairs, from what it left there.
 void launch_hist_roots(const MixedState* s, double* hist, int max_iter, cudaStream_t st);
 
@@ -151,6 +154,14 @@ struct OpF32 {
   bool pairs_built = false;
   DevBuf<float> rowf, colw, ediag, pdiag;
   DevBuf<float> p, q, r, z;         // FP32 iteration vectors (sorted, padded)
+  // the persistent form of the pair kernels' iteration (persist_pairs.cu)
+  bool rounds_built = false;
+  DevBuf<int4> rounds;
+  DevBuf<int> round_ptr, warp_ptr;
+  DevBuf<float4> round_sums, xiw;
+  DevBuf<float2> zp;
+  DevBuf<double> round_part;
+  DevBuf<unsigned int> round_bar;
   DevBuf<float> r2;                 // second r buffer of the band preconditioner
   DevBuf<MixedState> state;
   HostBuf<MixedState> h_state;      // pinned staging of the state

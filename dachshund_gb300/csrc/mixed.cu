@@ -900,6 +900,24 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   bool persisted = false;
   if (use_sg && pc && op->iter_form == DS_ITER_AUTO && !op->ctx->prof.enabled && max_iter > 0)
     persisted = run_mixed_persistent(op, f, pc, sv, X, rbuf[0], max_iter, st);
+  // The Jacobi form with the pair kernels: one cooperative launch of the iterations
+  // up to each update (persist_pairs.cu).
+  const bool rounds = fast && op->iter_form == DS_ITER_AUTO && !op->ctx->prof.enabled &&
+                      max_iter > 0 && mixed_pairs_usable(op, f);
+  if (rounds) {
+    persisted = true;
+    do {
+      launch_mixed_pairs(op, f, X, max_iter, st);
+      fast_update();
+      unsigned int bar[2];
+      DS_CUDA(cudaMemcpyAsync(bar, f.round_bar.p, sizeof(bar), cudaMemcpyDeviceToHost, st));
+      DS_CUDA(cudaMemcpyAsync(f.h_state.p, S, sizeof(h), cudaMemcpyDeviceToHost, st));
+      DS_CUDA(cudaStreamSynchronize(st));
+      if (bar[1])
+        throw Error{DS_ERR_TIMEOUT, "persistent mixed solve: a grid barrier wait timed out "
+                                    "(barrier " + std::to_string(bar[1]) + ")"};
+    } while (!f.h_state.p->done);
+  }
   if (!persisted)  // the host polls the done flag (the persistent launch needs no events)
     for (auto& e : evs) DS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   if (!persisted && !op->ctx->prof.enabled && !use_tc && max_iter > 0) {
@@ -959,7 +977,7 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
 
-  if (persisted) {
+  if (persisted && !rounds) {
     const int code = persistent_error(op, st);
     if (code)
       throw Error{DS_ERR_TIMEOUT, "persistent mixed solve: a grid barrier wait timed out "
