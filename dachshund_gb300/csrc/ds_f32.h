@@ -45,12 +45,6 @@ struct F32Args {
   double* alpha_out;
   double* den_out;
   const int* skip_flag;
-  // the mixed form's fused direction step (launch_pair_f32_dir): v = z + beta p,
-  // p the one of the two buffers that the iteration count names, the new p to the
-  // other
-  const float* z;
-  float* p[2];
-  struct MixedState* mst;
   // EPI_MAP
   const int* row_perm;
   double* out64;
@@ -63,7 +57,6 @@ struct F32Args {
 };
 
 void launch_pair_f32(int formula, int epi, const F32Args& a, cudaStream_t st);
-void launch_pair_f32_dir(int formula, const F32Args& a, cudaStream_t st);
 
 // The inner product q = A32 p with the pair exponents on the tensor cores
 // (pair_tc.cu): EXPANDED formula, EPI_PRODUCT epilogue, a.err set.
@@ -139,8 +132,11 @@ struct MixedState {
   FastState fast;     // the scalars of the forms that sum in float pairs
 };
 
-bool mixed_pairs_usable(ds_operator* op, struct OpF32& f);
-void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, cudaStream_t st);
+// The persistent form of the Jacobi iteration (persist_pairs.cu); g: the grid of
+// the per-kernel form's vector kernels, whose sums' order it keeps.
+bool mixed_pairs_usable(ds_operator* op, struct OpF32& f, int g);
+void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, int g,
+                        cudaStream_t st);
 
 // The |r| history of a form that sums in float pairs, from what it left there.
 void launch_hist_roots(const MixedState* s, double* hist, int max_iter, cudaStream_t st);
@@ -160,7 +156,7 @@ struct OpF32 {
   DevBuf<int> round_ptr, warp_ptr;
   DevBuf<float4> round_sums, xiw;
   DevBuf<float2> zp;
-  DevBuf<double> round_part;
+  DevBuf<double> round_part;  // p.q per tile, then r.z and |r|^2 per row block
   DevBuf<unsigned int> round_bar;
   DevBuf<float> r2;                 // second r buffer of the band preconditioner
   DevBuf<MixedState> state;

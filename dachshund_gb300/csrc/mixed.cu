@@ -25,7 +25,6 @@
 #include "ds_learned.h"
 #include "ds_skewer.h"
 #include "ds_mixed_dev.cuh"
-#include "ds_ffsum.cuh"
 #include "ds_ops.h"
 
 namespace ds {
@@ -244,59 +243,7 @@ __global__ void __launch_bounds__(VB) k_mx_update(int n, MixedState* st, double*
   }
 }
 
-// K2 of the Jacobi form with the pair kernels: the same with the direction read
-// from the buffer that the iteration count names, sums and scalars in float pairs
-// (the state's `fast`), no FP64 but the iterate's update.  Latency bound (44,237
-// pixels, 173 CTAs): 11.1 -> 7.9 us, FP64's ~400 clocks per dependent instruction
-// having been in its sums, division and root; with the direction step in the
-// product and the update's kernels every eighth iteration the solve takes 12.6 ->
-// 11.4 ms.  Vectors and x are those of FP64 sums to 4e-13.
-__global__ void __launch_bounds__(VB) k_mx_step(int n, MixedState* st, double* __restrict__ x,
-                                                float* __restrict__ r, float* __restrict__ z,
-                                                const float* __restrict__ p0,
-                                                const float* __restrict__ p1,
-                                                const float* __restrict__ q,
-                                                const float* __restrict__ pd,
-                                                double* __restrict__ part, double* hist) {
-  if (st->done || st->need_update) return;
-  __shared__ float2 red[2 * (VB / 32)];
-  const ff al = st->fast.alpha;
-  const float alpha = al.h;
-  const double alpha_d = (double)al.h + (double)al.l;
-  const float* p = st->iter & 1 ? p0 : p1;  // the new one
-  const float sr = st->fast.sr, sz = st->fast.sz;
-  ff rz{0.f, 0.f}, rr{0.f, 0.f};
-  for (int i = blockIdx.x * VB + threadIdx.x; i < n; i += gridDim.x * VB) {
-    const float ri = fmaf(-alpha, q[i], r[i]);
-    const float zi = ri / pd[i];
-    r[i] = ri;
-    z[i] = zi;
-    x[i] = fma(alpha_d, (double)p[i], x[i]);
-    const float rs = sr * ri;
-    ff_acc_prod(rz, rs, sz * zi);
-    ff_acc_prod(rr, rs, rs);
-  }
-  const ff s = block_sum2_ff<VB>(rz, rr, red);
-  if (threadIdx.x == 0 || threadIdx.x == 16)
-    store_part(part + 2 * blockIdx.x + (threadIdx.x >> 4), s);
-  if (last_block_arrive(&st->counter[1]) && threadIdx.x < 32) {
-    ff trz, trr;
-    warp_total2_ff(part, gridDim.x, trz, trr);
-    if (threadIdx.x == 0) {
-      fast_step(st->fast, *st, hist, st->iter + 1, trz, trr);
-      st->skip_update = !st->need_update;
-      st->counter[1] = 0;
-    }
-  }
-}
-
-__global__ void k_mx_fast(MixedState* st) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) fast_init(st->fast, *st);
-}
-
 // K6: r = float(r64); z = r / pd; r.z and |r64| (FP64); stop or continue.
-// FAST: between k_mx_step's iterations (float-pair scalars and history).
-template <bool FAST>
 __global__ void __launch_bounds__(VB) k_mx_replace(int n, MixedState* st,
                                                    const double* __restrict__ r64,
                                                    float* __restrict__ r, float* __restrict__ z,
@@ -326,13 +273,9 @@ __global__ void __launch_bounds__(VB) k_mx_replace(int n, MixedState* st,
     const double trr = reduce_partials<VB>(part, gridDim.x, 2, 1, red);
     if (threadIdx.x == 0) {
       const double rt = sqrt(trr);
-      if (FAST) fast_to(st->fast, *st);
       st->rtrue = rt;
       htrue[++st->n_updates] = rt;
-      if (FAST)
-        store_hist(hist + st->iter, st->fast, trr);
-      else
-        hist[st->iter] = rt;
+      hist[st->iter] = rt;
       if (rt <= st->tol_norm_b) {
         st->done = 1;
         st->converged = 1;
@@ -347,7 +290,6 @@ __global__ void __launch_bounds__(VB) k_mx_replace(int n, MixedState* st,
       st->need_update = 0;
       st->skip_update = 1;
       st->counter[1] = 0;
-      if (FAST) fast_from(st->fast, *st);
     }
   }
 }
@@ -815,38 +757,7 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   // r.z, update test), K5 (FP64-accurate residual when an update is due),
   // K6 (the update), K7 (p = z + beta p).  Every kernel returns at once once
   // the solve is done, so iterations launched past the end change nothing.
-  // The Jacobi form with the CUDA-core pair kernels has two kernels per iteration
-  // (the product with the direction step and alpha, k_mx_step), which return at
-  // once while an update is due; the residual and its replacement follow every
-  // eighth iteration: per iteration their two empty launches cost 5 us.
-  const bool fast = !pc && !op->sgrid && !use_tc;
-  if (fast) {
-    f.r2.alloc(np);  // the direction's second buffer
-    prod.z = f.z.p;
-    prod.p[0] = f.p.p;
-    prod.p[1] = f.r2.p;
-    prod.mst = S;
-    k_mx_fast<<<1, 32, 0, st>>>(S);
-    DS_CHECK_LAUNCH();
-  }
-  auto fast_iteration = [&] {
-    launch_pair_f32_dir(f.formula, prod, st);
-    k_mx_step<<<g, VB, 0, st>>>(np, S, X, f.r.p, f.z.p, prod.p[0], prod.p[1], f.q.p, PD,
-                                op->partial.p, f.hist.p);
-    DS_CHECK_LAUNCH();
-  };
-  auto fast_update = [&] {
-    outer_residual(upd);
-    k_mx_replace<true><<<g, VB, 0, st>>>(np, S, op->r.p, f.r.p, f.z.p, PD, op->partial.p,
-                                         f.hist.p, f.htrue.p);
-    DS_CHECK_LAUNCH();
-  };
   auto iteration = [&](int it) {
-    if (fast) {
-      fast_iteration();
-      if (op->ctx->prof.enabled || it % 8 == 0) fast_update();
-      return;
-    }
     if (use_sg)
       // K7 of the previous iteration (p = z + beta p) is done by K1 here
       skewer_product_f32(op, sv, f.p.p, prod.out, prod.counter, prod.num, prod.alpha_out,
@@ -875,8 +786,8 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
       a.part = pc_part;
       pc_iter<1>(a, st);
     } else {
-      k_mx_replace<false><<<g, VB, 0, st>>>(np, S, op->r.p, f.r.p, f.z.p, PD, op->partial.p,
-                                            f.hist.p, f.htrue.p);            // K6
+      k_mx_replace<<<g, VB, 0, st>>>(np, S, op->r.p, f.r.p, f.z.p, PD, op->partial.p, f.hist.p,
+                                     f.htrue.p);                             // K6
       DS_CHECK_LAUNCH();
     }
     if (!use_sg) {
@@ -901,14 +812,17 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   if (use_sg && pc && op->iter_form == DS_ITER_AUTO && !op->ctx->prof.enabled && max_iter > 0)
     persisted = run_mixed_persistent(op, f, pc, sv, X, rbuf[0], max_iter, st);
   // The Jacobi form with the pair kernels: one cooperative launch of the iterations
-  // up to each update (persist_pairs.cu).
-  const bool rounds = fast && op->iter_form == DS_ITER_AUTO && !op->ctx->prof.enabled &&
-                      max_iter > 0 && mixed_pairs_usable(op, f);
+  // up to each update (persist_pairs.cu), the same values as the kernels below.
+  const bool rounds = !op->sgrid && !pc && !use_tc && op->iter_form == DS_ITER_AUTO &&
+                      !op->ctx->prof.enabled && max_iter > 0 && mixed_pairs_usable(op, f, g);
   if (rounds) {
     persisted = true;
     do {
-      launch_mixed_pairs(op, f, X, max_iter, st);
-      fast_update();
+      launch_mixed_pairs(op, f, X, max_iter, g, st);
+      outer_residual(upd);
+      k_mx_replace<<<g, VB, 0, st>>>(np, S, op->r.p, f.r.p, f.z.p, PD, op->partial.p, f.hist.p,
+                                     f.htrue.p);
+      DS_CHECK_LAUNCH();
       unsigned int bar[2];
       DS_CUDA(cudaMemcpyAsync(bar, f.round_bar.p, sizeof(bar), cudaMemcpyDeviceToHost, st));
       DS_CUDA(cudaMemcpyAsync(f.h_state.p, S, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -965,7 +879,6 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
     cudaGraphExecDestroy(gexec);
   }
   if (use_sg) skewer_x_to_sorted(op, X, op->x.p, st);
-  if (fast) launch_hist_roots(S, f.hist.p, max_iter, st);
   DS_CUDA(cudaEventRecord(ev1, st));
   DS_CUDA(cudaMemcpyAsync(f.h_state.p, S, sizeof(h), cudaMemcpyDeviceToHost, st));
   DS_CUDA(cudaStreamSynchronize(st));

@@ -28,7 +28,6 @@
 // rows are summed in FP64 at the end.
 #include "ds_device.cuh"
 #include "ds_f32.h"
-#include "ds_ffsum.cuh"
 #include "ds_pair_f32.cuh"
 
 namespace ds {
@@ -42,14 +41,9 @@ namespace {
 constexpr int F32_MIN_CTAS = 5;
 constexpr int F32_QU = 2;  // groups of four columns unrolled
 
-// DIR: the mixed form's Jacobi iteration, v = p = z + beta p formed as the columns
-// are loaded (and stored by the row tiles), p.q and alpha in float pairs.
-template <int FORMULA, int EPI, bool DOT, bool DIR>
+template <int FORMULA, int EPI, bool DOT>
 __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
   if (a.skip_flag && *a.skip_flag) return;
-  if (DIR && (a.mst->done || a.mst->need_update)) return;
-  const float beta = DIR ? a.mst->fast.beta : 0.f;
-  const float* pold = DIR ? a.p[a.mst->iter & 1] : nullptr;
   // per warp: two staged work items (64 columns) and their column values
   __shared__ float4 sc[2 * TILE];
   __shared__ float4 su4[2 * TILE / 4];
@@ -83,10 +77,7 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
     const float4 o = a.corig[ct], q = a.cxi[j];
     c.o = make_float3(o.x, o.y, o.z);
     c.q = make_float3(q.x, q.y, q.z);
-    if (DIR)
-      c.u = a.colw[j] * fmaf(beta, pold[j], a.z[j]);
-    else
-      c.u = (EPI == EPI_PRODUCT) ? a.colw[j] * a.v[j] : a.v[j];
+    c.u = (EPI == EPI_PRODUCT) ? a.colw[j] * a.v[j] : a.v[j];
     c.m = it & 15u;
   };
   constexpr unsigned full = 0xffffffffu;
@@ -154,36 +145,9 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
   sred[warp][lane + 64] = s2 - c2;
   sred[warp][lane + 96] = s3 - c3;
   __syncthreads();
-  const int i = base + tid;
-  if (DIR) {
-    // the four slices in a float pair (exact but for the pair's last bits), then
-    // as below
-    ff a01, a23;
-    two_sum(sred[0][tid], sred[1][tid], a01.h, a01.l);
-    two_sum(sred[2][tid], sred[3][tid], a23.h, a23.l);
-    const float p = fmaf(beta, pold[i], a.z[i]);
-    const float q = fmaf(a.rowf[i], ff_add(a01, a23).h, a.ediag[i] * p);
-    a.out[i] = q;
-    a.p[(a.mst->iter & 1) ^ 1][i] = p;
-    __shared__ float2 red2[2 * (TILE / 32)];
-    ff dq{0.f, 0.f};
-    ff_acc_prod(dq, a.mst->fast.sz * p, a.mst->fast.sr * q);
-    const ff s = block_sum2_ff<TILE>(dq, ff{0.f, 0.f}, red2);
-    if (tid == 0) store_part(a.dot_partial + t, s);
-    if (last_block_arrive(a.counter)) {
-      if (warp == 0) {
-        const ff pq = warp_total_ff(a.dot_partial, gridDim.x);
-        if (tid == 0) {
-          a.mst->fast.pq = pq;
-          a.mst->fast.alpha = ff_div(a.mst->fast.rz, pq);
-          *a.counter = 0;
-        }
-      }
-    }
-    return;
-  }
   const double sum = ((double)sred[0][tid] + (double)sred[1][tid]) +
                      ((double)sred[2][tid] + (double)sred[3][tid]);
+  const int i = base + tid;
   if (EPI == EPI_PRODUCT) {
     // q_i = wl_i var_s 2^-a_i sum_j e_ij wr_j v_j + e_i v_i
     const float q = fmaf(a.rowf[i], (float)sum, a.ediag[i] * a.vrow[i]);
@@ -212,11 +176,11 @@ void launch_formula(int epi, const F32Args& a, cudaStream_t st) {
   const dim3 grid(a.n_row_tiles), block(TILE);
   if (epi == EPI_PRODUCT) {
     if (a.dot_partial)
-      k_pair_f32<FORMULA, EPI_PRODUCT, true, false><<<grid, block, 0, st>>>(a);
+      k_pair_f32<FORMULA, EPI_PRODUCT, true><<<grid, block, 0, st>>>(a);
     else
-      k_pair_f32<FORMULA, EPI_PRODUCT, false, false><<<grid, block, 0, st>>>(a);
+      k_pair_f32<FORMULA, EPI_PRODUCT, false><<<grid, block, 0, st>>>(a);
   } else if (epi == EPI_MAP) {
-    k_pair_f32<FORMULA, EPI_MAP, false, false><<<grid, block, 0, st>>>(a);
+    k_pair_f32<FORMULA, EPI_MAP, false><<<grid, block, 0, st>>>(a);
   } else {
     throw Error{DS_ERR_ARG, "bad FP32 pair epilogue"};
   }
@@ -224,46 +188,23 @@ void launch_formula(int epi, const F32Args& a, cudaStream_t st) {
 
 }  // namespace
 
-static void launch_profiled(const F32Args& a0, int kind, cudaStream_t st,
-                            void (*launch)(const F32Args&, int, int, cudaStream_t), int formula,
-                            int epi) {
+void launch_pair_f32(int formula, int epi, const F32Args& a0, cudaStream_t st) {
   if (a0.n_row_tiles <= 0) return;
   F32Args a = a0;
   cudaEvent_t ev = nullptr;
+  const int kind = epi == EPI_MAP ? 2 : 1;
   if (a.prof && a.prof->enabled) {
     a.prof_pairs = a.prof->d_pairs + kind;
     a.prof->begin(st, &ev);
   } else {
     a.prof_pairs = nullptr;
   }
-  launch(a, formula, epi, st);
+  if (formula == F32_EXPANDED)
+    launch_formula<F32_EXPANDED>(epi, a, st);
+  else
+    launch_formula<F32_DIRECT>(epi, a, st);
   DS_CHECK_LAUNCH();
   if (ev) a.prof->end(st, ev, kind);
-}
-
-void launch_pair_f32(int formula, int epi, const F32Args& a, cudaStream_t st) {
-  launch_profiled(
-      a, epi == EPI_MAP ? 2 : 1, st,
-      [](const F32Args& b, int fm, int ep, cudaStream_t s) {
-        if (fm == F32_EXPANDED)
-          launch_formula<F32_EXPANDED>(ep, b, s);
-        else
-          launch_formula<F32_DIRECT>(ep, b, s);
-      },
-      formula, epi);
-}
-
-// q = A32 p with p = z + beta p, alpha = rz / p.q (a.z, a.p, a.mst set).
-void launch_pair_f32_dir(int formula, const F32Args& a, cudaStream_t st) {
-  launch_profiled(
-      a, 1, st,
-      [](const F32Args& b, int fm, int, cudaStream_t s) {
-        if (fm == F32_EXPANDED)
-          k_pair_f32<F32_EXPANDED, EPI_PRODUCT, true, true><<<b.n_row_tiles, TILE, 0, s>>>(b);
-        else
-          k_pair_f32<F32_DIRECT, EPI_PRODUCT, true, true><<<b.n_row_tiles, TILE, 0, s>>>(b);
-      },
-      formula, EPI_PRODUCT);
 }
 
 }  // namespace ds

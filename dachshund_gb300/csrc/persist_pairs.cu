@@ -13,9 +13,13 @@
 // per-kernel form's order: every FP32 value is that form's bit for bit.
 //
 // Phases, a grid barrier after each: the rounds (p = z + beta p formed as the
-// columns are loaded); the rows' q and p.q; x, r, z and the sums r.z and |r|^2.
-// The four warps of a quad own a tile's rows (one per thread, r, z, p, x in
-// registers) and fold one slice each.
+// columns are loaded); the rows' q and p.q; r, z (then x) and the sums r.z, |r|^2.
+// Rows are owned by thread, and the FP64 sums are the per-kernel form's to the last
+// bit, order included: a Krylov recurrence in FP32 amplifies any flipped rounding to
+// a few percent of the final residual, which an FP32 evaluation of the map from x
+// shows.  A dependent FP64 addition takes 66 clocks with up to 4 warps of an SM at
+// it but 300 with 16, so one warp adds up what the shuffles of 4 or 8 would (tree).
+//
 #include <algorithm>
 #include <string>
 
@@ -23,7 +27,8 @@
 
 #include "ds_device.cuh"
 #include "ds_f32.h"
-#include "ds_ffsum.cuh"
+#include "ds_ff.cuh"
+#include "ds_mixed_dev.cuh"
 #include "ds_ops.h"
 #include "ds_pair_f32.cuh"
 
@@ -32,16 +37,17 @@ namespace ds {
 namespace {
 
 constexpr int NT = 512, W = NT / 32, QUADS = NT / TILE;
-constexpr int MAX_PER = 8;  // tiles per quad at most (160 KB of rows)
+constexpr int VB = 256;     // rows per block of the vector sums
+constexpr int MAX_PER = 8;  // rows per thread at most (160 KB)
 
-// A thread's row of a tile (registers are the rounds'); `per` of them per thread.
+// A thread's row (registers are the rounds'); `per` of them per thread.
 struct Row {
   double x;
   float p, r, z, q, pd, rowf, ed, pad;
 };
 
 struct Args {
-  int n_tiles, max_iter, per;
+  int n_tiles, max_iter, per, g;
   const int4* rounds;         // tile, item, item or 0, -
   const int* round_ptr;       // first round of (tile, slice); 4 n_tiles + 1
   const int* warp_ptr;        // first round of a warp; W G + 1
@@ -52,7 +58,7 @@ struct Args {
   float *p, *r, *z;
   float2* zp;                 // (z, p) of every pixel
   float4* sums;               // rounds x 32: lane l's rows l, l + 32, l + 64, l + 96
-  double* part;               // p.q per CTA, then (from P2) r.z and |r|^2
+  double* part;               // p.q per tile, then r.z and |r|^2 per row block
   MixedState* st;
   double* hist;
   unsigned int* bar;          // arrivals, error
@@ -62,13 +68,46 @@ struct Args {
 struct Shared {
   float4 sc[W * 64];   // per warp: 64 staged columns
   float4 su4[W * 16];  // and their values
-  FastState f;
+  double sum[2][NT];   // sums in progress (r.z and |r|^2)
   MixedState s;
-  ff alpha;
-  float2 red[2 * W];
   float slice[QUADS][4][TILE];
   int ok;
 };
+
+// The sum that NW warps' block_sum would form of v[0 .. 32 NW), by one warp (valid in
+// lane 0; v is overwritten).
+template <int NW>
+__device__ __forceinline__ double tree(double* v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+#pragma unroll
+    for (int e = lane; e < NW * s; e += 32) {
+      const int i = (e / s) * 32 + e % s;
+      v[i] += v[i + s];
+    }
+    __syncwarp();
+  }
+  double t = 0.0;
+  if (lane == 0)
+#pragma unroll
+    for (int w = 0; w < NW; ++w) t += v[32 * w];
+  return t;
+}
+
+// float(((s0 + s1) + s2 + s3) in FP64) of the slices' sums: in FP32 with the exact
+// errors, in FP64 where these leave the rounding open (one row in millions).
+__device__ __forceinline__ float slice_total(float s0, float s1, float s2, float s3) {
+  float a, ea, b, eb, s, es;
+  two_sum(s0, s1, a, ea);
+  two_sum(s2, s3, b, eb);
+  two_sum(a, b, s, es);
+  const float rest = __fadd_rn(__fadd_rn(ea, eb), es);
+  const float open = 4e-7f * (fabsf(ea) + fabsf(eb) + fabsf(es));
+  const float lo = __fadd_rn(s, __fadd_rn(rest, -open)), hi = __fadd_rn(s, __fadd_rn(rest, open));
+  if (lo == hi) return lo;
+  return (float)(((double)s0 + (double)s1) + ((double)s2 + (double)s3));
+}
 
 __device__ __forceinline__ void grid_arrive(const Args& a) {
   __syncthreads();
@@ -106,16 +145,16 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   Shared& sm = *reinterpret_cast<Shared*>(smraw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = gridDim.x;
-  const int P2 = (G + 1) & ~1;  // the pair partials start 16-byte aligned
   constexpr unsigned full = 0xffffffffu;
-  if (tid == 0) {
-    sm.s = *a.st;
-    sm.f = sm.s.fast;
-  }
-  // the quad's tiles and the thread's row of each
+  if (tid == 0) sm.s = *a.st;
+  // Half a CTA owns the rows of block vb of the vector sums, rows vb VB + ... and
+  // every g VB rows on; a quad of warps a tile of them.
   const int quad = tid / TILE, row = tid % TILE, slice = row >> 5;
+  const int vb = (int)blockIdx.x + G * (tid / VB);
   Row* const rows = reinterpret_cast<Row*>(smraw + sizeof(Shared)) + tid;  // k-th at k NT
-  auto tile_of = [&](int k) { return (k * QUADS + quad) * G + (int)blockIdx.x; };
+  auto tile_of = [&](int k) {
+    return vb < a.g ? 2 * (vb + k * a.g) + (quad & 1) : a.n_tiles;
+  };
   for (int k = 0; k < a.per; ++k) {
     const int t = tile_of(k);
     if (t >= a.n_tiles) break;
@@ -167,7 +206,7 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
   if (!grid_wait(a, sm, epoch)) return;
   while (!sm.s.need_update && !sm.s.done && sm.s.iter < a.max_iter) {
     const int it = sm.s.iter + 1;
-    const float beta = sm.f.beta;
+    const float beta = (float)sm.s.beta;
     // ---- the rounds
     if (nr > 0) {
       Col ca, cb;
@@ -210,7 +249,6 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
     grid_arrive(a);
     if (!grid_wait(a, sm, epoch)) return;
     // ---- the rows: q = A32 p and p.q
-    ff dq{0.f, 0.f};
     for (int k = 0; k < a.per; ++k) {
       const int t = tile_of(k);
       const bool own = t < a.n_tiles;
@@ -241,59 +279,90 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
       }
       __syncthreads();
       if (own) {
-        // the four slices in a float pair (exact but for the pair's last bits)
         Row& w = rows[k * NT];
-        ff a01, a23;
-        two_sum(sl[0][row], sl[1][row], a01.h, a01.l);
-        two_sum(sl[2][row], sl[3][row], a23.h, a23.l);
         const float p = fmaf(beta, w.p, w.z);
-        const float q = fmaf(w.rowf, ff_add(a01, a23).h, w.ed * p);
+        const float sum = slice_total(sl[0][row], sl[1][row], sl[2][row], sl[3][row]);
+        const float q = fmaf(w.rowf, sum, w.ed * p);
         w.p = p;
         w.q = q;
-        ff_acc_prod(dq, sm.f.sz * p, sm.f.sr * q);
+        sm.sum[0][tid] = (double)p * (double)q;
       }
-      if (k + 1 < a.per) __syncthreads();  // sl is written again
-    }
-    {
-      const ff bs = block_sum2_ff<NT>(dq, ff{0.f, 0.f}, sm.red);
-      if (tid == 0) store_part(a.part + blockIdx.x, bs);
+      __syncthreads();
+      if (own && slice == 0) {
+        const double d = tree<TILE / 32>(sm.sum[0] + tid - lane);
+        if (lane == 0) a.part[t] = d;
+      }
     }
     grid_arrive(a);
     if (!grid_wait(a, sm, epoch)) return;
     // ---- the step
+    if (warp < TILE / 32) {
+      double v = 0.0;
+      for (int k = tid; k < a.n_tiles; k += TILE) v += __ldcg(a.part + k);
+      sm.sum[0][tid] = v;
+    }
+    __syncthreads();
     if (warp == 0) {
-      const ff pq = warp_total_ff(a.part, G);
+      const double pq = tree<TILE / 32>(sm.sum[0]);
       if (lane == 0) {
-        sm.f.pq = pq;
-        sm.f.alpha = sm.alpha = ff_div(sm.f.rz, pq);
+        sm.s.pq = pq;
+        sm.s.alpha = sm.s.rz / pq;
       }
     }
     __syncthreads();
-    ff rz{0.f, 0.f}, rr{0.f, 0.f};
-    const ff al = sm.alpha;
-    const double alpha_d = (double)al.h + (double)al.l;
-    for (int k = 0; k < a.per && tile_of(k) < a.n_tiles; ++k) {
-      Row& w = rows[k * NT];
-      const float p = w.p, r = fmaf(-al.h, w.q, w.r), z = r / w.pd;
-      a.zp[tile_of(k) * TILE + row] = make_float2(z, p);
-      w.r = r;
-      w.z = z;
-      w.x = fma(alpha_d, (double)p, w.x);
-      const float rs = sm.f.sr * r;
-      ff_acc_prod(rz, rs, sm.f.sz * z);
-      ff_acc_prod(rr, rs, rs);
-    }
+    const double alpha_d = sm.s.alpha;
+    const float alpha = (float)alpha_d;
     {
-      const ff bs = block_sum2_ff<NT>(rz, rr, sm.red);
-      if (tid == 0 || tid == 16)
-        store_part(a.part + (size_t)P2 + 2 * blockIdx.x + (tid >> 4), bs);
+      double rz = 0.0, rr = 0.0;
+      for (int k = 0; k < a.per && tile_of(k) < a.n_tiles; ++k) {
+        Row& w = rows[k * NT];
+        const float r = fmaf(-alpha, w.q, w.r), z = r / w.pd;
+        a.zp[tile_of(k) * TILE + row] = make_float2(z, w.p);
+        w.r = r;
+        w.z = z;
+        rz = fma((double)r, (double)z, rz);
+        rr = fma((double)r, (double)r, rr);
+      }
+      sm.sum[0][tid] = rz;
+      sm.sum[1][tid] = rr;
+    }
+    __syncthreads();
+    if ((warp & 3) == 0) {  // warps 0, 4: r.z, |r|^2 of the first half; 8, 12: the second
+      const int h = (warp >> 2) & 1;
+      const double d = tree<VB / 32>(sm.sum[h] + (warp >> 3) * VB);
+      const int b = (int)blockIdx.x + G * (warp >> 3);
+      if (lane == 0 && b < a.g) a.part[a.n_tiles + 2 * b + h] = d;
     }
     grid_arrive(a);
+    for (int k = 0; k < a.per && tile_of(k) < a.n_tiles; ++k) {
+      Row& w = rows[k * NT];
+      w.x = fma(alpha_d, (double)w.p, w.x);
+    }
     if (!grid_wait(a, sm, epoch)) return;
+    {
+      const int h = tid / VB;  // r.z by the first half of the CTA, |r|^2 by the second
+      double v = 0.0;
+      for (int k = tid % VB; k < a.g; k += VB) v += __ldcg(a.part + a.n_tiles + 2 * k + h);
+      sm.sum[h][tid % VB] = v;
+    }
+    __syncthreads();
     if (warp == 0) {
-      ff trz, trr;
-      warp_total2_ff(a.part + P2, G, trz, trr);
-      if (lane == 0) fast_step(sm.f, sm.s, blockIdx.x == 0 ? a.hist : nullptr, it, trz, trr);
+      const double trz = tree<VB / 32>(sm.sum[0]);
+      if (lane == 0) {
+        sm.s.rz_old = sm.s.rz;
+        sm.s.rz = trz;
+        sm.s.beta = trz / sm.s.rz_old;
+      }
+    } else if (warp == VB / 32) {
+      const double trr = tree<VB / 32>(sm.sum[1]);
+      if (lane == 0) {
+        sm.s.rnorm = sqrt(trr);
+        sm.s.iter = it;
+        if (blockIdx.x == 0) a.hist[it] = sm.s.rnorm;
+        sm.s.rmax = fmax(sm.s.rmax, sm.s.rnorm);
+        sm.s.need_update = update_due(&sm.s, it) ? 1 : 0;
+        sm.s.skip_update = !sm.s.need_update;
+      }
     }
     __syncthreads();
   }
@@ -306,8 +375,6 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
     a.z[g] = w.z;
   }
   if (blockIdx.x == 0 && tid == 0) {
-    sm.s.fast = sm.f;
-    sm.s.skip_update = !sm.s.need_update;
     *a.st = sm.s;
   }
 }
@@ -375,10 +442,10 @@ static const void* kernel_of(const OpF32& f) {
 
 // Prepares the launches (kept with the operator's FP32 pair list); false when the
 // rows do not fit, and the per-kernel form runs.
-bool mixed_pairs_usable(ds_operator* op, OpF32& f) {
+bool mixed_pairs_usable(ds_operator* op, OpF32& f, int g) {
   const int nt = op->pix.n_tiles, G = op->ctx->num_sms;
-  const int per = (nt + QUADS * G - 1) / (QUADS * G);
-  if (per > MAX_PER) return false;
+  const int per = (op->pix.n_pad + g * VB - 1) / (g * VB);
+  if (per > MAX_PER || g > 2 * G) return false;
   const size_t smem = sizeof(Shared) + (size_t)per * NT * sizeof(Row);
   const void* fn = kernel_of(f);
   DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -422,7 +489,7 @@ bool mixed_pairs_usable(ds_operator* op, OpF32& f) {
                                                      f.xiw.p);
   DS_CHECK_LAUNCH();
   f.zp.alloc(op->pix.n_pad);
-  f.round_part.alloc((size_t)3 * G + 2);
+  f.round_part.alloc((size_t)nt + 4 * G);
   f.round_bar.alloc(2);
   f.rounds_built = true;
   return true;
@@ -430,13 +497,15 @@ bool mixed_pairs_usable(ds_operator* op, OpF32& f) {
 
 // Iterations up to the next reliable update (or the cap) from x, p, r, z and the
 // state.
-void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, cudaStream_t st) {
+void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, int g,
+                        cudaStream_t st) {
   DS_CUDA(cudaMemsetAsync(f.round_bar.p, 0, f.round_bar.bytes(), st));
   const int G = op->ctx->num_sms;
   Args a{};
   a.n_tiles = op->pix.n_tiles;
   a.max_iter = max_iter;
-  a.per = (a.n_tiles + QUADS * G - 1) / (QUADS * G);
+  a.g = g;
+  a.per = (op->pix.n_pad + g * VB - 1) / (g * VB);
   a.rounds = f.rounds.p;
   a.round_ptr = f.round_ptr.p;
   a.warp_ptr = f.warp_ptr.p;
