@@ -20,6 +20,11 @@
 // shows.  A dependent FP64 addition takes 66 clocks with up to 4 warps of an SM at
 // it but 300 with 16, so one warp adds up what the shuffles of 4 or 8 would (tree).
 //
+// Measured (solve and map on a kept operator, per-kernel form -> here): 2,048 pixels
+// 5.0 -> 3.1 ms, 10,240 7.4 -> 4.2, 24,000 8.9 -> 5.9, 44,237 12.2 -> 9.0.  An
+// iteration of 44,237 pixels takes 68,000 clocks: 36,000 the rounds (18,000 if the
+// exponentials alone bound them), 9,000 their uneven ends and barrier, 11,000 the rows,
+// 12,000 the step and its sums.
 #include <algorithm>
 #include <string>
 
@@ -38,7 +43,10 @@ namespace {
 
 constexpr int NT = 512, W = NT / 32, QUADS = NT / TILE;
 constexpr int VB = 256;     // rows per block of the vector sums
-constexpr int MAX_PER = 8;  // rows per thread at most (160 KB)
+// Rows per thread at most: 155,648 pixels.  131,072 pixels take 26.4 ms per solve in
+// the per-kernel form and 22.6 here; 262,144 take 44.4 and 45.8 (the tiles then fill
+// the SMs evenly without it, and the rounds' sums leave L2).
+constexpr int MAX_PER = 2;
 
 // A thread's row (registers are the rounds'); `per` of them per thread.
 struct Row {
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(NT, 1) k_mixed_pairs(Args a) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
         for (int h = 0; h < 2; ++h)
-          accumulate_item<FORMULA, 2>((masks >> (4 * h)) & 15u, scw + 32 * h,
+          accumulate_item<FORMULA, 8>((masks >> (4 * h)) & 15u, scw + 32 * h,
                                       sm.su4 + warp * 16 + 8 * h, R, acc);
         a.sums[(size_t)(r0 + k) * 32 + lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
       }
