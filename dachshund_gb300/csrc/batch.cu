@@ -35,6 +35,7 @@
 #include "ds_tc.cuh"
 #include "ds_device.cuh"
 #include "ds_ff.cuh"
+#include "ds_ffsum.cuh"
 
 namespace ds {
 namespace {
@@ -439,7 +440,7 @@ __global__ void k_ff_points_batch(int n_pad, const double* __restrict__ x,
   }
 }
 
-// ---- per-(pixel, RHS) vector kernels: one CTA per tile, thread = RHS ------------
+// ---- per-(pixel, RHS) vector kernels: one CTA per tile, thread = (RHS, row group) --
 
 struct BV {
   int R;
@@ -450,42 +451,97 @@ struct BV {
   const int* done;      // per (chunk, RHS)
   const double* alpha;  // per (chunk, RHS)
   const double* beta;
+  const float2* scale;  // (sr, sz) per (chunk, RHS), powers of two
 };
 
-// MODE 0 (U2): x_c += alpha p; r -= alpha q; z = r / pd.
+// Row groups of the vector and scalar kernels' CTAs: (RHS, group) threads, a
+// power of two of groups.
+inline int row_groups(int rt, int threads) {
+  int g = 1;
+  while (2 * g <= 8 && 2 * g * rt <= threads) g *= 2;
+  return g;
+}
+
+// U2: x_c += alpha p; r -= alpha q; z = r / pd.  Partials per (tile, RHS): r.z at
+// [t][r], |r|^2 at [t][R + r].  Bound by its 28 bytes per (pixel, RHS); the sums are
+// float pairs (exact products, compensated sums, of vectors scaled to about 1): in
+// FP64 they took 5 instructions of 16 clocks per element and the kernel 160 us at
+// 207,104 pixels x 64 instead of 73.
+__global__ void k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
+                          float* __restrict__ z, const float* __restrict__ p,
+                          const float* __restrict__ q, const float* __restrict__ pd,
+                          double* __restrict__ part) {
+  extern __shared__ float4 sums[];  // (group, RHS): r.z and |r|^2
+  const int t = blockIdx.x;
+  const int c = v.tile_chunk[t];
+  const int r = threadIdx.x, g = threadIdx.y, G = blockDim.y;
+  const int cr = c * v.R + r;
+  if (v.chunk_done[c]) return;
+  const bool on = r < v.R && !v.done[cr] && !v.hold[cr];
+  ff rz{0.f, 0.f}, rs{0.f, 0.f};
+  float2 sc = make_float2(1.f, 1.f);
+  if (on) {
+    const float alpha = (float)v.alpha[cr];
+    sc = v.scale[cr];
+    constexpr int U = 4;  // rows in flight
+    for (int k = g * (TILE / G); k < (g + 1) * (TILE / G); k += U) {
+      const int i = t * TILE + k;
+      const size_t ir = (size_t)i * v.R + r;
+      float pv[U], xv[U], qv[U], rv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        pv[u] = p[ir + (size_t)u * v.R];
+        xv[u] = xc[ir + (size_t)u * v.R];
+        qv[u] = q[ir + (size_t)u * v.R];
+        rv[u] = rr[ir + (size_t)u * v.R];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float ri = fmaf(-alpha, qv[u], rv[u]), zi = ri / pd[i + u];
+        xc[ir + (size_t)u * v.R] = fmaf(alpha, pv[u], xv[u]);
+        rr[ir + (size_t)u * v.R] = ri;
+        z[ir + (size_t)u * v.R] = zi;
+        const float rsc = sc.x * ri;
+        ff_acc_prod(rz, rsc, sc.y * zi);
+        ff_acc_prod(rs, rsc, rsc);
+      }
+    }
+  }
+  sums[g * blockDim.x + r] = make_float4(rz.h, rz.l, rs.h, rs.l);
+  __syncthreads();
+  if (g == 0 && on) {
+    for (int k = 1; k < G; ++k) {
+      const float4 o = sums[k * blockDim.x + r];
+      rz = ff_add(rz, ff{o.x, o.y});
+      rs = ff_add(rs, ff{o.z, o.w});
+    }
+    const double ur = (double)(1.f / sc.x), uz = (double)(1.f / sc.y);
+    part[(size_t)t * 2 * v.R + r] = ff_double(rz) * ur * uz;
+    part[(size_t)t * 2 * v.R + v.R + r] = ff_double(rs) * ur * ur;
+  }
+}
+
 // MODE 1 (U6): r = float(r64); z = r / pd (update pending).
 // MODE 2 (init): r = float(b); z = r / pd; p = z; x_c = 0.
-// Partials per (tile, RHS): r.z at [t][r], |r|^2 at [t][R + r] (FP64 r64 in
-// modes 1 and 2).
+// Partials as k_bu_step's, in FP64 of the FP64 r64.
 template <int MODE>
 __global__ void k_bu_update(BV v, float* __restrict__ xc, float* __restrict__ rr,
                             float* __restrict__ z, float* __restrict__ p,
-                            const float* __restrict__ q, const float* __restrict__ pd,
-                            const double* __restrict__ r64, double* __restrict__ part) {
+                            const float* __restrict__ pd, const double* __restrict__ r64,
+                            double* __restrict__ part) {
   const int t = blockIdx.x;
   const int c = v.tile_chunk[t];
   const int r = threadIdx.x;
   if (r >= v.R) return;
   const int cr = c * v.R + r;
-  if (MODE != 2 && (v.chunk_done[c] || v.done[cr])) return;
-  if (MODE == 0 && v.hold[cr]) return;
-  if (MODE == 1 && !v.need[cr]) return;
-  const float alpha = MODE == 0 ? (float)v.alpha[cr] : 0.f;
+  if (MODE == 1 && (v.chunk_done[c] || v.done[cr] || !v.need[cr])) return;
   double srz = 0.0, srr = 0.0;
   for (int k = 0; k < TILE; ++k) {
     const int i = t * TILE + k;
     const size_t ir = (size_t)i * v.R + r;
-    float ri;
-    double rd;
-    if (MODE == 0) {
-      xc[ir] = fmaf(alpha, p[ir], xc[ir]);
-      ri = fmaf(-alpha, q[ir], rr[ir]);
-      rd = (double)ri;
-    } else {
-      rd = r64[ir];
-      ri = (float)rd;
-      if (MODE == 2) xc[ir] = 0.f;
-    }
+    const double rd = r64[ir];
+    const float ri = (float)rd;
+    if (MODE == 2) xc[ir] = 0.f;
     rr[ir] = ri;
     const float zi = ri / pd[i];
     z[ir] = zi;
@@ -531,14 +587,32 @@ __global__ void k_bu_fold(BV v, double* __restrict__ x, float* __restrict__ xc) 
   }
 }
 
-// ---- per-(chunk, RHS) scalar kernels: one CTA per chunk, thread = RHS ------------
+// ---- per-(chunk, RHS) scalar kernels: one CTA per chunk, thread = (RHS, tile group) --
 
-// Sum over the chunk's tiles in tile order (deterministic).
-__device__ __forceinline__ double chunk_sum(const double* part, int t0, int t1, int stride,
-                                            int off) {
-  double s = 0.0;
-  for (int t = t0; t < t1; ++t) s += part[(size_t)t * stride + off];
-  return s;
+// Sums over the chunk's tiles: N of them per RHS at part[t stride + off + n step],
+// the groups' tiles in order, then the groups (a fixed order; valid in group 0).  One
+// thread per sum is a chain of dependent loads and FP64 additions over the chunk's
+// tiles: 41 us for 67 tiles instead of 10.
+template <int N>
+__device__ __forceinline__ void chunk_sums(double (&s)[N], const double* part, int t0, int t1,
+                                           int stride, int off, int step, bool on,
+                                           double* sm /* N x threads */) {
+  const int g = threadIdx.y, G = blockDim.y, nt = blockDim.x * G;
+  const int me = g * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int n = 0; n < N; ++n) s[n] = 0.0;
+  if (on)
+#pragma unroll 4
+    for (int t = t0 + g; t < t1; t += G)
+#pragma unroll
+      for (int n = 0; n < N; ++n) s[n] += part[(size_t)t * stride + off + n * step];
+#pragma unroll
+  for (int n = 0; n < N; ++n) sm[n * nt + me] = s[n];
+  __syncthreads();
+  if (g == 0)
+    for (int k = 1; k < G; ++k)
+#pragma unroll
+      for (int n = 0; n < N; ++n) s[n] += sm[n * nt + k * blockDim.x + threadIdx.x];
 }
 
 // MODE 0 (S1): alpha = r.z / p.q.
@@ -559,22 +633,36 @@ template <int MODE>
 __global__ void k_bs(BatchState s, const double* __restrict__ part) {
   const int c = blockIdx.x, r = threadIdx.x;
   const int R = s.R;
+  extern __shared__ double bs_sm[];
   __shared__ int any_active, any_iterating;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     any_active = 0;
     any_iterating = 0;
   }
   __syncthreads();
   if (MODE != 3 && s.chunk_done[c]) return;  // uniform over the block
   const int cr = c * R + r;
-  if (r < R) {
+  const bool head = threadIdx.y == 0;
+  double sum[2] = {0.0, 0.0};  // p.q, or r.z and |r|^2
+  if (MODE != 4) {
     const int t0 = s.chunk_tile0[c], t1 = s.chunk_tile0[c + 1];
     if (MODE == 0) {
-      if (!s.done[cr] && !s.hold[cr]) s.alpha[cr] = s.rz[cr] / chunk_sum(part, t0, t1, R, r);
+      double one[1];
+      chunk_sums(one, part, t0, t1, R, r, 0, r < R && !s.done[cr] && !s.hold[cr], bs_sm);
+      sum[0] = one[0];
+    } else {
+      const bool on = r < R && (MODE == 1   ? !s.done[cr] && !s.hold[cr]
+                                : MODE == 2 ? !s.done[cr] && s.need[cr]
+                                            : true);
+      chunk_sums(sum, part, t0, t1, 2 * R, r, R, on, bs_sm);
+    }
+  }
+  if (r < R && head) {
+    if (MODE == 0) {
+      if (!s.done[cr] && !s.hold[cr]) s.alpha[cr] = s.rz[cr] / sum[0];
     } else if (MODE == 1) {
       if (!s.done[cr] && !s.hold[cr]) {
-        const double rz = chunk_sum(part, t0, t1, 2 * R, r);
-        const double rn = sqrt(chunk_sum(part, t0, t1, 2 * R, R + r));
+        const double rz = sum[0], rn = sqrt(sum[1]);
         s.rz_old[cr] = s.rz[cr];
         s.rz[cr] = rz;
         const int it = ++s.iter[cr];
@@ -596,8 +684,7 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
       }
     } else if (MODE == 2) {
       if (!s.done[cr] && s.need[cr]) {
-        const double rz = chunk_sum(part, t0, t1, 2 * R, r);
-        const double rt = sqrt(chunk_sum(part, t0, t1, 2 * R, R + r));
+        const double rz = sum[0], rt = sqrt(sum[1]);
         s.rtrue[cr] = rt;
         ++s.n_updates[cr];
         s.hold[cr] = 0;
@@ -616,8 +703,10 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
         }
       }
     } else if (MODE == 3) {
-      const double rz = chunk_sum(part, t0, t1, 2 * R, r);
-      const double rt = sqrt(chunk_sum(part, t0, t1, 2 * R, R + r));
+      const double rz = sum[0], rt = sqrt(sum[1]);
+      const int er = rt > 0.0 ? ilogb(rt) : 0, ez = rz > 0.0 ? ilogb(rz) : 0;
+      s.scale[cr] = make_float2(pow2_neg(er), pow2_neg(ez - er));
+      s.beta[cr] = 0.0;
       s.rz[cr] = rz;
       s.rtrue[cr] = s.rmax[cr] = s.rbest[cr] = rt;
       s.it_best[cr] = 0;
@@ -642,8 +731,8 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
   }
   __syncthreads();
   const int update = MODE == 1 && any_active && !any_iterating;
-  if (update && r < R && !s.done[cr]) s.need[cr] = 1;
-  if (threadIdx.x == 0) {
+  if (update && head && r < R && !s.done[cr]) s.need[cr] = 1;
+  if (threadIdx.x == 0 && head) {
     if (MODE == 1) s.chunk_update[c] = update;
     if (MODE == 4) s.chunk_update[c] = 0;
     if ((MODE == 2 || MODE == 3) && !any_active) {
@@ -981,6 +1070,7 @@ void batch_build(ds_batch* B, const double* d_rec, const int* sizes) {
                   &B->s_rtrue,
                   &B->s_norm_b, &B->s_tol_norm_b})
     v->alloc(CR);
+  B->s_scale.alloc(CR);
   for (auto* v : {&B->s_iter, &B->s_n_updates, &B->s_need, &B->s_hold, &B->s_done,
                   &B->s_converged, &B->s_it_best, &B->s_stalled})
     v->alloc(CR);
@@ -1072,6 +1162,7 @@ BatchState state_args(ds_batch* B, const ds_mixed_params& mp) {
   s.rz_old = B->s_rz_old.p;
   s.alpha = B->s_alpha.p;
   s.beta = B->s_beta.p;
+  s.scale = B->s_scale.p;
   s.rmax = B->s_rmax.p;
   s.rbest = B->s_rbest.p;
   s.it_best = B->s_it_best.p;
@@ -1100,10 +1191,17 @@ std::map<std::tuple<int, int, int>, std::pair<int, int>> g_tune;
 // q = A32 p over every chunk not done, with the chosen variant.  With the
 // context's profiling on, the launch is timed (kind 1) and its pair x RHS
 // products counted.
-void batch_mv(ds_batch* B, cudaStream_t st) {
+// dir: p = z + beta p first (tensor-core variant), where the RHS iterates.
+void batch_mv(ds_batch* B, cudaStream_t st, bool dir) {
   if (B->variant == BV_TENSOR && !B->panel.p)
     B->panel.alloc(batch_tc_panel_elems(B->n_tiles, B->n_rhs));
   BatchF32Args a = mv_args(B);
+  if (dir) {
+    a.dir_z = B->zz.p;
+    a.dir_beta = B->s_beta.p;
+    a.dir_hold = B->s_hold.p;
+    a.dir_done = B->s_done.p;
+  }
   Profiler& pr = B->ctx->prof;
   cudaEvent_t ev = nullptr;
   if (pr.enabled) {
@@ -1268,41 +1366,50 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
 
   const BatchState S = state_args(B, mp);
   const BV v{R,           B->tile_chunk.p, B->chunk_done.p, B->s_need.p,
-             B->s_hold.p, B->s_done.p,     B->s_alpha.p,     B->s_beta.p};
+             B->s_hold.p, B->s_done.p,     B->s_alpha.p,     B->s_beta.p,  B->s_scale.p};
   const int RT = ((R + 31) / 32) * 32;
+  const dim3 rows(RT, row_groups(RT, 512)), tiles(RT, row_groups(RT, 1024));
+  const size_t row_smem = (size_t)rows.x * rows.y * sizeof(float4);
+  const size_t bs_smem = (size_t)tiles.x * tiles.y * 2 * sizeof(double);
+  // The tensor-core matvec forms p = z + beta p as it packs p (launch_batch_mv_tc).
+  const bool fused_dir = B->variant == BV_TENSOR;
 
   cudaEvent_t ev0, ev1;
   DS_CUDA(cudaEventCreate(&ev0));
   DS_CUDA(cudaEventCreate(&ev1));
   DS_CUDA(cudaEventRecord(ev0, st));
   // r = b (x0 = 0), z = M^-1 r, p = z, x_c = 0
-  k_bu_update<2><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, nullptr, B->pd32.p,
-                                   B->bv.p, B->part.p);
+  k_bu_update<2><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->pd32.p, B->bv.p,
+                                   B->part.p);
   DS_CHECK_LAUNCH();
-  k_bs<3><<<C, RT, 0, st>>>(S, B->part.p);
+  k_bs<3><<<C, tiles, bs_smem, st>>>(S, B->part.p);
   DS_CHECK_LAUNCH();
 
   auto issue_iteration = [&] {
-    batch_mv(B, st);                                                                 // MV
-    k_bs<0><<<C, RT, 0, st>>>(S, B->part.p);                                         // S1
+    batch_mv(B, st, fused_dir);                                                      // MV
+    k_bs<0><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S1
     DS_CHECK_LAUNCH();
-    k_bu_update<0><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->q.p,
-                                     B->pd32.p, nullptr, B->part.p);                 // U2
+    k_bu_step<<<T, rows, row_smem, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->q.p,
+                                         B->pd32.p, B->part.p);                      // U2
     DS_CHECK_LAUNCH();
-    k_bs<1><<<C, RT, 0, st>>>(S, B->part.p);                                         // S2
+    k_bs<1><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S2
     DS_CHECK_LAUNCH();
-    k_bu_dir<0><<<T, RT, 0, st>>>(v, B->zz.p, B->p.p);                               // U3
-    DS_CHECK_LAUNCH();
+    if (!fused_dir) {
+      k_bu_dir<0><<<T, RT, 0, st>>>(v, B->zz.p, B->p.p);                             // U3
+      DS_CHECK_LAUNCH();
+    }
     k_bu_fold<<<T, RT, 0, st>>>(v, B->xv.p, B->xc.p);                                // U4
     DS_CHECK_LAUNCH();
     batch_resid(B, st);                                                              // R5
-    k_bu_update<1><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, nullptr,
-                                     B->pd32.p, B->r64.p, B->part.p);                // U6
+    k_bu_update<1><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->pd32.p,
+                                     B->r64.p, B->part.p);                           // U6
     DS_CHECK_LAUNCH();
-    k_bs<2><<<C, RT, 0, st>>>(S, B->part.p);                                         // S6
+    k_bs<2><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S6
     DS_CHECK_LAUNCH();
-    k_bu_dir<1><<<T, RT, 0, st>>>(v, B->zz.p, B->p.p);                               // U7
-    DS_CHECK_LAUNCH();
+    if (!fused_dir) {
+      k_bu_dir<1><<<T, RT, 0, st>>>(v, B->zz.p, B->p.p);                             // U7
+      DS_CHECK_LAUNCH();
+    }
     k_bs<4><<<C, RT, 0, st>>>(S, B->part.p);                                         // S7
     DS_CHECK_LAUNCH();
   };

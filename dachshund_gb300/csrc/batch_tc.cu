@@ -497,9 +497,14 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
 // 2 NB-row operand [u_hi | u_lo] in the core-matrix layout above.  One
 // thread per (tile, group of 8 pixels, RHS): 8 strided reads (coalesced over
 // the RHS index), one 16-byte store per part.
+// With a.dir_z the direction step p = z + beta p of every RHS that iterates (neither
+// done nor held) comes first: a pass over p and z of its own took 65 us of the 81 of
+// both at 207,104 pixels x 64.
 template <int NB>
-__global__ void k_pack_panels(int n_tiles, int R, const float* __restrict__ p,
-                              const float* __restrict__ colw, __nv_bfloat16* __restrict__ panel) {
+__global__ void k_pack_panels(BatchF32Args a) {
+  const int n_tiles = a.n_row_tiles, R = a.n_rhs;
+  const float* __restrict__ colw = a.colw;
+  __nv_bfloat16* __restrict__ panel = reinterpret_cast<__nv_bfloat16*>(a.panel);
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)n_tiles * (TILE / 8) * R;
   if (k >= total) return;
@@ -510,7 +515,24 @@ __global__ void k_pack_panels(int n_tiles, int R, const float* __restrict__ p,
   const int j0 = ct * TILE + kg * 8;
   float u[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) u[e] = colw[j0 + e] * p[(size_t)(j0 + e) * R + r];
+  for (int e = 0; e < 8; ++e) u[e] = a.p[(size_t)(j0 + e) * R + r];
+  if (a.dir_z) {
+    const int c = a.tile_chunk[ct], cr = c * R + r;
+    if (a.chunk_done[c]) return;  // its panels are not read
+    if (!a.dir_done[cr] && !a.dir_hold[cr]) {
+      const float beta = (float)a.dir_beta[cr];
+      float z[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) z[e] = a.dir_z[(size_t)(j0 + e) * R + r];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        u[e] = fmaf(beta, u[e], z[e]);
+        a.p[(size_t)(j0 + e) * R + r] = u[e];
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) u[e] *= colw[j0 + e];
   uint4 vh, vl;
   split2(u[0], u[1], vh.x, vl.x);
   split2(u[2], u[3], vh.y, vl.y);
@@ -534,8 +556,7 @@ void tc_launch(const BatchF32Args& a, cudaStream_t st) {
     attr = true;
   }
   const size_t packs = (size_t)a.n_row_tiles * (TILE / 8) * a.n_rhs;
-  k_pack_panels<NB><<<(unsigned)((packs + 255) / 256), 256, 0, st>>>(
-      a.n_row_tiles, a.n_rhs, a.p, a.colw, reinterpret_cast<__nv_bfloat16*>(a.panel));
+  k_pack_panels<NB><<<(unsigned)((packs + 255) / 256), 256, 0, st>>>(a);
   DS_CHECK_LAUNCH();
   static int sms = 0;  // queried on the first (uncaptured) launch
   if (!sms) {

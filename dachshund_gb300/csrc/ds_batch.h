@@ -38,8 +38,11 @@ struct BatchF32Args {
   const float* rowf;
   const float* ediag;
   int n_rhs;
-  const float* p;  // [pixel][n_rhs]
+  float* p;        // [pixel][n_rhs]
   float* q;
+  const float* dir_z;  // tensor-core variant: p = z + beta p first (null: p as it is)
+  const double* dir_beta;
+  const int *dir_hold, *dir_done;
   double* part;    // per (tile, RHS): p . q over the tile
   unsigned int* work;  // work-queue counter of the persistent launch
   unsigned long long* prof_pairs;  // profiling: pair x RHS products evaluated
@@ -85,6 +88,7 @@ struct BatchState {
   double* rz_old;
   double* alpha;
   double* beta;
+  float2* scale;  // (sr, sz): powers of two that bring the first |r| and r.z near 1
   double* rmax;
   double* rbest;    // smallest recurrence |r| since the last halving
   double* rtrue;
@@ -140,6 +144,7 @@ struct ds_batch {
   ds::FFData ffd;  // float-pair coordinates of the FP64-accurate residual
   ds::DevBuf<float> p, q, rr, zz, xc;
   ds::DevBuf<double> part;
+  ds::DevBuf<float2> s_scale;
   ds::DevBuf<double> s_rz, s_rz_old, s_alpha, s_beta, s_rmax, s_rbest, s_rtrue, s_norm_b,
       s_tol_norm_b;
   ds::DevBuf<int> s_iter, s_n_updates, s_need, s_hold, s_done, s_converged, s_it_best, s_stalled;
@@ -159,7 +164,7 @@ struct ds_batch {
 namespace ds {
 bool batch_rb_supported(int R, int rb);
 void batch_build(ds_batch* B, const double* d_rec, const int* sizes);
-void batch_mv(ds_batch* B, cudaStream_t st);
+void batch_mv(ds_batch* B, cudaStream_t st, bool dir = false);
 void batch_resid(ds_batch* B, cudaStream_t st);
 void batch_autotune(ds_batch* B, bool force, double* best_ms_out);
 void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_dev, double* x_dev,
