@@ -218,18 +218,16 @@ __global__ void __launch_bounds__(TILE) k_batch_mv_f32(BatchF32Args a) {
 
 // u = var_s wl x of the chunks with an update pending, as an unevaluated
 // float pair (hi = float(u), lo = float(u - hi)): about 48 significant bits.
-__global__ void k_resid_prep(int R, double var_s, const int* __restrict__ tile_chunk,
-                             const int* __restrict__ chunk_done,
-                             const int* __restrict__ chunk_update, const double* __restrict__ wl,
+__global__ void k_resid_prep(int R, double var_s, UpdateList up, const double* __restrict__ wl,
                              const double* __restrict__ xv, float2* __restrict__ uu) {
-  const int t = blockIdx.x;
-  const int c = tile_chunk[t];
-  if (chunk_done[c] || !chunk_update[c]) return;
-  const size_t base = (size_t)t * TILE * R;
-  for (int k = threadIdx.x; k < TILE * R; k += blockDim.x) {
-    const double u = var_s * wl[t * TILE + k / R] * xv[base + k];
-    const float h = __double2float_rn(u);
-    uu[base + k] = make_float2(h, __double2float_rn(u - (double)h));
+  for (int k = blockIdx.x; k < *up.n; k += gridDim.x) {
+    const int t = up.tile[k];
+    const size_t base = (size_t)t * TILE * R;
+    for (int i = threadIdx.x; i < TILE * R; i += blockDim.x) {
+      const double u = var_s * wl[t * TILE + i / R] * xv[base + i];
+      const float h = __double2float_rn(u);
+      uu[base + i] = make_float2(h, __double2float_rn(u - (double)h));
+    }
   }
 }
 
@@ -292,6 +290,12 @@ __device__ __forceinline__ float ex2_br(float x) {
 // right-hand sides per item the extra accumulators spill a few registers at
 // 3 CTAs per SM; that still beats 2 CTAs per SM without spills and 16
 // right-hand sides per item on the 512-chunk batch.)
+//
+// The chunks' updates mostly come one chunk at a time (24 chunks: 87 launches with
+// work), whose tiles alone leave most of the chip idle and take as long as the
+// longest item: then an item's tile pairs go in up to 8 segments, whose float-pair
+// sums the last to finish adds up in segment order.  24 chunks x 64: 102 -> RESID_MS ms
+// a solve.
 template <int RB, bool FF>
 __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
   constexpr int ROWF = 2 * RB + 4;  // floats per staged column
@@ -313,25 +317,28 @@ __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
   const float cut = (float)kc.exact_cut;
   const int R = a.n_rhs;
   const int nblk = R / RB;
-  const int n_items = a.n_row_tiles * nblk;
+  const int n_whole = *a.up.n * nblk;
+  int S = 1;  // segments
+  while (S < 8 && 2 * S * n_whole <= a.seg_cap) S *= 2;
+  const int n_items = n_whole * S;
   float* suw = ustage + warp * SUBTILE * ROWF;
   for (;;) {
     __syncthreads();
-    if (tid == 0) s_item = (int)atomicAdd(a.work, 1u);
+    if (tid == 0) s_item = n_items ? (int)atomicAdd(a.work, 1u) : 0;
     __syncthreads();
     const int item = s_item;
     if (item >= n_items) break;
-    const int t = a.row_order[item / nblk];
-    const int r0 = (item % nblk) * RB;
-    const int c = a.tile_chunk[t];
-    if (a.chunk_done[c] || !a.chunk_update[c]) continue;
+    const int whole = item / S, seg = item % S;
+    const int t = a.up.tile[whole / nblk];
+    const int r0 = (whole % nblk) * RB;
     const int i = t * TILE + tid;
     const double xi = a.x[i], yi = a.y[i], zi = a.z[i];
     float ah[RB], al[RB], af[RB];
 #pragma unroll
     for (int r = 0; r < RB; ++r) ah[r] = al[r] = af[r] = 0.f;
     unsigned n_sub = 0;
-    for (int p = a.row_ptr[t]; p < a.row_ptr[t + 1]; ++p) {
+    const int q0 = a.row_ptr[t], nq = a.row_ptr[t + 1] - q0;
+    for (int p = q0 + nq * seg / S; p < q0 + nq * (seg + 1) / S; ++p) {
       const unsigned m = (a.mask[p] >> (4 * warp)) & 0xFu;
       if (!m) continue;
       n_sub += __popc(m);
@@ -360,10 +367,16 @@ __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
           sw[warp][1][lane] = a.y[j];
           sw[warp][2][lane] = a.z[j];
         }
-        const float2* src = a.uu + (size_t)j * R + r0;
-        float2* dst = reinterpret_cast<float2*>(suw + lane * ROWF);
-#pragma unroll
-        for (int r = 0; r < RB; ++r) dst[r] = src[r];
+        // u: the high parts of a column's RHS, then the low ones (far columns read
+        // the high parts alone)
+        const float2* src = a.uu + (size_t)(j - lane) * R + r0;
+#pragma unroll 8
+        for (int k = lane; k < SUBTILE * RB; k += 32) {
+          const float2 u = src[(size_t)(k / RB) * R + k % RB];
+          float* dst = suw + (k / RB) * ROWF + k % RB;
+          dst[0] = u.x;
+          dst[RB] = u.y;
+        }
         __syncwarp();
 #pragma unroll 1
         for (int jj = 0; jj < SUBTILE; ++jj) {
@@ -376,9 +389,9 @@ __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
             if (__all_sync(0xffffffffu, d2f >= BR_FAR)) {
               if (d2f < cut) {
                 const float g = ex2_br(-d2f * BR_LOG2E);
-                const float2* u2 = reinterpret_cast<const float2*>(suw + jj * ROWF);
+                const float* uh = suw + jj * ROWF;
 #pragma unroll
-                for (int r = 0; r < RB; ++r) af[r] = fmaf(g, u2[r].x, af[r]);
+                for (int r = 0; r < RB; ++r) af[r] = fmaf(g, uh[r], af[r]);
               }
               continue;
             }
@@ -396,17 +409,44 @@ __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
             const double g = arg < kc.exact_cut ? exp_neg_f64(arg, tf) : 0.0;
             split_f64(g, sh, sl);
           }
-          const float2* u2 = reinterpret_cast<const float2*>(suw + jj * ROWF);
+          const float* uh = suw + jj * ROWF;
 #pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            const float2 u = u2[r];
-            df_mac(ah[r], al[r], sh, sl, u.x, u.y);
-          }
+          for (int r = 0; r < RB; ++r) df_mac(ah[r], al[r], sh, sl, uh[r], uh[RB + r]);
         }
       }
     }
     if (a.prof_pairs && lane == 0)
       atomicAdd(a.prof_pairs, (unsigned long long)n_sub * SUBTILE * SUBTILE * RB);
+    if (S > 1) {
+      // (segment, RHS): ah, al, af of the 128 rows
+      float* out = a.seg + ((size_t)item * RB * 3) * TILE + tid;
+#pragma unroll
+      for (int r = 0; r < RB; ++r) {
+        out[(3 * r + 0) * TILE] = ah[r];
+        out[(3 * r + 1) * TILE] = al[r];
+        out[(3 * r + 2) * TILE] = af[r];
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_item = atomicAdd(a.seg_count + whole, 1u) == (unsigned)S - 1;
+      __syncthreads();
+      if (!s_item) continue;
+      __threadfence();
+      if (tid == 0) a.seg_count[whole] = 0;
+#pragma unroll
+      for (int r = 0; r < RB; ++r) ah[r] = al[r] = af[r] = 0.f;
+      for (int s = 0; s < S; ++s) {
+        const float* in = a.seg + ((size_t)(whole * S + s) * RB * 3) * TILE + tid;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          float h, e;
+          two_sum(ah[r], __ldcg(in + (3 * r + 0) * TILE), h, e);
+          ah[r] = h;
+          al[r] = __fadd_rn(al[r], __fadd_rn(e, __ldcg(in + (3 * r + 1) * TILE)));
+          af[r] += __ldcg(in + (3 * r + 2) * TILE);
+        }
+      }
+    }
     const double wli = a.wl[i], ei = a.e[i];
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
@@ -521,36 +561,51 @@ __global__ void k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
   }
 }
 
-// MODE 1 (U6): r = float(r64); z = r / pd (update pending).
-// MODE 2 (init): r = float(b); z = r / pd; p = z; x_c = 0.
+// MODE 1 (U6): r = float(r64); z = r / pd, of the tiles with an update pending.
+// MODE 2 (init): r = float(b); z = r / pd; p = z; x_c = 0, of all tiles.
 // Partials as k_bu_step's, in FP64 of the FP64 r64.
 template <int MODE>
-__global__ void k_bu_update(BV v, float* __restrict__ xc, float* __restrict__ rr,
-                            float* __restrict__ z, float* __restrict__ p,
-                            const float* __restrict__ pd, const double* __restrict__ r64,
-                            double* __restrict__ part) {
-  const int t = blockIdx.x;
-  const int c = v.tile_chunk[t];
-  const int r = threadIdx.x;
-  if (r >= v.R) return;
-  const int cr = c * v.R + r;
-  if (MODE == 1 && (v.chunk_done[c] || v.done[cr] || !v.need[cr])) return;
-  double srz = 0.0, srr = 0.0;
-  for (int k = 0; k < TILE; ++k) {
-    const int i = t * TILE + k;
-    const size_t ir = (size_t)i * v.R + r;
-    const double rd = r64[ir];
-    const float ri = (float)rd;
-    if (MODE == 2) xc[ir] = 0.f;
-    rr[ir] = ri;
-    const float zi = ri / pd[i];
-    z[ir] = zi;
-    if (MODE == 2) p[ir] = zi;
-    srz = fma((double)ri, (double)zi, srz);
-    srr = fma(rd, rd, srr);
+__global__ void k_bu_update(BV v, UpdateList up, int n_tiles, float* __restrict__ xc,
+                            float* __restrict__ rr, float* __restrict__ z,
+                            float* __restrict__ p, const float* __restrict__ pd,
+                            const double* __restrict__ r64, double* __restrict__ part) {
+  extern __shared__ double2 sums64[];  // (group, RHS): r.z and |r|^2
+  const int n = MODE == 1 ? *up.n : n_tiles;
+  const int r = threadIdx.x, g = threadIdx.y, G = blockDim.y;
+  for (int e = blockIdx.x; e < n; e += gridDim.x) {
+    const int t = MODE == 1 ? up.tile[e] : e;
+    const int cr = v.tile_chunk[t] * v.R + r;
+    const bool on = r < v.R && (MODE == 2 || (!v.done[cr] && v.need[cr]));
+    double srz = 0.0, srr = 0.0;
+    if (on) {
+#pragma unroll 4
+      for (int k = g * (TILE / G); k < (g + 1) * (TILE / G); ++k) {
+        const int i = t * TILE + k;
+        const size_t ir = (size_t)i * v.R + r;
+        const double rd = r64[ir];
+        const float ri = (float)rd;
+        if (MODE == 2) xc[ir] = 0.f;
+        rr[ir] = ri;
+        const float zi = ri / pd[i];
+        z[ir] = zi;
+        if (MODE == 2) p[ir] = zi;
+        srz = fma((double)ri, (double)zi, srz);
+        srr = fma(rd, rd, srr);
+      }
+    }
+    __syncthreads();
+    sums64[g * blockDim.x + r] = make_double2(srz, srr);
+    __syncthreads();
+    if (g == 0 && on) {
+      for (int k = 1; k < G; ++k) {
+        const double2 o = sums64[k * blockDim.x + r];
+        srz += o.x;
+        srr += o.y;
+      }
+      part[(size_t)t * 2 * v.R + r] = srz;
+      part[(size_t)t * 2 * v.R + v.R + r] = srr;
+    }
   }
-  part[(size_t)t * 2 * v.R + r] = srz;
-  part[(size_t)t * 2 * v.R + v.R + r] = srr;
 }
 
 // MODE 0 (U3): p = z + beta p where the RHS iterates on (not held).
@@ -573,17 +628,18 @@ __global__ void k_bu_dir(BV v, const float* __restrict__ z, float* __restrict__ 
 }
 
 // U4: x += x_c (FP64); x_c = 0 where an update is pending.
-__global__ void k_bu_fold(BV v, double* __restrict__ x, float* __restrict__ xc) {
-  const int t = blockIdx.x;
-  const int c = v.tile_chunk[t];
-  const int r = threadIdx.x;
-  if (r >= v.R || v.chunk_done[c]) return;
-  const int cr = c * v.R + r;
-  if (!v.need[cr] || v.done[cr]) return;
-  for (int k = 0; k < TILE; ++k) {
-    const size_t ir = (size_t)(t * TILE + k) * v.R + r;
-    x[ir] += (double)xc[ir];
-    xc[ir] = 0.f;
+__global__ void k_bu_fold(BV v, UpdateList up, double* __restrict__ x, float* __restrict__ xc) {
+  const int r = threadIdx.x, g = threadIdx.y, G = blockDim.y;
+  if (r >= v.R) return;
+  for (int e = blockIdx.x; e < *up.n; e += gridDim.x) {
+    const int t = up.tile[e], cr = v.tile_chunk[t] * v.R + r;
+    if (!v.need[cr] || v.done[cr]) continue;
+#pragma unroll 4
+    for (int k = g * (TILE / G); k < (g + 1) * (TILE / G); ++k) {
+      const size_t ir = (size_t)(t * TILE + k) * v.R + r;
+      x[ir] += (double)xc[ir];
+      xc[ir] = 0.f;
+    }
   }
 }
 
@@ -634,12 +690,13 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
   const int c = blockIdx.x, r = threadIdx.x;
   const int R = s.R;
   extern __shared__ double bs_sm[];
-  __shared__ int any_active, any_iterating;
+  __shared__ int any_active, any_iterating, first;
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     any_active = 0;
     any_iterating = 0;
   }
   __syncthreads();
+  if (MODE == 0 && c == 0 && threadIdx.x == 0 && threadIdx.y == 0) *s.up.n = 0;
   if (MODE != 3 && s.chunk_done[c]) return;  // uniform over the block
   const int cr = c * R + r;
   const bool head = threadIdx.y == 0;
@@ -733,12 +790,17 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
   const int update = MODE == 1 && any_active && !any_iterating;
   if (update && head && r < R && !s.done[cr]) s.need[cr] = 1;
   if (threadIdx.x == 0 && head) {
-    if (MODE == 1) s.chunk_update[c] = update;
-    if (MODE == 4) s.chunk_update[c] = 0;
     if ((MODE == 2 || MODE == 3) && !any_active) {
       s.chunk_done[c] = 1;
       atomicSub(s.active_chunks, 1);
     }
+    if (MODE == 1 && update) first = atomicAdd(s.up.n, s.chunk_tile0[c + 1] - s.chunk_tile0[c]);
+  }
+  if (MODE == 1 && update) {  // the chunk's tiles (any order of the chunks will do)
+    __syncthreads();
+    const int t0 = s.chunk_tile0[c], n = s.chunk_tile0[c + 1] - t0;
+    for (int k = threadIdx.y * blockDim.x + threadIdx.x; k < n; k += blockDim.x * blockDim.y)
+      s.up.tile[first + k] = t0 + k;
   }
 }
 
@@ -900,8 +962,8 @@ void launch_batch_mv_f32(const BatchF32Args& a, int formula, int rb, int grid, c
 }
 
 void launch_batch_resid_f64(const BatchF64Args& a, int grid, cudaStream_t st) {
-  k_resid_prep<<<a.n_row_tiles, 256, 0, st>>>(a.n_rhs, a.kc.var_s, a.tile_chunk, a.chunk_done,
-                                               a.chunk_update, a.wl, a.xv, a.uu);
+  k_resid_prep<<<std::min(a.n_row_tiles, 4 * sm_count()), 256, 0, st>>>(a.n_rhs, a.kc.var_s,
+                                                                       a.up, a.wl, a.xv, a.uu);
   DS_CHECK_LAUNCH();
   DS_CUDA(cudaMemsetAsync(a.work, 0, sizeof(unsigned int), st));
   switch (resid_block(a.n_rhs)) {
@@ -1075,7 +1137,12 @@ void batch_build(ds_batch* B, const double* d_rec, const int* sizes) {
                   &B->s_converged, &B->s_it_best, &B->s_stalled})
     v->alloc(CR);
   B->chunk_done.alloc(C);
-  B->chunk_update.alloc(C);
+  B->up_n.alloc(1);
+  B->up_tile.alloc(T);
+  B->seg_cap = 9 * sm_count();  // three times the residual's CTAs at 32 RHS per item
+  B->seg.alloc((size_t)B->seg_cap * resid_block(B->n_rhs) * 3 * TILE);
+  B->seg_count.alloc(B->seg_cap);
+  DS_CUDA(cudaMemsetAsync(B->seg_count.p, 0, B->seg_count.bytes(), st));
   B->active.alloc(1);
   B->work.alloc(2);
   B->err.alloc(1);
@@ -1139,11 +1206,11 @@ BatchF64Args resid_args(ds_batch* B) {
   a.row_ptr = B->pairs64.row_ptr.p;
   a.cols = B->pairs64.cols.p;
   a.mask = B->pairs64.mask.p;
-  a.row_order = B->pairs64.row_order.p;
   a.n_row_tiles = B->n_tiles;
-  a.tile_chunk = B->tile_chunk.p;
-  a.chunk_done = B->chunk_done.p;
-  a.chunk_update = B->chunk_update.p;
+  a.up = UpdateList{B->up_n.p, B->up_tile.p};
+  a.seg = B->seg.p;
+  a.seg_count = B->seg_count.p;
+  a.seg_cap = B->seg_cap;
   a.n_rhs = B->n_rhs;
   a.work = B->work.p + 1;
   a.uu = B->uu.p;
@@ -1177,7 +1244,7 @@ BatchState state_args(ds_batch* B, const ds_mixed_params& mp) {
   s.done = B->s_done.p;
   s.converged = B->s_converged.p;
   s.chunk_done = B->chunk_done.p;
-  s.chunk_update = B->chunk_update.p;
+  s.up = UpdateList{B->up_n.p, B->up_tile.p};
   s.active_chunks = B->active.p;
   return s;
 }
@@ -1232,7 +1299,7 @@ static void check_tc_error(ds_batch* B) {
   }
 }
 
-// r64 = b - A x (FP64) over the chunks flagged in chunk_update (profiled as
+// r64 = b - A x (FP64) over the update list's tiles (profiled as
 // kind 0).
 void batch_resid(ds_batch* B, cudaStream_t st) {
   BatchF64Args a = resid_args(B);
@@ -1359,7 +1426,7 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
   DS_CHECK_LAUNCH();
   DS_CUDA(cudaMemsetAsync(B->xv.p, 0, NR * sizeof(double), st));
   DS_CUDA(cudaMemsetAsync(B->chunk_done.p, 0, C * sizeof(int), st));
-  DS_CUDA(cudaMemsetAsync(B->chunk_update.p, 0, C * sizeof(int), st));
+  DS_CUDA(cudaMemsetAsync(B->up_n.p, 0, sizeof(int), st));
   const int h_active = C;
   DS_CUDA(cudaMemcpyAsync(B->active.p, &h_active, sizeof(int), cudaMemcpyHostToDevice, st));
   DS_CUDA(cudaStreamSynchronize(st));  // h_active is on this stack frame
@@ -1369,6 +1436,7 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
              B->s_hold.p, B->s_done.p,     B->s_alpha.p,     B->s_beta.p,  B->s_scale.p};
   const int RT = ((R + 31) / 32) * 32;
   const dim3 rows(RT, row_groups(RT, 512)), tiles(RT, row_groups(RT, 1024));
+  const int TU = std::min(T, 4 * sm_count());  // the list kernels' grid
   const size_t row_smem = (size_t)rows.x * rows.y * sizeof(float4);
   const size_t bs_smem = (size_t)tiles.x * tiles.y * 2 * sizeof(double);
   // The tensor-core matvec forms p = z + beta p as it packs p (launch_batch_mv_tc).
@@ -1379,8 +1447,8 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
   DS_CUDA(cudaEventCreate(&ev1));
   DS_CUDA(cudaEventRecord(ev0, st));
   // r = b (x0 = 0), z = M^-1 r, p = z, x_c = 0
-  k_bu_update<2><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->pd32.p, B->bv.p,
-                                   B->part.p);
+  k_bu_update<2><<<T, rows, row_smem, st>>>(v, S.up, T, B->xc.p, B->rr.p, B->zz.p, B->p.p,
+                                            B->pd32.p, B->bv.p, B->part.p);
   DS_CHECK_LAUNCH();
   k_bs<3><<<C, tiles, bs_smem, st>>>(S, B->part.p);
   DS_CHECK_LAUNCH();
@@ -1398,11 +1466,11 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
       k_bu_dir<0><<<T, RT, 0, st>>>(v, B->zz.p, B->p.p);                             // U3
       DS_CHECK_LAUNCH();
     }
-    k_bu_fold<<<T, RT, 0, st>>>(v, B->xv.p, B->xc.p);                                // U4
+    k_bu_fold<<<TU, rows, 0, st>>>(v, S.up, B->xv.p, B->xc.p);                       // U4
     DS_CHECK_LAUNCH();
     batch_resid(B, st);                                                              // R5
-    k_bu_update<1><<<T, RT, 0, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->pd32.p,
-                                     B->r64.p, B->part.p);                           // U6
+    k_bu_update<1><<<TU, rows, row_smem, st>>>(v, S.up, T, B->xc.p, B->rr.p, B->zz.p, B->p.p,
+                                               B->pd32.p, B->r64.p, B->part.p);      // U6
     DS_CHECK_LAUNCH();
     k_bs<2><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S6
     DS_CHECK_LAUNCH();

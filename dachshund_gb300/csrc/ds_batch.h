@@ -52,6 +52,12 @@ struct BatchF32Args {
   long long wait_limit;  // tensor-core variant: bound of its waits (SM clock cycles)
 };
 
+// The tiles of the chunks that take an update in this iteration.
+struct UpdateList {
+  int* n;
+  int* tile;
+};
+
 struct BatchF64Args {
   KernelConsts kc;
   const double* x;
@@ -67,11 +73,11 @@ struct BatchF64Args {
   const int* row_ptr;
   const int* cols;
   const unsigned short* mask;
-  const int* row_order;
   int n_row_tiles;
-  const int* tile_chunk;
-  const int* chunk_done;
-  const int* chunk_update;
+  UpdateList up;
+  float* seg;           // float-pair sums of an item's segments
+  unsigned* seg_count;  // their arrivals, per item (0 between launches)
+  int seg_cap;          // segments that fit
   int n_rhs;
   unsigned int* work;
   unsigned long long* prof_pairs;  // profiling: pair x RHS products evaluated
@@ -103,7 +109,7 @@ struct BatchState {
   int* done;
   int* converged;
   int* chunk_done;
-  int* chunk_update;
+  UpdateList up;
   int* active_chunks;
 };
 
@@ -148,7 +154,10 @@ struct ds_batch {
   ds::DevBuf<double> s_rz, s_rz_old, s_alpha, s_beta, s_rmax, s_rbest, s_rtrue, s_norm_b,
       s_tol_norm_b;
   ds::DevBuf<int> s_iter, s_n_updates, s_need, s_hold, s_done, s_converged, s_it_best, s_stalled;
-  ds::DevBuf<int> chunk_done, chunk_update, active;
+  ds::DevBuf<int> chunk_done, active, up_n, up_tile;
+  ds::DevBuf<float> seg;
+  ds::DevBuf<unsigned> seg_count;
+  int seg_cap = 0;
   ds::DevBuf<int> loop_it;  // iterations run by the device-side loop of a solve
   ds::DevBuf<unsigned int> work;  // work-queue counters
   ds::DevBuf<unsigned short> panel;  // tensor-core variant: BF16 u panels (lazy)
