@@ -294,7 +294,7 @@ __device__ __forceinline__ float ex2_br(float x) {
 // The chunks' updates mostly come one chunk at a time (24 chunks: 87 launches with
 // work), whose tiles alone leave most of the chip idle and take as long as the
 // longest item: then an item's tile pairs go in up to 8 segments, whose float-pair
-// sums the last to finish adds up in segment order.  24 chunks x 64: 102 -> RESID_MS ms
+// sums the last to finish adds up in segment order.  24 chunks x 64: 102 -> 54 ms
 // a solve.
 template <int RB, bool FF>
 __global__ void __launch_bounds__(TILE, 3) k_batch_resid_f64(BatchF64Args a) {
@@ -506,7 +506,7 @@ inline int row_groups(int rt, int threads) {
 // [t][r], |r|^2 at [t][R + r].  Bound by its 28 bytes per (pixel, RHS); the sums are
 // float pairs (exact products, compensated sums, of vectors scaled to about 1): in
 // FP64 they took 5 instructions of 16 clocks per element and the kernel 160 us at
-// 207,104 pixels x 64 instead of 73.
+// 207,104 pixels x 64 instead of 88.
 __global__ void k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
                           float* __restrict__ z, const float* __restrict__ p,
                           const float* __restrict__ q, const float* __restrict__ pd,

@@ -10,9 +10,11 @@
 // and a 32 KB panel, against 1,024 clocks of MMA issue at N = 128 and 512
 // clocks of ex2 for the S values.  MMAs with N = 64 run at about half their
 // peak rate on this part (67-95 clocks each against 32), so the panel is one
-// N = 2 NB operand.  Measured (64 chunks x 64 RHS): tensor pipe 21% busy,
-// shared-memory pipes 29% (LSU) and 23% (tensor core), issue 42%: the
-// two-stage S pipeline leaves latency exposed rather than saturating a pipe.
+// N = 2 NB operand.  Measured (24 chunks x 64 RHS, 25,530 tiles): a tile's 16 MMAs
+// take 1,950 clocks (their operand reads beside the stores), its generation 1,000
+// and its stores 500 beside them; the rest of 3,300 clocks a tile is the hand-offs
+// and the items' ends.  With the panel copies issued by the coordinates' warp and
+// the epilogue run by the generation warps it was 3,900 (370 -> 330 us a product).
 //
 // Precision: S and u = w p are split into BF16 hi + lo parts.  The u panel
 // of a column tile is one B operand of N = 2 NB rows, [u_hi | u_lo], so two
@@ -22,22 +24,22 @@
 // significant bits per term with an FP32 accumulator, an operator error near
 // 1e-5 relative, which the FP64 reliable updates of the solver remove.
 //
-// Per CTA (one per SM, GEN_WARPS + 2 warps, persistent over (row tile, RHS
-// block) items), warp-specialized with mbarrier hand-offs:
+// Per CTA (one per SM, GEN_WARPS + EPI_WARPS + 3 warps, persistent over (row tile,
+// RHS block) items), warp-specialized with mbarrier hand-offs:
 //   * warps 0 .. GEN_WARPS - 1 generate S for the current column tile (row
 //     sub-tile warp % 4, 128 / (GEN_WARPS / 4) columns per warp; EXPANDED
 //     exponent: 3 FFMA + ex2 per pair; DIRECT when the tiles are too wide for
 //     it), split it into BF16 hi / lo and store both into shared memory in
 //     the canonical K-major no-swizzle layout (8 x 16-byte core matrices); a
-//     32 x 32 sub-tile outside the cutoff is zero.  After an item's last tile
-//     they read D back (tcgen05.ld; warp w may read TMEM lanes
-//     32 (w % 4) .. + 31, its own rows), form q = rowf D + ediag p and the
-//     tile's p.q per RHS;
-//   * warp GEN_WARPS stages the column coordinates of each column tile and
-//     issues the cp.async.bulk copy of its u panel (pre-packed in HBM by
-//     k_pack_panels in the same core-matrix layout);
-//   * lane 0 of warp GEN_WARPS + 1 issues the MMAs (K steps whose column
+//     32 x 32 sub-tile outside the cutoff is zero;
+//   * the EPI_WARPS warps after them read D back after an item's last tile
+//     (tcgen05.ld; warp w may read TMEM lanes 32 (w % 4) .. + 31, its own rows),
+//     form q = rowf D + ediag p and the tile's p.q per RHS;
+//   * PROD_WARP stages the column coordinates of each column tile;
+//   * lane 0 of MMA_WARP issues the MMAs (K steps whose column
 //     sub-tile interacts with no row sub-tile are skipped) and commits them;
+//   * lane 0 of PANEL_WARP issues the cp.async.bulk copy of each column tile's u
+//     panel (pre-packed in HBM by k_pack_panels in the same core-matrix layout);
 //   * S tiles, panels and coordinates are double-buffered and the
 //     accumulator has two TMEM buffers, so generation of tile g + 1 overlaps
 //     the MMAs of tile g and an item's epilogue overlaps the next item.
@@ -55,10 +57,14 @@
 namespace ds {
 namespace {
 
-constexpr int GEN_WARPS = 8;                       // S generation + epilogue (8 or 16)
+constexpr int GEN_WARPS = 8;                       // S generation (8 or 16)
+constexpr int EPI_WARPS = 4;                       // epilogue: one per TMEM lane quarter
+constexpr int PROD_WARP = GEN_WARPS + EPI_WARPS;   // column coordinates
+constexpr int MMA_WARP = PROD_WARP + 1;            // MMA issue
+constexpr int PANEL_WARP = PROD_WARP + 2;          // panel copies
 constexpr int GEN_CW = GEN_WARPS / 4;              // warps per row sub-tile
 constexpr int GEN_CS = 4 / GEN_CW;                 // column sub-tiles per warp
-constexpr int TC_THREADS = (GEN_WARPS + 2) * 32;   // + producer warp + MMA warp
+constexpr int TC_THREADS = (GEN_WARPS + EPI_WARPS + 3) * 32;
 // One CTA per SM: the warps are spread over the 4 SM sub-partitions, each
 // with 16,384 registers, so the busiest one holds ceil(warps / 4) warps.
 constexpr int TC_MAXNREG = (16384 / (32 * ((TC_THREADS / 32 + 3) / 4))) & ~7;
@@ -93,14 +99,14 @@ struct TcSmem {
   __nv_bfloat16 s[2][2][S_ELEMS];     // [buffer][hi, lo] generated S tiles
   __nv_bfloat16 u[2][2 * NB * TILE];  // [buffer] u panel, hi then lo
   float4 sc[2][TILE];                 // [buffer] column coordinates of the tile
-  float red[2][GEN_WARPS][32];        // [D buffer][warp] per-column p.q sums
+  float red[2][EPI_WARPS][NB];        // [D buffer][warp] per-column p.q sums
   uint64_t sc_full[2];   // column coordinates staged       (1 arrive)
   uint64_t u_full[2];    // u panel landed                  (1 arrive + tx bytes)
   uint64_t s_full[2];    // S tile written                  (GEN_WARPS arrives)
   uint64_t mma_done[2];  // MMAs reading buffer b completed (tcgen05.commit)
   uint64_t d_full[2];    // all MMAs of an item completed   (tcgen05.commit)
-  uint64_t d_empty[2];   // D read back by the epilogue     (GEN_WARPS arrives)
-  uint64_t red_full[2];  // per-warp column sums written    (GEN_WARPS arrives)
+  uint64_t d_empty[2];   // D read back by the epilogue     (EPI_WARPS arrives)
+  uint64_t red_full[2];  // per-warp column sums written    (EPI_WARPS arrives)
   uint32_t tmem_addr;
   int abort;
 };
@@ -156,15 +162,12 @@ __device__ __forceinline__ float warp_column_sums(float (&v)[HN], int lane) {
   return r;
 }
 
-// Warp roles: warps 0 .. GEN_WARPS - 1 generate S and run the epilogue; warp
-// GEN_WARPS stages the column coordinates and issues the u-panel copy of each
-// column tile; lane 0 of warp GEN_WARPS + 1 issues the MMAs.  The
-// hand-offs are mbarriers, so no role waits for another except for data:
-// generation of tile g + 1 overlaps the MMAs of tile g, and the epilogue of
+// Warp roles as above.  The hand-offs are mbarriers, so no role waits for another
+// except for data: generation of tile g + 1 overlaps the MMAs of tile g, and the epilogue of
 // an item (its accumulator in one of two TMEM buffers) overlaps the MMAs of
-// the next.  Items are dealt round-robin (item = CTA + k * grid), in the
-// launch order (chunks by decreasing work), so every role walks the same
-// sequence without a queue.
+// the next.  Items are dealt in turns of one per CTA (item_of) in the launch
+// order (tiles by decreasing work), so every role walks the same sequence
+// without a queue.
 template <int NB, int FORMULA>
 __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
   static_assert(NB == 16 || NB == 32 || NB == 64, "RHS block");
@@ -173,7 +176,7 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
   constexpr uint32_t PANEL_BYTES = 2u * NB * TILE * 2u;
   constexpr uint32_t U_LBO = (2 * NB / 8) * 128;
   constexpr uint32_t IDESC = idesc_bf16(128, 2 * NB);
-  constexpr int HN = NB / GEN_CW;  // RHS columns of D per generation warp
+  constexpr int HN = NB < 32 ? NB : 32;  // RHS columns of D per epilogue pass
   extern __shared__ uint8_t smem_raw[];
   TcSmem<NB>& sm = *reinterpret_cast<TcSmem<NB>*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -185,8 +188,8 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
       mbar_init(&sm.s_full[b], GEN_WARPS);
       mbar_init(&sm.mma_done[b], 1);
       mbar_init(&sm.d_full[b], 1);
-      mbar_init(&sm.d_empty[b], GEN_WARPS);
-      mbar_init(&sm.red_full[b], GEN_WARPS);
+      mbar_init(&sm.d_empty[b], EPI_WARPS);
+      mbar_init(&sm.red_full[b], EPI_WARPS);
     }
     sm.abort = 0;
     mbar_fence_init();
@@ -200,37 +203,40 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
   const int nblk = R / NB;
   const int n_items = a.n_row_tiles * nblk;
   const __nv_bfloat16* panels = reinterpret_cast<const __nv_bfloat16*>(a.panel);
+  // The CTA's items, every gridDim-th of the tiles by decreasing work, every other
+  // time from the end: even shares (in one direction the first CTA's were 16% above
+  // the mean).
+  const int n_turns = (n_items + (int)gridDim.x - 1) / (int)gridDim.x;
+  auto item_of = [&](int turn) {
+    return turn * (int)gridDim.x +
+           ((turn & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+  };
   int last_g = -1;  // last tile of this role's walk (MMA commit / panel copy in flight)
 
   if (warp < GEN_WARPS) {
-    // ---- generation and epilogue ------------------------------------------
-    // warp = 4 cw + rs: row sub-tile rs (TMEM lanes 32 rs ..), column
-    // sub-tiles GEN_CS cw .. GEN_CS cw + GEN_CS - 1 of S, D columns cw HN ..
-    // In generation lane l forms rows 32 rs + 8 j + (l & 7), j = 0..3, times
-    // the 8 columns 8 (l >> 3) .. of each column sub-tile, so each staged
-    // column is read once per 4 rows.  128-bit shared accesses are served
+    // ---- generation ---------------------------------------------------------
+    // warp = 4 cw + rs: row sub-tile rs, column sub-tiles GEN_CS cw ..
+    // GEN_CS cw + GEN_CS - 1 of S.  Lane l forms rows 32 rs + 8 j + (l & 7),
+    // j = 0..3, times the 8 columns 8 (l >> 3) .. of each column sub-tile, so each
+    // staged column is read once per 4 rows.  128-bit shared accesses are served
     // 8 lanes at a time: lanes 8q .. 8q + 7 read the same coordinates
-    // (broadcast) and store 8 consecutive rows (128 contiguous bytes).  In
-    // the epilogue lane l owns row 32 rs + l (its TMEM lane).
+    // (broadcast) and store 8 consecutive rows (128 contiguous bytes).
     const int rs = warp & 3, cw = warp >> 2;
     const int kq = lane >> 3, rl = lane & 7;
-    const int row = 32 * rs + lane;
-    uint32_t g = 0, k = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    uint32_t g = 0;
+    for (int turn = 0; turn < n_turns; ++turn) {
+      const int item = item_of(turn);
+      if (item >= n_items) break;  // the last turn
       const int t = a.row_order[item / nblk];
-      const int rb = item % nblk;
       if (a.chunk_done[a.tile_chunk[t]]) continue;
-      const int i = t * TILE + row;
       float4 me[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) me[j] = a.xi[t * TILE + 32 * rs + 8 * j + rl];
       const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
-      bool any = false;
       unsigned m = a.mask[p0];
       for (int p = p0; p < p1; ++p, ++g) {
         const uint32_t b = g & 1;
         const unsigned mnext = p + 1 < p1 ? a.mask[p + 1] : 0u;
-        any |= m != 0u;
         // S values of this warp's sub-tiles are formed in registers as soon as
         // the coordinates are staged; the S buffer is awaited only for the
         // stores
@@ -300,83 +306,103 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
         m = mnext;
       }
       if (aborted(&sm.abort)) break;
-      // epilogue: D of this item in TMEM buffer db; the row's p values and
-      // coefficients are loaded before the wait
+    }
+  } else if (warp < PROD_WARP) {
+    // ---- epilogue: D of an item in TMEM buffer db, while the next is generated ----
+    // Warp rs owns row sub-tile rs (its TMEM lanes), lane l row 32 rs + l.
+    const int rs = warp & 3;
+    uint32_t k = 0;
+    for (int turn = 0; turn < n_turns; ++turn) {
+      const int item = item_of(turn);
+      if (item >= n_items) break;  // the last turn
+      const int t = a.row_order[item / nblk];
+      const int rb = item % nblk;
+      if (a.chunk_done[a.tile_chunk[t]]) continue;
+      const int i = t * TILE + 32 * rs + lane;
+      const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
+      unsigned mine = 0;
+      for (int p = p0 + lane; p < p1; p += 32) mine |= a.mask[p];
+      const bool any = __any_sync(0xffffffffu, mine != 0u);  // else D was not written
       const uint32_t db = k & 1;
       const float rf = a.rowf[i], ed = a.ediag[i];
-      const int r0 = rb * NB + cw * HN;
-      const float4* pv4 = reinterpret_cast<const float4*>(a.p + (size_t)i * R + r0);
-      float4* qv4 = reinterpret_cast<float4*>(a.q + (size_t)i * R + r0);
-      float4 pvr[HN / 4];
+      bool ok = true;
+#pragma unroll 1
+      for (int h = 0; h < NB / HN; ++h) {
+        const int r0 = rb * NB + h * HN;
+        const float4* pv4 = reinterpret_cast<const float4*>(a.p + (size_t)i * R + r0);
+        float4* qv4 = reinterpret_cast<float4*>(a.q + (size_t)i * R + r0);
+        float4 pvr[HN / 4];
 #pragma unroll
-      for (int k4 = 0; k4 < HN / 4; ++k4) pvr[k4] = pv4[k4];
-      if (!warp_wait_or_abort(sm, &sm.d_full[db], (k >> 1) & 1u, a.err, 13, a.wait_limit,
-                              lane))
-        break;
-      __syncwarp();
-      tc_fence_after();
-      float d[HN], dl[HN];
-      const uint32_t tl = tmem + ((uint32_t)(32 * rs) << 16) + db * D_COLS + (uint32_t)(cw * HN);
-      tmem_ld<HN>(tl, d);        // S u_hi
-      tmem_ld<HN>(tl + NB, dl);  // S u_lo
+        for (int k4 = 0; k4 < HN / 4; ++k4) pvr[k4] = pv4[k4];
+        if (h == 0) {
+          ok = warp_wait_or_abort(sm, &sm.d_full[db], (k >> 1) & 1u, a.err, 13, a.wait_limit,
+                                  lane);
+          if (!ok) break;
+          __syncwarp();
+          tc_fence_after();
+        }
+        float d[HN], dl[HN];
+        const uint32_t tl = tmem + ((uint32_t)(32 * rs) << 16) + db * D_COLS + (uint32_t)(h * HN);
+        tmem_ld<HN>(tl, d);        // S u_hi
+        tmem_ld<HN>(tl + NB, dl);  // S u_lo
 #pragma unroll
-      for (int j = 0; j < HN; ++j) d[j] += dl[j];
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.d_empty[db]);
-      if (!any) {
+        for (int j = 0; j < HN; ++j) d[j] += dl[j];
+        if (h == NB / HN - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.d_empty[db]);
+        }
+        if (!any) {
 #pragma unroll
-        for (int j = 0; j < HN; ++j) d[j] = 0.f;
+          for (int j = 0; j < HN; ++j) d[j] = 0.f;
+        }
+#pragma unroll
+        for (int k4 = 0; k4 < HN / 4; ++k4) {
+          const float4 pv = pvr[k4];
+          float4 qv;
+          qv.x = fmaf(rf, d[4 * k4 + 0], ed * pv.x);
+          qv.y = fmaf(rf, d[4 * k4 + 1], ed * pv.y);
+          qv.z = fmaf(rf, d[4 * k4 + 2], ed * pv.z);
+          qv.w = fmaf(rf, d[4 * k4 + 3], ed * pv.w);
+          qv4[k4] = qv;
+          d[4 * k4 + 0] = pv.x * qv.x;  // d now holds the p.q products
+          d[4 * k4 + 1] = pv.y * qv.y;
+          d[4 * k4 + 2] = pv.z * qv.z;
+          d[4 * k4 + 3] = pv.w * qv.w;
+        }
+        const float csum = warp_column_sums<HN>(d, lane);
+        if (lane < HN) sm.red[db][rs][h * HN + lane] = csum;
       }
-#pragma unroll
-      for (int k4 = 0; k4 < HN / 4; ++k4) {
-        const float4 pv = pvr[k4];
-        float4 qv;
-        qv.x = fmaf(rf, d[4 * k4 + 0], ed * pv.x);
-        qv.y = fmaf(rf, d[4 * k4 + 1], ed * pv.y);
-        qv.z = fmaf(rf, d[4 * k4 + 2], ed * pv.z);
-        qv.w = fmaf(rf, d[4 * k4 + 3], ed * pv.w);
-        qv4[k4] = qv;
-        d[4 * k4 + 0] = pv.x * qv.x;  // d now holds the p.q products
-        d[4 * k4 + 1] = pv.y * qv.y;
-        d[4 * k4 + 2] = pv.z * qv.z;
-        d[4 * k4 + 3] = pv.w * qv.w;
-      }
-      const float csum = warp_column_sums<HN>(d, lane);
-      if (lane < HN) sm.red[db][warp][lane] = csum;
+      if (!ok) break;
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.red_full[db]);
-      // The sums of buffer db are read before this item's column sums of
-      // buffer db are rewritten two items later: those need D of that item,
-      // i.e. the S tiles of the item in between from every generation warp.
-      if (warp < NB / 32 + (NB < 32) &&
-          !warp_wait_or_abort(sm, &sm.red_full[db], (k >> 1) & 1u, a.err, 14, a.wait_limit,
-                              lane))
+      // All four warps wait, so that none rewrites red[db] two items on before the
+      // others have read it: it passes the item in between with them.
+      if (!warp_wait_or_abort(sm, &sm.red_full[db], (k >> 1) & 1u, a.err, 14, a.wait_limit, lane))
         break;
-      if (tid < NB) {
-        // column tid of the block: warp column group h = tid / HN, summed
-        // over the four row sub-tiles (warps 4 h .. 4 h + 3)
-        const int h = tid / HN, j = tid % HN;
+      const int col = tid - GEN_WARPS * 32;
+      if (col < NB) {
         double sum = 0.0;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) sum += (double)sm.red[db][h * 4 + w][j];
-        a.part[(size_t)t * R + rb * NB + tid] = sum;
+        for (int w = 0; w < EPI_WARPS; ++w) sum += (double)sm.red[db][w][col];
+        a.part[(size_t)t * R + rb * NB + col] = sum;
       }
-      if (a.prof_pairs && tid == 0) {
+      if (a.prof_pairs && col == 0) {
         unsigned long long n_sub = 0;
         for (int p = p0; p < p1; ++p) n_sub += __popc(a.mask[p]);
         atomicAdd(a.prof_pairs, n_sub * SUBTILE * SUBTILE * NB);
       }
       ++k;
     }
-  } else if (warp == GEN_WARPS) {
-    // ---- producer: column coordinates and u panels ------------------------------
+  } else if (warp == PROD_WARP) {
+    // ---- producer: column coordinates ---------------------------------------------
     // The next tile's indices and coordinates are loaded into registers
     // before waiting for its buffer, so their latency overlaps that wait.
     uint32_t g = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    for (int turn = 0; turn < n_turns; ++turn) {
+      const int item = item_of(turn);
+      if (item >= n_items) break;  // the last turn
       const int t = a.row_order[item / nblk];
-      const int rb = item % nblk;
       if (a.chunk_done[a.tile_chunk[t]]) continue;
       const float4 ot = a.orig[t];
       const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
@@ -412,17 +438,6 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.sc_full[b]);
-        // u[b] is free once the MMAs of tile g - 2 completed
-        if (g >= 2 &&
-            !warp_wait_or_abort(sm, &sm.mma_done[b], ((g >> 1) - 1) & 1u, a.err, 21,
-                                a.wait_limit, lane))
-          break;
-        if (lane == 0) {
-          mbar_expect_tx(&sm.u_full[b], PANEL_BYTES);
-          bulk_g2s(sm.u[b], panels + ((size_t)ct * nblk + rb) * (2 * NB * TILE), PANEL_BYTES,
-                   &sm.u_full[b]);
-        }
-        last_g = (int)g;
         ct = ct_n;
         co = co_n;
 #pragma unroll
@@ -430,10 +445,41 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
       }
       if (aborted(&sm.abort)) break;
     }
+  } else if (warp == PANEL_WARP) {
+    // ---- u panels.  A warp of its own: in the producer, the wait for the MMAs of
+    // tile g - 2 held the coordinates of tile g + 1 back and with them the generation
+    // (1,000 of 3,600 clocks a tile).
+    uint32_t g = 0;
+    for (int turn = 0; turn < n_turns && lane == 0; ++turn) {
+      const int item = item_of(turn);
+      if (item >= n_items) break;  // the last turn
+      const int t = a.row_order[item / nblk];
+      const int rb = item % nblk;
+      if (a.chunk_done[a.tile_chunk[t]]) continue;
+      const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
+      int ct = p0 < p1 ? a.cols[p0] : 0;
+      for (int p = p0; p < p1; ++p, ++g) {
+        const uint32_t b = g & 1;
+        const int ct_n = p + 1 < p1 ? a.cols[p + 1] : ct;
+        // u[b] is free once the MMAs of tile g - 2 completed
+        if (aborted(&sm.abort) ||
+            (g >= 2 && !wait_or_abort(sm, &sm.mma_done[b], ((g >> 1) - 1) & 1u, a.err, 21,
+                                      a.wait_limit)))
+          break;
+        mbar_expect_tx(&sm.u_full[b], PANEL_BYTES);
+        bulk_g2s(sm.u[b], panels + ((size_t)ct * nblk + rb) * (2 * NB * TILE), PANEL_BYTES,
+                 &sm.u_full[b]);
+        last_g = (int)g;
+        ct = ct_n;
+      }
+      if (aborted(&sm.abort)) break;
+    }
   } else if (lane == 0) {
     // ---- MMA issue ------------------------------------------------------------
     uint32_t g = 0, k = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    for (int turn = 0; turn < n_turns; ++turn) {
+      const int item = item_of(turn);
+      if (item >= n_items) break;  // the last turn
       const int t = a.row_order[item / nblk];
       if (a.chunk_done[a.tile_chunk[t]]) continue;
       const int p0 = a.row_ptr[t], p1 = a.row_ptr[t + 1];
@@ -481,11 +527,11 @@ __global__ void __maxnreg__(TC_MAXNREG) k_batch_mv_tc(BatchF32Args a) {
   // earlier MMA of the thread) and the last two panel copies (a copy into a
   // buffer is issued only after the copy before it in that buffer was used).
   if (aborted(&sm.abort) && last_g >= 0 && lane == 0) {
-    if (warp == GEN_WARPS) {
+    if (warp == PANEL_WARP) {
       mbar_wait(&sm.u_full[last_g & 1], (last_g >> 1) & 1u);
       if (last_g >= 1) mbar_wait(&sm.u_full[(last_g - 1) & 1], ((last_g - 1) >> 1) & 1u);
     }
-    if (warp == GEN_WARPS + 1) mbar_wait(&sm.mma_done[last_g & 1], (last_g >> 1) & 1u);
+    if (warp == MMA_WARP) mbar_wait(&sm.mma_done[last_g & 1], (last_g >> 1) & 1u);
   }
   tc_fence_before();
   __syncthreads();
