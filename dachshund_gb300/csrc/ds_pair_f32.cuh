@@ -1,5 +1,5 @@
 // Evaluation of staged columns by the FP32 pair kernels (pair_f32.cu: the
-// formulations and the lane layout; persist_pairs.cu).
+// formulations and the lane layout; persist_pairs.cu), the latter's packing.
 #pragma once
 
 #include "ds_f32.h"
@@ -20,10 +20,12 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
 }
 
 // A lane's four rows (lane, +32, +64, +96), each coordinate twice: the packed
-// operations take one row and two neighbouring columns.  (Two rows and one column
-// need the column's four values duplicated into register pairs: 8 moves a column,
-// which made the loop bound by instruction issue, 24 instructions a column where 4
-// exponentials take 16 clocks.)
+// operations take one row and two neighbouring columns.  (Two rows and one column, as
+// in pair_f32.cu, need the column's four values duplicated into register pairs: 24
+// issued instructions a column instead of 15, where 4 exponentials take 16 clocks.
+// With 4 warps per scheduler here that is 10.7 -> 9.6 ms a solve at 44,237 pixels; the
+// 20 warps per SM of the per-kernel form, at 96 registers, are faster with it: 43.5
+// against 45.6 ms at 262,144.)
 struct RowRegs {
   float2 x[4], y[4], z[4];
   __device__ __forceinline__ void set(int k, float4 v) {

@@ -39,7 +39,78 @@ namespace {
 // on the 262,144-pixel workload 5 CTAs per SM beat 4, 6, 7 (with spills) and
 // the one-tile prefetch at 8.
 constexpr int F32_MIN_CTAS = 5;
-constexpr int F32_QU = 2;  // groups of four columns unrolled
+
+// One warp's 32 staged columns against its lane's four rows, as two f32x2 row
+// pairs (01: rows lane and lane+32, 23: rows lane+64 and lane+96).  A pair
+// whose two row sub-tiles are both beyond the cutoff from the column
+// sub-tile is skipped (DO01 / DO23 false).  The column values come four to a
+// shared-memory load.
+template <int FORMULA, bool DO01, bool DO23>
+__device__ __forceinline__ void accumulate32_rows(const float4* __restrict__ col,
+                                             const float4* __restrict__ cu4, float2 x01,
+                                             float2 y01, float2 z01, float2 x23, float2 y23,
+                                             float2 z23, float2& acc01, float2& acc23) {
+#pragma unroll
+  for (int qd = 0; qd < 8; ++qd) {
+    const float4 u4 = cu4[qd];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 c4 = col[4 * qd + k];
+      const float uk = k == 0 ? u4.x : k == 1 ? u4.y : k == 2 ? u4.z : u4.w;
+      const float2 u2 = make_float2(uk, uk);
+      float2 t01, t23;
+      if (FORMULA == F32_EXPANDED) {
+        const float2 cx = make_float2(c4.x, c4.x), cy = make_float2(c4.y, c4.y);
+        const float2 cz = make_float2(c4.z, c4.z), cw = make_float2(c4.w, c4.w);
+        if (DO01) {
+          t01 = __ffma2_rn(x01, cx, cw);
+          t01 = __ffma2_rn(y01, cy, t01);
+          t01 = __ffma2_rn(z01, cz, t01);
+        }
+        if (DO23) {
+          t23 = __ffma2_rn(x23, cx, cw);
+          t23 = __ffma2_rn(y23, cy, t23);
+          t23 = __ffma2_rn(z23, cz, t23);
+        }
+      } else {
+        const float2 ncx = make_float2(-c4.x, -c4.x), ncy = make_float2(-c4.y, -c4.y);
+        const float2 ncz = make_float2(-c4.z, -c4.z);
+        if (DO01) {
+          const float2 dx = __fadd2_rn(x01, ncx), dy = __fadd2_rn(y01, ncy);
+          const float2 dz = __fadd2_rn(z01, ncz);
+          t01 = __fmul2_rn(dx, make_float2(-dx.x, -dx.y));
+          t01 = __ffma2_rn(dy, make_float2(-dy.x, -dy.y), t01);
+          t01 = __ffma2_rn(dz, make_float2(-dz.x, -dz.y), t01);
+        }
+        if (DO23) {
+          const float2 dx = __fadd2_rn(x23, ncx), dy = __fadd2_rn(y23, ncy);
+          const float2 dz = __fadd2_rn(z23, ncz);
+          t23 = __fmul2_rn(dx, make_float2(-dx.x, -dx.y));
+          t23 = __ffma2_rn(dy, make_float2(-dy.x, -dy.y), t23);
+          t23 = __ffma2_rn(dz, make_float2(-dz.x, -dz.y), t23);
+        }
+      }
+      if (DO01) acc01 = __ffma2_rn(make_float2(ex2f(t01.x), ex2f(t01.y)), u2, acc01);
+      if (DO23) acc23 = __ffma2_rn(make_float2(ex2f(t23.x), ex2f(t23.y)), u2, acc23);
+    }
+  }
+}
+
+// The 32 columns of one staged work item with the row pairs its mask names.
+template <int FORMULA>
+__device__ __forceinline__ void accumulate_item_rows(unsigned m, const float4* __restrict__ col,
+                                                const float4* __restrict__ cu4, float2 x01,
+                                                float2 y01, float2 z01, float2 x23, float2 y23,
+                                                float2 z23, float2& acc01, float2& acc23) {
+  const bool do01 = (m & 3u) != 0;   // row sub-tile 0 or 1
+  const bool do23 = (m & 12u) != 0;  // row sub-tile 2 or 3
+  if (do01 && do23)
+    accumulate32_rows<FORMULA, true, true>(col, cu4, x01, y01, z01, x23, y23, z23, acc01, acc23);
+  else if (do01)
+    accumulate32_rows<FORMULA, true, false>(col, cu4, x01, y01, z01, x23, y23, z23, acc01, acc23);
+  else if (do23)
+    accumulate32_rows<FORMULA, false, true>(col, cu4, x01, y01, z01, x23, y23, z23, acc01, acc23);
+}
 
 template <int FORMULA, int EPI, bool DOT>
 __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
@@ -53,9 +124,13 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int base = t * TILE;
 
-  RowRegs R;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) R.set(k, a.rxi[base + lane + 32 * k]);
+  float2 x01, y01, z01, x23, y23, z23;
+  {
+    const float4 r0 = a.rxi[base + lane], r1 = a.rxi[base + lane + 32];
+    const float4 r2 = a.rxi[base + lane + 64], r3 = a.rxi[base + lane + 96];
+    x01 = make_float2(r0.x, r1.x); y01 = make_float2(r0.y, r1.y); z01 = make_float2(r0.z, r1.z);
+    x23 = make_float2(r2.x, r3.x); y23 = make_float2(r2.y, r3.y); z23 = make_float2(r2.z, r3.z);
+  }
   const float4 ot = a.rorig[t];
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
@@ -71,6 +146,11 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
   // item) and folds them into the compensated sums once; the column inputs
   // of the next round are loaded into registers while a round is computed.
   const int i1 = a.item_ptr[t + 1];
+  struct ColRegs {
+    float3 q, o;   // this lane's column (tile-relative) and the tile's origin
+    float u;       // colw v (product) or v (map)
+    unsigned m;    // row sub-tiles interacting with the item's columns (bit k)
+  };
   auto load = [&](ColRegs& c, unsigned it) {
     const int ct = (int)(it >> 6);
     const int j = ct * TILE + 32 * (int)((it >> 4) & 3u) + lane;
@@ -103,7 +183,14 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
   float4* const scw = sc + warp * 64;
   float* const suw = reinterpret_cast<float*>(su4 + warp * 16);
   auto stage = [&](const ColRegs& c, int slot) {
-    stage_columns(scw + slot, column_in_frame<FORMULA>(c, ot));
+    const float dx = ot.x - c.o.x, dy = ot.y - c.o.y, dz = ot.z - c.o.z;
+    const float zx = c.q.x - dx, zy = c.q.y - dy, zz = c.q.z - dz;
+    if (FORMULA == F32_EXPANDED) {
+      const float aj = fmaf(zx, zx, fmaf(zy, zy, zz * zz));
+      scw[slot + lane] = make_float4(2.f * zx, 2.f * zy, 2.f * zz, -aj);
+    } else {
+      scw[slot + lane] = make_float4(zx, zy, zz, 0.f);
+    }
     suw[slot + lane] = c.u;
   };
   ColRegs ca, cb;
@@ -120,21 +207,24 @@ __global__ void __launch_bounds__(TILE, F32_MIN_CTAS) k_pair_f32(F32Args a) {
     if (a.prof_pairs)
       evaluated += 2 * SUBTILE * 32 * (((ma & 3u) != 0) + ((ma & 12u) != 0) +
                                        ((mb & 3u) != 0) + ((mb & 12u) != 0));
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    accumulate_item<FORMULA, F32_QU>(ma, scw, su4 + warp * 16, R, acc);
+    float2 acc01 = make_float2(0.f, 0.f), acc23 = make_float2(0.f, 0.f);
+    accumulate_item_rows<FORMULA>(ma, scw, su4 + warp * 16, x01, y01, z01, x23, y23, z23, acc01,
+                             acc23);
     if (EPI == EPI_MAP) {
       // the map keeps 32-term FP32 partials: each item is folded on its own
-      kahan_add(s0, c0, acc[0]);
-      kahan_add(s1, c1, acc[1]);
-      kahan_add(s2, c2, acc[2]);
-      kahan_add(s3, c3, acc[3]);
-      acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+      kahan_add(s0, c0, acc01.x);
+      kahan_add(s1, c1, acc01.y);
+      kahan_add(s2, c2, acc23.x);
+      kahan_add(s3, c3, acc23.y);
+      acc01 = make_float2(0.f, 0.f);
+      acc23 = make_float2(0.f, 0.f);
     }
-    accumulate_item<FORMULA, F32_QU>(mb, scw + 32, su4 + warp * 16 + 8, R, acc);
-    kahan_add(s0, c0, acc[0]);
-    kahan_add(s1, c1, acc[1]);
-    kahan_add(s2, c2, acc[2]);
-    kahan_add(s3, c3, acc[3]);
+    accumulate_item_rows<FORMULA>(mb, scw + 32, su4 + warp * 16 + 8, x01, y01, z01, x23, y23, z23,
+                             acc01, acc23);
+    kahan_add(s0, c0, acc01.x);
+    kahan_add(s1, c1, acc01.y);
+    kahan_add(s2, c2, acc23.x);
+    kahan_add(s3, c3, acc23.y);
     va = na;
     vb = nbv;
   }

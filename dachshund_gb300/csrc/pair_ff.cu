@@ -69,27 +69,33 @@ __global__ void k_ff_points(int n_pad, const double* __restrict__ x, const doubl
   }
 }
 
-// One warp per CTA: its 32 rows need nothing of the tile's other warps, and the grid
-// fills the SMs evenly where 128-row CTAs left 2 on one and 3 on the next.  Columns
-// go in groups of FF_G, neighbours and mostly on the same side of FF_FAR: the
-// group's terms are evaluated together (one column's are a chain of some 30 dependent
-// operations), then added in column order.  Latency bound up to some 100,000 pixels
-// (7 warps per SM, issue 0.54 -> 0.61 a clock): 44,237 pixels 0.72 -> 0.67 ms; 131,072
-// pixels' solve 23.3 -> 22.6 ms (groups of 1: 22.7, of 4: 23.0, of 8: 23.4).
+// A warp's 32 rows need nothing of the tile's other warps: up to FF_TILES tiles a warp
+// is a CTA, and the grid fills the SMs evenly where 128-row CTAs left 2 on one and 3
+// on the next.  Columns go in groups of FF_G, neighbours and mostly on the same side
+// of FF_FAR: the group's terms are evaluated together (one column's are a chain of
+// some 30 dependent operations), then added in column order.  Latency bound up to
+// some 100,000 pixels (7 warps per SM, issue 0.54 -> 0.61 a clock): 44,237 pixels
+// 0.72 -> 0.67 ms; 131,072 pixels' solve 23.3 -> 22.6 ms (groups of 1: 22.7, of 4:
+// 23.0, of 8: 23.4); 262,144 pixels' solve 44.0 ms in CTAs of a warp, 43.5 in whole
+// tiles.
+constexpr int FF_TILES = 1216;
 constexpr int FF_G = 2;
-__global__ void __launch_bounds__(32) k_pair_ff_resid(KernelConsts kc, PairArgs a, FFPoints f) {
+__global__ void __launch_bounds__(TILE) k_pair_ff_resid(KernelConsts kc, PairArgs a, FFPoints f) {
   if (a.skip_flag && *a.skip_flag) return;
-  __shared__ float4 sxy[SUBTILE], szu[SUBTILE];  // xh xl yh yl; zh zl uh ul
+  __shared__ float4 sxy_w[TILE / 32][SUBTILE], szu_w[TILE / 32][SUBTILE];  // xh xl yh yl; zh zl uh ul
   __shared__ float tab_h[32], tab_l[32];
-  const int t = a.row_order ? a.row_order[blockIdx.x >> 2] : (int)(blockIdx.x >> 2);
-  const int warp = blockIdx.x & 3, lane = threadIdx.x;
+  const int lane = threadIdx.x & 31, mine = threadIdx.x >> 5;
+  const int gw = blockIdx.x * (blockDim.x >> 5) + mine;  // a row sub-tile of the grid
+  const int t = a.row_order ? a.row_order[gw >> 2] : gw >> 2;
+  const int warp = gw & 3;
+  float4 *const sxy = sxy_w[mine], *const szu = szu_w[mine];
   const int i = t * TILE + warp * 32 + lane;
-  {
+  if (threadIdx.x < 32) {
     const ff v = ff_from_double(exp2(-(double)lane / 32.0));
     tab_h[lane] = v.h;
     tab_l[lane] = v.l;
   }
-  __syncwarp();
+  __syncthreads();
   const float cut = (float)kc.exact_cut;
   const double xi = a.rx[i] * f.sp, yi = a.ry[i] * f.sp, zi = a.rz[i] * f.sq;
   float ah = 0.f, al = 0.f;
@@ -197,7 +203,8 @@ void launch_pair_ff_resid(const KernelConsts& kc, const PairArgs& a0, const FFPo
   } else {
     a.prof_pairs = nullptr;
   }
-  k_pair_ff_resid<<<a.n_row_tiles * (TILE / 32), 32, 0, st>>>(kc, a, f);
+  const int nt = a.n_row_tiles > FF_TILES ? TILE : 32;
+  k_pair_ff_resid<<<a.n_row_tiles * (TILE / nt), nt, 0, st>>>(kc, a, f);
   DS_CHECK_LAUNCH();
   if (ev) a.prof->end(st, ev, 0);
 }
