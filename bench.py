@@ -49,14 +49,12 @@ K_PAIR_F32_DRAM_BYTES = 9_174_528
 K_SG32_DRAM_BYTES = 16_603_136  # k_sg32_levels 4,202,496 + k_sg32_apply 12,400,640
 # DRAM bytes (read + write) of one launch of the persistent solve on the
 # 262,144-pixel workload (profiles/k_mixed_resident_wf262144.md)
-K_PERSIST_DRAM_BYTES = 44_619_520  # read 43,064,576 + write 1,554,944
+K_PERSIST_DRAM_BYTES = 44_860_000  # read 43.07 MB + write 1.79 MB
 # the structured inner operator's cutoff (DS_DEFAULT_STRUCTURED_INNER_CUTOFF)
 SG_INNER_CUT = 14.0
-# FP64-pipe instructions per evaluated pair of the plain FP64 kernel
-# k_pair_f64<EXACT, PRODUCT> on the 262,144-pixel workload, from one ncu
-# capture (FP64-pipe busy fraction x 2 per clock x active SM cycles / the
-# launch's evaluated pairs; profiles/k_pair_f64_exact_wf262144.md)
-K_PAIR_F64_EXACT_OPS = 17.4
+# Bytes of a stored pair of the plain FP64 operator beyond 65,536 pixels (value and
+# 32-bit column index), streamed once per product.
+PAIR_VALS_BYTES = 12.0
 # Plain FP64 iteration count of the workload (tol 1e-8, exact kernel), for the
 # CPU-baseline extrapolation of the reference arm.
 REF_ITERS = {"wf-262144px-grf": 162, "wf-32768px-grf": 150}
@@ -888,18 +886,19 @@ def run_ours(args, rank, world, local):
         pprof = ctx.profile()
         ctx.set_profiling(False)
         p_gps = pprof["f64_evaluated"] / (pprof["f64_ms"] * 1e-3) if pprof["f64_ms"] else None
-        p_peak = DFMA_RATE / K_PAIR_F64_EXACT_OPS * SMS * sm_hz
+        p_hbm = measured_peaks().get("hbm_gbs")
+        p_peak = p_hbm * 1e9 / PAIR_VALS_BYTES if p_hbm else None
         kernels["fp64_plain_matvec"] = {
-            "kernel": "k_pair_f64<EXACT> (plain FP64 PCG products and residuals)",
+            "kernel": "FP64 products and residuals of the plain PCG from the stored pair values",
             "launches_per_solve": pprof["f64_launches"],
             "ms_per_launch": pprof["f64_ms"] / max(pprof["f64_launches"], 1),
             "Gpair_per_s": p_gps / 1e9 if p_gps else None,
-            "fp64_ops_per_pair": K_PAIR_F64_EXACT_OPS,
-            "peak_Gpair_per_s": p_peak / 1e9,
-            "frac": p_gps / p_peak if p_gps else None,
-            "peak_basis": (f"FP64 pipe: {DFMA_RATE:.0f} FP64 instructions/clk/SM x {SMS} SMs "
-                           f"x median SM clock / {K_PAIR_F64_EXACT_OPS} FP64 instructions per "
-                           "evaluated pair (ncu capture)")}
+            "bytes_per_pair": PAIR_VALS_BYTES,
+            "peak_Gpair_per_s": p_peak / 1e9 if p_peak else None,
+            "frac": p_gps / p_peak if p_gps and p_peak else None,
+            "peak_basis": (f"measured HBM bandwidth / {PAIR_VALS_BYTES:.0f} bytes per pair (value "
+                           "and column index; vectors and gathers stay in L2); launches that a "
+                           "flag skips included")}
         t0 = time.perf_counter()
         grid.product_dev(op, xp, mpl)
         ctx.synchronize()
