@@ -5,22 +5,23 @@
 // but the launches: every reduction is segmented by chunk, and a chunk whose
 // right-hand sides have all converged is skipped by every kernel.
 //
-// One iteration (captured once as a CUDA graph and replayed):
+// One iteration (the body of one graph's WHILE node):
 //   MV   q = A32 p for every RHS; persistent launch pulling (row tile, RHS
 //        block) items heaviest-first from a work queue; the S value of a pair
 //        is generated once per item and applied to RB right-hand sides
 //   S1   alpha = r.z / p.q per (chunk, RHS)
 //   U2   x_c += alpha p; r -= alpha q; z = r / pd; partial r.z, r.r per tile
 //   S2   new r.z, |r|, beta; hold the RHS that want a reliable update; the
-//        chunk updates once all its active RHS are held
-//   U3   p = z + beta p (RHS still iterating)
+//        chunk updates once all its active RHS are held: its tiles join the
+//        list that U4 to U6 run over
+//   U3   p = z + beta p (RHS still iterating; tensor-core variant: U3 and U7
+//        are part of the next MV's packing of p)
 //   U4   x += x_c in FP64; x_c = 0 (update pending)
 //   R5   r64 = b - A x in FP64 for chunks with an update pending
 //   U6   r = float(r64); z = r / pd; partial r.z, |r64|^2
 //   S6   FP64 stopping test, restart of the recurrence, beta
 //   U7   p = z + beta p after an update;  S7 clears the update flags
-// The host replays the graph and reads the number of active chunks every
-// 8 iterations.
+// The loop ends on the device when no chunk is active.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>

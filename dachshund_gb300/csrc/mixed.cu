@@ -815,6 +815,7 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   // up to each update (persist_pairs.cu), the same values as the kernels below.
   const bool rounds = !op->sgrid && !pc && !use_tc && op->iter_form == DS_ITER_AUTO &&
                       !op->ctx->prof.enabled && max_iter > 0 && mixed_pairs_usable(op, f, g);
+  unsigned int rounds_err = 0;  // barrier whose wait ran out
   if (rounds) {
     persisted = true;
     do {
@@ -827,10 +828,8 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
       DS_CUDA(cudaMemcpyAsync(bar, f.round_bar.p, sizeof(bar), cudaMemcpyDeviceToHost, st));
       DS_CUDA(cudaMemcpyAsync(f.h_state.p, S, sizeof(h), cudaMemcpyDeviceToHost, st));
       DS_CUDA(cudaStreamSynchronize(st));
-      if (bar[1])
-        throw Error{DS_ERR_TIMEOUT, "persistent mixed solve: a grid barrier wait timed out "
-                                    "(barrier " + std::to_string(bar[1]) + ")"};
-    } while (!f.h_state.p->done);
+      rounds_err = bar[1];
+    } while (!rounds_err && !f.h_state.p->done);
   }
   if (!persisted)  // the host polls the done flag (the persistent launch needs no events)
     for (auto& e : evs) DS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -890,6 +889,9 @@ void run_mixed(ds_operator* op, const ds_mixed_params& mp, ds_pcg_result& res,
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
 
+  if (rounds_err)
+    throw Error{DS_ERR_TIMEOUT, "persistent mixed solve: a grid barrier wait timed out "
+                                "(barrier " + std::to_string(rounds_err) + ")"};
   if (persisted && !rounds) {
     const int code = persistent_error(op, st);
     if (code)

@@ -250,10 +250,13 @@ int ds_operator_set_inner_matvec(ds_operator* op, int variant);
  * and a band preconditioner (cluster or learned), the whole iteration loop
  * is one cooperative launch whose CTAs stay resident and meet at bounded
  * grid barriers (the call returns DS_ERR_TIMEOUT if a barrier wait runs out,
- * see ds_context_set_wait_limit); otherwise, and with DS_ITER_GRAPH, eight
- * iterations are one CUDA graph replayed until the solve ends.  Both run the
- * same recurrence; sums are taken in a different order, so iteration counts
- * can differ by rounding. */
+ * see ds_context_set_wait_limit); with the CUDA-core pair kernels and the
+ * Jacobi preconditioner (up to 155,648 pixels) the iterations up to each
+ * reliable update are one such launch, with every value of the graph form;
+ * otherwise, and with DS_ITER_GRAPH, eight iterations are one CUDA graph
+ * replayed until the solve ends.  All run the same recurrence; with a
+ * preconditioner sums are taken in a different order, so iteration counts can
+ * differ by rounding. */
 enum { DS_ITER_AUTO = 0, DS_ITER_GRAPH = 1 };
 int ds_operator_set_iteration_form(ds_operator* op, int form);
 
