@@ -3,8 +3,8 @@
 // stands in for WFVector{SN,W}::solve_cf (lib/wf_vector.cc:123-155, 276-319).
 //
 // Dense matvec: A streamed once per product (8 n^2 bytes) by a persistent
-// grid over 64 x 2048 blocks, HBM-bound with float-pair arithmetic on the
-// FP32 pipe (see the matvec section below).
+// grid over 64-row items of its nonzero 64 x 64 blocks, HBM-bound with float-pair
+// arithmetic on the FP32 pipe (see the matvec section below).
 // Cholesky: right-looking, 32-wide panels: diagonal block in shared memory by
 // one CTA, the panel by a triangular solve per row, the trailing lower
 // triangle by 64 x 64 tiles (each thread a 4 x 4 block).
@@ -27,9 +27,24 @@ constexpr int DTILE = 64;    // trailing-update tile
 constexpr int DM_WARPS = 8;
 constexpr int DM_ROWS = 8;                  // rows per warp
 constexpr int DM_RB = DM_WARPS * DM_ROWS;   // rows per work item
-constexpr int DM_CW = 2048;                 // columns per work item
-constexpr int DM_STEP = 64;                 // columns per warp step: DM_CW / 32
+constexpr int DM_STEP = 64;                 // columns per warp step: a block
+constexpr int DM_CW = 32 * DM_STEP;         // columns per word of the nonzero blocks' mask
+constexpr int DM_WORDS = 2;                 // mask words per work item at most
 constexpr int DM_CTAS_PER_SM = 2;
+
+// Blocks per work item: the most (an item's FP64 row sums, arrival and partials take
+// some 15,000 clocks, as long as its loads of 8 blocks) that leave four items per
+// resident CTA, not less than 4.  Rows of up to 2,048 columns stay one item and one
+// running sum.  Solves to 1e-11 (items of 32 blocks -> this rule): 32,768 pixels 61.1
+// -> 58.1 ms (64 blocks; 73 with 128: uneven shares), 8,192 18.2 -> 14.4 ms (8).
+inline int dense_span(int n, int sms) {
+  int span = 32 * DM_WORDS;
+  const int least = n <= DM_CW ? 32 : 4;
+  while (span > least && (long long)(n / DM_RB) * ((n / DM_STEP + span - 1) / span) <
+                             4ll * DM_CTAS_PER_SM * sms)
+    span /= 2;
+  return span;
+}
 
 // A_ij of the operator for every (i, j) < n (row-major, leading dim ld), in
 // the order of the given coordinate/coefficient arrays (sorted or caller);
@@ -84,13 +99,13 @@ __global__ void k_dense_build(KernelConsts kc, int n, size_t ld, const double* _
 // ---- dense matvec ------------------------------------------------------------
 //
 // q = A v (+ the last CTA's alpha = delta / (dotv . q)) or r = b - A v, A in
-// HBM (n x n FP64, row-major, sorted order).  Work items are 64-row x
-// 2048-column blocks of A pulled by a persistent grid (CTA count a multiple
-// of the SM count); each warp streams 8 rows of its block with 16-byte
+// HBM (n x n FP64, row-major, sorted order).  Work items are 64 rows times 256 to
+// 4,096 columns of A (dense_span) pulled by a persistent grid (CTA count a multiple
+// of the SM count); each warp streams 8 rows of its item, a 64-column block ahead, with 16-byte
 // evict-first loads (every byte of A read once per product), and the column
-// slice of v is read through L1 (the 8 warps of a CTA share it).  Per-block
-// row sums go to a partial buffer; the last block of a row block to finish
-// (an atomic count) adds its rows' partials in column-block order, so the
+// slice of v is read through L1 (the 8 warps of a CTA share it).  Per-item
+// row sums go to a partial buffer; the last item of a row block to finish
+// (an atomic count) adds its rows' partials in column order, so the
 // result does not depend on the finishing order.
 //
 // Two arithmetics:
@@ -116,14 +131,16 @@ __global__ void k_dense_build(KernelConsts kc, int n, size_t ld, const double* _
 struct DenseMv {
   int n;     // rows = columns (n_pad, a multiple of 128)
   int nrb;   // row blocks
-  int ncb;   // column blocks
+  int ncb;   // mask words per row block
+  int span;  // blocks per work item: 4, 8, ..., 32 DM_WORDS
+  int nsp;   // work items per row block
   const double* A;
   const double* v;    // FP64 arithmetic
   const float2* vff;  // FLOAT_PAIR arithmetic: v as (head, tail) floats
   const double* b;
   double* out;
   const double* dotv;
-  double* part;       // ncb x n row partials
+  double* part;       // nsp x n row partials
   double* dot_part;   // nrb
   unsigned int* rb_cnt;  // nrb arrival counts (zero between launches)
   unsigned int* cnt;     // row blocks finished (zero between launches)
@@ -131,7 +148,8 @@ struct DenseMv {
   const int* skip;
   unsigned long long* prof_pairs;
   const unsigned* mask;      // nonzero 64 x 64 blocks, nrb x ncb words
-  const unsigned* need;      // per row block: its words that are not 0
+  const unsigned* need;      // per row block: its items with a nonzero block
+  const unsigned char* on;   // nrb x nsp: the item has a nonzero block
   const unsigned* nonfinite; // v holds an infinity or a NaN
 };
 
@@ -189,30 +207,50 @@ __global__ void k_split_vec(int n, const double* __restrict__ v, float2* __restr
   }
 }
 
+// Mask words of an item (all zero past the last one): the first is shifted so that
+// bit 0 is its word's first block.
+__device__ __forceinline__ void item_words(const DenseMv& a, int item, bool full,
+                                           unsigned (&w)[DM_WORDS]) {
+  const int sp = item / a.nrb, rb = item - sp * a.nrb, b0 = sp * a.span;
+#pragma unroll
+  for (int k = 0; k < DM_WORDS; ++k) {
+    const int wi = b0 / 32 + k;
+    w[k] = 0;
+    if (sp >= a.nsp || wi >= a.ncb || (k > 0 && 32 * k >= a.span)) continue;
+    w[k] = full ? 0xffffffffu >> (32 - min(DM_CW, a.n - wi * DM_CW) / DM_STEP)
+                : a.mask[(size_t)rb * a.ncb + wi];
+    if (a.span < 32) w[k] &= ((1u << a.span) - 1) << (b0 & 31);
+  }
+}
+
 template <bool FF, bool SIGNED, bool RESIDUAL, bool DOT>
 __global__ void __launch_bounds__(DM_WARPS * 32, DM_CTAS_PER_SM) k_dense_mv(DenseMv a) {
   if (a.skip && *a.skip) return;
   __shared__ double red[DM_WARPS];
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int n_items = a.nrb * a.ncb;
+  const int n_items = a.nrb * a.nsp;
   const bool full = *a.nonfinite != 0;
   if (a.prof_pairs && blockIdx.x == 0) {  // entries read
     unsigned long long steps = 0;
-    for (int k = tid; k < n_items; k += DM_WARPS * 32)
+    for (int k = tid; k < a.nrb * a.ncb; k += DM_WARPS * 32)
       steps += full ? min(DM_CW, a.n - k % a.ncb * DM_CW) / DM_STEP : __popc(a.mask[k]);
     atomicAdd(a.prof_pairs, steps * DM_RB * DM_STEP);
   }
   // row blocks fastest: the items of one CTA lie all over the matrix, whose
   // nonzero blocks gather near the diagonal
+  unsigned next[DM_WORDS];  // the next item's mask words
+  item_words(a, blockIdx.x, full, next);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int cb = item / a.nrb, rb = item - cb * a.nrb;
-    const int c0 = cb * DM_CW;
-    unsigned todo = a.mask[(size_t)rb * a.ncb + cb];
-    if (full) todo = 0xffffffffu >> (32 - min(DM_CW, a.n - c0) / DM_STEP);
-    if (!todo) continue;
+    const int sp = item / a.nrb, rb = item - sp * a.nrb;
+    unsigned w[DM_WORDS];
+#pragma unroll
+    for (int k = 0; k < DM_WORDS; ++k) w[k] = next[k];
+    item_words(a, item + (int)gridDim.x, full, next);
+    if (!(w[0] | w[1])) continue;
+    int c0 = sp * a.span / 32 * DM_CW;  // the current word's first column
     const int r0 = rb * DM_RB + warp * DM_ROWS;
-    const double* Ab = a.A + (size_t)r0 * a.n + c0 + 2 * lane;
+    const double* Ab = a.A + (size_t)r0 * a.n + 2 * lane;
     float sh[DM_ROWS], sl[DM_ROWS];
     double acc[DM_ROWS];
 #pragma unroll
@@ -220,45 +258,56 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_CTAS_PER_SM) k_dense_mv(Dens
       sh[r] = sl[r] = 0.f;
       acc[r] = 0.0;
     }
-    // two blocks at a time, their loads first
-    while (todo) {
-      const int s0 = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int s1 = todo ? __ffs(todo) - 1 : s0;
-      const bool two = todo != 0;
-      todo &= todo - 1;
-      uint4 q[2][DM_ROWS];
-#pragma unroll
-      for (int r = 0; r < DM_ROWS; ++r)
-        q[0][r] = ld_stream16(Ab + (size_t)r * a.n + DM_STEP * s0);
-      if (two) {
-#pragma unroll
-        for (int r = 0; r < DM_ROWS; ++r)
-          q[1][r] = ld_stream16(Ab + (size_t)r * a.n + DM_STEP * s1);
+    // one block ahead: block k + 1 is in flight while block k is multiplied
+    struct Blk {
+      uint4 q[DM_ROWS];
+      float4 v;  // two float pairs, or two doubles
+      bool any;
+    };
+    auto fetch = [&](Blk& k) {
+      if (!w[0]) {
+        w[0] = w[1];
+        w[1] = 0;
+        c0 += DM_CW;
       }
+      k.any = w[0] != 0;
+      if (!w[0]) return;
+      const int c = c0 + DM_STEP * (__ffs(w[0]) - 1);
+      w[0] &= w[0] - 1;
 #pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {
-        if (h2 == 1 && !two) break;
-        const int c = c0 + DM_STEP * (h2 ? s1 : s0) + 2 * lane;
-        if (FF) {
-          const float4 vv = __ldg(reinterpret_cast<const float4*>(a.vff + c));
+      for (int r = 0; r < DM_ROWS; ++r) k.q[r] = ld_stream16(Ab + (size_t)r * a.n + c);
+      k.v = FF ? __ldg(reinterpret_cast<const float4*>(a.vff + c + 2 * lane))
+               : __ldg(reinterpret_cast<const float4*>(a.v + c + 2 * lane));
+    };
+    auto multiply = [&](const Blk& k) {
+      if (FF) {
 #pragma unroll
-          for (int r = 0; r < DM_ROWS; ++r) {
-            float h, l;
-            split_f64<SIGNED>(q[h2][r].x, q[h2][r].y, h, l);
-            ff_mac(h, l, vv.x, vv.y, sh[r], sl[r]);
-            split_f64<SIGNED>(q[h2][r].z, q[h2][r].w, h, l);
-            ff_mac(h, l, vv.z, vv.w, sh[r], sl[r]);
-          }
-        } else {
-          const double2 vv = __ldg(reinterpret_cast<const double2*>(a.v + c));
+        for (int r = 0; r < DM_ROWS; ++r) {
+          float h, l;
+          split_f64<SIGNED>(k.q[r].x, k.q[r].y, h, l);
+          ff_mac(h, l, k.v.x, k.v.y, sh[r], sl[r]);
+          split_f64<SIGNED>(k.q[r].z, k.q[r].w, h, l);
+          ff_mac(h, l, k.v.z, k.v.w, sh[r], sl[r]);
+        }
+      } else {
+        const double v0 = __hiloint2double(__float_as_int(k.v.y), __float_as_int(k.v.x));
+        const double v1 = __hiloint2double(__float_as_int(k.v.w), __float_as_int(k.v.z));
 #pragma unroll
-          for (int r = 0; r < DM_ROWS; ++r) {
-            acc[r] = fma(__hiloint2double((int)q[h2][r].y, (int)q[h2][r].x), vv.x, acc[r]);
-            acc[r] = fma(__hiloint2double((int)q[h2][r].w, (int)q[h2][r].z), vv.y, acc[r]);
-          }
+        for (int r = 0; r < DM_ROWS; ++r) {
+          acc[r] = fma(__hiloint2double((int)k.q[r].y, (int)k.q[r].x), v0, acc[r]);
+          acc[r] = fma(__hiloint2double((int)k.q[r].w, (int)k.q[r].z), v1, acc[r]);
         }
       }
+    };
+    Blk k0, k1;
+    fetch(k0);
+    for (;;) {
+      fetch(k1);
+      multiply(k0);
+      if (!k1.any) break;
+      fetch(k0);
+      multiply(k1);
+      if (!k0.any) break;
     }
     // this block's row sums: lane partials in FP64, fixed tree.  Every lane
     // halves its rows three times (9 FP64 additions instead of 40).
@@ -276,19 +325,29 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_CTAS_PER_SM) k_dense_mv(Dens
     }
     t[0] += __shfl_xor_sync(0xffffffffu, t[0], 2);
     t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
-    if ((lane & 3) == 0) a.part[(size_t)cb * a.n + r0 + (lane >> 2)] = t[0];
+    if ((lane & 3) == 0) a.part[(size_t)sp * a.n + r0 + (lane >> 2)] = t[0];
     __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&a.rb_cnt[rb], 1u) == (full ? a.ncb : a.need[rb]) - 1;
+    if (tid == 0) s_last = atomicAdd(&a.rb_cnt[rb], 1u) == (full ? (unsigned)a.nsp : a.need[rb]) - 1;
     __syncthreads();
-    if (s_last) {  // every (nonzero) column block of this row block is in: finish its rows
+    if (s_last) {  // every (nonzero) item of this row block is in: finish its rows
       __threadfence();
       double dot = 0.0;
       if (tid < DM_RB) {
         const int row = rb * DM_RB + tid;
         double sum = 0.0;
-        for (int k = 0; k < a.ncb; ++k)
-          if (full || a.mask[(size_t)rb * a.ncb + k]) sum += __ldcg(a.part + (size_t)k * a.n + row);
+        const unsigned char* on = a.on + (size_t)rb * a.nsp;
+        constexpr int U = 8;  // partials in flight
+        for (int k = 0; k < a.nsp; k += U) {
+          double v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            v[u] = k + u < a.nsp && (full || on[k + u]) ? __ldcg(a.part + (size_t)(k + u) * a.n + row)
+                                                        : 0.0;
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (k + u < a.nsp && (full || on[k + u])) sum += v[u];
+        }
         const double o = RESIDUAL ? a.b[row] - sum : sum;
         a.out[row] = o;
         if (DOT) dot = a.dotv[row] * o;
@@ -316,15 +375,24 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_CTAS_PER_SM) k_dense_mv(Dens
   }
 }
 
-// Per row block the number of mask words that are not 0; a row block of
+// Per row block its items with a nonzero block and their number; a row block of
 // padding alone gets one block to read, so that its rows are written.
-__global__ void k_dense_need(int nrb, int ncb, unsigned* __restrict__ mask,
-                             unsigned* __restrict__ need) {
+__global__ void k_dense_need(int nrb, int ncb, int span, int nsp, unsigned* __restrict__ mask,
+                             unsigned char* __restrict__ on, unsigned* __restrict__ need) {
   const int rb = blockIdx.x * blockDim.x + threadIdx.x;
   if (rb >= nrb) return;
+  unsigned* m = mask + (size_t)rb * ncb;
+  bool any = false;
+  for (int k = 0; k < ncb; ++k) any |= m[k] != 0;
+  if (!any) m[0] = 1;
   unsigned c = 0;
-  for (int k = 0; k < ncb; ++k) c += mask[(size_t)rb * ncb + k] != 0;
-  if (!c) mask[(size_t)rb * ncb] = c = 1;
+  for (int s = 0; s < nsp; ++s) {
+    unsigned bits = 0;
+    for (int b = s * span; b < (s + 1) * span && b < 32 * ncb; ++b)
+      bits |= (m[b / 32] >> (b % 32)) & 1u;
+    on[(size_t)rb * nsp + s] = (unsigned char)bits;
+    c += bits;
+  }
   need[rb] = c;
 }
 
@@ -491,6 +559,7 @@ void op_free_dense(ds_operator* op) {
   op->dense.release();
   op->dense_vff.release();
   op->dense_part.release();
+  op->dense_on.release();
   op->dense_dot.release();
   op->dense_cnt.release();
   op->dense_mask.release();
@@ -514,8 +583,10 @@ void op_build_dense(ds_operator* op) {
       op->kc, (int)np, np, op->pix.x.p, op->pix.y.p, op->pix.z.p, op->wl.p, op->e.p,
       op->table.p, op->dense.p, stats.p, op->dense_mask.p);
   DS_CHECK_LAUNCH();
-  k_dense_need<<<(unsigned)((nrb + 127) / 128), 128, 0, st>>>((int)nrb, (int)ncb,
-                                                              op->dense_mask.p, op->dense_need.p);
+  const int span = dense_span((int)np, sms), nsp = ((int)np / DM_STEP + span - 1) / span;
+  op->dense_on.alloc(nrb * nsp);
+  k_dense_need<<<(unsigned)((nrb + 127) / 128), 128, 0, st>>>(
+      (int)nrb, (int)ncb, span, nsp, op->dense_mask.p, op->dense_on.p, op->dense_need.p);
   DS_CHECK_LAUNCH();
   unsigned long long h[3];
   DS_CUDA(cudaMemcpyAsync(h, stats.p, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -527,7 +598,7 @@ void op_build_dense(ds_operator* op) {
   op->dense_ff_ok = mx <= hi && (h[0] == ~0ull || mn >= lo);
   op->dense_signed = h[2] != 0;
   op->dense_vff.alloc(np);
-  op->dense_part.alloc(ncb * np);
+  op->dense_part.alloc((size_t)nsp * np);
   op->dense_dot.alloc(nrb);
   op->dense_cnt.alloc(nrb + 1);
   DS_CUDA(cudaMemsetAsync(op->dense_cnt.p, 0, (nrb + 1) * sizeof(unsigned int), st));
@@ -561,6 +632,10 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
   a.n = np;
   a.nrb = np / DM_RB;
   a.ncb = (np + DM_CW - 1) / DM_CW;
+  const int sms = op->ctx->num_sms > 0 ? op->ctx->num_sms : 152;
+  a.span = dense_span(np, sms);
+  a.nsp = (np / DM_STEP + a.span - 1) / a.span;
+  a.on = op->dense_on.p;
   a.A = op->dense.p;
   a.v = v;
   a.vff = op->dense_vff.p;
@@ -577,8 +652,7 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
   a.need = op->dense_need.p;
   a.nonfinite = op->dense_need.p + a.nrb;
   const bool ff = dense_arith_in_use(op) == DS_DENSE_FLOAT_PAIR;
-  const int sms = op->ctx->num_sms > 0 ? op->ctx->num_sms : 152;
-  const int grid = std::min(a.nrb * a.ncb, sms * DM_CTAS_PER_SM);
+  const int grid = std::min(a.nrb * a.nsp, sms * DM_CTAS_PER_SM);
   Profiler& prof = op->ctx->prof;
   cudaEvent_t ev = nullptr;
   if (prof.enabled) {
