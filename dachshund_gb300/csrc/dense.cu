@@ -199,12 +199,8 @@ __device__ __forceinline__ uint4 ld_stream16(const double* p) {
 __global__ void k_split_vec(int n, const double* __restrict__ v, float2* __restrict__ vff,
                             unsigned* nonfinite, const int* skip) {
   if (skip && *skip) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double x = v[i];
-    if (!isfinite(x)) *nonfinite = 1u;
-    const float h = __double2float_rn(x);
-    vff[i] = make_float2(h, __double2float_rn(x - (double)h));
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    vff[i] = dense_split(v[i], nonfinite);
 }
 
 // Mask words of an item (all zero past the last one): the first is shifted so that
@@ -624,8 +620,13 @@ void launch_dense_mv(const DenseMv& a, bool residual, bool dot, int grid, cudaSt
 
 }  // namespace
 
+unsigned* dense_nonfinite(ds_operator* op) {
+  return op->dense_need.p + op->pix.n_pad / DM_RB;
+}
+
 void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
-                 const double* dotv, PcgState* pcg, const int* skip, cudaStream_t st) {
+                 const double* dotv, PcgState* pcg, const int* skip, cudaStream_t st,
+                 bool is_split) {
   const int np = op->pix.n_pad;
   require(np % DM_RB == 0 && op->dense.p, "dense operator not built");
   DenseMv a{};
@@ -650,7 +651,7 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
   a.skip = skip;
   a.mask = op->dense_mask.p;
   a.need = op->dense_need.p;
-  a.nonfinite = op->dense_need.p + a.nrb;
+  a.nonfinite = dense_nonfinite(op);
   const bool ff = dense_arith_in_use(op) == DS_DENSE_FLOAT_PAIR;
   const int grid = std::min(a.nrb * a.nsp, sms * DM_CTAS_PER_SM);
   Profiler& prof = op->ctx->prof;
@@ -659,10 +660,12 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
     a.prof_pairs = prof.d_pairs + 3;
     prof.begin(st, &ev);
   }
-  DS_CUDA(cudaMemsetAsync(op->dense_need.p + a.nrb, 0, sizeof(unsigned), st));
-  k_split_vec<<<std::min((np + 255) / 256, 4 * sms), 256, 0, st>>>(
-      np, v, op->dense_vff.p, op->dense_need.p + a.nrb, skip);
-  DS_CHECK_LAUNCH();
+  if (!is_split) {
+    DS_CUDA(cudaMemsetAsync(dense_nonfinite(op), 0, sizeof(unsigned), st));
+    k_split_vec<<<std::min((np + 255) / 256, 4 * sms), 256, 0, st>>>(
+        np, v, op->dense_vff.p, dense_nonfinite(op), skip);
+    DS_CHECK_LAUNCH();
+  }
   if (ff) {
     if (op->dense_signed)
       launch_dense_mv<true, true>(a, residual, dotv != nullptr, grid, st);

@@ -23,6 +23,14 @@ __device__ __forceinline__ double block_sum(double v, double* sm /* NT/32 */) {
   return s;
 }
 
+// An element of the dense product's vector as a float pair; *nonfinite = 1 for an
+// infinity or a NaN.
+__device__ __forceinline__ float2 dense_split(double x, unsigned* nonfinite) {
+  if (!isfinite(x)) *nonfinite = 1u;
+  const float h = __double2float_rn(x);
+  return make_float2(h, __double2float_rn(x - (double)h));
+}
+
 // Every block calls this once after writing its partial result (thread 0);
 // returns true in exactly one block, the last to arrive, which then sees all
 // partials.  The counter is reset by that block.

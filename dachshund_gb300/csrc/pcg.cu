@@ -107,13 +107,16 @@ __global__ void __launch_bounds__(VB) k_pcg_direction(int n, const PcgState* st,
                                                       const double* __restrict__ s,
                                                       double* __restrict__ d, double var_s,
                                                       const double* __restrict__ wr,
-                                                      double* __restrict__ u) {
+                                                      double* __restrict__ u,
+                                                      float2* __restrict__ vff,
+                                                      unsigned* nonfinite) {
   if (st->done) return;
   const double beta = st->beta;
   for (int i = blockIdx.x * VB + threadIdx.x; i < n; i += gridDim.x * VB) {
     const double di = fma(beta, d[i], s[i]);
     d[i] = di;
     if (u) u[i] = var_s * (wr[i] * di);
+    if (vff) vff[i] = dense_split(di, nonfinite);
   }
 }
 
@@ -275,7 +278,7 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   int issued = 0, waited = 0;
   for (int it = 1; it < pp.max_iter && !persistent; ++it) {
     if (op->use_dense)  // q = A d, alpha
-      dense_apply(op, false, op->d.p, op->q.p, op->d.p, S, &S->done, st);
+      dense_apply(op, false, op->d.p, op->q.p, op->d.p, S, &S->done, st, it > 1);
     else if (vals)
       launch_pair_vals(op, EPI_PRODUCT, prod, st);
     else
@@ -298,7 +301,15 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
                                         op->pdiag.p, op->partial.p, op->hist.p, op->dhist.p);
     }
     DS_CHECK_LAUNCH();
-    k_pcg_direction<<<g, VB, 0, st>>>(np, S, op->s.p, op->d.p, op->kc.var_s, op->wr.p, u);
+    // (the dense product's float pairs of d are formed here: a launch of their own
+    // took 4 of some 30 us an iteration at 1,280 pixels)
+    unsigned* flag = nullptr;
+    if (op->use_dense) {
+      flag = dense_nonfinite(op);
+      DS_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
+    }
+    k_pcg_direction<<<g, VB, 0, st>>>(np, S, op->s.p, op->d.p, op->kc.var_s, op->wr.p, u,
+                                      op->use_dense ? op->dense_vff.p : nullptr, flag);
     DS_CHECK_LAUNCH();
     if (it % CHECK == 0) {
       const int slot = issued % NSLOT;
