@@ -1,5 +1,5 @@
-// Sums and CG scalars of the mixed-precision solves in float pairs, shared by the
-// persistent (persist.cu) and the per-kernel form (mixed.cu, pair_f32.cu).
+// Sums and CG scalars of the mixed-precision solves in float pairs: the persistent
+// structured form (persist.cu) and the batched solve's vector sums (batch.cu).
 #pragma once
 
 #include "ds_f32.h"
@@ -26,9 +26,9 @@ __device__ __forceinline__ ff ff_shfl_down(ff v, int o, int width = 32) {
 // Sums over the CTA of two float pairs per thread (float-pair shuffle trees, a
 // fixed order), valid in lanes 0 and 16 of warp 0.  The Krylov vectors' dot
 // products are summed this way from the threads to the grid (exact products by
-// FMA, compensated sums, about 44 bits): a dependent FP64 instruction has a
-// latency of some 400 clocks on GB300, and the FP64 sums and scalars of a
-// persistent iteration took 14,000 of its 22,000 clocks at 16 CTAs.
+// FMA, compensated sums, about 44 bits): a dependent FP64 addition takes 300
+// clocks with the SM's 16 warps at it (66 with 4), and the FP64 sums and scalars
+// of a persistent iteration took 14,000 of its 22,000 clocks at 16 CTAs.
 template <int NT>
 __device__ __forceinline__ ff block_sum2_ff(ff v, ff w, float2* sm /* 2 NT / 32 */) {
   constexpr int W = NT / 32;
