@@ -88,19 +88,6 @@ void build_ff_points(FFData& f, const PointSet& ps, const KernelConsts& kc, cuda
 void launch_pair_ff_resid(const KernelConsts& kc, const PairArgs& a, const FFPoints& f,
                           cudaStream_t st);
 
-// The recurrence's scalars between two updates in float pairs and FP32 (see
-// ds_ffsum.cuh); a MixedState holds them in FP64 at the ends and across updates.
-// The norms only decide when an update is due, whose FP64-accurate residual
-// decides the solve.  The sums take sr r, sz z, sr q and sz p, powers of two that
-// bring the first |r| and r.z to about 1: the squares of vectors in units far
-// from 1 (fluxes of 1e-17) would leave FP32's range.
-struct FastState {
-  ff rz, rz_old, alpha, pq;  // rz, rz_old, pq times sr sz
-  float beta, rnorm, rmax, rbest, delta, tol;  // the norms times sr
-  float sr, sz;
-  int it_best;
-};
-
 // Device state of the reliable-update mixed-precision PCG.
 struct MixedState {
   double rz;          // r . z (FP32 vectors, FP64 sum)
@@ -129,7 +116,6 @@ struct MixedState {
                       // FP32 one is far above tol)
   int pad2;
   unsigned int counter[4];
-  FastState fast;     // the scalars of the forms that sum in float pairs
 };
 
 // The persistent form of the Jacobi iteration (persist_pairs.cu); g: the grid of
@@ -137,9 +123,6 @@ struct MixedState {
 bool mixed_pairs_usable(ds_operator* op, struct OpF32& f, int g);
 void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, int g,
                         cudaStream_t st);
-
-// The |r| history of a form that sums in float pairs, from what it left there.
-void launch_hist_roots(const MixedState* s, double* hist, int max_iter, cudaStream_t st);
 
 // FP32 operator data, built on the first mixed-precision call.
 struct OpF32 {

@@ -165,24 +165,26 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // may work on its own data (writing nothing another CTA reads in the next
 // phase), which hides that work behind the barrier's latency.
 constexpr int BAR_WORDS = 32;  // one 128-byte line
-// Thread 0's barrier state.  The phase timers accumulate in shared memory and
-// go to global memory once, at the kernel's end: a read-modify-write of global
-// memory in front of the arrival's release held up every barrier.
+// Thread 0's barrier state and phase timers, in shared memory (timers go to global
+// memory once, at the kernel's end): a read-modify-write of global memory or a
+// register spilled to local memory in front of the arrival's release held up every
+// barrier (1.0 -> 1.25 us with 16 CTAs for 48 bytes of spills).
 struct BarState {
-  unsigned int epoch = 0;          // barriers passed
-  unsigned long long exit_ns = 0;  // last exit (%globaltimer)
-  int last = 0;                    // this CTA completed the current epoch (RET)
-};
-struct PhaseTimers {
   unsigned long long phase[8], visits[8], work[8];
+  unsigned long long exit_ns;  // last exit (%globaltimer)
+  unsigned int epoch;          // barriers passed
+  int last;                    // this CTA completed the current epoch (RET)
 };
-__shared__ PhaseTimers s_timers;
+__shared__ BarState s_bar;
 
-__device__ void timers_start(const PersistArgs& a, BarState& b) {
+__device__ void timers_start(const PersistArgs& a) {
+  BarState& b = s_bar;
   if (threadIdx.x < 8)
-    s_timers.phase[threadIdx.x] = s_timers.visits[threadIdx.x] = s_timers.work[threadIdx.x] = 0;
+    s_bar.phase[threadIdx.x] = s_bar.visits[threadIdx.x] = s_bar.work[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     b.exit_ns = global_ns();
+    b.epoch = 0;
+    b.last = 0;
     if (blockIdx.x == 0) {
       a.pt[PT_START] = b.exit_ns;
       a.pt[PT_GRID] = gridDim.x;
@@ -194,20 +196,21 @@ __device__ void timers_start(const PersistArgs& a, BarState& b) {
 __device__ void timers_end(const PersistArgs& a) {
   __syncthreads();
   if (threadIdx.x < 8) {
-    a.pt[PT_CTA + 8 * blockIdx.x + threadIdx.x] += s_timers.work[threadIdx.x];
+    a.pt[PT_CTA + 8 * blockIdx.x + threadIdx.x] += s_bar.work[threadIdx.x];
     if (blockIdx.x == 0) {
-      a.pt[PT_PHASE + threadIdx.x] += s_timers.phase[threadIdx.x];
-      a.pt[PT_VISITS + threadIdx.x] += s_timers.visits[threadIdx.x];
+      a.pt[PT_PHASE + threadIdx.x] += s_bar.phase[threadIdx.x];
+      a.pt[PT_VISITS + threadIdx.x] += s_bar.visits[threadIdx.x];
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.pt[PT_KERNEL] += global_ns() - a.pt[PT_START];
 }
 
 template <bool RET>
-__device__ void grid_arrive(const PersistArgs& a, int code, BarState& b) {
+__device__ void grid_arrive(const PersistArgs& a, int code) {
+  BarState& b = s_bar;
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (b.epoch > 0) s_timers.work[code] += global_ns() - b.exit_ns;
+    if (b.epoch > 0) s_bar.work[code] += global_ns() - b.exit_ns;
     ++b.epoch;
     if (RET) {
       unsigned int old;
@@ -223,7 +226,8 @@ __device__ void grid_arrive(const PersistArgs& a, int code, BarState& b) {
 }
 
 template <bool RET>
-__device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
+__device__ bool grid_wait(const PersistArgs& a, int code) {
+  BarState& b = s_bar;
   __shared__ int ok_s;
   if (threadIdx.x == 0) {
     int ok = 1;
@@ -250,8 +254,8 @@ __device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
       ok = 0;
     }
     const unsigned long long now = global_ns();
-    s_timers.phase[code] += now - b.exit_ns;  // reported for CTA 0
-    s_timers.visits[code] += 1;
+    s_bar.phase[code] += now - b.exit_ns;  // reported for CTA 0
+    s_bar.visits[code] += 1;
     b.exit_ns = now;
     ok_s = ok;
   }
@@ -260,19 +264,19 @@ __device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
 }
 
 template <bool RET>
-__device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code, BarState& b) {
-  grid_arrive<RET>(a, code, b);
-  return grid_wait<RET>(a, code, b);
+__device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code) {
+  grid_arrive<RET>(a, code);
+  return grid_wait<RET>(a, code);
 }
 
 // Sum of n partials in a fixed order by one warp (valid in lane 0), the same in
 // every CTA: lane l takes l, l + 32, ..., then a shuffle tree, so the FP64 pipe
 // (2 operations per clock per SM on GB300) sees n + 5 additions per CTA instead
 // of a CTA-wide tree.
-__device__ __forceinline__ double warp_total(const double* part, int n) {
+__device__ __forceinline__ double warp_total(const double* part, int n, int stride = 1) {
   double v = 0.0;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < n; i += 32) v += __ldcg(part + i);
+  for (int i = threadIdx.x & 31; i < n; i += 32) v += __ldcg(part + (size_t)i * stride);
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
@@ -529,11 +533,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
   const int G = gridDim.x;
   const int P2 = (G + 1) & ~1;  // the pair partials start 16-byte aligned
   const size_t ns = (size_t)a.n_blocks * a.S;
-  BarState bst;  // barrier state (thread 0)
   if (tid == 0) sS = *a.S_;
-  timers_start(a, bst);
+  timers_start(a);
   __syncthreads();
-  for (int k = 0; k < N_CALIB; ++k) grid_sync<true>(a, B_CALIB, bst);
+  for (int k = 0; k < N_CALIB; ++k) grid_sync<true>(a, B_CALIB);
   // the recurrence sets done by iteration max_iter at the latest (the
   // update it forces there ends the solve); the bound keeps hist in range
   while (!sS.done && sS.iter < a.max_iter) {
@@ -548,7 +551,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
           return (float)a.wr[r] * pv;
         });
     }
-    if (!grid_sync<true>(a, B_LEVELS, bst)) break;
+    if (!grid_sync<true>(a, B_LEVELS)) break;
     // ---- B: q = A32 p, partial p.q
     double dq = 0.0;
     for (int blk = blockIdx.x; blk < a.n_blocks; blk += G) {
@@ -573,7 +576,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
       const double bs = block_sum<NT>(dq, red);
       if (tid == 0) a.part[blockIdx.x] = bs;
     }
-    if (!grid_sync<true>(a, B_PRODUCT, bst)) break;
+    if (!grid_sync<true>(a, B_PRODUCT)) break;
     // ---- C: alpha; x, r, z per owned block; partials r.z, |r|^2
     const double pq = partial_total(a.part, G, tot);
     if (tid == 0) tot[0] = sS.rz / pq;
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
         a.part[(size_t)P2 + 2 * blockIdx.x + 1] = b2;
       }
     }
-    if (!grid_sync<true>(a, B_STEP, bst)) break;
+    if (!grid_sync<true>(a, B_STEP)) break;
     {
       const double2 t2 = partial_total2(a.part + P2, G, tot);
       if (tid == 0) step_scalars(sS, a, it, alpha_d, pq, t2.x, t2.y);
@@ -630,7 +633,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
     for (int blk = blockIdx.x; blk < a.n_blocks; blk += G)
       block_levels<double>(a, blk, a.olmax, a.taps64, a.V64, su64,
                            [&](size_t r) { return a.wr[r] * __ldcg(a.x + r); });
-    if (!grid_sync<true>(a, B_LEVELS64, bst)) break;
+    if (!grid_sync<true>(a, B_LEVELS64)) break;
     // ---- E, F: r64 = b - A x per owned skewer; r = r64, z = G G^T r
     rz = 0.0;
     rr = 0.0;
@@ -684,7 +687,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
         a.part[(size_t)P2 + 2 * blockIdx.x + 1] = b2;
       }
     }
-    if (!grid_sync<true>(a, B_UPDATE, bst)) break;
+    if (!grid_sync<true>(a, B_UPDATE)) break;
     {
       const double2 t2 = partial_total2(a.part + P2, G, tot);
       if (tid == 0) update_scalars(sS, a, t2.x, t2.y);
@@ -781,12 +784,17 @@ __device__ __forceinline__ void block_product_ff(const PersistArgs& a, int blk, 
 //
 // With at most one block per CTA (the cooperative grid holds every block),
 // each CTA keeps its block's FP32 vectors p, z, q (record-local order j n_per
-// + k), r (slot order), the FP64 iterate x, the FP32 coefficients and its
-// skewers' FP32 neighbour lists in shared memory for the whole solve: the
-// phases then read global memory only for the neighbours' levels (B), the
-// factor (C) and the partials, and the levels they publish (A, D).  x goes
-// back to global memory at the end.  Same recurrence, same sums in the same
-// order as the general form.
+// + k), r (slot order), the iterate x (float pairs), the FP32 coefficients, its
+// FP16 factor and its product items in shared memory for the whole solve: the
+// phases then read global memory only for the neighbours' levels and the
+// partials, and write the levels they publish.  x goes back to global memory at
+// the end.  The general form's recurrence, rearranged; sums in float pairs within
+// the warps and FP64 from there up (ds_ffsum.cuh).
+//
+// What the sums and scalars cost: 16 CTAs (64 x 64 pixels, 82 iterations) 0.82 ms a
+// launch, 256 CTAs (1,024 x 256, 130 iterations) 3.30; with FP64 sums by all warps,
+// scalars by FP64 divisions and roots, 1.16 and 4.17; in float pairs throughout, of
+// 44 bits, 0.72 and 3.11.
 constexpr int NI = 512;   // product items of a block kept in shared memory
 constexpr int GI = 4;     // skewers per block of the item form at most
 
@@ -940,12 +948,11 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   const int m = a.g * npr;  // records of the block (record-local index j n_per + k)
   const size_t n = (size_t)a.n;
   const size_t ns = (size_t)a.n_blocks * a.S;
-  BarState bst;  // barrier state (thread 0)
   if (tid == 0) {
     sS = *a.S_;
-    fast_init(sF, sS);
+    fast_from(sF, sS, sS.rnorm);
   }
-  timers_start(a, bst);
+  timers_start(a);
   if (tid < MAX_G) sk[tid] = tid < a.g ? skewer_of(a, blk, tid) : -1;
   {  // the block's product items
     const size_t i0 = (size_t)blk * NI;
@@ -960,7 +967,6 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     }
   }
   __syncthreads();
-  const float sr = sF.sr, sz = sF.sz;  // the sums' scales
   for (int i = tid; i < m; i += NT) {
     const int j = i / npr;
     const int s = sk[j];
@@ -1078,10 +1084,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     if (has_pixel) product_rows(part * no / tk, (part + 1) * no / tk);
   };
   levels_z();
-  grid_arrive<false>(a, B_LEVELS, bst);
+  grid_arrive<false>(a, B_LEVELS);
   own_rows();
-  if (grid_wait<false>(a, B_LEVELS, bst)) {
-    for (int k = 0; k < N_CALIB; ++k) grid_sync<false>(a, B_CALIB, bst);
+  if (grid_wait<false>(a, B_LEVELS)) {
+    for (int k = 0; k < N_CALIB; ++k) grid_sync<false>(a, B_CALIB);
   }
   while (!sS.done && sS.iter < a.max_iter) {
       const int it = sS.iter + 1;
@@ -1099,7 +1105,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           for (int j = 0; j < GI; ++j) red_w[(part * GI + j) * npr + kq] = acc[j];
         }
         __syncthreads();  // red_w, s_ab
-        const float beta = s_ab;
+        const float beta = s_ab, sr = sF.sr, sz = sF.sz;
 #pragma unroll
         for (int t = 0; t < RPT; ++t) {
           if (jj[t] < 0) continue;
@@ -1116,17 +1122,17 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       {
-        const ff bs = block_sum2_ff<NT>(dq, ff{0.f, 0.f}, red);
-        if (tid == 0) store_part(a.part + blk, bs);
+        const double bs = block_sum2<NT, false>(dq, ff{0.f, 0.f}, red);
+        if (tid == 0) a.part[blk] = bs;
       }
-      if (!grid_sync<false>(a, B_PRODUCT, bst)) break;
+      if (!grid_sync<false>(a, B_PRODUCT)) break;
       // ---- step: alpha; x, r, z of the block; levels of z; partials.  Warp 0
       // alone adds the CTAs' partials and forms the scalars.
       if (tid < 32) {
-        const ff pq = warp_total_ff(a.part, G);
+        const double pq = warp_total(a.part, G);
         if (tid == 0) {
           sF.pq = pq;
-          sF.alpha = s_alpha = ff_div(sF.rz, pq);
+          sF.alpha = s_alpha = quotient_ff(sF.rz, pq);
           s_ab = s_alpha.h;
         }
       }
@@ -1149,6 +1155,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       {
         float zk[RPT];
         block_precond_h<BAND>(a, Lh, rs, ts, zk);
+        const float sr = sF.sr, sz = sF.sz;
 #pragma unroll
         for (int t = 0; t < RPT; ++t) {
           if (li[t] < 0) continue;
@@ -1161,18 +1168,19 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       }
       levels_z();  // published first: the stores drain while the sums are formed
       {
-        const ff bs = block_sum2_ff<NT>(rz, rr, red);
-        if (tid == 0 || tid == 16) store_part(a.part + (size_t)P2 + 2 * blk + (tid >> 4), bs);
+        const double bs = block_sum2<NT, true>(rz, rr, red);
+        if (tid == 0 || tid == 16) a.part[(size_t)P2 + 2 * blk + (tid >> 4)] = bs;
       }
-      grid_arrive<false>(a, B_STEP, bst);
+      grid_arrive<false>(a, B_STEP);
       own_rows();
-      if (!grid_wait<false>(a, B_STEP, bst)) break;
-      if (tid < 32) {
-        ff trz, trr;
-        warp_total2_ff(a.part + P2, G, trz, trr);
-        if (tid == 0) fast_step(sF, sS, blockIdx.x == 0 ? a.hist : nullptr, it, trz, trr);
+      if (!grid_wait<false>(a, B_STEP)) break;
+      if (tid < 64) {  // warp 0: r.z and beta; warp 1: |r| and the update test
+        const double t = warp_total(a.part + P2 + (tid >> 5), G, 2);
+        if (tid == 0) fast_beta(sF, t);
+        if (tid == 32) fast_norm(sF, sS, it, t);
       }
       __syncthreads();
+      if (blockIdx.x == 0 && tid == 32) a.hist[it] = sF.rr * sF.urr;
       if (!sS.need_update) continue;
       // ---- FP64-accurate update in float pairs (GB300 issues FP64 at 1/64 of
       // FP32): levels of u = wr x, stored as float pairs in the FP64 levels'
@@ -1203,7 +1211,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           V2[(size_t)l * n + rg[t]] = make_float2(acc.h, acc.l);
         }
       }
-      if (!grid_sync<false>(a, B_LEVELS64, bst)) break;
+      if (!grid_sync<false>(a, B_LEVELS64)) break;
       // r64 = b - A x of the block (into us); r = r64, z = G G^T r, levels of z
       {
         ff acc[RPT];
@@ -1242,28 +1250,28 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         for (int t = 0; t < RPT; ++t) {
           if (li[t] < 0) continue;
           zs[li[t]] = zk[t];
-          ff_acc_prod(rz_u, sr * rs[slot_of(a.S, t)], sz * zk[t]);
+          ff_acc_prod(rz_u, sF.sr * rs[slot_of(a.S, t)], sF.sz * zk[t]);
         }
       }
       {
-        const ff b1 = block_sum2_ff<NT>(rz_u, ff{0.f, 0.f}, red);
+        const double b1 = block_sum2<NT, false>(rz_u, ff{0.f, 0.f}, red);
         const double b2 = block_sum<NT>(rr_u, red64);
         if (tid == 0) {
-          a.part[(size_t)P2 + 2 * blk] = ff_double(b1) * (1.0 / ((double)sr * (double)sz));
+          a.part[(size_t)P2 + 2 * blk] = b1 * (1.0 / ((double)sF.sr * (double)sF.sz));
           a.part[(size_t)P2 + 2 * blk + 1] = b2;
         }
       }
       levels_z();
-      grid_arrive<false>(a, B_UPDATE, bst);
+      grid_arrive<false>(a, B_UPDATE);
       own_rows();
-      if (!grid_wait<false>(a, B_UPDATE, bst)) break;
+      if (!grid_wait<false>(a, B_UPDATE)) break;
       if (tid < 32) {
         const double2 t2 = warp_total2(a.part + P2, G);
         if (tid == 0) {
           fast_to(sF, sS);
           update_scalars(sS, a, t2.x, t2.y);
-          if (blockIdx.x == 0) store_hist(a.hist + sS.iter, sF, t2.y);
-          fast_from(sF, sS);
+          if (blockIdx.x == 0) a.hist[sS.iter] = t2.y;
+          fast_from(sF, sS, sS.rtrue);
         }
       }
       __syncthreads();
@@ -1276,7 +1284,6 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
   if (blockIdx.x == 0 && tid == 0) {
     fast_to(sF, sS);
     sS.skip_update = 1;
-    sS.fast = sF;
     *a.S_ = sS;
   }
 }
@@ -1405,15 +1412,11 @@ __global__ void __launch_bounds__(NT) k_build_items(int g, int n_per, int n,
   }
 }
 
-// The roots of the |sr r|^2 that a form with float-pair sums left in
-// hist[1 .. iter].
+// The roots of the |r|^2 that the resident form left in hist[1 .. iter].
 __global__ void k_hist_roots(const MixedState* st, double* __restrict__ hist) {
-  const double ur = 1.0 / (double)st->fast.sr;
   for (int i = 1 + blockIdx.x * blockDim.x + threadIdx.x; i <= st->iter;
-       i += gridDim.x * blockDim.x) {
-    const float2 v = reinterpret_cast<const float2*>(hist)[i];
-    hist[i] = sqrt((double)v.x + (double)v.y) * ur;
-  }
+       i += gridDim.x * blockDim.x)
+    hist[i] = sqrt(hist[i]);
 }
 
 // out = in as float pairs.
@@ -1615,13 +1618,12 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   DS_CUDA(cudaLaunchCooperativeKernel(pick(resident), dim3(grid), dim3(NT), args,
                                       resident ? res_bytes : 0, st));
   DS_CHECK_LAUNCH();
-  if (resident) launch_hist_roots(f.state.p, f.hist.p, max_iter, st);
+  if (resident) {
+    k_hist_roots<<<std::max(1, std::min(64, (max_iter + 255) / 256)), 256, 0, st>>>(f.state.p,
+                                                                                  f.hist.p);
+    DS_CHECK_LAUNCH();
+  }
   return true;
-}
-
-void launch_hist_roots(const MixedState* s, double* hist, int max_iter, cudaStream_t st) {
-  k_hist_roots<<<std::max(1, std::min(64, (max_iter + 255) / 256)), 256, 0, st>>>(s, hist);
-  DS_CHECK_LAUNCH();
 }
 
 int persistent_error(ds_operator* op, cudaStream_t st) {
