@@ -166,6 +166,12 @@ struct KernelConsts {
   double exact_cut;  // exponent cutoff of the exact kernel
   double cull_arg;   // tile-pair culling threshold on c_perp dperp^2 + c_para dz^2
   int eval;          // DS_EVAL_TABLE / DS_EVAL_EXACT
+  // the FP32 pair search (ds_pairhit.cuh): its scales sqrt(c_perp), sqrt(c_para),
+  // times the inverse of powers of two that coordinates take first (hit_units set), and
+  // whether it tells pairs apart at all
+  float hit_perp, hit_para;
+  int hit_units, hit_ok;
+  double unit_perp, unit_para;
 };
 
 KernelConsts make_consts(const ds_kernel_params& kp);

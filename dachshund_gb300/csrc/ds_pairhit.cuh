@@ -13,8 +13,12 @@
 // the warp's rows, S = sqrt(cutoff)) with a relative error below 2^-22, and
 // the squared distance is off by less than 2^-18 (cutoff + S (E + S)), which
 // the threshold adds; beyond E + S = 2^20 S every pair passes, and so does a
-// pair whose test overflows to NaN.  A pair that passes without interacting
-// costs one evaluation that gives zero.
+// pair whose test overflows to NaN.  The scales are FP64 roots rounded once (a
+// coefficient of lengths beyond 1e19 units is subnormal in FP32); where a scale lies
+// outside 2^-100 .. 2^100 its power of two multiplies the coordinates in FP64 first,
+// so that no interacting pair's leave FP32's range; with a cutoff outside 2^-20 ..
+// 2^40 every pair passes (make_consts).  A pair that passes without interacting costs
+// one evaluation that gives zero.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -26,12 +30,19 @@ namespace ds {
 // One warp's reference frame: a row's coordinates, the scales and the
 // threshold (warp-uniform).
 struct HitFrame {
-  double ox, oy, oz;
+  double ox, oy, oz, up, uq;
   float sp, sq, thr;
+  int units;
 };
 
 __device__ __forceinline__ float3 hit_point(const HitFrame& f, double x, double y, double z) {
-  return make_float3((float)(x - f.ox) * f.sp, (float)(y - f.oy) * f.sp, (float)(z - f.oz) * f.sq);
+  double dx = x - f.ox, dy = y - f.oy, dz = z - f.oz;
+  if (f.units) {
+    dx *= f.up;
+    dy *= f.up;
+    dz *= f.uq;
+  }
+  return make_float3((float)dx * f.sp, (float)dy * f.sp, (float)dz * f.sq);
 }
 
 // The frame of the warp's 32 rows (every lane its own row's coordinates) and
@@ -43,14 +54,17 @@ __device__ __forceinline__ HitFrame hit_frame(const KernelConsts& k, double x, d
   f.ox = __shfl_sync(full, x, 0);
   f.oy = __shfl_sync(full, y, 0);
   f.oz = __shfl_sync(full, z, 0);
-  f.sp = sqrtf((float)k.c_perp);
-  f.sq = sqrtf((float)k.c_para);
+  f.sp = k.hit_perp;
+  f.sq = k.hit_para;
+  f.up = k.unit_perp;
+  f.uq = k.unit_para;
+  f.units = k.hit_units;
   row = hit_point(f, x, y, z);
   float e = fmaxf(fabsf(row.x), fmaxf(fabsf(row.y), fabsf(row.z)));
   for (int o = 16; o > 0; o >>= 1) e = fmaxf(e, __shfl_xor_sync(full, e, o));
   const float cut = __double2float_ru(k.cull_arg), s = sqrtf(cut);
   const float eps = 1.f / (1 << 18);
-  f.thr = e + s < (float)(1 << 20) * s ? cut + eps * (cut + s * (e + s)) : INFINITY;
+  f.thr = k.hit_ok && e + s < (float)(1 << 20) * s ? cut + eps * (cut + s * (e + s)) : INFINITY;
   return f;
 }
 

@@ -41,6 +41,16 @@ KernelConsts make_consts(const ds_kernel_params& kp) {
   // Table: S == 0 once xx = arg * dx_inv reaches TABLE_N - 1.
   const double cut = kp.eval == DS_EVAL_TABLE ? (TABLE_N - 1) / k.dx_inv : k.exact_cut;
   k.cull_arg = cut * (1.0 + 1e-9);
+  auto unit = [](double s) {
+    return s == 0.0 || (s >= 0x1p-100 && s <= 0x1p100) ? 1.0 : std::ldexp(1.0, std::ilogb(s));
+  };
+  const double sp = std::sqrt(k.c_perp), sq = std::sqrt(k.c_para);
+  k.unit_perp = unit(sp);
+  k.unit_para = unit(sq);
+  k.hit_units = k.unit_perp != 1.0 || k.unit_para != 1.0;
+  k.hit_perp = (float)(sp / k.unit_perp);
+  k.hit_para = (float)(sq / k.unit_para);
+  k.hit_ok = k.cull_arg >= 0x1p-20 && k.cull_arg <= 0x1p40;
   return k;
 }
 
