@@ -78,6 +78,7 @@ bool run_pcg_persistent(ds_operator* op, const ds_pcg_params& pp, cudaStream_t s
 
 // Pair values in fixed point (pair_fx.cu).
 bool fx_usable(const KernelConsts& kc, const PointSet& rows, const PointSet& cols);
+bool vals_fx_usable(const KernelConsts& kc, const PointSet& ps);
 void launch_pair_fx(const KernelConsts& kc, int epi, const PairArgs& a, const PointSet& rows,
                     const PointSet& cols, cudaStream_t st);
 void fill_vals_fx(ds_operator* op, const dim3& grid, cudaStream_t st);

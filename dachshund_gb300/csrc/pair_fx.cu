@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(TILE) k_pair_fx(FxArgs f, PairArgs a) {
 }
 
 // Values of the stored pairs, as k_vals_eval (pair_vals.cu): one thread per
-// entry.  A pair of the list that passed the FP32 test without interacting may
-// lie beyond the fixed-point range by less than the test's margin.
+// entry.  A pair of the list that passed the FP32 test without interacting lies
+// beyond the cutoff by less than the test's margin (vals_fx_usable).
 template <class I>
 __global__ void __launch_bounds__(TILE) k_vals_fx(FxArgs f, const int* __restrict__ cnt,
                                                   const long long* __restrict__ start,
@@ -182,7 +182,8 @@ FxScale fx_scale(const KernelConsts& kc, const double* lo, const double* hi) {
   double ext = 1.0;
   for (int a = 0; a < 3; ++a) {
     f.hi[a] = std::sqrt(c[a]);
-    f.lo[a] = std::fma(-f.hi[a], f.hi[a], c[a]) / (2.0 * f.hi[a]);
+    // (0 for an infinite correlation length)
+    f.lo[a] = f.hi[a] > 0.0 ? std::fma(-f.hi[a], f.hi[a], c[a]) / (2.0 * f.hi[a]) : 0.0;
     f.o[a] = 0.5 * lo[a] + 0.5 * hi[a];
     ext = std::max(ext, (hi[a] - lo[a]) * f.hi[a]);
   }
@@ -236,6 +237,18 @@ bool fx_usable(const KernelConsts& kc, const PointSet& rows, const PointSet& col
         (std::max(rows.hi[a], cols.hi[a]) - std::min(rows.lo[a], cols.lo[a])) * s[a];
     if (!(ext <= 65536.0)) return false;
   }
+  return true;
+}
+
+// The list's values besides: its search (ds_pairhit.cuh) must not pass pairs from
+// beyond the fixed-point range, whose differences wrap.  With a threshold in use
+// everywhere (hit_ok, E + S < 2^20 S for E the extent) a pair that passes has |dX|^2
+// at most 2^-18 S (2^16 + S) + 2^-18 cut above the cutoff, below 50 at 48.
+bool vals_fx_usable(const KernelConsts& kc, const PointSet& ps) {
+  if (!kc.hit_ok || !fx_usable(kc, ps, ps)) return false;
+  const double s[3] = {std::sqrt(kc.c_perp), std::sqrt(kc.c_perp), std::sqrt(kc.c_para)};
+  for (int a = 0; a < 3; ++a)
+    if (!((ps.hi[a] - ps.lo[a]) * s[a] < 0x1p19 * std::sqrt(kc.cull_arg))) return false;
   return true;
 }
 

@@ -200,7 +200,7 @@ void fill(ds_operator* op, PairVals& pv, const PairArgs& a, DevBuf<I>& cols, cud
   // enough CTAs for 16 per SM (152) when there are few slices
   const int ns = op->pix.n_pad / 32;
   const dim3 grid(ns, std::max(1, std::min(32, (2432 + ns - 1) / ns)));
-  if (fx_usable(op->kc, op->pix, op->pix)) {
+  if (vals_fx_usable(op->kc, op->pix)) {
     fill_vals_fx(op, grid, st);
     return;
   }

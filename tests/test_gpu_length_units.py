@@ -65,6 +65,22 @@ def test_covariance_in_units(ctx):
         np.testing.assert_array_equal(u, v)
 
 
+def test_sparse_set_with_a_small_cutoff(ctx):
+    """32 points 2,048 scaled units apart (a multiple of the fixed-point
+    coordinates' period) and a cutoff of 1e-3: no two interact, although the search's
+    threshold does not resolve them."""
+    n = 32
+    rec = np.zeros((n, 5))
+    rec[:, 0] = 64.0 * 128 * np.arange(n)
+    rec[:, 3] = 0.01
+    a = np.random.default_rng(2).standard_normal(n)
+    lp = 4 / np.sqrt(2.0)  # sqrt(c_perp) = 1/4 to rounding
+    op = WFVectorSN(ctx, rec, SignalCovarParams(VS, lp, LQ, eval="exact", exact_cutoff=1e-3))
+    ref = (VS + 0.01) * a
+    assert np.all(np.abs(op.A_product(a) - ref) <= 8 * 2.0 ** -53 * np.abs(ref))
+    op.close()
+
+
 @pytest.mark.parametrize("ev", ["table", "exact"])
 def test_infinite_length(ctx, ev):
     """An infinite perpendicular length: the kernel depends on z alone."""
