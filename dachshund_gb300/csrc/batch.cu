@@ -507,15 +507,17 @@ inline int row_groups(int rt, int threads) {
 // [t][r], |r|^2 at [t][R + r].  Bound by its 28 bytes per (pixel, RHS); the sums are
 // float pairs (exact products, compensated sums, of vectors scaled to about 1): in
 // FP64 they took 5 instructions of 16 clocks per element and the kernel 160 us at
-// 207,104 pixels x 64 instead of 88.
-__global__ void k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
+// 207,104 pixels x 64 instead of 88.  CTA (tile, y): right-hand sides [y blockDim.x,
+// (y + 1) blockDim.x); 512 threads at most (its 80 registers allow 768).
+constexpr int STEP_THREADS = 512;
+__global__ void __launch_bounds__(STEP_THREADS) k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
                           float* __restrict__ z, const float* __restrict__ p,
                           const float* __restrict__ q, const float* __restrict__ pd,
                           double* __restrict__ part) {
   extern __shared__ float4 sums[];  // (group, RHS): r.z and |r|^2
   const int t = blockIdx.x;
   const int c = v.tile_chunk[t];
-  const int r = threadIdx.x, g = threadIdx.y, G = blockDim.y;
+  const int r = blockIdx.y * blockDim.x + threadIdx.x, g = threadIdx.y, G = blockDim.y;
   const int cr = c * v.R + r;
   if (v.chunk_done[c]) return;
   const bool on = r < v.R && !v.done[cr] && !v.hold[cr];
@@ -548,11 +550,11 @@ __global__ void k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
       }
     }
   }
-  sums[g * blockDim.x + r] = make_float4(rz.h, rz.l, rs.h, rs.l);
+  sums[g * blockDim.x + threadIdx.x] = make_float4(rz.h, rz.l, rs.h, rs.l);
   __syncthreads();
   if (g == 0 && on) {
     for (int k = 1; k < G; ++k) {
-      const float4 o = sums[k * blockDim.x + r];
+      const float4 o = sums[k * blockDim.x + threadIdx.x];
       rz = ff_add(rz, ff{o.x, o.y});
       rs = ff_add(rs, ff{o.z, o.w});
     }
@@ -1437,6 +1439,10 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
              B->s_hold.p, B->s_done.p,     B->s_alpha.p,     B->s_beta.p,  B->s_scale.p};
   const int RT = ((R + 31) / 32) * 32;
   const dim3 rows(RT, row_groups(RT, 512)), tiles(RT, row_groups(RT, 1024));
+  // the step's CTAs (row_smem is enough for them)
+  const unsigned step_y = (RT + STEP_THREADS - 1) / STEP_THREADS;
+  const unsigned step_x = (RT / 32 + step_y - 1) / step_y * 32;
+  const dim3 step_rows(step_x, row_groups(step_x, STEP_THREADS)), step_grid(T, step_y);
   const int TU = std::min(T, 4 * sm_count());  // the list kernels' grid
   const size_t row_smem = (size_t)rows.x * rows.y * sizeof(float4);
   const size_t bs_smem = (size_t)tiles.x * tiles.y * 2 * sizeof(double);
@@ -1458,8 +1464,8 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
     batch_mv(B, st, fused_dir);                                                      // MV
     k_bs<0><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S1
     DS_CHECK_LAUNCH();
-    k_bu_step<<<T, rows, row_smem, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p, B->q.p,
-                                         B->pd32.p, B->part.p);                      // U2
+    k_bu_step<<<step_grid, step_rows, row_smem, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p,
+                                                      B->q.p, B->pd32.p, B->part.p);  // U2
     DS_CHECK_LAUNCH();
     k_bs<1><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S2
     DS_CHECK_LAUNCH();
