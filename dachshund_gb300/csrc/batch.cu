@@ -505,23 +505,25 @@ inline int row_groups(int rt, int threads) {
 
 // U2: x_c += alpha p; r -= alpha q; z = r / pd.  Partials per (tile, RHS): r.z at
 // [t][r], |r|^2 at [t][R + r].  Bound by its 28 bytes per (pixel, RHS); the sums are
-// float pairs (exact products, compensated sums, of vectors scaled to about 1): in
-// FP64 they took 5 instructions of 16 clocks per element and the kernel 160 us at
-// 207,104 pixels x 64 instead of 88.  CTA (tile, y): right-hand sides [y blockDim.x,
-// (y + 1) blockDim.x); 512 threads at most (its 80 registers allow 768).
+// in three floats (exact products of vectors scaled to about 1, as good as FP64 or
+// better): in FP64 they took 5 instructions of 16 clocks per element and the kernel
+// 160 us at 207,104 pixels x 64 where float pairs take 88; in three floats, with 64
+// registers instead of 80, the solve is faster again (24 chunks x 64: 169 -> 165 ms).
+// CTA (tile, y): right-hand sides [y blockDim.x, (y + 1) blockDim.x), 512 threads at
+// most (two such CTAs fill an SM's registers).
 constexpr int STEP_THREADS = 512;
 __global__ void __launch_bounds__(STEP_THREADS) k_bu_step(BV v, float* __restrict__ xc, float* __restrict__ rr,
                           float* __restrict__ z, const float* __restrict__ p,
                           const float* __restrict__ q, const float* __restrict__ pd,
                           double* __restrict__ part) {
-  extern __shared__ float4 sums[];  // (group, RHS): r.z and |r|^2
+  extern __shared__ f3 sums[];  // (group, RHS): r.z and |r|^2
   const int t = blockIdx.x;
   const int c = v.tile_chunk[t];
   const int r = blockIdx.y * blockDim.x + threadIdx.x, g = threadIdx.y, G = blockDim.y;
   const int cr = c * v.R + r;
   if (v.chunk_done[c]) return;
   const bool on = r < v.R && !v.done[cr] && !v.hold[cr];
-  ff rz{0.f, 0.f}, rs{0.f, 0.f};
+  f3 rz{0.f, 0.f, 0.f}, rs{0.f, 0.f, 0.f};
   float2 sc = make_float2(1.f, 1.f);
   if (on) {
     const float alpha = (float)v.alpha[cr];
@@ -545,22 +547,23 @@ __global__ void __launch_bounds__(STEP_THREADS) k_bu_step(BV v, float* __restric
         rr[ir + (size_t)u * v.R] = ri;
         z[ir + (size_t)u * v.R] = zi;
         const float rsc = sc.x * ri;
-        ff_acc_prod(rz, rsc, sc.y * zi);
-        ff_acc_prod(rs, rsc, rsc);
+        f3_acc_prod(rz, rsc, sc.y * zi);
+        f3_acc_prod(rs, rsc, rsc);
       }
     }
   }
-  sums[g * blockDim.x + threadIdx.x] = make_float4(rz.h, rz.l, rs.h, rs.l);
+  f3* const mine = sums + 2 * (g * blockDim.x + threadIdx.x);
+  mine[0] = rz;
+  mine[1] = rs;
   __syncthreads();
   if (g == 0 && on) {
     for (int k = 1; k < G; ++k) {
-      const float4 o = sums[k * blockDim.x + threadIdx.x];
-      rz = ff_add(rz, ff{o.x, o.y});
-      rs = ff_add(rs, ff{o.z, o.w});
+      f3_add(rz, mine[2 * k * blockDim.x]);
+      f3_add(rs, mine[2 * k * blockDim.x + 1]);
     }
     const double ur = (double)(1.f / sc.x), uz = (double)(1.f / sc.y);
-    part[(size_t)t * 2 * v.R + r] = ff_double(rz) * ur * uz;
-    part[(size_t)t * 2 * v.R + v.R + r] = ff_double(rs) * ur * ur;
+    part[(size_t)t * 2 * v.R + r] = f3_double(rz) * ur * uz;
+    part[(size_t)t * 2 * v.R + v.R + r] = f3_double(rs) * ur * ur;
   }
 }
 
@@ -674,6 +677,12 @@ __device__ __forceinline__ void chunk_sums(double (&s)[N], const double* part, i
       for (int n = 0; n < N; ++n) s[n] += sm[n * nt + k * blockDim.x + threadIdx.x];
 }
 
+// The scales (sr, sz) of the step's sums, from the last |r| and r.z in FP64.
+__device__ __forceinline__ float2 step_scale(double rn, double rz) {
+  const int er = rn > 0.0 ? ilogb(rn) : 0, ez = rz > 0.0 ? ilogb(rz) : 0;
+  return make_float2(pow2_neg(er), pow2_neg(ez - er));
+}
+
 // MODE 0 (S1): alpha = r.z / p.q.
 // MODE 1 (S2): new r.z and |r|, beta.  A right-hand side whose recurrence
 //              residual fell by delta since its last update, reached tol |b|,
@@ -755,6 +764,7 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
           s.done[cr] = 1;
         } else {
           s.rz[cr] = rz;  // rz_old keeps the r.z before the held iteration
+          s.scale[cr] = step_scale(rt, rz);
           s.beta[cr] = s.stalled[cr] ? 0.0 : rz / s.rz_old[cr];
           s.rmax[cr] = rt;
           s.rbest[cr] = rt;
@@ -764,8 +774,7 @@ __global__ void k_bs(BatchState s, const double* __restrict__ part) {
       }
     } else if (MODE == 3) {
       const double rz = sum[0], rt = sqrt(sum[1]);
-      const int er = rt > 0.0 ? ilogb(rt) : 0, ez = rz > 0.0 ? ilogb(rz) : 0;
-      s.scale[cr] = make_float2(pow2_neg(er), pow2_neg(ez - er));
+      s.scale[cr] = step_scale(rt, rz);
       s.beta[cr] = 0.0;
       s.rz[cr] = rz;
       s.rtrue[cr] = s.rmax[cr] = s.rbest[cr] = rt;
@@ -1439,12 +1448,13 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
              B->s_hold.p, B->s_done.p,     B->s_alpha.p,     B->s_beta.p,  B->s_scale.p};
   const int RT = ((R + 31) / 32) * 32;
   const dim3 rows(RT, row_groups(RT, 512)), tiles(RT, row_groups(RT, 1024));
-  // the step's CTAs (row_smem is enough for them)
+  // the step's CTAs
   const unsigned step_y = (RT + STEP_THREADS - 1) / STEP_THREADS;
   const unsigned step_x = (RT / 32 + step_y - 1) / step_y * 32;
   const dim3 step_rows(step_x, row_groups(step_x, STEP_THREADS)), step_grid(T, step_y);
   const int TU = std::min(T, 4 * sm_count());  // the list kernels' grid
-  const size_t row_smem = (size_t)rows.x * rows.y * sizeof(float4);
+  const size_t row_smem = (size_t)rows.x * rows.y * sizeof(double2);
+  const size_t step_smem = (size_t)step_rows.x * step_rows.y * 2 * sizeof(f3);
   const size_t bs_smem = (size_t)tiles.x * tiles.y * 2 * sizeof(double);
   // The tensor-core matvec forms p = z + beta p as it packs p (launch_batch_mv_tc).
   const bool fused_dir = B->variant == BV_TENSOR;
@@ -1464,7 +1474,7 @@ void batch_solve_dev(ds_batch* B, const ds_mixed_params& mp, const double* rhs_d
     batch_mv(B, st, fused_dir);                                                      // MV
     k_bs<0><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S1
     DS_CHECK_LAUNCH();
-    k_bu_step<<<step_grid, step_rows, row_smem, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p,
+    k_bu_step<<<step_grid, step_rows, step_smem, st>>>(v, B->xc.p, B->rr.p, B->zz.p, B->p.p,
                                                       B->q.p, B->pd32.p, B->part.p);  // U2
     DS_CHECK_LAUNCH();
     k_bs<1><<<C, tiles, bs_smem, st>>>(S, B->part.p);                                // S2

@@ -94,7 +94,7 @@ struct BatchState {
   double* rz_old;
   double* alpha;
   double* beta;
-  float2* scale;  // (sr, sz): powers of two that bring the first |r| and r.z near 1
+  float2* scale;  // (sr, sz): powers of two that bring the last update's |r| and r.z near 1
   double* rmax;
   double* rbest;    // smallest recurrence |r| since the last halving
   double* rtrue;

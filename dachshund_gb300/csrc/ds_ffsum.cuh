@@ -1,6 +1,7 @@
-// Dot products of FP32 vectors in float pairs (exact products by FMA, compensated
-// sums, about 44 bits) over vectors scaled by powers of two, and their sums in FP64
-// from the warps up: the persistent structured form (persist.cu).
+// Dot products of FP32 vectors scaled by powers of two: in float pairs (exact
+// products by FMA, compensated sums, about 44 bits) within a warp and FP64 from there
+// up, the persistent structured form (persist.cu); in three floats (more bits than
+// FP64 sums) within a tile, the batched solve (batch.cu).
 #pragma once
 
 #include "ds_f32.h"
@@ -15,6 +16,35 @@ __device__ __forceinline__ void ff_acc_prod(ff& a, float x, float y) {
   p.h = __fmul_rn(x, y);
   p.l = __fmaf_rn(x, y, -p.h);
   a = ff_add(a, p);
+}
+
+// Sums in three floats: every rounding error of the first is added to the second
+// and that sum's to the third, so that a sum of n terms is within n^3 2^-72 of the
+// exact one, better than FP64's n 2^-53 up to some 700 terms.
+struct f3 {
+  float a, b, c;
+};
+
+// v += x y (the product's error by FMA).
+__device__ __forceinline__ void f3_acc_prod(f3& v, float x, float y) {
+  const float p = __fmul_rn(x, y), e = __fmaf_rn(x, y, -p);
+  float e1, e2, e3;
+  two_sum(v.a, p, v.a, e1);
+  two_sum(v.b, e1, v.b, e2);
+  two_sum(v.b, e, v.b, e3);
+  v.c = __fadd_rn(v.c, __fadd_rn(e2, e3));
+}
+
+__device__ __forceinline__ void f3_add(f3& v, const f3& w) {
+  float e1, e2, e3;
+  two_sum(v.a, w.a, v.a, e1);
+  two_sum(v.b, e1, v.b, e2);
+  two_sum(v.b, w.b, v.b, e3);
+  v.c = __fadd_rn(__fadd_rn(v.c, w.c), __fadd_rn(e2, e3));
+}
+
+__device__ __forceinline__ double f3_double(const f3& v) {
+  return (double)v.a + ((double)v.b + (double)v.c);
 }
 
 __device__ __forceinline__ ff ff_shfl_down(ff v, int o) {

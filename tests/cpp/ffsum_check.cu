@@ -1,5 +1,5 @@
-// The persistent solve's sums and scalars (csrc/ds_ffsum.cuh) on the device, against
-// the same in exact or FP64 arithmetic on the host.  Prints "name error bound" lines.
+// The persistent and batched solves' sums and scalars (csrc/ds_ffsum.cuh) on the
+// device, against the same in exact or FP64 arithmetic on the host.  Prints "name error bound" lines.
 #include <cmath>
 #include <cstdio>
 #include <random>
@@ -49,6 +49,21 @@ __global__ void k_norms(int n, const double* rr, double unit, double delta, doub
   f.alpha = ff{1.f, 0.f};
   fast_to(f, s);
   back[i] = s.rnorm;
+}
+
+// A tile's dot product as the batched step forms it: 8 groups of 16 rows.
+__global__ void k_tile(const float* x, const float* y, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  f3 total{0.f, 0.f, 0.f};
+  for (int g = 0; g < 8; ++g) {
+    f3 v{0.f, 0.f, 0.f};
+    for (int k = 0; k < 16; ++k) {
+      const size_t e = (size_t)i * 128 + 16 * g + k;
+      f3_acc_prod(v, x[e], y[e]);
+    }
+    f3_add(total, v);
+  }
+  out[i] = f3_double(total);
 }
 
 template <class T>
@@ -124,6 +139,31 @@ int main() {
     eq = fmax(eq, (double)fabsl(((long double)q[i].x + q[i].y - ref) / ref));
   }
   printf("quotient %g %g\n", eq, ldexp(1.0, -45));
+  // A tile's sum in three floats: 128^3 2^-72 of the terms' magnitudes and the three
+  // roundings to FP64.
+  const int nt = 1024;
+  std::vector<float> x((size_t)nt * 128), y(x.size());
+  for (size_t i = 0; i < x.size(); ++i) {
+    x[i] = (float)((U(rng) - 0.5) * exp(6 * U(rng)));
+    y[i] = i % 3 ? (float)((U(rng) - 0.3) * exp(6 * U(rng))) : x[i];
+  }
+  double* dt = up(std::vector<double>(nt));
+  k_tile<<<nt / 128, 128>>>(up(x), up(y), dt);
+  const auto tiles = down(dt, nt);
+  double et = 0;
+  for (int i = 0; i < nt; ++i) {
+    // the exact products' sum by long double (64 bits or more), compensated
+    long double sum = 0, low = 0, mag = 0;
+    for (int k = 0; k < 128; ++k) {
+      const long double p = (long double)x[(size_t)i * 128 + k] * y[(size_t)i * 128 + k];
+      const long double t = sum + p, bb = t - sum;
+      low += (sum - (t - bb)) + (p - bb);
+      sum = t;
+      mag += fabsl(p);
+    }
+    et = fmax(et, (double)(fabsl((tiles[i] - sum) - low) / mag));
+  }
+  printf("tile %g %g\n", et, ldexp(1.0, 21 - 72) + 3 * u53);
   // The update test 2^-46 on either side of delta^2 and of tol^2, in three units.
   for (double unit : {1.0, 1e-17, 1e12}) {
     const double delta = 1e-4, tol = 3e-3, d = ldexp(1.0, -46);
