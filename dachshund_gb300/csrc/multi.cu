@@ -293,11 +293,6 @@ void mproduct(ds_operator* op, const MPairArgs& a, int R, bool vals, cudaStream_
   DS_CHECK_LAUNCH();
 }
 
-__global__ void k_recip(int n, const double* __restrict__ v, double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = 1.0 / v[i];
-}
-
 // Per right-hand side sums over the grid of two values each thread holds
 // for r = threadIdx.x % R (R divides the block and the grid stride); the
 // last CTA gets them in tot[0..R) and tot[R..2R).  Fixed order: the block's
@@ -358,7 +353,7 @@ __global__ void __launch_bounds__(MVB) k_mnorm(size_t n, const double* __restric
 // mode 2: precondition + dots only (full-residual step, after the residual)
 // mode 3: start from x = 0: r = b, d = M^-1 r + dots
 // CTA (x, y): right-hand sides [32 y, 32 y + 32) (the lanes) of rows 8 x + warp,
-// + 8 gridDim.x, ..., four rows in flight; ipd = 1 / the Jacobi diagonal.
+// + 8 gridDim.x, ..., four rows in flight.
 template <int MODE>
 __global__ void __launch_bounds__(MVB) k_mupdate(int n, MState* st, MShared* sh,
                                                  double* __restrict__ x, double* __restrict__ r,
@@ -366,7 +361,7 @@ __global__ void __launch_bounds__(MVB) k_mupdate(int n, MState* st, MShared* sh,
                                                  const double* __restrict__ q,
                                                  double* __restrict__ s,
                                                  const double* __restrict__ b,
-                                                 const double* __restrict__ ipd,
+                                                 const double* __restrict__ pdiag,
                                                  double* part, double* hist, int hist_stride) {
   if (MODE != 3 && sh->all_done) return;
   __shared__ double red[MVB];
@@ -392,7 +387,7 @@ __global__ void __launch_bounds__(MVB) k_mupdate(int n, MState* st, MShared* sh,
         ri = fma(-alpha, q[e], ri);  // lib/pcg.h:48
         r[e] = ri;
       }
-      const double si = ri * ipd[i];  // lib/pcg.h:52
+      const double si = ri / pdiag[i];  // lib/pcg.h:52
       s[e] = si;
       if (MODE == 3) d[e] = si;
       rs = fma(ri, si, rs);
@@ -515,7 +510,7 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
   const dim3 ug(std::min(np / (MVB / 32), std::max(1, 1216 * 32 / R)), R / 32);
   const int hist_stride = std::max(pp.max_iter, 1) + 1;
   const bool vals = ensure_pair_vals(op);
-  DevBuf<double> b, x, r, d, q, s, part, hist, mp, sig, ipd;
+  DevBuf<double> b, x, r, d, q, s, part, hist, mp, sig;
   DevBuf<MState> dst;
   DevBuf<MShared> dsh;
   b.alloc(nv);
@@ -525,9 +520,6 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
   q.alloc(nv);
   s.alloc(nv);
   part.alloc(std::max<size_t>((size_t)2 * R * std::max<size_t>(g, ug.x), (size_t)np / 8 * R));
-  ipd.alloc(np);
-  k_recip<<<(np + MVB - 1) / MVB, MVB, 0, st>>>(np, op->pdiag.p, ipd.p);
-  DS_CHECK_LAUNCH();
   hist.alloc((size_t)R * hist_stride);
   mp.alloc(3 * (size_t)R);
   sig.alloc(R);
@@ -578,20 +570,20 @@ void map_covar_diag_multi(ds_operator* op, int n_map, const double* map_pts,
     DS_CHECK_LAUNCH();
     // r = b (x = 0), d = M^-1 r, delta, |r|  (lib/pcg.h:95-108)
     k_mupdate<3><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                    ipd.p, part.p, hist.p, hist_stride);
+                                    op->pdiag.p, part.p, hist.p, hist_stride);
     DS_CHECK_LAUNCH();
     for (int it = 1; it < pp.max_iter; ++it) {
       mproduct<false, true>(op, prod, R, vals, st);
       if (it % pp.step_r == 0) {
         k_mupdate<1><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        ipd.p, part.p, hist.p, hist_stride);
+                                        op->pdiag.p, part.p, hist.p, hist_stride);
         DS_CHECK_LAUNCH();
         mproduct<true, false>(op, resid, R, vals, st);
         k_mupdate<2><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        ipd.p, part.p, hist.p, hist_stride);
+                                        op->pdiag.p, part.p, hist.p, hist_stride);
       } else {
         k_mupdate<0><<<ug, MVB, 0, st>>>(np, dst.p, dsh.p, x.p, r.p, d.p, q.p, s.p, b.p,
-                                        ipd.p, part.p, hist.p, hist_stride);
+                                        op->pdiag.p, part.p, hist.p, hist_stride);
       }
       DS_CHECK_LAUNCH();
       k_mdir<<<gd, MVB, 0, st>>>(nv, dst.p, dsh.p, s.p, d.p);
