@@ -34,12 +34,14 @@ constexpr int DM_CTAS_PER_SM = 2;
 
 // Blocks per work item: the most (an item's FP64 row sums, arrival and partials take
 // some 15,000 clocks, as long as its loads of 8 blocks) that leave four items per
-// resident CTA, not less than 4.  Rows of up to 2,048 columns stay one item and one
-// running sum.  Solves to 1e-11 (items of 32 blocks -> this rule): 32,768 pixels 61.1
-// -> 58.1 ms (64 blocks; 73 with 128: uneven shares), 8,192 18.2 -> 14.4 ms (8).
+// resident CTA, not less than 16.  Rows of up to 2,048 columns stay one item and one
+// running sum.  Us per PCG iteration with 4, 8, 16, 32, 64 blocks: 5,000 pixels in a
+// box where every block is nonzero 91, 74, 70, 67, 83, at the survey's density 89, 69,
+// 66, 63, 81; 8,190 pixels 175, 139, 125, 116, 121 and 141, 103, 96, 103, 96; 15,000
+// pixels 523, 385, 332, 323, 329 and 334, 238, 178, 184, 222.
 inline int dense_span(int n, int sms) {
   int span = 32 * DM_WORDS;
-  const int least = n <= DM_CW ? 32 : 4;
+  const int least = n <= DM_CW ? 32 : 16;
   while (span > least && (long long)(n / DM_RB) * ((n / DM_STEP + span - 1) / span) <
                              4ll * DM_CTAS_PER_SM * sms)
     span /= 2;
@@ -99,7 +101,7 @@ __global__ void k_dense_build(KernelConsts kc, int n, size_t ld, const double* _
 // ---- dense matvec ------------------------------------------------------------
 //
 // q = A v (+ the last CTA's alpha = delta / (dotv . q)) or r = b - A v, A in
-// HBM (n x n FP64, row-major, sorted order).  Work items are 64 rows times 256 to
+// HBM (n x n FP64, row-major, sorted order).  Work items are 64 rows times 1,024 to
 // 4,096 columns of A (dense_span) pulled by a persistent grid (CTA count a multiple
 // of the SM count); each warp streams 8 rows of its item, a 64-column block ahead, with 16-byte
 // evict-first loads (every byte of A read once per product), and the column
@@ -132,7 +134,7 @@ struct DenseMv {
   int n;     // rows = columns (n_pad, a multiple of 128)
   int nrb;   // row blocks
   int ncb;   // mask words per row block
-  int span;  // blocks per work item: 4, 8, ..., 32 DM_WORDS
+  int span;  // blocks per work item: 16, 32 or 32 DM_WORDS
   int nsp;   // work items per row block
   const double* A;
   const double* v;    // FP64 arithmetic
