@@ -152,7 +152,9 @@ struct DenseMv {
   const unsigned* mask;      // nonzero 64 x 64 blocks, nrb x ncb words
   const unsigned* need;      // per row block: its items with a nonzero block
   const unsigned char* on;   // nrb x nsp: the item has a nonzero block
-  const unsigned* nonfinite; // v holds an infinity or a NaN
+  const unsigned* nonfinite; // == mark: v holds an infinity or a NaN
+  unsigned mark;
+  int whole;                 // the whole matrix in any case
 };
 
 // a = h + l to 2^-46 |a| for a = 0 or 2^-100 <= |a| <= 2^100: h holds the
@@ -199,10 +201,10 @@ __device__ __forceinline__ uint4 ld_stream16(const double* p) {
 }
 
 __global__ void k_split_vec(int n, const double* __restrict__ v, float2* __restrict__ vff,
-                            unsigned* nonfinite, const int* skip) {
+                            unsigned* nonfinite, unsigned mark, const int* skip) {
   if (skip && *skip) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    vff[i] = dense_split(v[i], nonfinite);
+    vff[i] = dense_split(v[i], nonfinite, mark);
 }
 
 // Mask words of an item (all zero past the last one): the first is shifted so that
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_CTAS_PER_SM) k_dense_mv(Dens
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_items = a.nrb * a.nsp;
-  const bool full = *a.nonfinite != 0;
+  const bool full = a.whole || *a.nonfinite == a.mark;
   if (a.prof_pairs && blockIdx.x == 0) {  // entries read
     unsigned long long steps = 0;
     for (int k = tid; k < a.nrb * a.ncb; k += DM_WARPS * 32)
@@ -577,6 +579,7 @@ void op_build_dense(ds_operator* op) {
   op->dense_mask.alloc(nrb * ncb);
   op->dense_need.alloc(nrb + 1);  // + the nonfinite flag
   DS_CUDA(cudaMemsetAsync(op->dense_mask.p, 0, op->dense_mask.bytes(), st));
+  DS_CUDA(cudaMemsetAsync(op->dense_need.p + nrb, 0, sizeof(unsigned), st));
   k_dense_build<<<std::min<size_t>(np, (size_t)sms * 8), 256, 0, st>>>(
       op->kc, (int)np, np, op->pix.x.p, op->pix.y.p, op->pix.z.p, op->wl.p, op->e.p,
       op->table.p, op->dense.p, stats.p, op->dense_mask.p);
@@ -622,8 +625,13 @@ void launch_dense_mv(const DenseMv& a, bool residual, bool dot, int grid, cudaSt
 
 }  // namespace
 
-unsigned* dense_nonfinite(ds_operator* op) {
+static unsigned* nonfinite_word(ds_operator* op) {
   return op->dense_need.p + op->pix.n_pad / DM_RB;
+}
+
+DenseNonfinite dense_next_vector(ds_operator* op) {
+  if (++op->dense_mark == 0) ++op->dense_mark;  // 0: the word as built
+  return {nonfinite_word(op), op->dense_mark};
 }
 
 void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
@@ -653,8 +661,13 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
   a.skip = skip;
   a.mask = op->dense_mask.p;
   a.need = op->dense_need.p;
-  a.nonfinite = dense_nonfinite(op);
   const bool ff = dense_arith_in_use(op) == DS_DENSE_FLOAT_PAIR;
+  // FP64 products need no split: where a row is one item (little to skip, and a launch
+  // to look for infinities takes 2 us of 38) they multiply the whole matrix
+  a.whole = !ff && np <= DM_CW;
+  if (!is_split && !a.whole) dense_next_vector(op);
+  a.nonfinite = nonfinite_word(op);
+  a.mark = op->dense_mark;
   const int grid = std::min(a.nrb * a.nsp, sms * DM_CTAS_PER_SM);
   Profiler& prof = op->ctx->prof;
   cudaEvent_t ev = nullptr;
@@ -662,10 +675,9 @@ void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
     a.prof_pairs = prof.d_pairs + 3;
     prof.begin(st, &ev);
   }
-  if (!is_split) {
-    DS_CUDA(cudaMemsetAsync(dense_nonfinite(op), 0, sizeof(unsigned), st));
+  if (!is_split && !a.whole) {
     k_split_vec<<<std::min((np + 255) / 256, 4 * sms), 256, 0, st>>>(
-        np, v, op->dense_vff.p, dense_nonfinite(op), skip);
+        np, v, op->dense_vff.p, nonfinite_word(op), a.mark, skip);
     DS_CHECK_LAUNCH();
   }
   if (ff) {

@@ -23,10 +23,10 @@ __device__ __forceinline__ double block_sum(double v, double* sm /* NT/32 */) {
   return s;
 }
 
-// An element of the dense product's vector as a float pair; *nonfinite = 1 for an
+// An element of the dense product's vector as a float pair; *nonfinite = mark for an
 // infinity or a NaN.
-__device__ __forceinline__ float2 dense_split(double x, unsigned* nonfinite) {
-  if (!isfinite(x)) *nonfinite = 1u;
+__device__ __forceinline__ float2 dense_split(double x, unsigned* nonfinite, unsigned mark) {
+  if (!isfinite(x)) *nonfinite = mark;
   const float h = __double2float_rn(x);
   return make_float2(h, __double2float_rn(x - (double)h));
 }

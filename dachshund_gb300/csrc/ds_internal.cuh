@@ -387,6 +387,7 @@ struct ds_operator {
   // nonzero 64 x 64 blocks (a word per work item), their words per row block
   // and a flag (dense.cu)
   ds::DevBuf<unsigned int> dense_mask, dense_need;
+  unsigned int dense_mark = 0;  // of the vector being multiplied (dense_next_vector)
   ds::DevBuf<unsigned char> dense_on;
   bool pairs_built = false;  // `pairs` (ensure_op_pairs)
   ds::PairVals vals;         // the pairs' values (ensure_pair_vals)

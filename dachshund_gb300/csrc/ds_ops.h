@@ -51,10 +51,15 @@ int dense_arith_in_use(const ds_operator* op);  // DS_DENSE_FLOAT_PAIR or DS_DEN
 void dense_apply(ds_operator* op, bool residual, const double* v, double* out,
                  const double* dotv, PcgState* pcg, const int* skip, cudaStream_t st,
                  bool is_split = false);
-// The flag in device memory that the vector being multiplied holds an infinity or a
-// NaN; with it and op->dense_vff (dense_split of every element) set by the caller,
-// dense_apply takes is_split.
-unsigned* dense_nonfinite(ds_operator* op);
+// For a caller that splits the next product's vector itself (dense_apply with
+// is_split): dense_split of every element into op->dense_vff with this word and mark.
+// The word holds the mark when the vector has an infinity or a NaN; every vector has a
+// mark of its own, so that the word needs no clearing.
+struct DenseNonfinite {
+  unsigned* word;
+  unsigned mark;
+};
+DenseNonfinite dense_next_vector(ds_operator* op);
 void solve_cf_dev(ds_context* ctx, int form, int n, const double* d_rec, const KernelConsts& kc,
                   const double* d_table, double* d_x);
 // MapCovarDiag with the operator's table kernel: groups of map points as the

@@ -109,14 +109,14 @@ __global__ void __launch_bounds__(VB) k_pcg_direction(int n, const PcgState* st,
                                                       const double* __restrict__ wr,
                                                       double* __restrict__ u,
                                                       float2* __restrict__ vff,
-                                                      unsigned* nonfinite) {
+                                                      DenseNonfinite nonfinite) {
   if (st->done) return;
   const double beta = st->beta;
   for (int i = blockIdx.x * VB + threadIdx.x; i < n; i += gridDim.x * VB) {
     const double di = fma(beta, d[i], s[i]);
     d[i] = di;
     if (u) u[i] = var_s * (wr[i] * di);
-    if (vff) vff[i] = dense_split(di, nonfinite);
+    if (vff) vff[i] = dense_split(di, nonfinite.word, nonfinite.mark);
   }
 }
 
@@ -303,11 +303,8 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
     DS_CHECK_LAUNCH();
     // (the dense product's float pairs of d are formed here: a launch of their own
     // took 4 of some 30 us an iteration at 1,280 pixels)
-    unsigned* flag = nullptr;
-    if (op->use_dense) {
-      flag = dense_nonfinite(op);
-      DS_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
-    }
+    DenseNonfinite flag{};
+    if (op->use_dense) flag = dense_next_vector(op);
     k_pcg_direction<<<g, VB, 0, st>>>(np, S, op->s.p, op->d.p, op->kc.var_s, op->wr.p, u,
                                       op->use_dense ? op->dense_vff.p : nullptr, flag);
     DS_CHECK_LAUNCH();
