@@ -157,6 +157,13 @@ struct HostBuf {
   }
 };
 
+// A kernel's limit of dynamic shared memory belongs to the device, not to a context:
+// it is only ever raised, so that a launch on another thread between this one's call
+// and its launch cannot fall below it.  resident_ctas raises it and returns the CTAs
+// per SM (0: the size does not fit); all_shared: the largest carveout first.
+void raise_dynamic_smem(const void* fn, size_t bytes);
+int resident_ctas(const void* fn, int threads, size_t bytes, bool all_shared = false);
+
 // Kernel constants shared by every pair kernel.
 struct KernelConsts {
   double var_s;

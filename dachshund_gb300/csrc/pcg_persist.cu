@@ -257,8 +257,8 @@ __global__ void __launch_bounds__(NT) k_pcg_persistent(Args a, const I* __restri
 // The whole iteration of run_pcg (x, the state's norm and tolerance set) when
 // every slice gets a resident CTA, two to an SM at most (n up to 9,728 on 152
 // SMs); false leaves it to the per-kernel form, which at larger n spends its time
-// in the product and not between kernels.  err_code: nonzero when a barrier wait
-// ran out (synchronises the stream).
+// in the product and not between kernels.  Launches only: the caller reads the error
+// word pcg_sync[1] once the stream has finished.
 bool run_pcg_persistent(ds_operator* op, const ds_pcg_params& pp, cudaStream_t st) {
   const PairVals& pv = op->vals;
   const int ns = op->pix.n_pad / 32, sms = op->ctx->num_sms;
@@ -268,10 +268,7 @@ bool run_pcg_persistent(ds_operator* op, const ds_pcg_params& pp, cudaStream_t s
                           : (const void*)k_pcg_persistent<int>;
   // shared memory of one CTA per SM, or of two
   const size_t bytes = ns <= sms ? 200 * 1024 : 96 * 1024;
-  DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  int per_sm = 0;
-  DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, bytes));
-  if ((long long)per_sm * sms < ns) return false;
+  if ((long long)resident_ctas(fn, NT, bytes) * sms < ns) return false;
   op->ud.alloc(op->pix.n_pad);
   op->u.alloc(op->pix.n_pad);
   op->pcg_sync.alloc(2);

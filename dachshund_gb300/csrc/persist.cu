@@ -1434,23 +1434,6 @@ void to_ff(DevBuf<float2>& out, const double* in, size_t n, cudaStream_t st) {
   DS_CHECK_LAUNCH();
 }
 
-// Resident CTAs per SM of a kernel at `smem` dynamic bytes (0: does not fit).
-int resident_per_sm(const void* fn, size_t smem) {
-  cudaFuncAttributes fa;
-  DS_CUDA(cudaFuncGetAttributes(&fa, fn));
-  int dev = 0, optin = 0;
-  DS_CUDA(cudaGetDevice(&dev));
-  DS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (fa.sharedSizeBytes + smem > (size_t)optin) return 0;
-  DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared));
-  if (smem > 48 * 1024)
-    DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem));
-  return per_sm;
-}
-
 // The block of each CTA.  The slowest block sets the product phase (an interior
 // cluster has up to 1.7 times the mean's rows), and the first CTAs of a launch
 // go one to an SM, the rest second to the same SMs in order: the blocks with the
@@ -1527,20 +1510,13 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
     g.res_cut = g.inner.cut;
   }
   const size_t res_bytes = ResLayout::bytes(band, pc->n_per);
-  static int per_sm0[3] = {-1, -1, -1};
-  static int per_sm1[3] = {-1, -1, -1};
-  static size_t res_last[3] = {0, 0, 0};
-  const int bi = band == 16 ? 0 : band == 2 ? 1 : 2;
-  if (per_sm0[bi] < 0) per_sm0[bi] = resident_per_sm(pick(false), 0);
-  if (res_last[bi] != res_bytes) {
-    per_sm1[bi] = resident_per_sm(pick(true), res_bytes);
-    res_last[bi] = res_bytes;
-  }
   const int nsm = op->ctx->num_sms;
   // the item form: 32-bit offsets into the levels, <= GI skewers per block,
   // a thread for every pixel, every block's items in shared memory
-  const bool resident = g.res_max_list <= NI && per_sm1[bi] * nsm >= pc->n_sk;
-  const int grid = resident ? pc->n_sk : std::min(per_sm0[bi] * nsm, pc->n_sk);
+  const bool resident = g.res_max_list <= NI &&
+                        resident_ctas(pick(true), NT, res_bytes, true) * nsm >= pc->n_sk;
+  const int grid =
+      resident ? pc->n_sk : std::min(resident_ctas(pick(false), NT, 0, true) * nsm, pc->n_sk);
   if (grid <= 0) return false;
   g.p_part.alloc((size_t)3 * grid + 1);
   const size_t n_pt = PT_CTA + 8 * (size_t)grid;

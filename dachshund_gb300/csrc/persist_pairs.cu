@@ -456,10 +456,7 @@ bool mixed_pairs_usable(ds_operator* op, OpF32& f, int g) {
   if (per > MAX_PER || g > 2 * G) return false;
   const size_t smem = sizeof(Shared) + (size_t)per * NT * sizeof(Row);
   const void* fn = kernel_of(f);
-  DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem));
-  if (per_sm < 1) return false;
+  if (resident_ctas(fn, NT, smem) < 1) return false;
   if (f.rounds_built) return true;
   cudaStream_t st = op->ctx->stream;
   const int n = 4 * nt, nw = W * G;

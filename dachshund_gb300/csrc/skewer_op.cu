@@ -967,9 +967,7 @@ bool skewer_map_product(ds_map* map, ds_operator* op, const double* x_dev, doubl
     const int K = (g.n_per + MF_T - 1) / MF_T;
     auto fn = K == 1 ? k_mc_fused<1> : K == 2 ? k_mc_fused<2> : K == 3 ? k_mc_fused<3>
                                                                          : k_mc_fused<4>;
-    if (zs_bytes > 48 * 1024)
-      DS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)zs_bytes));
+    raise_dynamic_smem((const void*)fn, zs_bytes);
     const int n = g.n_sk * g.n_per;
     mc.xff.alloc(n);
     k_mc_split<<<std::min(1024, (n + 255) / 256), 256, 0, st>>>(n, x_dev, mc.xff.p);
