@@ -164,6 +164,12 @@ struct HostBuf {
 void raise_dynamic_smem(const void* fn, size_t bytes);
 int resident_ctas(const void* fn, int threads, size_t bytes, bool all_shared = false);
 
+// A cooperative launch after every earlier one of the process on this device: the CTAs
+// of two grids that each fill the GPU, in streams of two contexts, could otherwise be
+// resident in part and wait for each other's room at their barriers.
+void launch_cooperative(const void* fn, int ctas, int threads, void** args, size_t bytes,
+                        cudaStream_t st);
+
 // Kernel constants shared by every pair kernel.
 struct KernelConsts {
   double var_s;

@@ -298,8 +298,7 @@ bool run_pcg_persistent(ds_operator* op, const ds_pcg_params& pp, cudaStream_t s
   const unsigned short* c16 = pv.col16.p;
   const int* c32 = pv.col32.p;
   void* args[] = {&a, narrow ? (void*)&c16 : (void*)&c32};
-  DS_CUDA(cudaLaunchCooperativeKernel(fn, dim3(ns), dim3(NT), args, bytes, st));
-  DS_CHECK_LAUNCH();
+  launch_cooperative(fn, ns, NT, args, bytes, st);
   return true;
 }
 

@@ -1591,9 +1591,7 @@ bool run_mixed_persistent(ds_operator* op, OpF32& f, const SkewerPC* pc, const S
   a.op_ff = g.ff_op.p;
   a.taps64_ff = g.ff_taps.p;
   void* args[] = {&a};
-  DS_CUDA(cudaLaunchCooperativeKernel(pick(resident), dim3(grid), dim3(NT), args,
-                                      resident ? res_bytes : 0, st));
-  DS_CHECK_LAUNCH();
+  launch_cooperative(pick(resident), grid, NT, args, resident ? res_bytes : 0, st);
   if (resident) {
     k_hist_roots<<<std::max(1, std::min(64, (max_iter + 255) / 256)), 256, 0, st>>>(f.state.p,
                                                                                   f.hist.p);

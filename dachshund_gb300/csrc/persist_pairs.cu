@@ -531,9 +531,8 @@ void launch_mixed_pairs(ds_operator* op, OpF32& f, double* X, int max_iter, int 
   a.bar = f.round_bar.p;
   a.limit = op->ctx->wait_limit > 0 ? op->ctx->wait_limit : 4000000000LL;
   void* args[] = {&a};
-  DS_CUDA(cudaLaunchCooperativeKernel(kernel_of(f), dim3(G), dim3(NT), args,
-                                      sizeof(Shared) + (size_t)a.per * NT * sizeof(Row), st));
-  DS_CHECK_LAUNCH();
+  launch_cooperative(kernel_of(f), G, NT, args, sizeof(Shared) + (size_t)a.per * NT * sizeof(Row),
+                     st);
 }
 
 }  // namespace ds
