@@ -264,10 +264,12 @@ class _WFVector:
                        "ds_operator_set_inner_matvec")
 
     def set_iteration_form(self, form: str = "auto"):
-        """How solve_mixed launches its iterations: "auto" (one persistent
-        cooperative launch with the structured inner operator and a band
-        preconditioner, else a replayed CUDA graph) or "graph" (always the
-        graph of eight iterations)."""
+        """How solve_mixed and solve_pcg launch their iterations: "auto" (one
+        persistent cooperative launch with the structured inner operator and a
+        band preconditioner or for a small plain solve, one up to each update
+        with the pair kernels, else a replayed CUDA graph or, plain, the
+        kernels one by one) or "graph" (always the graph of eight iterations,
+        plain the kernels one by one: no bounded waits)."""
         v = {"auto": _lib.DS_ITER_AUTO, "graph": _lib.DS_ITER_GRAPH}[form]
         self.ctx.check(self._lib.ds_operator_set_iteration_form(self.handle, v),
                        "ds_operator_set_iteration_form")

@@ -246,8 +246,8 @@ void run_pcg(ds_operator* op, const ds_pcg_params& pp, ds_pcg_result& res, doubl
   const int g = vgrid(np);
   const bool vals = !op->use_dense && ensure_pair_vals(op);
   // (profiling times the products one by one)
-  const bool persistent =
-      vals && !op->ctx->prof.enabled && run_pcg_persistent(op, pp, st);
+  const bool persistent = vals && op->iter_form == DS_ITER_AUTO && !op->ctx->prof.enabled &&
+                          run_pcg_persistent(op, pp, st);
   if (!persistent) {
     // r = b - A x; d = M^-1 r; delta = r.d; |r|  (lib/pcg.h:95-108)
     op_apply_sorted(op, EPI_RESIDUAL, op->x.p, op->r.p, st);

@@ -256,7 +256,10 @@ int ds_operator_set_inner_matvec(ds_operator* op, int variant);
  * otherwise, and with DS_ITER_GRAPH, eight iterations are one CUDA graph
  * replayed until the solve ends.  All run the same recurrence; with a
  * preconditioner sums are taken in a different order, so iteration counts can
- * differ by rounding. */
+ * differ by rounding.  The form holds for plain solves (ds_solve_pcg*) too: with
+ * DS_ITER_AUTO those of up to 9,728 pixels are one cooperative launch with bounded
+ * barriers, with DS_ITER_GRAPH the kernels of each iteration are launched one by one,
+ * which waits for nothing and cannot time out. */
 enum { DS_ITER_AUTO = 0, DS_ITER_GRAPH = 1 };
 int ds_operator_set_iteration_form(ds_operator* op, int form);
 
