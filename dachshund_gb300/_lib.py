@@ -149,6 +149,8 @@ SIGNATURES = {
     "ds_context_last_error": (C.c_char_p, [_vp]),
     "ds_context_set_profiling": (_i, [_vp, _i]),
     "ds_context_set_wait_limit": (_i, [_vp, C.c_longlong]),
+    "ds_context_set_store_share": (_i, [_vp, C.c_double]),
+    "ds_operator_get_stored_bytes": (_i, [_vp, C.POINTER(C.c_size_t)]),
     "ds_context_get_profile": (_i, [_vp, C.POINTER(ProfileC)]),
     "ds_operator_create": (_i, [_vp, _i, _i, _dp, C.POINTER(KernelParamsC), C.POINTER(_vp)]),
     "ds_operator_destroy": (None, [_vp]),

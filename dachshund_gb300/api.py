@@ -178,6 +178,12 @@ class Context:
         out makes the call raise DsError with code DS_ERR_TIMEOUT."""
         self.check(self._lib.ds_context_set_wait_limit(self.handle, int(cycles)), "wait limit")
 
+    def set_store_share(self, share: float = 0.125):
+        """Share of the free device memory that each operator may take to store
+        its interacting pairs' values (and the persistent pair form's row
+        sums); 0 stores nothing and gives back what is stored."""
+        self.check(self._lib.ds_context_set_store_share(self.handle, float(share)), "store share")
+
     def profile(self) -> dict:
         p = _lib.ProfileC()
         self.check(self._lib.ds_context_get_profile(self.handle, C.byref(p)), "profile")
@@ -333,6 +339,13 @@ class _WFVector:
             C.c_void_p(out.data_ptr())), "ds_operator_skewer_product_dev")
         self.ctx.synchronize()
         return out.cpu().numpy()
+
+    def stored_bytes(self) -> int:
+        """Bytes of the stored pair values; 0 when products evaluate the pairs."""
+        v = C.c_size_t()
+        self.ctx.check(self._lib.ds_operator_get_stored_bytes(self.handle, C.byref(v)),
+                       "ds_operator_get_stored_bytes")
+        return v.value
 
     def info(self) -> dict:
         inf = _lib.OperatorInfoC()

@@ -336,6 +336,21 @@ int ds_context_set_wait_limit(ds_context* ctx, long long cycles) {
   return DS_OK;
 }
 
+int ds_context_set_store_share(ds_context* ctx, double share) {
+  if (!ctx || !(share >= 0.0 && share <= 1.0)) return DS_ERR_ARG;
+  ctx->store_share = share;
+  ++ctx->share_serial;
+  return DS_OK;
+}
+
+int ds_operator_get_stored_bytes(ds_operator* op, size_t* bytes) {
+  if (!op || !bytes) return DS_ERR_ARG;
+  const PairVals& v = op->vals;
+  *bytes = v.ok ? v.cnt.bytes() + v.start.bytes() + v.val.bytes() + v.col16.bytes() + v.col32.bytes()
+                : 0;
+  return DS_OK;
+}
+
 int ds_context_get_profile(ds_context* ctx, ds_profile* out) {
   if (!ctx || !out) return DS_ERR_ARG;
   return guarded(ctx, [&] {

@@ -323,7 +323,7 @@ struct FxPoints {
 // The FP64 operator's interacting pairs as stored values (pair_vals.cu):
 // slices of 32 rows, entry e of lane l of slice s at (start[s] + e) * 32 + l.
 struct PairVals {
-  bool tried = false;  // built or given up
+  unsigned decided = 0;  // the context's share_serial when built or given up
   bool ok = false;
   DevBuf<int> cnt;          // entries per row
   DevBuf<long long> start;  // per slice (+ 1)
@@ -356,6 +356,8 @@ struct ds_context {
   int device = 0;
   int num_sms = 0;  // streaming multiprocessors of the device (persistent grids)
   long long wait_limit = 0;  // bound of tensor-core mbarrier waits (0: default)
+  double store_share = 0.125;  // ds_context_set_store_share
+  unsigned share_serial = 1;   // its settings so far
   cudaStream_t stream = nullptr;
   std::string last_error;
   ds::Profiler prof;

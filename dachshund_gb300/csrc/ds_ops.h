@@ -74,6 +74,9 @@ void ensure_op_pairs(ds_operator* op);
 // The operator's pair values, built on the first FP64 product; false when
 // they would take too much memory (pair_vals.cu).
 bool ensure_pair_vals(ds_operator* op);
+// Device memory that stored forms of one object may take: the context's share of what
+// is free, the memory cached in the device's pool included.
+size_t store_budget(ds_context* ctx);
 // out = A v or b - A v from them (a as for launch_pair_f64, a.u formed).
 void launch_pair_vals(ds_operator* op, int epi, const PairArgs& a, cudaStream_t st);
 

@@ -215,14 +215,55 @@ void fill(ds_operator* op, PairVals& pv, const PairArgs& a, DevBuf<I>& cols, cud
 
 }  // namespace
 
-// Builds the list on the operator's first product (counting pass, scan,
-// indices, values); false when the operator evaluates its pairs on every
-// product instead: when the list would take more than an eighth of the
-// device memory that is free, so that it never crowds out what the caller
-// allocates later, or when its allocation fails.
+size_t store_budget(ds_context* ctx) {
+  size_t free_b = 0, total_b = 0;
+  DS_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  cudaMemPool_t pool;
+  DS_CUDA(cudaDeviceGetDefaultMemPool(&pool, ctx->device));
+  unsigned long long held = 0, used = 0;
+  DS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+  DS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return (size_t)(ctx->store_share * (double)(free_b + (held > used ? held - used : 0)));
+}
+
+static void drop_vals(PairVals& pv) {
+  pv.ok = false;
+  pv.cnt.release();
+  pv.start.release();
+  pv.val.release();
+  pv.col16.release();
+  pv.col32.release();
+}
+
+static bool build_vals(ds_operator* op);
+
+// Builds the list on the operator's first product; false when the operator
+// evaluates its pairs on every product instead: when the list would take more
+// than the context's share (an eighth unless set) of the device memory that is
+// free, so that it does not crowd out what the caller allocates later, or when an
+// allocation fails.  Decided again when the share is set; share 0 gives the list
+// back.
 bool ensure_pair_vals(ds_operator* op) {
   PairVals& pv = op->vals;
-  if (pv.tried) return pv.ok;
+  if (pv.decided == op->ctx->share_serial) return pv.ok;
+  if (!(pv.ok && op->ctx->store_share > 0.0)) {
+    drop_vals(pv);
+    try {
+      pv.ok = op->ctx->store_share > 0.0 && build_vals(op);
+    } catch (const Error& e) {
+      drop_vals(pv);
+      if (e.code != DS_ERR_OOM) throw;
+      cudaGetLastError();  // the failed allocation's
+    }
+    if (!pv.ok) drop_vals(pv);
+  }
+  pv.decided = op->ctx->share_serial;
+  return pv.ok;
+}
+
+// Counting pass, scan, indices, values; false when over the budget.
+static bool build_vals(ds_operator* op) {
+  PairVals& pv = op->vals;
   PairArgs a = op_pair_args(op, nullptr, nullptr);
   cudaStream_t st = op->ctx->stream;
   const int ns = op->pix.n_pad / 32;
@@ -244,28 +285,15 @@ bool ensure_pair_vals(ds_operator* op) {
   DS_CUDA(cudaStreamSynchronize(st));
   const bool narrow = op->pix.n_pad <= 65536;
   const size_t n = (size_t)std::max<long long>(rows, 1) * 32;
-  size_t free_b = 0, total_b = 0;
-  DS_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  pv.tried = true;
-  if (n * (narrow ? 10 : 12) > free_b / 8) return false;
-  try {
-    pv.val.alloc(n);
-    if (narrow)
-      pv.col16.alloc(n);
-    else
-      pv.col32.alloc(n);
-  } catch (const Error& e) {
-    if (e.code != DS_ERR_OOM) throw;
-    cudaGetLastError();  // the failed allocation's
-    pv.val.release();
-    pv.col16.release();
-    return false;
-  }
-  if (narrow)
+  if (n * (narrow ? 10 : 12) > store_budget(op->ctx)) return false;
+  pv.val.alloc(n);
+  if (narrow) {
+    pv.col16.alloc(n);
     fill(op, pv, a, pv.col16, st);
-  else
+  } else {
+    pv.col32.alloc(n);
     fill(op, pv, a, pv.col32, st);
-  pv.ok = true;
+  }
   return true;
 }
 

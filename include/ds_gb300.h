@@ -160,6 +160,18 @@ int ds_context_set_wait_limit(ds_context* ctx, long long cycles);
 /* ---- the operator A over one pixel set --------------------------------- */
 typedef struct ds_operator ds_operator;
 
+/* Share (0 to 1; default 1/8) of the device memory free at the time, the memory the
+ * library's pool holds in reserve included, that each operator on the context may take
+ * to store what its products otherwise evaluate: the values of its interacting pairs
+ * (ds_A_product) and the row sums of the mixed solve's persistent pair form
+ * (ds_operator_set_iteration_form).  An operator decides at its first product, and
+ * again after every call of this function; with 0 it stores nothing, and gives back
+ * at its next product what it stored.  ds_operator_get_stored_bytes reports the bytes of
+ * an operator's stored pair values, 0 when it evaluates its pairs.  No reference
+ * counterpart. */
+int ds_context_set_store_share(ds_context* ctx, double share);
+int ds_operator_get_stored_bytes(ds_operator* op, size_t* bytes);
+
 /* WFVectorSN / WFVectorW ctor (lib/wf_vector.h:37-46, 72-81).  ``records``:
  * n NPixel (form SN) or WPixel (form W) records.  Copies them to the device
  * in a spatially sorted, tiled layout and builds the culled tile-pair list. */
@@ -185,8 +197,9 @@ int ds_operator_get_info(ds_operator* op, ds_operator_info* info);
  * every interacting pair once and keeps the values on the device (10 to 12
  * bytes per pair: about 0.6 GB at 32,768 pixels and 8 GB at 262,144 with the
  * exact kernel); later products read them.  An operator whose values would take
- * more than an eighth of the free device memory evaluates its pairs on every
- * call instead, with the same results to rounding. */
+ * more than the context's share of the free device memory (an eighth unless set:
+ * ds_context_set_store_share) evaluates its pairs on every call instead, with the
+ * same results to rounding. */
 int ds_A_product(ds_operator* op, const double* a, double* b);
 int ds_A_product_dev(ds_operator* op, const double* a, double* b);
 
