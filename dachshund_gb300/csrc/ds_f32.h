@@ -134,6 +134,7 @@ struct OpF32 {
   DevBuf<float> rowf, colw, ediag, pdiag;
   DevBuf<float> p, q, r, z;         // FP32 iteration vectors (sorted, padded)
   // the persistent form of the pair kernels' iteration (persist_pairs.cu)
+  unsigned rounds_decided = 0;  // the context's share_serial when built or given up
   bool rounds_built = false;
   DevBuf<int4> rounds;
   DevBuf<int> round_ptr, warp_ptr;

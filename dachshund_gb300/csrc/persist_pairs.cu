@@ -448,16 +448,49 @@ static const void* kernel_of(const OpF32& f) {
                                    : (const void*)k_mixed_pairs<F32_DIRECT>;
 }
 
+static void drop_rounds(OpF32& f) {
+  f.rounds_built = false;
+  for (auto* b : {&f.round_ptr, &f.warp_ptr}) b->release();
+  f.rounds.release();
+  f.round_sums.release();
+  f.xiw.release();
+  f.zp.release();
+  f.round_part.release();
+  f.round_bar.release();
+}
+
+static bool build_rounds(ds_operator* op, OpF32& f);
+
 // Prepares the launches (kept with the operator's FP32 pair list); false when the
-// rows do not fit, and the per-kernel form runs.
+// rows do not fit or the rounds (536 bytes each; clumped pixels have millions) would
+// take more than the context's share of the device memory, and the per-kernel form
+// runs.  Decided again when the share is set; share 0 gives them back.
 bool mixed_pairs_usable(ds_operator* op, OpF32& f, int g) {
-  const int nt = op->pix.n_tiles, G = op->ctx->num_sms;
+  const int G = op->ctx->num_sms;
   const int per = (op->pix.n_pad + g * VB - 1) / (g * VB);
   if (per > MAX_PER || g > 2 * G) return false;
   const size_t smem = sizeof(Shared) + (size_t)per * NT * sizeof(Row);
   const void* fn = kernel_of(f);
   if (resident_ctas(fn, NT, smem) < 1) return false;
-  if (f.rounds_built) return true;
+  if (f.rounds_decided == op->ctx->share_serial) return f.rounds_built;
+  if (!(f.rounds_built && op->ctx->store_share > 0.0)) {
+    drop_rounds(f);
+    try {
+      f.rounds_built = op->ctx->store_share > 0.0 && build_rounds(op, f);
+    } catch (const Error& e) {
+      drop_rounds(f);
+      if (e.code != DS_ERR_OOM) throw;
+      cudaGetLastError();  // the failed allocation's
+    }
+    if (!f.rounds_built) drop_rounds(f);
+  }
+  f.rounds_decided = op->ctx->share_serial;
+  return f.rounds_built;
+}
+
+// The rounds, their shares and the buffers; false when over the budget.
+static bool build_rounds(ds_operator* op, OpF32& f) {
+  const int nt = op->pix.n_tiles, G = op->ctx->num_sms;
   cudaStream_t st = op->ctx->stream;
   const int n = 4 * nt, nw = W * G;
   DevBuf<int> cnt, before;
@@ -476,6 +509,9 @@ bool mixed_pairs_usable(ds_operator* op, OpF32& f, int g) {
   int total = 0;
   DS_CUDA(cudaMemcpyAsync(&total, f.round_ptr.p + n, sizeof(int), cudaMemcpyDeviceToHost, st));
   DS_CUDA(cudaStreamSynchronize(st));
+  if ((size_t)total * (32 * sizeof(float4) + sizeof(int4) + 2 * sizeof(int)) >
+      store_budget(op->ctx))
+    return false;
   f.rounds.alloc(std::max(total, 1));
   DevBuf<int> weight;
   weight.alloc(total + 1);
@@ -496,7 +532,6 @@ bool mixed_pairs_usable(ds_operator* op, OpF32& f, int g) {
   f.zp.alloc(op->pix.n_pad);
   f.round_part.alloc((size_t)nt + 4 * G);
   f.round_bar.alloc(2);
-  f.rounds_built = true;
   return true;
 }
 

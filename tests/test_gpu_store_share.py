@@ -104,9 +104,15 @@ def test_mixed_forms_equal(ctx, n):
     op = WFVectorW(ctx, records("w", n), params(True))
     x1, r1 = op.solve_mixed(MixedParams(tol=1e-10))
     with share(ctx, 0.0):
-        x0, r0 = op.solve_mixed(MixedParams(tol=1e-10))
-    assert r1.success and r0.num_iters == r1.num_iters
+        ctx.set_wait_limit(1)  # (the persistent form would time out)
+        try:
+            x0, r0 = op.solve_mixed(MixedParams(tol=1e-10))
+        finally:
+            ctx.set_wait_limit(0)
+    x2, r2 = op.solve_mixed(MixedParams(tol=1e-10))
+    assert r1.success and r0.num_iters == r1.num_iters == r2.num_iters
     np.testing.assert_array_equal(x0, x1)
+    np.testing.assert_array_equal(x2, x1)
     op.close()
 
 
