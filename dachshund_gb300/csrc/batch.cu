@@ -1151,8 +1151,17 @@ void batch_build(ds_batch* B, const double* d_rec, const int* sizes) {
   B->chunk_done.alloc(C);
   B->up_n.alloc(1);
   B->up_tile.alloc(T);
-  B->seg_cap = 9 * sm_count();  // three times the residual's CTAs at 32 RHS per item
-  B->seg.alloc((size_t)B->seg_cap * resid_block(B->n_rhs) * 3 * TILE);
+  // segments of the residual's items: three times its CTAs at 32 RHS per item, or all
+  // that the batch's items can have; without room for them items stay whole
+  const int rb = resid_block(B->n_rhs);
+  B->seg_cap = (int)std::min<long long>(9 * sm_count(), 8ll * T * (B->n_rhs / rb));
+  try {
+    B->seg.alloc((size_t)B->seg_cap * rb * 3 * TILE);
+  } catch (const Error& e) {
+    if (e.code != DS_ERR_OOM) throw;
+    cudaGetLastError();  // the failed allocation's
+    B->seg_cap = 1;
+  }
   B->seg_count.alloc(B->seg_cap);
   DS_CUDA(cudaMemsetAsync(B->seg_count.p, 0, B->seg_count.bytes(), st));
   B->active.alloc(1);
