@@ -389,23 +389,23 @@ __global__ void k_rev_fill(int n, const int* __restrict__ nbr, const float* __re
   if (e < n && g[e] != 0.f) src[ptr[nbr[e]] + atomicSub(&cnt[nbr[e]], 1) - 1] = e;
 }
 
-// Sorts each list (of entry numbers: the order does not depend on the atomics)
-// and writes the skewer and weight of every entry.
-__global__ void k_rev_sort(int n_sk, const int* __restrict__ ptr, int* __restrict__ src,
+// Writes the skewer and weight of every entry in ascending order of the entry numbers
+// (it does not depend on the atomics): a warp per list, each entry at its rank.  The
+// lists have some 8 entries; where many skewers share a line of sight, 8 of them are
+// named by all (a training step of 4,000 such skewers x 4 pixels: 166 ms with one
+// thread's insertion sort per list, 7.5 here).
+__global__ void k_rev_sort(int n_sk, const int* __restrict__ ptr, const int* __restrict__ src,
                            const float* __restrict__ g, int* __restrict__ idx,
                            float* __restrict__ w) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   if (s >= n_sk) return;
   const int a = ptr[s], b = ptr[s + 1];
-  for (int i = a + 1; i < b; ++i) {
+  for (int i = a + (threadIdx.x & 31); i < b; i += 32) {
     const int v = src[i];
-    int j = i - 1;
-    for (; j >= a && src[j] > v; --j) src[j + 1] = src[j];
-    src[j + 1] = v;
-  }
-  for (int i = a; i < b; ++i) {
-    idx[i] = src[i] / 8;
-    w[i] = g[src[i]];
+    int rank = 0;
+    for (int j = a; j < b; ++j) rank += src[j] < v;
+    idx[a + rank] = v / 8;
+    w[a + rank] = g[v];
   }
 }
 
@@ -533,7 +533,8 @@ void build_rev_lists(int n_sk, const int* nbr, const float* g, RevLists& rev, cu
   DS_CUDA(cub::DeviceScan::ExclusiveSum(rev.tmp.p, bytes, rev.cnt.p, rev.ptr.p, n_sk + 1, st));
   k_rev_fill<<<grid1(n), 256, 0, st>>>(n, nbr, g, rev.ptr.p, rev.cnt.p, rev.src.p);
   DS_CHECK_LAUNCH();
-  k_rev_sort<<<grid1(n_sk, 64), 64, 0, st>>>(n_sk, rev.ptr.p, rev.src.p, g, rev.idx.p, rev.w.p);
+  k_rev_sort<<<grid1(32 * (size_t)n_sk), 256, 0, st>>>(n_sk, rev.ptr.p, rev.src.p, g, rev.idx.p,
+                                                       rev.w.p);
   DS_CHECK_LAUNCH();
 }
 
