@@ -96,12 +96,15 @@ __device__ __forceinline__ float pow2_neg(int e) {
 // and across updates).  The sums take sr r, sz z, sr q and sz p, powers of two that
 // bring |r| and r.z at the last update to about 1 (the squares of vectors in units
 // far from 1, fluxes of 1e-17, would leave FP32's range), and stay in those units.
-// The norms are kept as squares: they only decide when an update is due, and an FP64
-// root takes as long as a dozen additions.
+// The norms are kept as squares, with their thresholds, and compared as the integers of
+// the same order that the numbers' bits are: they only decide when an update is due, an
+// FP64 root takes as long as a dozen additions, and an FP64 instruction of one lane
+// holds its scheduler's pipe for 64 clocks.
 struct FastState {
   float sr, sz;
   double rz, rz_old, pq;               // times sr sz
-  double rr, rrmax, rrbest, tol2;      // squares, times sr^2
+  double rr, rrmax, tol2;              // squares, times sr^2 (tol2 < 0: no tolerance)
+  double due, half;                    // delta^2 rrmax; a quarter of the best rr
   double delta2, urr;                  // delta^2; 1 / sr^2
   ff alpha;
   float beta;
@@ -129,9 +132,10 @@ __device__ __forceinline__ void fast_from(FastState& f, const MixedState& s, dou
   f.rz_old = s.rz_old * sq;
   f.rr = square(rnorm);
   f.rrmax = square(s.rmax);
-  f.rrbest = square(s.rbest);
+  f.half = 0.25 * square(s.rbest);
   f.tol2 = s.tol_norm_b >= 0.0 ? square(s.tol_norm_b) : -1.0;
   f.delta2 = s.delta * s.delta;
+  f.due = f.delta2 * f.rrmax;
   f.urr = 1.0 / (sr * sr);
   f.beta = (float)s.beta;
   f.it_best = s.it_best;
@@ -146,7 +150,7 @@ __device__ __forceinline__ void fast_to(const FastState& f, MixedState& s) {
   s.beta = f.beta;
   s.rnorm = sqrt(f.rr) * ur;
   s.rmax = sqrt(f.rrmax) * ur;
-  s.rbest = sqrt(f.rrbest) * ur;
+  s.rbest = sqrt(4.0 * f.half) * ur;
   s.it_best = f.it_best;
 }
 
@@ -159,17 +163,22 @@ __device__ __forceinline__ void fast_beta(FastState& f, double trz) {
 }
 
 __device__ __forceinline__ void fast_norm(FastState& f, MixedState& s, int it, double trr) {
+  auto bits = [](double v) { return __double_as_longlong(v); };  // (a NaN: above all)
   f.rr = trr;
   s.iter = it;
-  f.rrmax = fmax(f.rrmax, trr);
-  if (trr < 0.25 * f.rrbest) {
-    f.rrbest = trr;
+  if (bits(trr) > bits(f.rrmax) && bits(trr) <= 0x7ff0000000000000ll) {
+    f.rrmax = trr;
+    f.due = f.delta2 * trr;
+  }
+  if (bits(trr) < bits(f.half)) {
+    f.half = 0.25 * trr;
     f.it_best = it;
   }
   const bool stall = it - f.it_best >= STALL_ITERS;
   if (stall) s.stalled = 1;
-  s.need_update =
-      trr < f.delta2 * f.rrmax || trr <= f.tol2 || it >= s.max_iter || stall ? 1 : 0;
+  s.need_update = bits(trr) < bits(f.due) || bits(trr) <= bits(f.tol2) || it >= s.max_iter || stall
+                      ? 1
+                      : 0;
 }
 
 }  // namespace ds

@@ -273,12 +273,37 @@ __device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code) {
 // every CTA: lane l takes l, l + 32, ..., then a shuffle tree, so the FP64 pipe
 // (2 operations per clock per SM on GB300) sees n + 5 additions per CTA instead
 // of a CTA-wide tree.
-__device__ __forceinline__ double warp_total(const double* part, int n, int stride = 1) {
+__device__ __forceinline__ double warp_total(const double* part, int n) {
   double v = 0.0;
 #pragma unroll 4
-  for (int i = threadIdx.x & 31; i < n; i += 32) v += __ldcg(part + (size_t)i * stride);
+  for (int i = threadIdx.x & 31; i < n; i += 32) v += __ldcg(part + i);
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Sum of n partials `stride` apart by any one warp (valid in lane 0), in another fixed
+// order for its latency: four chains per lane, the first addition of each and the
+// tree's levels above n left out.
+__device__ __forceinline__ double warp_total4(const double* part, int n, int stride) {
+  const int lane = threadIdx.x & 31;
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (lane + 32 * u < n) v[u] = __ldcg(part + (size_t)(lane + 32 * u) * stride);
+  for (int i = lane + 128; i < n; i += 128) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + 32 * u < n) v[u] += __ldcg(part + (size_t)(i + 32 * u) * stride);
+  }
+  if (n > 64) {
+    v[0] += v[2];
+    v[1] += v[3];
+  }
+  if (n > 32) v[0] += v[1];
+  int o = 16;
+  while (o >= n && o > 1) o >>= 1;
+  for (; o > 0; o >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
+  return v[0];
 }
 
 // The same for n pairs of partials (both sums from one pass over them).
@@ -791,8 +816,8 @@ __device__ __forceinline__ void block_product_ff(const PersistArgs& a, int blk, 
 // the end.  The general form's recurrence, rearranged; sums in float pairs within
 // the warps and FP64 from there up (ds_ffsum.cuh).
 //
-// What the sums and scalars cost: 16 CTAs (64 x 64 pixels, 82 iterations) 0.82 ms a
-// launch, 256 CTAs (1,024 x 256, 130 iterations) 3.30; with FP64 sums by all warps,
+// What the sums and scalars cost: 16 CTAs (64 x 64 pixels, 82 iterations) 0.81 ms a
+// launch, 256 CTAs (1,024 x 256, 130 iterations) 3.23; with FP64 sums by all warps,
 // scalars by FP64 divisions and roots, 1.16 and 4.17; in float pairs throughout, of
 // 44 bits, 0.72 and 3.11.
 constexpr int NI = 512;   // product items of a block kept in shared memory
@@ -1129,7 +1154,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       // ---- step: alpha; x, r, z of the block; levels of z; partials.  Warp 0
       // alone adds the CTAs' partials and forms the scalars.
       if (tid < 32) {
-        const double pq = warp_total(a.part, G);
+        const double pq = warp_total4(a.part, G, 1);
         if (tid == 0) {
           sF.pq = pq;
           sF.alpha = s_alpha = quotient_ff(sF.rz, pq);
@@ -1175,7 +1200,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
       own_rows();
       if (!grid_wait<false>(a, B_STEP)) break;
       if (tid < 64) {  // warp 0: r.z and beta; warp 1: |r| and the update test
-        const double t = warp_total(a.part + P2 + (tid >> 5), G, 2);
+        const double t = warp_total4(a.part + P2 + (tid >> 5), G, 2);
         if (tid == 0) fast_beta(sF, t);
         if (tid == 32) fast_norm(sF, sS, it, t);
       }
@@ -1435,10 +1460,11 @@ void to_ff(DevBuf<float2>& out, const double* in, size_t n, cudaStream_t st) {
 }
 
 // The block of each CTA.  The slowest block sets the product phase (an interior
-// cluster has up to 1.7 times the mean's rows), and the first CTAs of a launch
-// go one to an SM, the rest second to the same SMs in order: the blocks with the
-// most items get the SMs that hold one CTA, the others are paired most with
-// fewest.
+// cluster has up to 1.7 times the mean's rows).  The order assumes that the first CTAs
+// of a launch go one to an SM and the rest second to the same SMs in order, as they do
+// here though nothing promises it: the blocks with the most items get the SMs that hold
+// one CTA, the others are paired most with fewest (15.0 -> 13.3 us a product phase at
+// 1,024 x 256 pixels).  Only the time depends on it.
 std::vector<int> launch_order(const std::vector<int>& cnt, int n, int sms) {
   std::vector<int> by(n), order(n);
   std::iota(by.begin(), by.end(), 0);
