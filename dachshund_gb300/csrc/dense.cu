@@ -2,9 +2,9 @@
 // used by PCG when the matrix fits, and the closed-form solve (Cholesky) that
 // stands in for WFVector{SN,W}::solve_cf (lib/wf_vector.cc:123-155, 276-319).
 //
-// Dense matvec: A streamed once per product (8 n^2 bytes) by a persistent
-// grid over 64-row items of its nonzero 64 x 64 blocks, HBM-bound with float-pair
-// arithmetic on the FP32 pipe (see the matvec section below).
+// Dense matvec: the nonzero 64 x 64 blocks of A streamed once per product by a
+// persistent grid over 64-row items, HBM-bound with float-pair arithmetic on the
+// FP32 pipe (see the matvec section below).
 // Cholesky: right-looking, 32-wide panels: diagonal block in shared memory by
 // one CTA, the panel by a triangular solve per row, the trailing lower
 // triangle by 64 x 64 tiles (each thread a 4 x 4 block).

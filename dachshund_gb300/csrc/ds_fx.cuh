@@ -3,7 +3,7 @@
 //
 // GB300 issues FP64 at 2 lanes per clock per SM and 32-bit integer
 // multiply-adds at 32 times that and more: a pair value takes ~20 FP64
-// instructions (10 clocks of an SM) or ~70 integer ones (~0.7 clocks), and
+// instructions (10 clocks of an SM) or ~70 integer ones (~1.1 clocks), and
 // fixed point keeps more bits than FP64 on the way:
 //  * coordinates scaled by sqrt(c) are held in units of 2^-60, modulo 2^64
 //    (formed once per point in double-double arithmetic); a difference of two

@@ -3,8 +3,8 @@
 //
 // GB300 issues FP64 at 2 lanes per clock per SM, so evaluating a pair (~20
 // FP64 instructions, pair_f64.cu) takes 10 clocks of an SM; the same pair read
-// from HBM as an FP64 value and a column index takes 10 or 12 bytes (0.27
-// clocks at the measured rate) and one FP64 FMA (0.5 clocks).  An iterative
+// from HBM as an FP64 value and a column index takes 10 or 12 bytes (0.47 or
+// 0.56 clocks at the measured rate) and one FP64 FMA (0.5 clocks).  An iterative
 // solve multiplies by the same S a hundred times and more, so the first product
 // of an operator evaluates every interacting pair once into this list, and all
 // products and residuals read it.  Bound then by the FP64 FMA and HBM about

@@ -817,9 +817,9 @@ __device__ __forceinline__ void block_product_ff(const PersistArgs& a, int blk, 
 // the warps and FP64 from there up (ds_ffsum.cuh).
 //
 // What the sums and scalars cost: 16 CTAs (64 x 64 pixels, 82 iterations) 0.81 ms a
-// launch, 256 CTAs (1,024 x 256, 130 iterations) 3.23; with FP64 sums by all warps,
-// scalars by FP64 divisions and roots, 1.16 and 4.17; in float pairs throughout, of
-// 44 bits, 0.72 and 3.11.
+// launch, 256 CTAs (1,024 x 256, 130 iterations) 3.23; in float pairs throughout, of
+// 44 bits, 0.73 and 3.07; with FP64 sums by all warps and scalars by FP64 divisions and
+// roots (and the timers in global memory), 1.16 and 4.17.
 constexpr int NI = 512;   // product items of a block kept in shared memory
 constexpr int GI = 4;     // skewers per block of the item form at most
 

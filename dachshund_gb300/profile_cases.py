@@ -17,6 +17,9 @@ leaves the GPU's clocks as they are):
                  (the start kernels, then one persistent launch of
                  k_mixed_resident) and the 80 x 80 x 512 structured map
                  (k_mc_split + k_mc_fused)
+  mixed_pairs    one mixed-precision Jacobi solve of 192 skewers x 256 pixels
+                 with z offsets of their own and a tenth of the pixels
+                 masked out (k_mixed_pairs, one launch per reliable update)
   tc_matvec      one batched FP32 product of 64 chunks x 64 RHS with the
                  tensor-core variant (k_pack_panels + k_batch_mv_tc)
   tc_inner       one mixed-precision solve of the 262,144-pixel system with
@@ -127,6 +130,18 @@ def main(argv=None):
                 op.set_inner_matvec("tensor")
             x, res = op.solve_mixed(MixedParams(tol=1e-8))
             print(case, "iters", res.num_iters)
+    elif case == "mixed_pairs":
+        rng = np.random.default_rng(7)
+        n_sk, n_per = 192, 256
+        pix = np.empty((n_sk, n_per, 5))
+        pix[:, :, :2] = rng.uniform(0, 2.5 * np.sqrt(n_sk), (n_sk, 1, 2))
+        pix[:, :, 2] = synth.DZ * (np.arange(n_per) + rng.uniform(0, 1, (n_sk, 1)))
+        pix[:, :, 3] = rng.uniform(0.05, 0.3, (n_sk, n_per))
+        pix[:, :, 4] = rng.standard_normal((n_sk, n_per))
+        pix = pix.reshape(-1, 5)[rng.uniform(0, 1, n_sk * n_per) < 0.9]
+        op = WFVectorW(ctx, pixel_to_wpixel(pix), sp)
+        x, res = op.solve_mixed(MixedParams(tol=1e-11))
+        print(case, len(pix), "pixels, iters", res.num_iters, "updates", res.n_outer)
     elif case == "dense_matvec":
         w = synth.grf_workload("wf-16384px-grf", 128, 128, 40.0 / np.sqrt(2.0), 0,
                                (28, 28, 256), 1e-8)

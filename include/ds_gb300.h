@@ -118,14 +118,16 @@ const char* ds_context_last_error(ds_context* ctx);
  * clocks, lib/timer.h:13-26).  When enabled, every launch of a pair kernel
  * (the matvec / residual / map kernels) on this context is bracketed by CUDA
  * events on the context's stream; the profile accumulates their device time,
- * their count and the tile-evaluated pairs they covered (for the batched
+ * their count and the pairs they evaluated (for the batched
  * kernels of ds_batch_*: pair x right-hand-side products, and a profiled
  * batched solve runs its iterations without the CUDA graph so that each
  * launch can be timed).  Disabling keeps the totals until the next enable. */
 typedef struct {
   long long pair_launches;   /* pair-kernel launches timed (FP64 + FP32) */
   double pair_ms;            /* their summed device time */
-  double pair_evaluated;     /* pairs evaluated (tile pairs x tile^2) */
+  double pair_evaluated;     /* pairs evaluated: the FP64 kernels' interacting pairs
+                                (as their search finds them), the FP32 kernels' row
+                                and column sub-tiles in reach */
   long long kernel_launches; /* every kernel this library launched (process-wide) */
   long long f64_launches;    /* the FP64 pair kernels alone */
   double f64_ms;
@@ -166,7 +168,8 @@ typedef struct ds_operator ds_operator;
  * (ds_A_product) and the row sums of the mixed solve's persistent pair form
  * (ds_operator_set_iteration_form).  An operator decides at its first product, and
  * again after every call of this function; with 0 it stores nothing, and gives back
- * at its next product what it stored.  ds_operator_get_stored_bytes reports the bytes of
+ * at its next product what it stored (a graph that the caller captured before must not
+ * be replayed then).  ds_operator_get_stored_bytes reports the bytes of
  * an operator's stored pair values, 0 when it evaluates its pairs.  No reference
  * counterpart. */
 int ds_context_set_store_share(ds_context* ctx, double share);
