@@ -165,22 +165,24 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // may work on its own data (writing nothing another CTA reads in the next
 // phase), which hides that work behind the barrier's latency.
 constexpr int BAR_WORDS = 32;  // one 128-byte line
-// Thread 0's barrier state and phase timers, in shared memory (timers go to global
-// memory once, at the kernel's end): a read-modify-write of global memory or a
-// register spilled to local memory in front of the arrival's release held up every
-// barrier (1.0 -> 1.25 us with 16 CTAs for 48 bytes of spills).
+// Thread 0's barrier state: the resident form keeps it in shared memory (its registers
+// would spill, and stores to local memory in front of the arrival's release hold up the
+// barrier: 1.0 -> 1.25 us with 16 CTAs for 48 bytes of spills), the general form in
+// registers (1,500 x 128 pixels 6.5 ms a solve, 7.4 with it in shared memory).  The
+// phase timers are in shared memory and go to global memory once, at the kernel's end.
 struct BarState {
-  unsigned long long phase[8], visits[8], work[8];
   unsigned long long exit_ns;  // last exit (%globaltimer)
   unsigned int epoch;          // barriers passed
   int last;                    // this CTA completed the current epoch (RET)
 };
-__shared__ BarState s_bar;
+struct PhaseTimers {
+  unsigned long long phase[8], visits[8], work[8];
+};
+__shared__ PhaseTimers s_timers;
 
-__device__ void timers_start(const PersistArgs& a) {
-  BarState& b = s_bar;
+__device__ void timers_start(const PersistArgs& a, BarState& b) {
   if (threadIdx.x < 8)
-    s_bar.phase[threadIdx.x] = s_bar.visits[threadIdx.x] = s_bar.work[threadIdx.x] = 0;
+    s_timers.phase[threadIdx.x] = s_timers.visits[threadIdx.x] = s_timers.work[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     b.exit_ns = global_ns();
     b.epoch = 0;
@@ -196,21 +198,20 @@ __device__ void timers_start(const PersistArgs& a) {
 __device__ void timers_end(const PersistArgs& a) {
   __syncthreads();
   if (threadIdx.x < 8) {
-    a.pt[PT_CTA + 8 * blockIdx.x + threadIdx.x] += s_bar.work[threadIdx.x];
+    a.pt[PT_CTA + 8 * blockIdx.x + threadIdx.x] += s_timers.work[threadIdx.x];
     if (blockIdx.x == 0) {
-      a.pt[PT_PHASE + threadIdx.x] += s_bar.phase[threadIdx.x];
-      a.pt[PT_VISITS + threadIdx.x] += s_bar.visits[threadIdx.x];
+      a.pt[PT_PHASE + threadIdx.x] += s_timers.phase[threadIdx.x];
+      a.pt[PT_VISITS + threadIdx.x] += s_timers.visits[threadIdx.x];
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.pt[PT_KERNEL] += global_ns() - a.pt[PT_START];
 }
 
 template <bool RET>
-__device__ void grid_arrive(const PersistArgs& a, int code) {
-  BarState& b = s_bar;
+__device__ void grid_arrive(const PersistArgs& a, int code, BarState& b) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (b.epoch > 0) s_bar.work[code] += global_ns() - b.exit_ns;
+    if (b.epoch > 0) s_timers.work[code] += global_ns() - b.exit_ns;
     ++b.epoch;
     if (RET) {
       unsigned int old;
@@ -226,8 +227,7 @@ __device__ void grid_arrive(const PersistArgs& a, int code) {
 }
 
 template <bool RET>
-__device__ bool grid_wait(const PersistArgs& a, int code) {
-  BarState& b = s_bar;
+__device__ bool grid_wait(const PersistArgs& a, int code, BarState& b) {
   __shared__ int ok_s;
   if (threadIdx.x == 0) {
     int ok = 1;
@@ -254,8 +254,8 @@ __device__ bool grid_wait(const PersistArgs& a, int code) {
       ok = 0;
     }
     const unsigned long long now = global_ns();
-    s_bar.phase[code] += now - b.exit_ns;  // reported for CTA 0
-    s_bar.visits[code] += 1;
+    s_timers.phase[code] += now - b.exit_ns;  // reported for CTA 0
+    s_timers.visits[code] += 1;
     b.exit_ns = now;
     ok_s = ok;
   }
@@ -264,9 +264,9 @@ __device__ bool grid_wait(const PersistArgs& a, int code) {
 }
 
 template <bool RET>
-__device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code) {
-  grid_arrive<RET>(a, code);
-  return grid_wait<RET>(a, code);
+__device__ __forceinline__ bool grid_sync(const PersistArgs& a, int code, BarState& b) {
+  grid_arrive<RET>(a, code, b);
+  return grid_wait<RET>(a, code, b);
 }
 
 // Sum of n partials in a fixed order by one warp (valid in lane 0), the same in
@@ -543,6 +543,7 @@ __device__ __forceinline__ void update_scalars(MixedState& sS, const PersistArgs
 // ---- general form: any number of blocks per CTA, vectors in global memory
 template <int BAND>
 __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
+  BarState bst;  // thread 0's
   __shared__ MixedState sS;
   __shared__ double red[NT / 32];
   __shared__ double tot[2];
@@ -559,9 +560,9 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
   const int P2 = (G + 1) & ~1;  // the pair partials start 16-byte aligned
   const size_t ns = (size_t)a.n_blocks * a.S;
   if (tid == 0) sS = *a.S_;
-  timers_start(a);
+  timers_start(a, bst);
   __syncthreads();
-  for (int k = 0; k < N_CALIB; ++k) grid_sync<true>(a, B_CALIB);
+  for (int k = 0; k < N_CALIB; ++k) grid_sync<true>(a, B_CALIB, bst);
   // the recurrence sets done by iteration max_iter at the latest (the
   // update it forces there ends the solve); the bound keeps hist in range
   while (!sS.done && sS.iter < a.max_iter) {
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
           return (float)a.wr[r] * pv;
         });
     }
-    if (!grid_sync<true>(a, B_LEVELS)) break;
+    if (!grid_sync<true>(a, B_LEVELS, bst)) break;
     // ---- B: q = A32 p, partial p.q
     double dq = 0.0;
     for (int blk = blockIdx.x; blk < a.n_blocks; blk += G) {
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
       const double bs = block_sum<NT>(dq, red);
       if (tid == 0) a.part[blockIdx.x] = bs;
     }
-    if (!grid_sync<true>(a, B_PRODUCT)) break;
+    if (!grid_sync<true>(a, B_PRODUCT, bst)) break;
     // ---- C: alpha; x, r, z per owned block; partials r.z, |r|^2
     const double pq = partial_total(a.part, G, tot);
     if (tid == 0) tot[0] = sS.rz / pq;
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
         a.part[(size_t)P2 + 2 * blockIdx.x + 1] = b2;
       }
     }
-    if (!grid_sync<true>(a, B_STEP)) break;
+    if (!grid_sync<true>(a, B_STEP, bst)) break;
     {
       const double2 t2 = partial_total2(a.part + P2, G, tot);
       if (tid == 0) step_scalars(sS, a, it, alpha_d, pq, t2.x, t2.y);
@@ -658,7 +659,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
     for (int blk = blockIdx.x; blk < a.n_blocks; blk += G)
       block_levels<double>(a, blk, a.olmax, a.taps64, a.V64, su64,
                            [&](size_t r) { return a.wr[r] * __ldcg(a.x + r); });
-    if (!grid_sync<true>(a, B_LEVELS64)) break;
+    if (!grid_sync<true>(a, B_LEVELS64, bst)) break;
     // ---- E, F: r64 = b - A x per owned skewer; r = r64, z = G G^T r
     rz = 0.0;
     rr = 0.0;
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_persistent(PersistArgs a) {
         a.part[(size_t)P2 + 2 * blockIdx.x + 1] = b2;
       }
     }
-    if (!grid_sync<true>(a, B_UPDATE)) break;
+    if (!grid_sync<true>(a, B_UPDATE, bst)) break;
     {
       const double2 t2 = partial_total2(a.part + P2, G, tot);
       if (tid == 0) update_scalars(sS, a, t2.x, t2.y);
@@ -939,6 +940,7 @@ __device__ __forceinline__ void block_precond_h(const PersistArgs& a, const __ha
 
 template <int BAND>
 __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
+  __shared__ BarState bst;
   extern __shared__ __align__(16) unsigned char smraw[];
   ff* xs = reinterpret_cast<ff*>(smraw + ResLayout::xs);  // the iterate, float pairs
   double* us = reinterpret_cast<double*>(smraw + ResLayout::us);
@@ -977,7 +979,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     sS = *a.S_;
     fast_from(sF, sS, sS.rnorm);
   }
-  timers_start(a);
+  timers_start(a, bst);
   if (tid < MAX_G) sk[tid] = tid < a.g ? skewer_of(a, blk, tid) : -1;
   {  // the block's product items
     const size_t i0 = (size_t)blk * NI;
@@ -1109,10 +1111,10 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
     if (has_pixel) product_rows(part * no / tk, (part + 1) * no / tk);
   };
   levels_z();
-  grid_arrive<false>(a, B_LEVELS);
+  grid_arrive<false>(a, B_LEVELS, bst);
   own_rows();
-  if (grid_wait<false>(a, B_LEVELS)) {
-    for (int k = 0; k < N_CALIB; ++k) grid_sync<false>(a, B_CALIB);
+  if (grid_wait<false>(a, B_LEVELS, bst)) {
+    for (int k = 0; k < N_CALIB; ++k) grid_sync<false>(a, B_CALIB, bst);
   }
   while (!sS.done && sS.iter < a.max_iter) {
       const int it = sS.iter + 1;
@@ -1150,7 +1152,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         const double bs = block_sum2<NT, false>(dq, ff{0.f, 0.f}, red);
         if (tid == 0) a.part[blk] = bs;
       }
-      if (!grid_sync<false>(a, B_PRODUCT)) break;
+      if (!grid_sync<false>(a, B_PRODUCT, bst)) break;
       // ---- step: alpha; x, r, z of the block; levels of z; partials.  Warp 0
       // alone adds the CTAs' partials and forms the scalars.
       if (tid < 32) {
@@ -1196,9 +1198,9 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         const double bs = block_sum2<NT, true>(rz, rr, red);
         if (tid == 0 || tid == 16) a.part[(size_t)P2 + 2 * blk + (tid >> 4)] = bs;
       }
-      grid_arrive<false>(a, B_STEP);
+      grid_arrive<false>(a, B_STEP, bst);
       own_rows();
-      if (!grid_wait<false>(a, B_STEP)) break;
+      if (!grid_wait<false>(a, B_STEP, bst)) break;
       if (tid < 64) {  // warp 0: r.z and beta; warp 1: |r| and the update test
         const double t = warp_total4(a.part + P2 + (tid >> 5), G, 2);
         if (tid == 0) fast_beta(sF, t);
@@ -1236,7 +1238,7 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
           V2[(size_t)l * n + rg[t]] = make_float2(acc.h, acc.l);
         }
       }
-      if (!grid_sync<false>(a, B_LEVELS64)) break;
+      if (!grid_sync<false>(a, B_LEVELS64, bst)) break;
       // r64 = b - A x of the block (into us); r = r64, z = G G^T r, levels of z
       {
         ff acc[RPT];
@@ -1287,9 +1289,9 @@ __global__ void __launch_bounds__(NT, 2) k_mixed_resident(PersistArgs a) {
         }
       }
       levels_z();
-      grid_arrive<false>(a, B_UPDATE);
+      grid_arrive<false>(a, B_UPDATE, bst);
       own_rows();
-      if (!grid_wait<false>(a, B_UPDATE)) break;
+      if (!grid_wait<false>(a, B_UPDATE, bst)) break;
       if (tid < 32) {
         const double2 t2 = warp_total2(a.part + P2, G);
         if (tid == 0) {
