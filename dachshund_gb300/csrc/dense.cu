@@ -569,7 +569,14 @@ void op_free_dense(ds_operator* op) {
 void op_build_dense(ds_operator* op) {
   cudaStream_t st = op->ctx->stream;
   const size_t np = op->pix.n_pad;
-  op->dense.alloc(np * np);
+  try {
+    op->dense.alloc(np * np);
+  } catch (const Error& e) {
+    // the dense products read no stored pair values: their memory may be what is missing
+    if (e.code != DS_ERR_OOM || !drop_pair_vals(op)) throw;
+    cudaGetLastError();  // the failed allocation's
+    op->dense.alloc(np * np);
+  }
   DevBuf<unsigned long long> stats;
   stats.alloc(3);
   const unsigned long long init[3] = {~0ull, 0ull, 0ull};

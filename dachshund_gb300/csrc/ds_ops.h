@@ -74,6 +74,9 @@ void ensure_op_pairs(ds_operator* op);
 // The operator's pair values, built on the first FP64 product; false when
 // they would take too much memory (pair_vals.cu).
 bool ensure_pair_vals(ds_operator* op);
+// Gives the pair values back until the next product that wants them; false when there
+// are none.
+bool drop_pair_vals(ds_operator* op);
 // Device memory that stored forms of one object may take: the context's share of what
 // is free, the memory cached in the device's pool included.
 size_t store_budget(ds_context* ctx);

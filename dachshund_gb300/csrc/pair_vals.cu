@@ -235,6 +235,13 @@ static void drop_vals(PairVals& pv) {
   pv.col32.release();
 }
 
+bool drop_pair_vals(ds_operator* op) {
+  if (!op->vals.ok) return false;
+  drop_vals(op->vals);
+  op->vals.decided = 0;
+  return true;
+}
+
 static bool build_vals(ds_operator* op);
 
 // Builds the list on the operator's first product; false when the operator
